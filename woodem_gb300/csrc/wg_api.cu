@@ -14,6 +14,11 @@
 #include "wg_math.cuh"
 
 namespace wg {
+// the rounded reciprocals of a node's inertia and mass (0 for a zero: no division takes place)
+static double4_32a reciprocals(const double4_32a& m) {
+    auto r = [](double v) { return v != 0 ? 1. / v : 0.; };
+    return make_double4_32a(r(m.x), r(m.y), r(m.z), r(m.w));
+}
 // Scene.nextDt of a configuration: a positive finite value (0 and NaN: none)
 static double validNextDt(const wg_config& c) {
     return (c.next_dt > 0 && std::isfinite(c.next_dt)) ? c.next_dt : std::numeric_limits<double>::quiet_NaN();
@@ -553,6 +558,7 @@ int Sim::upload() {
     N.force = (double4_32a*)dalloc(sizeof(double4_32a) * nSlots);
     N.torque = (double4_32a*)dalloc(sizeof(double4_32a) * nSlots);
     N.minert = (double4_32a*)dalloc(sizeof(double4_32a) * nSlots);
+    N.rinv = prec == WG_PREC_FP64 ? (double4_32a*)dalloc(sizeof(double4_32a) * nSlots) : nullptr;
     N.lastPos = (double4_32a*)dalloc(sizeof(double4_32a) * nSlots);
     N.flags = (uint32_t*)dalloc(sizeof(uint32_t) * nSlots);
     P.n = (int32_t)nPar;
@@ -601,6 +607,13 @@ int Sim::upload() {
     WG_CUDA_TRY(cudaMemcpyAsync(N.force, force.data(), sizeof(double4_32a) * nSlots, cudaMemcpyHostToDevice, S.stream));
     WG_CUDA_TRY(cudaMemcpyAsync(N.torque, torque.data(), sizeof(double4_32a) * nSlots, cudaMemcpyHostToDevice, S.stream));
     WG_CUDA_TRY(cudaMemcpyAsync(N.minert, minert.data(), sizeof(double4_32a) * nSlots, cudaMemcpyHostToDevice, S.stream));
+    std::vector<double4_32a> rinv;
+    if (prec == WG_PREC_FP64) {
+        if (!N.rinv) return fail(WG_ERR_CUDA, "out of device memory (scene)");
+        rinv.resize(nSlots);
+        for (int64_t q = 0; q < nSlots; q++) rinv[q] = reciprocals(minert[q]);
+        WG_CUDA_TRY(cudaMemcpyAsync(N.rinv, rinv.data(), sizeof(double4_32a) * nSlots, cudaMemcpyHostToDevice, S.stream));
+    }
     WG_CUDA_TRY(cudaMemcpyAsync(N.lastPos, posr.data(), sizeof(double4_32a) * nSlots, cudaMemcpyHostToDevice, S.stream));
     WG_CUDA_TRY(cudaMemcpyAsync(N.flags, flags.data(), sizeof(uint32_t) * nSlots, cudaMemcpyHostToDevice, S.stream));
     WG_CUDA_TRY(cudaMemcpyAsync(P.shape, shape.data(), sizeof(int32_t) * nPar, cudaMemcpyHostToDevice, S.stream));
@@ -1483,6 +1496,12 @@ static int writeSlot(Sim& S, int64_t p0, int64_t cap, int64_t n, const double* p
         put(S.P.aux + p0, aux.data(), sizeof(int4) * cap) || put(S.P.facet + p0, fac.data(), d4 * cap) ||
         put(S.P.mat + p0, mt.data(), sizeof(int32_t) * cap) || put(S.P.mask + p0, mk.data(), sizeof(uint32_t) * cap))
         return S.fail(WG_ERR_CUDA, "slot upload failed");
+    std::vector<double4_32a> rinv;
+    if (S.N.rinv) {
+        rinv.resize(cap);
+        for (int64_t q = 0; q < cap; q++) rinv[q] = reciprocals(mi[q]);
+        if (put(S.N.rinv + p0, rinv.data(), d4 * cap)) return S.fail(WG_ERR_CUDA, "slot upload failed");
+    }
     if (S.prec == WG_PREC_FP32) {
         std::vector<NodeConst32> nc(cap);
         std::vector<float4> ph(cap), pl(cap), vh(cap), vl(cap), of(cap);

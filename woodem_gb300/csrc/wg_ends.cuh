@@ -139,6 +139,17 @@ __device__ __forceinline__ void warpSumEnds(const EA* __restrict__ endA, const E
     }
 }
 
+// FP64 ends: every lane adds its own particle's slots straight from memory, all lanes of the warp at
+// once. The FP64 pipe takes a warp instruction's time whether 1 or 32 lanes are active, so a sum
+// staged through shared memory a few particles at a time (as the FP32 one above) spends it
+// many times over; the lines read by neighbouring lanes are shared through L1.
+__device__ __forceinline__ void laneSumEnds(const double4_32a* __restrict__ endA, const double2* __restrict__ endB, bool take, int e0,
+                                            int e1, SumD& acc) {
+    if (!take) return;
+#pragma unroll 2
+    for (int e = e0; e < e1; e++) acc.add(endA[e], endB[e]);
+}
+
 // Degree of particle p in the incidence and the first of its end slots.
 __device__ __forceinline__ void endRange(const DevIncidence& I, int p, int& e0, int& e1) {
     e0 = I.hiStart[p] + I.loStart[p];

@@ -84,6 +84,7 @@ struct DevNodes {
     double4_32a* force;   // fx fy fz 0
     double4_32a* torque;  // tx ty tz 0
     double4_32a* minert;  // ix iy iz mass
+    double4_32a* rinv;    // FP64 mode: the rounded reciprocals 1/ix 1/iy 1/iz 1/mass (0 for a zero)
     double4_32a* lastPos; // verlet reference position
     uint32_t* flags;
     // FP32-force mode: double-float mirrors written by Leapfrog for the sphere-sphere contacts

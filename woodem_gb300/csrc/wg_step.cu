@@ -6,6 +6,7 @@
 // the reference expression cited beside it.
 #include <algorithm>
 
+#include "wg_div.cuh"
 #include "wg_ends.cuh"
 #include "wg_energy.cuh"
 #include "wg_geom.cuh"
@@ -31,6 +32,12 @@ __device__ __forceinline__ double sgn(double s) { return s < 0 ? -1 : (s > 0 ? 1
 // are out-of-line functions: inlined, the compiler turns them into predicated FP64 instructions,
 // which occupy the FP64 pipe (1/64 of the FP32 rate on GB300) in every warp. The operations, and
 // so the results, are the same either way. PERI: the periodic corrections (Cell velocity gradient).
+// Bound by the FP64 pipe. Each lane sums its own end slots with the whole warp active (staged through
+// shared memory a few particles at a time, the sums and all that followed from them ran 12 lanes a
+// warp instruction: 747 FP64 instructions a warp for 246 operations a node), and the divisions by
+// mass, inertia and norms take one reciprocal per divisor (wg_div.cuh). With both and one-warp
+// blocks for small scenes: 10 000 settling spheres, 200 steps, 29.9 -> 19.3 ms; a drum of 250 000,
+// 40 steps, 50.8 -> 38.6 ms.
 __device__ __noinline__ D3 linAccelPartial(D3 f, double mass, uint32_t flags) {
     D3 a{0, 0, 0};
     if (!(flags & 1u)) a.x = 0. + f.x / mass;
@@ -63,10 +70,9 @@ __device__ __noinline__ void resetForce(DevNodes N, int i, double mass, bool gra
     N.torque[i] = make_double4_32a(0., 0., 0., 0.);
 }
 template <bool PERI, bool ENERGY>
-__global__ void __launch_bounds__(256) k_leapfrog(DevNodes N, DevParticles P, DevIncidence I, const ScenePar* __restrict__ spp,
+__global__ void __launch_bounds__(128) k_leapfrog(DevNodes N, DevParticles P, DevIncidence I, const ScenePar* __restrict__ spp,
                                                   int* __restrict__ dFlags, int fromEnds, const long long* __restrict__ dStepC,
                                                   EnergyCols E) {
-    __shared__ EndStage<double4_32a, double2, 32> stage[8];
     if (halted(dFlags)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < N.n;
@@ -100,7 +106,7 @@ __global__ void __launch_bounds__(256) k_leapfrog(DevNodes N, DevParticles P, De
         t = ld3(N.torque[i]);
     }
     SumD acc{f, t};
-    warpSumEnds(I.endA, I.endB, take, e0, e1, stage[threadIdx.x >> 5], acc);
+    laneSumEnds(I.endA, I.endB, take, e0, e1, acc);
     f = acc.F;
     t = acc.T;
     if (!valid || (flags & F_CLUMPED) || frozen) return;
@@ -134,7 +140,8 @@ __global__ void __launch_bounds__(256) k_leapfrog(DevNodes N, DevParticles P, De
         }
     }
     if (!blockedAll) {
-        if ((flags & F_DOF_ALL) == 0) linAccel = f / mass;
+        const double4_32a ri = N.rinv[i];
+        if ((flags & F_DOF_ALL) == 0) linAccel = divBy(f, mass, ri.w);
         else linAccel = linAccelPartial(f, mass, flags);
         D3 pvf = vel, pva = angVel;
         if (PERI) {
@@ -150,7 +157,7 @@ __global__ void __launch_bounds__(256) k_leapfrog(DevNodes N, DevParticles P, De
             vel = vel + dt * linAccel;
         if (!isZero(inertia)) {
             D3 angAccel{0, 0, 0};
-            if ((flags & F_DOF_ALL) == 0) angAccel = D3{t.x / inertia.x, t.y / inertia.y, t.z / inertia.z};
+            if ((flags & F_DOF_ALL) == 0) angAccel = divBy3(t, inertia, D3{ri.x, ri.y, ri.z});
             else angAccel = angAccelPartial(t, inertia, flags);
             if (damp) angAccel = dampAccel(angAccel, t, pva, damping, dt);
             angVel = angVel + dt * angAccel;
@@ -184,14 +191,14 @@ __global__ void __launch_bounds__(256) k_leapfrog(DevNodes N, DevParticles P, De
     DQ ori{o4.x, o4.y, o4.z, o4.w};
     if (!isZero(angVel)) {
         const double angle = sqrt(sqn(angVel));
-        const D3 axis = angVel / angle;
+        const D3 axis = divBy(angVel, angle);
         const double ha = 0.5 * (angle * dt);
         double s, c;
         sincos(ha, &s, &c);
         const DQ q{c, s * axis.x, s * axis.y, s * axis.z};
         ori = qmul(q, ori);
     }
-    ori = qnormalized(ori);
+    ori = qnormalizedQ(ori);
     N.posr[i] = st4(pos, pr.w);
     N.vel[i] = st4(vel, 0.);
     N.angv[i] = st4(angVel, 0.);
@@ -203,17 +210,23 @@ __global__ void __launch_bounds__(256) k_leapfrog(DevNodes N, DevParticles P, De
     if (d2 + 0. > sp.maxD2) atomicOr(dFlags + FL_FULL, 1);
 }
 
+// Threads per block of the FP64 kernels over n items: one warp per block while the blocks of one
+// warp can all be resident (32 a SM on 152 SMs), so that a small scene's warps spread over every
+// SM's FP64 pipe instead of queueing for a few of them; 128 beyond that.
+static int fp64Block(int64_t n) { return n <= 152 * 32 * 32 ? 32 : 128; }
+
 void launch_leapfrog(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevIncidence& I, const ScenePar* sp,
                      int* dFlags, int fromEnds, const long long* dStep, bool periodic, const EnergyCols* energy) {
     if (N.n == 0) return;
-    const unsigned g = (N.n + 255) / 256;
+    const int b = fp64Block(N.n);
+    const unsigned g = (N.n + b - 1) / b;
     const EnergyCols E = energy ? *energy : EnergyCols{};
     if (energy) {
-        if (periodic) k_leapfrog<true, true><<<g, 256, 0, st>>>(N, P, I, sp, dFlags, fromEnds, dStep, E);
-        else k_leapfrog<false, true><<<g, 256, 0, st>>>(N, P, I, sp, dFlags, fromEnds, dStep, E);
+        if (periodic) k_leapfrog<true, true><<<g, b, 0, st>>>(N, P, I, sp, dFlags, fromEnds, dStep, E);
+        else k_leapfrog<false, true><<<g, b, 0, st>>>(N, P, I, sp, dFlags, fromEnds, dStep, E);
     } else {
-        if (periodic) k_leapfrog<true, false><<<g, 256, 0, st>>>(N, P, I, sp, dFlags, fromEnds, dStep, E);
-        else k_leapfrog<false, false><<<g, 256, 0, st>>>(N, P, I, sp, dFlags, fromEnds, dStep, E);
+        if (periodic) k_leapfrog<true, false><<<g, b, 0, st>>>(N, P, I, sp, dFlags, fromEnds, dStep, E);
+        else k_leapfrog<false, false><<<g, b, 0, st>>>(N, P, I, sp, dFlags, fromEnds, dStep, E);
     }
 }
 
@@ -685,8 +698,7 @@ void launch_energy_sum(cudaStream_t st, const EnergyCols& E, int which, int64_t 
 // DemData.force/torque for reporting after a run: the sum of the Leapfrog kernel (m*g, then every
 // end slot of the particle in slot order) written to the node, for every particle whose degree
 // is at most kHeavyThreshold.
-__global__ void __launch_bounds__(256) k_forces(DevNodes N, DevParticles P, DevIncidence I, const ScenePar* __restrict__ spp) {
-    __shared__ EndStage<double4_32a, double2, 32> stage[8];
+__global__ void __launch_bounds__(128) k_forces(DevNodes N, DevParticles P, DevIncidence I, const ScenePar* __restrict__ spp) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const ScenePar& sp = spp[p < P.n ? sceneOfP(P, p) : 0];
     const bool uni = p < P.n && P.shape[p] != WG_SHAPE_FACET;
@@ -703,7 +715,7 @@ __global__ void __launch_bounds__(256) k_forces(DevNodes N, DevParticles P, DevI
         }
     }
     SumD acc{F, T};
-    warpSumEnds(I.endA, I.endB, take, e0, e1, stage[threadIdx.x >> 5], acc);
+    laneSumEnds(I.endA, I.endB, take, e0, e1, acc);
     if (uni && (take || !sp.applyForces)) {
         N.force[p] = st4(acc.F, 0.);
         N.torque[p] = st4(acc.T, 0.);
@@ -962,7 +974,8 @@ void launch_forces(cudaStream_t st, const DevNodes& N, const DevParticles& P, co
         if (I.nHeavyFree > 0) k_forces_heavy<<<(I.nHeavyFree + 3) / 4, 128, 0, st>>>(N, I, I.heavyFree, I.nHeavyFree, sp, dFlags);
         return;
     }
-    k_forces<<<(P.n + 255) / 256, 256, 0, st>>>(N, P, I, sp);
+    const int b = fp64Block(P.n);
+    k_forces<<<(P.n + b - 1) / b, b, 0, st>>>(N, P, I, sp);
     if (I.nHeavy > 0) k_forces_heavy<<<(I.nHeavy + 3) / 4, 128, 0, st>>>(N, I, I.heavy, I.nHeavy, sp, nullptr);
 }
 
