@@ -1062,7 +1062,7 @@ int Sim::run(int64_t n) {
         else if (trackE) {
             cudaMemsetAsync(eCon.col, 0, sizeof(double) * EN_CON_NCOL * eCon.cap, stream);
             launch_contact_fp64(stream, N, P, C, I, dMats, sp, dStep, dFlags, cfg.periodic != 0,
-                                (contactBlock > 0 && contactBlock <= 128) ? contactBlock : 128, &eCon);
+                                std::min(contactBlock, 128), &eCon);
             launch_energy_sum(stream, eCon, 1, I.nAct, dEPartial, dEnergy, dECreated, dFlags, false);
             launches += 2;
             if (cfg.periodic && cfg.eval_stress) {
@@ -1073,7 +1073,7 @@ int Sim::run(int64_t n) {
             }
         } else
             launch_contact_fp64(stream, N, P, C, I, dMats, sp, dStep, dFlags, cfg.periodic != 0,
-                                (contactBlock > 0 && contactBlock <= 128) ? contactBlock : 128);  // launch bounds 128
+                                std::min(contactBlock, 128));  // launch bounds 128; <= 0: by the number of contacts
         if (!advanced) launch_advance(stream, dStep, dFlags);
         launches += advanced ? 1 : 2;
     };

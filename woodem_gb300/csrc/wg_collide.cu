@@ -18,7 +18,8 @@
 //      set, carrying their persistent state                      (k_mark_orphans .. k_gather)
 //   6. CSR incidence for the deterministic force sum              (k_lo_start, hi sort, k_hi_start)
 #include <cub/cub.cuh>
-
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
 #include <cmath>
@@ -83,8 +84,8 @@ struct CollideWork {
     int32_t* orphSrc = nullptr;
     int32_t* src = nullptr;
     int64_t mergeCap = 0, orphCap = 0, srcCap = 0;
-    int32_t* act = nullptr;       // exclusive scan of the active contacts
-    int32_t* actSS = nullptr;     // exclusive scan of the active sphere-sphere contacts
+    uint64_t* act = nullptr;      // exclusive scan of the active contacts (low half) and the plain ones of them (high)
+    uint64_t* actReal = nullptr;  // FP64 mode: the same of the real contacts
     uint32_t* hiKeys = nullptr;
     uint32_t* hiKeysSorted = nullptr;
     int32_t* hiVals = nullptr;
@@ -842,23 +843,30 @@ __global__ void k_dormant(DevContacts C, DevNodes N, DevParticles P, const Scene
 }
 
 // ---------------------------------------------------------------- CSR incidence
-// Only active contacts (a functor applies and the pair is not dormant) own end slots; act is
-// their exclusive scan over the key-sorted contacts, act[n] = number of active contacts.
+// Only active contacts (a functor applies and the pair is not dormant) own end slots.
 __device__ __forceinline__ bool activeContact(uint32_t fl) { return ctype(fl) != CT_NONE && !(fl & C_DORMANT); }
-__global__ void k_active(const uint32_t* __restrict__ flags, int64_t n, int32_t* __restrict__ act, int32_t* __restrict__ actSS) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    const uint32_t fl = flags[c];
-    const bool a = activeContact(fl);
-    act[c] = a ? 1 : 0;
-    actSS[c] = (a && ctype(fl) == CT_SS) ? 1 : 0;
-}
+// a plain contact joins two spheres of the same period
+__device__ __forceinline__ bool plainContact(uint32_t fl, int32_t cd) { return ctype(fl) == CT_SS && cd == packCellDist(0, 0, 0); }
+// What one contact adds to the running counts that place the active contacts in the work list: 1 in
+// the low half, and 1 in the high half if it is plain; with `real`, real contacts alone.
+struct WorkClass {
+    const uint32_t* flags;
+    const int32_t* cdist;
+    int64_t n;
+    uint32_t real;
+    __device__ __forceinline__ uint64_t operator()(int64_t c) const {
+        if (c >= n) return 0;
+        const uint32_t fl = flags[c];
+        if (!activeContact(fl) || (fl & real) != real) return 0;
+        return 1ull | (plainContact(fl, cdist[c]) ? 1ull << 32 : 0ull);
+    }
+};
 // loStart[p] = active contacts with lo < p
-__global__ void k_lo_start(const uint64_t* __restrict__ key, int64_t n, int nPar, const int32_t* __restrict__ act,
+__global__ void k_lo_start(const uint64_t* __restrict__ key, int64_t n, int nPar, const uint64_t* __restrict__ act,
                            int32_t* __restrict__ loStart) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p > nPar) return;
-    loStart[p] = act[lowerBound64(key, n, (uint64_t)(uint32_t)p << 32)];
+    loStart[p] = (int32_t)(uint32_t)act[lowerBound64(key, n, (uint64_t)(uint32_t)p << 32)];
 }
 // hi id of the active contacts, nPar for the others (sorted past every particle)
 __global__ void k_hi_keys(const uint64_t* __restrict__ key, const uint32_t* __restrict__ flags, int64_t n, uint32_t nPar,
@@ -874,25 +882,43 @@ __global__ void k_hi_start(const uint32_t* __restrict__ hks, int64_t n, int nPar
     hiStart[p] = (int32_t)lowerBound32(hks, n, (uint32_t)p);
 }
 // end slots: active contact c with hi==p sits at loStart[p] + (its index k in hiList); with lo==p
-// at hiStart[p+1] + act[c] (see DevIncidence); inactive contacts have no slot (-1)
-// The work list holds the active contacts other than sphere-sphere first, then the sphere-sphere
-// ones, each group in ascending contact order (actSS: exclusive scan of the active sphere-sphere
-// contacts; nOther = active contacts that are not sphere-sphere).
-__global__ void k_slots(const uint64_t* __restrict__ key, const uint32_t* __restrict__ flags, int64_t n, int64_t nAct,
-                        const int32_t* __restrict__ act, const int32_t* __restrict__ actSS, int64_t nOther, DevIncidence I) {
+// at hiStart[p+1] + (active contacts before c) (see DevIncidence); inactive contacts have no slot (-1).
+// The work list holds the nOther active contacts that are not plain (walls, facets, spheres of
+// different periods) and then the plain ones, each group in ascending contact order. In the FP64 mode
+// (actReal) the real contacts of a group come before its others: a warp of the contact kernel then
+// holds contacts that all go through the functor chain or that all leave after the distance test.
+// Mixed, the FP64 pipe, which takes a warp instruction's time whatever its lanes do, ran the chain
+// for the two fifths of the lanes that were not real (drum of 250 000: contact loop 0.70 -> 0.49 ms a
+// step). The FP32 kernel is bound by the gathered mirror records, which the mixed order reads
+// once for both kinds (1M drum: 0.161 ms a step mixed, 0.168 split).
+// tot, totReal: the counts over all contacts.
+__global__ void k_slots(const uint64_t* __restrict__ key, const uint32_t* __restrict__ flags, const int32_t* __restrict__ cdist, int64_t n,
+                        const uint64_t* __restrict__ act, const uint64_t* __restrict__ actReal, uint64_t tot, uint64_t totReal,
+                        DevIncidence I) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
+    const int nAct = (int)(uint32_t)tot, nPlain = (int)(tot >> 32);
     if (k < nAct) {
         const int32_t ch = I.hiList[k];
         const int hiP = (int)(key[ch] & 0xffffffffu);
         I.slotHi[ch] = I.loStart[hiP] + (int32_t)k;
     }
-    if (activeContact(flags[k])) {
-        const int loP = (int)(key[k] >> 32);
-        I.slotLo[k] = I.hiStart[loP + 1] + act[k];
-        const uint32_t fl = flags[k];
-        const int hiP = (int)(key[k] & 0xffffffffu);
-        const int64_t w = (ctype(fl) == CT_SS) ? nOther + actSS[k] : act[k] - actSS[k];
+    const uint32_t fl = flags[k];
+    if (activeContact(fl)) {
+        const uint64_t a = act[k];
+        const int all = (int)(uint32_t)a, plain = (int)(a >> 32);
+        const int loP = (int)(key[k] >> 32), hiP = (int)(key[k] & 0xffffffffu);
+        I.slotLo[k] = I.hiStart[loP + 1] + all;
+        const bool isPlain = plainContact(fl, cdist[k]);
+        int w = isPlain ? plain : all - plain;  // place within the group
+        if (actReal) {
+            const uint64_t r = actReal[k];
+            const int rAll = (int)(uint32_t)r, rPlain = (int)(r >> 32);
+            const int before = isPlain ? rPlain : rAll - rPlain;  // real ones of the group before this contact
+            const int real = isPlain ? (int)(totReal >> 32) : (int)(uint32_t)totReal - (int)(totReal >> 32);
+            w = (fl & C_REAL) ? before : real + (w - before);
+        }
+        if (isPlain) w += nAct - nPlain;
         I.work[w] = (fl & C_SWAP) ? make_int4((int)k, hiP, loP, (int)(fl & 0xeu)) : make_int4((int)k, loP, hiP, (int)(fl & 0xeu));
     } else {
         I.slotLo[k] = -1;
@@ -1280,7 +1306,7 @@ int collide_full_run(Sim& S) {
     if (W.hiCap < std::max<int64_t>(n, 1)) {
         if (W.hiKeys) {
             S.dfree(W.hiKeys); S.dfree(W.hiKeysSorted); S.dfree(W.hiVals); S.dfree(S.I.hiList);
-            S.dfree(S.I.slotLo); S.dfree(S.I.slotHi); S.dfree(W.act); S.dfree(W.actSS); S.dfree(S.I.work);
+            S.dfree(S.I.slotLo); S.dfree(S.I.slotHi); S.dfree(W.act); S.dfree(W.actReal); S.dfree(S.I.work);
         }
         W.hiCap = std::max<int64_t>(n, 1) * 3 / 2 + 1024;
         W.hiKeys = (uint32_t*)S.dalloc(sizeof(uint32_t) * W.hiCap);
@@ -1289,32 +1315,32 @@ int collide_full_run(Sim& S) {
         S.I.hiList = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
         S.I.slotLo = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
         S.I.slotHi = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-        W.act = (int32_t*)S.dalloc(sizeof(int32_t) * (W.hiCap + 1));
-        W.actSS = (int32_t*)S.dalloc(sizeof(int32_t) * (W.hiCap + 1));
+        W.act = (uint64_t*)S.dalloc(sizeof(uint64_t) * (W.hiCap + 1));
+        W.actReal = S.prec == WG_PREC_FP64 ? (uint64_t*)S.dalloc(sizeof(uint64_t) * (W.hiCap + 1)) : nullptr;
         S.I.work = (int4*)S.dalloc(sizeof(int4) * W.hiCap);
-        if (!S.I.slotHi || !W.act || !S.I.work) return S.fail(WG_ERR_CUDA, "out of device memory (incidence)");
+        if (!S.I.slotHi || !W.act || !S.I.work || (S.prec == WG_PREC_FP64 && !W.actReal)) return S.fail(WG_ERR_CUDA, "out of device memory (incidence)");
     }
-    int64_t nAct = 0, nSS = 0;
+    uint64_t tot = 0, totReal = 0;
     {
-        WG_CUDA_TRY(cudaMemsetAsync(W.act, 0, sizeof(int32_t) * (n + 1), st));
-        WG_CUDA_TRY(cudaMemsetAsync(W.actSS, 0, sizeof(int32_t) * (n + 1), st));
-        if (n > 0) {
-            k_active<<<(unsigned)((n + BS - 1) / BS), BS, 0, st>>>(S.C.flags, n, W.act, W.actSS);
+        auto scan = [&](uint32_t real, uint64_t* out, uint64_t* total) -> int {
+            const auto in = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), WorkClass{S.C.flags, S.C.cdist, n, real});
             size_t tb = 0;
-            cub::DeviceScan::ExclusiveSum(nullptr, tb, W.act, W.act, (int)(n + 1), st);
+            cub::DeviceScan::ExclusiveSum(nullptr, tb, in, out, (int)(n + 1), st);
             if (ensureCub(S, tb)) return WG_ERR_CUDA;
             tb = W.cubBytes;
-            WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, W.act, W.act, (int)(n + 1), st));
-            tb = W.cubBytes;
-            WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, W.actSS, W.actSS, (int)(n + 1), st));
+            WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, in, out, (int)(n + 1), st));
+            WG_CUDA_TRY(cudaMemcpyAsync(total, out + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+            return 0;
+        };
+        int q = scan(0, W.act, &tot);
+        if (q) return q;
+        if (W.actReal) {
+            q = scan(C_REAL, W.actReal, &totReal);
+            if (q) return q;
         }
-        int32_t h[2] = {0, 0};
-        WG_CUDA_TRY(cudaMemcpyAsync(&h[0], W.act + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        WG_CUDA_TRY(cudaMemcpyAsync(&h[1], W.actSS + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         WG_CUDA_TRY(cudaStreamSynchronize(st));
-        nAct = h[0];
-        nSS = h[1];
     }
+    const int64_t nAct = (int64_t)(uint32_t)tot, nSS = (int64_t)(tot >> 32);
     k_lo_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, n, (int)S.nPar, W.act, S.I.loStart);
     if (S.I.endCap < 2 * std::max<int64_t>(nAct, 1)) {
         if (S.I.endA) { S.dfree(S.I.endA); S.dfree(S.I.endB); }
@@ -1342,7 +1368,8 @@ int collide_full_run(Sim& S) {
         WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiBits, st));
     }
     k_hi_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.hiKeysSorted, n, (int)S.nPar, S.I.hiStart);
-    if (n > 0) k_slots<<<(unsigned)((n + BS - 1) / BS), BS, 0, st>>>(S.C.key, S.C.flags, n, nAct, W.act, W.actSS, nAct - nSS, S.I);
+    if (n > 0) k_slots<<<(unsigned)((n + BS - 1) / BS), BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, tot, totReal,
+                                                                           S.I);
     S.I.nAct = nAct;
     S.nMixed = nAct - nSS;
     // every end starts without a contribution; the contact kernel fills the real ones this step

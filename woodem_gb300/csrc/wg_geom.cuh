@@ -1,6 +1,7 @@
 // Cg2 geometry functors in FP64 (shared by the FP64 and FP32 contact kernels).
 // Every expression keeps the operand order of the reference expression it restates.
 #pragma once
+#include "wg_div.cuh"
 #include "wg_internal.h"
 #include "wg_math.cuh"
 
@@ -76,7 +77,7 @@ __device__ __forceinline__ bool geomSS(const DevNodes& N, int A, int B, D3 shift
     if (unDistSq > 0 && !real) return false;
     const double dist = sqrt(sqn(relPos));
     g.uN = dist - (r1 + r2);
-    g.normal = relPos / dist;
+    g.normal = divBy(relPos, dist);
     g.contPt = p1 + (r1 + 0.5 * g.uN) * g.normal;
     g.pos1 = p1;
     g.vel1 = ld3(N.vel[A]);
@@ -144,7 +145,7 @@ __device__ __forceinline__ bool geomFS(const DevNodes& N, const DevParticles& P,
     const D3 sC = ld3(ps) + shift2;
     const D3 p0 = ld3(N.posr[fn.x]), p1 = ld3(N.posr[fn.y]), p2 = ld3(N.posr[fn.z]);
     const D3 nn = cross(p1 - p0, p2 - p0);
-    const D3 fNormal = normalized(nn);
+    const D3 fNormal = normalizedQ(nn);
     const double planeDist = dot(sC - p0, fNormal);
     if (fabs(planeDist) > (radius + halfThick) && !real) return false;
     const D3 fC = sC - planeDist * fNormal;
@@ -167,7 +168,7 @@ __device__ __forceinline__ bool geomFS(const DevNodes& N, const DevParticles& P,
     const double rh = radius + halfThick;
     if (sqn(normal) > rh * rh && !real) return false;
     const double dist = sqrt(sqn(normal));
-    normal = normal / dist;
+    normal = divBy(normal, dist);
     if (halfThick > 0) contPt = contPt + normal * halfThick;
     g.uN = (dist - radius) - halfThick;
     // barycentric interpolation of the facet node velocities at contPt

@@ -161,8 +161,9 @@ struct DevIncidence {
     int32_t* loStart;  // nPar+1: contacts with lo==p are [loStart[p], loStart[p+1])
     int32_t* hiStart;  // nPar+1: hiList[hiStart[p] .. hiStart[p+1]) are contacts with hi==p, ascending
     int32_t* hiList;
-    int4* work;        // active contacts (contact, pA, pB, type|swap flag bits): those that are not
-                       // sphere-sphere first, then the sphere-sphere ones, each in ascending order
+    int4* work;        // active contacts (contact, pA, pB, type|swap flag bits): walls, facets and
+                       // spheres of different periods first, then the plain pairs of spheres (FP64
+                       // mode: in both the real ones before the others), in ascending order
     int64_t nAct;
     int32_t* slotLo;   // per contact: end slot of its lo particle (-1: no slot, the contact is inactive)
     int32_t* slotHi;   // per contact: end slot of its hi particle
@@ -232,7 +233,7 @@ void launch_leapfrog(cudaStream_t st, const DevNodes& N, const DevParticles& P, 
                      int* dFlags, int fromEnds, const long long* dStep, bool periodic, const EnergyCols* energy = nullptr);
 void launch_contact_fp64(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C,
                          const DevIncidence& I, const double4_32a* mats, const ScenePar* sp, const long long* dStep, int* dFlags,
-                         bool periodic, int block = 128, const EnergyCols* energy = nullptr);
+                         bool periodic, int block = 0, const EnergyCols* energy = nullptr);
 // perStep: only the heavy particles with a free DOF (guarded by the flags), before Leapfrog;
 // otherwise every particle's DemData.force/torque (reporting at the end of a run).
 void launch_forces(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevIncidence& I, const ScenePar* sp,
@@ -263,8 +264,8 @@ void launch_leapfrog32(cudaStream_t st, const DevNodes& N, const DevParticles& P
                        const ScenePar* sp, int* dFlags, int fromEnds, const long long* dStep, bool periodic,
                        const EnergyCols* energy = nullptr);
 // The kernels walk the active contacts I.work[0, I.nAct). Items [0, nMixed) are facet and wall
-// contacts; [nMixed, I.nAct) join two spheres and, in an aperiodic scene, go to a
-// sphere-sphere-only kernel.
+// contacts and pairs of spheres across a periodic boundary; [nMixed, I.nAct) join two spheres
+// of the same period and, in an aperiodic scene, go to a sphere-sphere-only kernel.
 // With a side stream the mixed range runs beside the sphere-sphere range (joined on st).
 struct SideStream {
     cudaStream_t st = nullptr;
@@ -354,7 +355,7 @@ struct Sim {
     DevContacts C{}, Cb{};  // current and spare (merge target)
     DevIncidence I{};
     int64_t cCap = 0;
-    int64_t nMixed = 0;   // work items [0, nMixed) are not sphere-sphere (see launch_contact_fp32)
+    int64_t nMixed = 0;   // work items [0, nMixed) are not plain pairs of spheres (see launch_contact_fp32)
     DevPackedSS K{};      // FP32-force mode: packed state of the active sphere-sphere contacts
     bool packDirty = false;  // K changed since it was last written back to the contact arrays
     double4_32a* dMats = nullptr;
@@ -386,7 +387,7 @@ struct Sim {
     bool fromEnds = false;   // the end slots hold the forces of the last contact loop
     // launch shape (wg_set_launch): threads per block of the contact kernels, steps queued per host
     // check, and whether a chunk of steps is replayed as a CUDA graph
-    int contactBlock = 0;    // 0: default (FP32: the resident-grid sphere-sphere kernel; FP64: 128)
+    int contactBlock = 0;    // 0: default (FP32: the resident-grid sphere-sphere kernel; FP64: by the contacts' number)
     int chunkSteps = 32;
     bool useGraph = false;
     bool concurrentContacts = true;   // facet/wall contacts beside, not before, the sphere-sphere ones

@@ -85,6 +85,29 @@ __host__ __device__ __forceinline__ DQ quatFromCols(D3 c0, D3 c1, D3 c2) {
     }
     return q;
 }
+// The same on the device with one square root and one division for all four branches: their operands
+// are selected first (a warp whose frames fall into several branches would run each of them).
+__device__ __forceinline__ DQ quatFromColsSel(D3 c0, D3 c1, D3 c2) {
+    const double m00 = c0.x, m11 = c1.y, m22 = c2.z;
+    const double tr = (m00 + m11) + m22;
+    const double d0 = c1.z - c2.y, d1 = c2.x - c0.z, d2 = c0.y - c1.x;  // m21-m12, m02-m20, m10-m01
+    const double s01 = c0.y + c1.x, s02 = c0.z + c2.x, s12 = c1.z + c2.y;
+    const bool pos = tr > 0;
+    int i = 0;
+    if (m11 > m00) i = 1;
+    if (m22 > (i == 1 ? m11 : m00)) i = 2;
+    const double a = i == 0 ? m00 : (i == 1 ? m11 : m22), b = i == 0 ? m11 : (i == 1 ? m22 : m00), c = i == 0 ? m22 : (i == 1 ? m00 : m11);
+    const double s = sqrt((pos ? tr : (a - b) - c) + 1.0);
+    const double h = 0.5 * s, v = 0.5 / s;
+    // the three products (w, x, y or z is h itself)
+    const double p = (pos ? d0 : (i == 0 ? d0 : (i == 1 ? d1 : d2))) * v;
+    const double q = (pos ? d1 : (i == 2 ? s02 : s01)) * v;
+    const double r = (pos ? d2 : (i == 0 ? s02 : s12)) * v;
+    if (pos) return DQ{h, p, q, r};
+    if (i == 0) return DQ{p, h, q, r};
+    if (i == 1) return DQ{p, q, h, r};
+    return DQ{p, q, r, h};
+}
 // v' = v + w*(2 q x v) + q x (2 q x v)
 __host__ __device__ __forceinline__ D3 qrot(DQ q, D3 v) {
     D3 qv{q.x, q.y, q.z};
