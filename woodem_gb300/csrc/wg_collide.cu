@@ -31,6 +31,7 @@
 
 namespace wg {
 
+struct PeriBox;
 struct CollideWork {
     // sphere and "large" (non-sphere) id lists, built at upload
     int32_t* sphereIds = nullptr;
@@ -48,7 +49,7 @@ struct CollideWork {
     int32_t* sid = nullptr;       // sorted sphere ids
     double4_32a* smn = nullptr;
     double4_32a* smx = nullptr;
-    uint32_t* smask = nullptr;
+    PeriBox* speri = nullptr;     // periodic: the sorted boxes in fractions of the cell
     float4* smnf = nullptr;       // box min rounded down, mask in w
     float4* smxf = nullptr;       // box max rounded up, particle id in w
     int32_t* newLo = nullptr;     // first index of each lo id in the sorted new pairs (merge)
@@ -264,7 +265,7 @@ __global__ void k_cell_off(const uint32_t* __restrict__ skey, int n, int64_t nce
 }
 
 __global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ sid, int n, double4_32a* __restrict__ smn,
-                                double4_32a* __restrict__ smx, uint32_t* __restrict__ smask, float4* __restrict__ smnf,
+                                double4_32a* __restrict__ smx, float4* __restrict__ smnf,
                                 float4* __restrict__ smxf, float4* __restrict__ smnfi, float4* __restrict__ smxfi) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -273,7 +274,6 @@ __global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ sid,
     const uint32_t m = P.mask[p];
     smn[i] = a;
     smx[i] = b;
-    smask[i] = m;
     smnf[i] = make_float4(__double2float_rd(a.x), __double2float_rd(a.y), __double2float_rd(a.z), __uint_as_float(m));
     smxf[i] = make_float4(__double2float_ru(b.x), __double2float_ru(b.y), __double2float_ru(b.z), __int_as_float(p));
     smnfi[i] = make_float4(__double2float_ru(a.x), __double2float_ru(a.y), __double2float_ru(a.z), 0.f);
@@ -505,64 +505,136 @@ __device__ __forceinline__ void flushPairsCd(uint64_t (&buf)[kPairBuf], int32_t 
         }
     nb = 0;
 }
+// A sphere's box in the periodic sweep, in sorted order: the box minimum as a fraction of the cell in
+// [0, 1) with its period taken off, and the box's edges as fractions.
+struct PeriBox {
+    float4 u;  // fraction per axis, mask in w
+    float4 l;  // edges per axis
+    int4 p;    // periods per axis, particle id in w
+};
+// How far the FP32 fractions above may be from the exact ones: below 3 roundings of 2^-24 each with
+// those of the FP64 quotients behind them; ten times that is decided in FP64.
+constexpr float kPeriEps = 2e-6f;
+__global__ void k_gather_peri(DevParticles P, const int32_t* __restrict__ sid, int n, const ScenePar* __restrict__ spp,
+                              PeriBox* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int q = sid[i];
+    const double4_32a a = P.mn[q], b = P.mx[q];
+    const double m[3] = {a.x, a.y, a.z}, x[3] = {b.x, b.y, b.z};
+    float u[3], l[3];
+    int p[3];
+    for (int k = 0; k < 3; k++) {
+        const double d = 1. / spp->cellSize[k], f = m[k] * d, fl = floor(f);
+        p[k] = (int)fl;
+        u[k] = (float)(f - fl);
+        l[k] = (float)((x[k] - m[k]) * d);
+    }
+    out[i].u = make_float4(u[0], u[1], u[2], __uint_as_float(P.mask[q]));
+    out[i].l = make_float4(l[0], l[1], l[2], 0.f);
+    out[i].p = make_int4(p[0], p[1], p[2], q);
+}
+// out of line: a few pairs in ten thousand come here
+static __device__ __noinline__ int overlapPeriExact(const DevParticles& P, int lo, int hi, const ScenePar* __restrict__ spp, int* per) {
+    return overlapPeri(P.mn[lo], P.mx[lo], P.mn[hi], P.mx[hi], spp->cellSize, per);
+}
+// One axis of the periodic overlap of boxes i and j in fractions of the cell: d, the distance from i's
+// minimum to the nearest image of j's, taken modulo 1; r the period taken off. The boxes overlap where
+// the one that starts later starts within the other (boxes shorter than half the cell). Returns the
+// gap (negative: overlap).
+__device__ __forceinline__ float periGap(float ui, float li, float uj, float lj, float& d, int& r) {
+    d = uj - ui;
+    const float f = rintf(d);
+    r = (int)f;
+    d -= f;
+    return d >= 0.f ? d - li : -d - lj;
+}
 // Periodic sweep: particle i tests the spheres of higher id in the (up to 27, wrapped, distinct)
-// cells around its own with the periodic overlap test; each pair is met once, from its lo id.
-__global__ void k_pairs_ss_peri(const uint32_t* __restrict__ skey, const int32_t* __restrict__ sid, const double4_32a* __restrict__ smn,
-                                const double4_32a* __restrict__ smx, const uint32_t* __restrict__ smask, int n, Grid G,
-                                const int32_t* __restrict__ off, uint32_t lone, const ScenePar* __restrict__ spp,
-                                uint64_t* __restrict__ pairs, int32_t* __restrict__ cds, int64_t cap,
-                                unsigned long long* __restrict__ counter, int* __restrict__ dErr) {
+// cells around its own; each pair is met once, from its lo id.
+// The exact test (overlapPeri: 18 FP64 divisions a pair) decides only the pairs with a gap or a
+// distance within kPeriEps of zero; every other one is rejected, or accepted with its periods, from
+// the FP32 fractions:
+//   the origin of overlapPeri's wrap is the box that starts first (d > 0: i's, d < 0: j's), so that
+//   the periods are p_i - p_j - r either way, and the overlap is a gap of zero or less.
+// exactOnly: some box is about half the cell or longer on an axis, where overlapPeri raises an error;
+// every candidate then goes through it.
+// Bound by instruction issue over about 85 candidates a sphere. With the exact test on every candidate
+// the sweep took nearly all of a full run of 200 000 spheres: 9.0 -> 0.48 ms.
+__global__ void __launch_bounds__(128) k_pairs_ss_peri(DevParticles P, const uint32_t* __restrict__ skey, const PeriBox* __restrict__ box,
+                                                       int n, Grid G, const int32_t* __restrict__ off, uint32_t lone, int exactOnly,
+                                                       const ScenePar* __restrict__ spp, uint64_t* __restrict__ pairs,
+                                                       int32_t* __restrict__ cds, int64_t cap, unsigned long long* __restrict__ counter,
+                                                       int* __restrict__ dErr) {
     const unsigned FULL = 0xffffffffu;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < n;
-    const ScenePar& sp = *spp;
-    int cx = 0, cy = 0, cz = 0, pi = 0;
-    uint32_t m1 = 0;
-    double4_32a mn1 = make_double4_32a(0., 0., 0., 0.), mx1 = mn1;
+    const int nx = G.nx, ny = G.ny, nz = G.nz;
+    int cx = 0, cy = 0, cz = 0;
+    PeriBox me{};
     if (valid) {
         const uint32_t k = skey[i];
-        cx = (int)(k % (uint32_t)G.nx);
-        cy = (int)((k / (uint32_t)G.nx) % (uint32_t)G.ny);
-        cz = (int)(k / ((uint32_t)G.nx * (uint32_t)G.ny));
-        pi = sid[i];
-        m1 = smask[i];
-        mn1 = smn[i];
-        mx1 = smx[i];
+        cx = (int)(k % (uint32_t)nx);
+        cy = (int)((k / (uint32_t)nx) % (uint32_t)ny);
+        cz = (int)(k / ((uint32_t)nx * (uint32_t)ny));
+        me = box[i];
     }
-    const int nx = G.nx, ny = G.ny, nz = G.nz;
-    // distinct wrapped offsets per axis
-    const int ox = nx >= 3 ? 3 : nx, oy = ny >= 3 ? 3 : ny, oz = nz >= 3 ? 3 : nz;
+    const uint32_t m1 = __float_as_uint(me.u.w);
+    const int pi = me.p.w;
+    // distinct wrapped rows; along x the cells cx-1 .. cx+1 as one run of sorted spheres, and the cell
+    // across the boundary as a second one
+    const int oy = ny >= 3 ? 3 : ny, oz = nz >= 3 ? 3 : nz;
+    const int xa = nx >= 3 ? max(cx - 1, 0) : 0, xb = nx >= 3 ? min(cx + 1, nx - 1) : nx - 1;
+    const int xw = nx >= 3 ? (cx == 0 ? nx - 1 : (cx == nx - 1 ? 0 : -1)) : -1;
     uint64_t buf[kPairBuf];
     int32_t cbuf[kPairBuf];
     int nb = 0;
-    for (int q = 0; q < ox * oy * oz; q++) {
-        const int dx = q % ox - (ox == 3 ? 1 : 0), dy = (q / ox) % oy - (oy == 3 ? 1 : 0), dz = q / (ox * oy) - (oz == 3 ? 1 : 0);
-        const int x = ((cx + dx) % nx + nx) % nx, y = ((cy + dy) % ny + ny) % ny, z = ((cz + dz) % nz + nz) % nz;
-        const int64_t cell = ((int64_t)z * ny + y) * nx + x;
-        const int beg = valid ? off[cell] : 0, end = valid ? off[cell + 1] : 0;
-        int j = beg;
-        for (;;) {
-            const bool has = j < end;
-            if (!__any_sync(FULL, has)) break;
-            if (has) {
-                const int pj = sid[j];
-                if (pj > pi && maskOk(m1, smask[j], lone)) {
-                    int per[3];
-                    const int r = overlapPeri(mn1, mx1, smn[j], smx[j], sp.cellSize, per);
-                    if (r < 0) atomicCAS(dErr, 0, 103);
-                    else if (r > 0) {
-                        const uint64_t key = pairKey(pi, pj);
-                        const int32_t cd = packCellDist(per[0], per[1], per[2]);
+    for (int q = 0; q < 2 * oy * oz; q++) {
+        const int row = q >> 1;
+        const int dy = row % oy - (oy == 3 ? 1 : 0), dz = row / oy - (oz == 3 ? 1 : 0);
+        int y = cy + dy, z = cz + dz;
+        y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
+        z = z < 0 ? z + nz : (z >= nz ? z - nz : z);
+        const int64_t rowBase = ((int64_t)z * ny + y) * nx;
+        int j = 0, end = 0;
+        if (valid) {
+            if (!(q & 1)) {
+                j = off[rowBase + xa];
+                end = off[rowBase + xb + 1];
+            } else if (xw >= 0) {
+                j = off[rowBase + xw];
+                end = off[rowBase + xw + 1];
+            }
+        }
+        for (; __any_sync(FULL, j < end); j++) {
+            if (j < end) {
+                const float4 u = box[j].u, l = box[j].l;
+                float dx, dyy, dzz;
+                int rx, ry, rz;
+                const float gx = periGap(me.u.x, me.l.x, u.x, l.x, dx, rx), gy = periGap(me.u.y, me.l.y, u.y, l.y, dyy, ry),
+                            gz = periGap(me.u.z, me.l.z, u.z, l.z, dzz, rz);
+                const float gap = fmaxf(fmaxf(gx, gy), gz);
+                if (gap <= kPeriEps || exactOnly) {
+                    const int4 p = box[j].p;
+                    const int pj = p.w;
+                    if (pj > pi && maskOk(m1, __float_as_uint(u.w), lone)) {
+                        int per[3] = {me.p.x - p.x - rx, me.p.y - p.y - ry, me.p.z - p.z - rz};
+                        int r = 1;
+                        if (exactOnly || gap >= -kPeriEps || fminf(fminf(fabsf(dx), fabsf(dyy)), fabsf(dzz)) <= kPeriEps)
+                            r = overlapPeriExact(P, pi, pj, spp, per);
+                        if (r < 0) atomicCAS(dErr, 0, 103);
+                        else if (r > 0) {
+                            const uint64_t key = pairKey(pi, pj);
+                            const int32_t cd = packCellDist(per[0], per[1], per[2]);
 #pragma unroll
-                        for (int q = 0; q < kPairBuf; q++)
-                            if (q == nb) {
-                                buf[q] = key;
-                                cbuf[q] = cd;
-                            }
-                        nb++;
+                            for (int v = 0; v < kPairBuf; v++)
+                                if (v == nb) {
+                                    buf[v] = key;
+                                    cbuf[v] = cd;
+                                }
+                            nb++;
+                        }
                     }
                 }
-                j++;
             }
             if (__any_sync(FULL, nb == kPairBuf)) flushPairsCd(buf, cbuf, nb, pairs, cds, cap, counter);
         }
@@ -1043,6 +1115,7 @@ int collide_full_run(Sim& S) {
     const int K = S.nScenes;
     std::vector<Grid> hG(K, Grid{0, 0, 0, 1, 1, 1, 1, 1, 0});
     Grid G = hG[0];
+    bool periExact = false;
     const int ns = W.nSph;
     if (ns > 0) {
         const int nb = (int)W.hChunk.size() - 1;
@@ -1104,14 +1177,19 @@ int collide_full_run(Sim& S) {
             W.cellKeySorted = (uint32_t*)S.dalloc(sizeof(uint32_t) * cap);
             W.cellVal = (int32_t*)S.dalloc(sizeof(int32_t) * cap);
             W.sid = (int32_t*)S.dalloc(sizeof(int32_t) * cap);
-            W.smn = (double4_32a*)S.dalloc(sizeof(double4_32a) * cap);
-            W.smx = (double4_32a*)S.dalloc(sizeof(double4_32a) * cap);
-            W.smask = (uint32_t*)S.dalloc(sizeof(uint32_t) * cap);
-            W.smnf = (float4*)S.dalloc(sizeof(float4) * cap);
-            W.smxf = (float4*)S.dalloc(sizeof(float4) * cap);
-            W.smnfi = (float4*)S.dalloc(sizeof(float4) * cap);
-            W.smxfi = (float4*)S.dalloc(sizeof(float4) * cap);
-            if (!W.smask || !W.smxf || !W.smxfi) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
+            if (!W.sid) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
+            if (S.cfg.periodic) {
+                W.speri = (PeriBox*)S.dalloc(sizeof(PeriBox) * cap);
+                if (!W.speri) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
+            } else {
+                W.smn = (double4_32a*)S.dalloc(sizeof(double4_32a) * cap);
+                W.smx = (double4_32a*)S.dalloc(sizeof(double4_32a) * cap);
+                W.smnf = (float4*)S.dalloc(sizeof(float4) * cap);
+                W.smxf = (float4*)S.dalloc(sizeof(float4) * cap);
+                W.smnfi = (float4*)S.dalloc(sizeof(float4) * cap);
+                W.smxfi = (float4*)S.dalloc(sizeof(float4) * cap);
+                if (!W.smn || !W.smx || !W.smnf || !W.smxf || !W.smnfi || !W.smxfi) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
+            }
         }
         W.cellOff = grow(S, W.cellOff, W.cellOffCap, ncellAll + 1);
         if (S.cfg.periodic) k_cellkey_peri<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.sphereIds, ns, G, S.dPar, W.cellKey, W.cellVal);
@@ -1124,7 +1202,12 @@ int collide_full_run(Sim& S) {
         tb = W.cubBytes;
         WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.cellKey, W.cellKeySorted, W.cellVal, W.sid, ns, 0, endBit, st));
         k_cell_off<<<(unsigned)((ncellAll + 1 + BS - 1) / BS), BS, 0, st>>>(W.cellKeySorted, ns, ncellAll, W.cellOff);
-        k_gather_sorted<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.sid, ns, W.smn, W.smx, W.smask, W.smnf, W.smxf, W.smnfi, W.smxfi);
+        if (S.cfg.periodic) {
+            k_gather_peri<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.sid, ns, S.dPar, W.speri);
+            // the grid's cells are no shorter than the longest box edge
+            for (int q = 0; q < 3; q++) periExact = periExact || !(hG[0].h <= 0.49 * S.hPar.cellSize[q]);
+        } else
+            k_gather_sorted<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.sid, ns, W.smn, W.smx, W.smnf, W.smxf, W.smnfi, W.smxfi);
     }
     // lists of large particles: facets with boxes spanning a few cells use the grid, the rest are global
     {
@@ -1178,8 +1261,8 @@ int collide_full_run(Sim& S) {
                 if (!W.pairCd || !W.pairCdSorted) return S.fail(WG_ERR_CUDA, "out of device memory (pairs)");
             }
             if (ns > 0)
-                k_pairs_ss_peri<<<(ns + BS - 1) / BS, BS, 0, st>>>(W.cellKeySorted, W.sid, W.smn, W.smx, W.smask, ns, G, W.cellOff, lone,
-                                                                 S.dPar, W.pairs, W.pairCd, W.pairCap, W.counter, S.dFlags + FL_ERR);
+                k_pairs_ss_peri<<<(ns + 127) / 128, 128, 0, st>>>(S.P, W.cellKeySorted, W.speri, ns, G, W.cellOff, lone, periExact ? 1 : 0,
+                                                                  S.dPar, W.pairs, W.pairCd, W.pairCap, W.counter, S.dFlags + FL_ERR);
             if (ns > 0 && W.nGlobal > 0)
                 k_pairs_global_peri<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.globalIds, W.nGlobal, W.sphereIds, ns, lone, S.dPar,
                                                                      W.pairs, W.pairCd, W.pairCap, W.counter, S.dFlags + FL_ERR);
