@@ -199,6 +199,10 @@ int wg_put_state(wg_scene* s, const double* pos, const double* ori, const double
 int wg_get_nodes(wg_scene* s, double* pos, double* ori, double* vel, double* ang_vel,
                  double* force, double* torque);
 int wg_get_stats(wg_scene* s, wg_stats* out);
+/* Scene.step, Scene.time, nFullRuns and ContactLoop.stress (9, row-major) of scene k (0: a single
+   scene) as wg_get_stats and wg_get_scene_stats give them, from the host side alone: no contact is
+   counted and the device is not waited for. Null pointers are skipped. */
+int wg_get_clock(wg_scene* s, int32_t k, int64_t* step, double* time, int64_t* n_full_runs, double* stress9);
 /* Scene.dt/nextDt and the DynDt counters after the last run (DynDt::run, pkg/dem/DynDt.cpp:93-113;
    PeriodicEngine::isActivated, core/Engine.cpp:169-194). */
 int wg_get_dyndt(wg_scene* s, wg_dyndt_state* out);

@@ -84,10 +84,11 @@ class Batch:
         L, h = self.H.L, self.H.h
         self.H.check(L.wg_run(h, int(n)), "run")
         self.stale = True
+        step, time = C.c_int64(), C.c_double()
         for k, S in enumerate(self.scenes):
-            st = self.scene_stats(k)
-            S.step = int(st.step)
-            S.time = float(st.time)
+            self.H.check(L.wg_get_clock(h, k, C.byref(step), C.byref(time), None, None), "get_clock")
+            S.step = step.value
+            S.time = time.value
             d = _native.wg_dyndt_state()
             self.H.check(L.wg_get_scene_dyndt(h, k, C.byref(d)), "get_scene_dyndt")
             S.dt = float(d.dt)
@@ -107,8 +108,7 @@ class Batch:
         """Bring the node state of every scene back into its host containers."""
         if not self.stale:
             return
-        out = {k: np.empty((self.n_nodes, w)) for k, w in (("pos", 3), ("ori", 4), ("vel", 3), ("angVel", 3), ("force", 3),
-                                                            ("torque", 3))}
+        out = _plan.node_arrays(self.n_nodes)
         self.H.check(self.H.L.wg_get_nodes(self.H.h, *[_native.ptr(out[k]) for k in ("pos", "ori", "vel", "angVel", "force",
                                                                                          "torque")]), "get_nodes")
         for k, S in enumerate(self.scenes):

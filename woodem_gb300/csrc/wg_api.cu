@@ -8,6 +8,7 @@
 #include <cstring>
 #include <limits>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "wg_internal.h"
@@ -51,6 +52,7 @@ Sim::~Sim() {
     for (void* p : allocs) cudaFree(p);
     allocs.clear();
     if (hFlags) cudaFreeHost(hFlags);
+    if (hDown) cudaFreeHost(hDown);
     for (int i = 0; i < 8; i++)
         if (ev[i]) cudaEventDestroy(ev[i]);
     for (cudaEvent_t e : evPool) cudaEventDestroy(e);
@@ -269,6 +271,52 @@ static cudaError_t copyState(double* stage, int64_t na, double* const host[6], i
         q = e;
     }
     return cudaSuccess;
+}
+
+// The state from the staging buffer into the caller's pageable arrays (null ones skipped), a large one:
+// threads take chunks in turn, each through a page-locked buffer of its own. Straight into pageable
+// memory the 152 MB of a million nodes take between 1 and 25 ms, depending on where its pages
+// lie, and 17 through the driver's own staging and a second copy; this way 3.
+constexpr int64_t kDownloadChunk = int64_t(1) << 18;  // doubles: 2 MB
+constexpr int kDownloadThreads = 8;
+static int downloadState(Sim& S, double* stage, int64_t na, double* const host[6]) {
+    if (!S.hDown) WG_CUDA_TRY(cudaMallocHost(&S.hDown, sizeof(double) * kDownloadChunk * kDownloadThreads));
+    const int64_t off[7] = {0, 3, 7, 10, 13, 16, 19};
+    struct Piece {
+        double *to, *from;
+        int64_t n;
+    };
+    std::vector<Piece> todo;
+    for (int q = 0; q < 6; q++)
+        if (host[q])
+            for (int64_t a = 0, n = (off[q + 1] - off[q]) * na; a < n; a += kDownloadChunk)
+                todo.push_back({host[q] + a, stage + off[q] * na + a, std::min(kDownloadChunk, n - a)});
+    std::vector<cudaError_t> res(kDownloadThreads, cudaSuccess);
+    auto work = [&](int t) {
+        double* buf = S.hDown + kDownloadChunk * t;
+        cudaEvent_t e = nullptr;
+        cudaError_t r = cudaSetDevice(S.device);
+        if (r == cudaSuccess) r = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+        for (size_t q = t; q < todo.size() && r == cudaSuccess; q += kDownloadThreads) {
+            r = cudaMemcpyAsync(buf, todo[q].from, sizeof(double) * todo[q].n, cudaMemcpyDeviceToHost, S.stream);
+            if (r == cudaSuccess) r = cudaEventRecord(e, S.stream);
+            if (r == cudaSuccess) r = cudaEventSynchronize(e);
+            if (r == cudaSuccess) std::memcpy(todo[q].to, buf, sizeof(double) * todo[q].n);
+        }
+        if (e) cudaEventDestroy(e);
+        res[t] = r;
+    };
+    std::vector<std::thread> pool;
+    try {
+        for (int t = 1; t < kDownloadThreads; t++) pool.emplace_back(work, t);
+    } catch (...) {  // no more threads: this one takes the rest
+    }
+    const int started = 1 + (int)pool.size();
+    work(0);
+    for (int t = started; t < kDownloadThreads; t++) work(t);
+    for (std::thread& t : pool) t.join();
+    for (cudaError_t r : res) WG_CUDA_TRY(r);
+    return 0;
 }
 
 // The early part of wg_run_host's copy-out (see Sim::earlyOut), issued right after the run's
@@ -1705,8 +1753,6 @@ int wg_get_scene_stats(wg_scene* s, int32_t k, wg_stats* o) {
     if (!s || !o) return WG_ERR_ARG;
     Sim& S = *SIM(s);
     if (k < 0 || k >= S.nScenes) return S.fail(WG_ERR_ARG, "scene index out of range");
-    int r = S.syncContacts();
-    if (r) return r;
     std::memset(o, 0, sizeof(*o));
     const wg_config& c = S.nScenes > 1 ? S.cfgs[k] : S.cfg;
     const int64_t done = S.step - S.cfg.step;
@@ -1714,20 +1760,23 @@ int wg_get_scene_stats(wg_scene* s, int32_t k, wg_stats* o) {
     o->time = S.nScenes > 1 ? S.bTime[k] : S.time;
     o->n_full_runs = S.nFullRuns;
     o->verlet_dist = S.nScenes > 1 && S.uploaded ? S.hPars[k].verletDist : S.hPar.verletDist;
-    if (S.uploaded && S.C.n > 0) {
-        const int64_t n = S.C.n;
-        std::vector<uint32_t> fl(n);
-        std::vector<uint64_t> key(n);
-        WG_CUDA_TRY(cudaMemcpyAsync(fl.data(), S.C.flags, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, S.stream));
-        WG_CUDA_TRY(cudaMemcpyAsync(key.data(), S.C.key, sizeof(uint64_t) * n, cudaMemcpyDeviceToHost, S.stream));
-        const int64_t p0 = S.nScenes > 1 ? S.sceneStart[k] : 0, p1 = S.nScenes > 1 ? S.sceneStart[k + 1] : S.nPar;
-        for (int64_t c2 = 0; c2 < n; c2++) {
-            const int64_t lo = (int64_t)(key[c2] >> 32);
-            if (lo < p0 || lo >= p1 || (fl[c2] & C_REMOVED)) continue;
-            o->n_contacts++;
-            if (fl[c2] & C_REAL) o->n_real++;
-        }
-    }
+    int64_t h[2];
+    const int r = count_contacts(S, S.nScenes > 1 ? S.sceneStart[k] : 0, S.nScenes > 1 ? S.sceneStart[k + 1] : S.nPar, h);
+    if (r) return r;
+    o->n_contacts = h[0];
+    o->n_real = h[1];
+    return WG_OK;
+}
+
+int wg_get_clock(wg_scene* s, int32_t k, int64_t* step, double* time, int64_t* n_full_runs, double* stress9) {
+    if (!s) return WG_ERR_ARG;
+    Sim& S = *SIM(s);
+    if (k < 0 || k >= S.nScenes) return S.fail(WG_ERR_ARG, "scene index out of range");
+    if (step) *step = S.nScenes > 1 ? S.cfgs[k].step + (S.step - S.cfg.step) : S.step;
+    if (time) *time = S.nScenes > 1 ? S.bTime[k] : S.time;
+    if (n_full_runs) *n_full_runs = S.nFullRuns;
+    if (stress9)
+        for (int q = 0; q < 9; q++) stress9[q] = S.stress[q];
     return WG_OK;
 }
 
@@ -1841,6 +1890,18 @@ int wg_put_state(wg_scene* s, const double* pos, const double* ori, const double
     return WG_OK;
 }
 
+namespace {
+bool pageLocked(const void* p) {
+    cudaPointerAttributes a;
+    if (!p) return true;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+}
+}  // namespace
+
 int wg_get_nodes(wg_scene* s, double* pos, double* ori, double* vel, double* ang_vel, double* force, double* torque) {
     if (!s) return WG_ERR_ARG;
     Sim& S = *SIM(s);
@@ -1855,23 +1916,19 @@ int wg_get_nodes(wg_scene* s, double* pos, double* ori, double* vel, double* ang
     }
     const int part = (pos || ori || vel || ang_vel) ? ((force || torque) ? 0 : 1) : 2;
     k_get_state<<<(unsigned)((na + 255) / 256), 256, 0, S.stream>>>(S.N, X.dApiMap, na, stagedArrays(X.dStage, na), part);
+    int64_t bytes = 0;
+    bool locked = true;
+    for (int q = 0; q < 6; q++)
+        if (dst[q]) {
+            bytes += (int64_t)sizeof(double) * w[q] * na;
+            locked = locked && pageLocked(dst[q]);
+        }
+    if (!locked && bytes >= (int64_t(4) << 20)) return downloadState(S, X.dStage, na, dst);
     WG_CUDA_TRY(copyState(X.dStage, na, dst, 0, 6, false, S.stream));
     WG_CUDA_TRY(cudaGetLastError());
     WG_CUDA_TRY(cudaStreamSynchronize(S.stream));
     return WG_OK;
 }
-
-namespace {
-bool pageLocked(const void* p) {
-    cudaPointerAttributes a;
-    if (!p) return true;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeHost;
-}
-}  // namespace
 
 int wg_run_host(wg_scene* s, int64_t n_steps, double* pos, double* ori, double* vel, double* ang_vel, double* force, double* torque) {
     int r = wg_put_state(s, pos, ori, vel, ang_vel, force, torque);
@@ -1989,8 +2046,6 @@ int wg_get_scene_dyndt(wg_scene* s, int32_t k, wg_dyndt_state* o) {
 int wg_get_stats(wg_scene* s, wg_stats* o) {
     if (!s || !o) return WG_ERR_ARG;
     Sim& S = *SIM(s);
-    int r = S.syncContacts();
-    if (r) return r;
     std::memset(o, 0, sizeof(*o));
     o->step = S.step;
     o->time = S.time;
@@ -1998,13 +2053,10 @@ int wg_get_stats(wg_scene* s, wg_stats* o) {
     o->n_contacts = S.uploaded ? S.C.n : 0;
     o->verlet_dist = S.hPar.verletDist;
     for (int q = 0; q < 9; q++) o->stress[q] = S.stress[q];
-    if (S.uploaded && S.C.n > 0) {
-        std::vector<uint32_t> fl(S.C.n);
-        WG_CUDA_TRY(cudaMemcpyAsync(fl.data(), S.C.flags, sizeof(uint32_t) * S.C.n, cudaMemcpyDeviceToHost, S.stream));
-        int64_t r = 0;
-        for (uint32_t f : fl) r += (f & C_REAL) ? 1 : 0;
-        o->n_real = r;
-    }
+    int64_t h[2];
+    const int r = count_contacts(S, 0, S.nPar, h);
+    if (r) return r;
+    o->n_real = h[1];
     return WG_OK;
 }
 

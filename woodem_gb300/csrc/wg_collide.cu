@@ -1013,6 +1013,57 @@ __global__ void k_heavy(DevIncidence I, DevParticles P, const uint32_t* __restri
     }
 }
 
+// ---------------------------------------------------------------- counting
+// Contacts whose lo id is in [p0, p1): out[0] those not removed, out[1] the real ones. packed: the plain
+// active contacts have their flags in the packed state and are counted there.
+__device__ __forceinline__ void addCounts(bool there, bool real, unsigned long long* __restrict__ out) {
+    const int a = __syncthreads_count(there), r = __syncthreads_count(real);
+    if (threadIdx.x == 0) {
+        if (a) atomicAdd(out, (unsigned long long)a);
+        if (r) atomicAdd(out + 1, (unsigned long long)r);
+    }
+}
+__global__ void k_count(DevContacts C, int packed, int64_t p0, int64_t p1, unsigned long long* __restrict__ out) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t fl = C_REMOVED;
+    if (c < C.n) {
+        const int64_t lo = (int64_t)(C.key[c] >> 32);
+        fl = C.flags[c];
+        if (lo < p0 || lo >= p1 || (packed && activeContact(fl) && plainContact(fl, C.cdist[c]))) fl = C_REMOVED;
+    }
+    addCounts(!(fl & C_REMOVED), (fl & C_REAL) && !(fl & C_REMOVED), out);
+}
+__global__ void k_count_packed(DevPackedSS K, int64_t p0, int64_t p1, unsigned long long* __restrict__ out) {
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t fl = C_REMOVED;
+    if (j < K.n) {
+        const int4 it = K.item[j];
+        const int lo = min(it.x, it.y);
+        fl = lo >= p0 && lo < p1 ? K.flags[j] : (uint32_t)C_REMOVED;
+    }
+    addCounts(!(fl & C_REMOVED), (fl & C_REAL) && !(fl & C_REMOVED), out);
+}
+int count_contacts(Sim& S, int64_t p0, int64_t p1, int64_t out[2]) {
+    out[0] = out[1] = 0;
+    if (!S.uploaded || S.C.n == 0) return 0;
+    WG_CUDA_TRY(cudaSetDevice(S.device));
+    if (!S.dCount) {
+        S.dCount = (unsigned long long*)S.dalloc(2 * sizeof(unsigned long long));
+        if (!S.dCount) return S.fail(WG_ERR_CUDA, "out of device memory (counts)");
+    }
+    const bool packed = S.packDirty && S.K.n > 0;
+    unsigned long long h[2];
+    WG_CUDA_TRY(cudaMemsetAsync(S.dCount, 0, sizeof(h), S.stream));
+    k_count<<<(unsigned)((S.C.n + 255) / 256), 256, 0, S.stream>>>(S.C, packed ? 1 : 0, p0, p1, S.dCount);
+    if (packed) k_count_packed<<<(unsigned)((S.K.n + 255) / 256), 256, 0, S.stream>>>(S.K, p0, p1, S.dCount);
+    WG_CUDA_TRY(cudaGetLastError());
+    WG_CUDA_TRY(cudaMemcpyAsync(h, S.dCount, sizeof(h), cudaMemcpyDeviceToHost, S.stream));
+    WG_CUDA_TRY(cudaStreamSynchronize(S.stream));
+    out[0] = (int64_t)h[0];
+    out[1] = (int64_t)h[1];
+    return 0;
+}
+
 // ---------------------------------------------------------------- host orchestration
 static int ensureCub(Sim& S, size_t bytes) {
     CollideWork& W = *S.cw;

@@ -296,6 +296,8 @@ struct Grid {
 struct CollideWork;  // scratch owned by the simulation
 struct Sim;
 int collide_full_run(Sim& S);
+// contacts with their lo id in [p0, p1): out[0] not removed, out[1] real
+int count_contacts(Sim& S, int64_t p0, int64_t p1, int64_t out[2]);
 
 // DynDt after ContactLoop (pkg/dem/DynDt.hpp:19-23) with the counters of its PeriodicEngine.
 struct DynDtState;
@@ -378,6 +380,7 @@ struct Sim {
     long long* dStep = nullptr;
     int* dFlags = nullptr;   // [0] full run requested, [1] error code
     int* hFlags = nullptr;   // pinned mirror
+    double* hDown = nullptr; // pinned buffers of the threads that download a large state
     std::vector<void*> allocs;
     CollideWork* cw = nullptr;
     bool uploaded = false, initialized = false;
@@ -396,6 +399,7 @@ struct Sim {
     int64_t graphSteps = 0;  // steps in the captured chunk, 0: none valid
     int64_t graphEpoch = -1; // nFullRuns when it was captured
     int64_t graphLaunches = 0;
+    unsigned long long* dCount = nullptr;  // count_contacts
     double* dStress = nullptr;       // 9 doubles + per-block partials
     int64_t stressCap = 0;
     double stress[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // ContactLoop.stress of the last step
