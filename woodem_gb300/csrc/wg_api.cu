@@ -640,12 +640,13 @@ int Sim::upload() {
         WG_CUDA_TRY(cudaMemcpyAsync(P.scene, hSceneOfPar.data(), sizeof(int32_t) * nPar, cudaMemcpyHostToDevice, S.stream));
         WG_CUDA_TRY(cudaMemcpyAsync(N.scene, nsc.data(), sizeof(int32_t) * nSlots, cudaMemcpyHostToDevice, S.stream));
     }
-    dStep = (long long*)dalloc(sizeof(long long));
-    dFlags = (int*)dalloc(sizeof(int) * FL_WORDS);
+    dFlags = (int*)dalloc(CTL_BYTES);
+    if (!dFlags) return fail(WG_ERR_CUDA, "out of device memory (scene)");
+    dStep = (long long*)(dFlags + FL_WORDS);
     X.dApiMap = (int32_t*)dalloc(sizeof(int32_t) * std::max<int64_t>(1, na));
     X.dStage = (double*)dalloc(sizeof(double) * 19 * std::max<int64_t>(1, na));
     if (!X.dStage) return fail(WG_ERR_CUDA, "out of device memory (scene)");
-    WG_CUDA_TRY(cudaMallocHost(&hFlags, sizeof(int) * 4 + sizeof(long long)));
+    WG_CUDA_TRY(cudaMallocHost(&hFlags, CTL_BYTES));
     std::vector<double4_32a> mats(hDensity.size());
     for (size_t m = 0; m < hDensity.size(); m++) mats[m] = make_double4_32a(hDensity[m], hYoung[m], hTanPhi[m], hKtDivKn[m]);
     WG_CUDA_TRY(cudaMemcpyAsync(N.posr, posr.data(), sizeof(double4_32a) * nSlots, cudaMemcpyHostToDevice, S.stream));
@@ -797,6 +798,7 @@ int Sim::checkErr() {
     if (hFlags[1] == 102) return fail(WG_ERR_NAN, "InsertionSortCollider: NaN in a particle bounding box (NaN position)");
     if (hFlags[1] == 103) return fail(WG_ERR_PERIODIC, "InsertionSortCollider: Particle larger than half of the cell size encountered.");
     if (hFlags[1] == 100) return fail(WG_ERR_ARG, "Cg2_Facet_Sphere_L3Geom: Impossible sphere-facet intersection (all points are outside the edges). (please report bug)");
+    if (hFlags[1] == 105) return fail(WG_ERR_CUDA, "a launch of several steps gave up waiting at a barrier");
     if (hFlags[1] != 0) return fail(WG_ERR_STATE, "device error code " + std::to_string(hFlags[1]));
     return 0;
 }
@@ -805,6 +807,7 @@ int Sim::checkErr() {
 __global__ void k_set_flags(int* f, int full) {
     f[FL_FULL] = full;
     f[FL_HALT] = 0;
+    f[FL_BAR] = 0;
 }
 
 // Scene::doOneStep (core/Scene.cpp:319-389) for n steps. Steps are queued on the stream in
@@ -1063,7 +1066,8 @@ int Sim::run(int64_t n) {
         }
     }
     cudaEvent_t* E = evPool.data();
-    long long* hStepPin = (long long*)(hFlags + 4);
+    const long long* hStepPin = (const long long*)(hFlags + FL_WORDS);
+    long long* dNs = dStep + 1;
     const bool fp32 = prec == WG_PREC_FP32;
     bool anyLaw0 = cfg.law == 0;
     for (const wg_config& c : cfgs) anyLaw0 = anyLaw0 || c.law == 0;
@@ -1126,7 +1130,9 @@ int Sim::run(int64_t n) {
         launches += advanced ? 1 : 2;
     };
     WG_CUDA_TRY(cudaMemsetAsync(dFlags, 0, sizeof(int) * FL_WORDS, stream));
+    WG_CUDA_TRY(cudaMemsetAsync(dNs, 0, 2 * sizeof(long long), stream));
     WG_CUDA_TRY(cudaEventRecord(ev[6], stream));
+    long long nsA = 0, nsB = 0;  // phases of the launches of several steps
     int64_t done = 0;
     while (done < n) {
         // the sphere-sphere kernel updates the packed state from here on
@@ -1135,7 +1141,11 @@ int Sim::run(int64_t n) {
             int r = ensureEnergyCapacity();
             if (r) return r;
         }
-        int64_t k = std::min<int64_t>(n - done, maxChunk);
+        // a small scene runs its steps in one launch, which ends by itself where a full run is due: the
+        // chunk only bounds its length (in a periodic cell every step has its own record)
+        const bool small = N.n <= kSmallNodes && I.nAct <= kSmallContacts && !trackE && !useGraph && contactBlock <= 0 &&
+                           I.nHeavyFree == 0 && (!fp32 || P.nFacets == 0 || facetsStatic);
+        int64_t k = std::min<int64_t>(n - done, small && !cfg.periodic && !anyZeroVd ? 8 * maxChunk : maxChunk);
         // dt may change after a step (Scene.nextDt, DynDt): such a step ends its chunk
         if (std::isfinite(nextDt)) k = 1;
         // wg_run_host's early copy-out: the run's last step gets a chunk of its own, whose first
@@ -1192,7 +1202,23 @@ int Sim::run(int64_t n) {
         // CUDA graph (re-captured after every full run, whose contact arrays it refers to)
         const bool lastEarly = earlyWanted && !earlyIssued && done + k == n && k == 1;
         const bool graphChunk = useGraph && fromEnds && !needFull && k == maxChunk && !cfg.periodic && !lastEarly;
-        if (graphChunk) {
+        bool oneLaunch = small && !lastEarly;
+        if (oneLaunch) {
+            unsigned* bar = (unsigned*)(dFlags + FL_BAR);
+            unsigned long long* ns = (unsigned long long*)dNs;
+            const int from = fromEnds ? 1 : 0;
+            const int r = fp32 ? launch_steps32(stream, N, P, C, I, K, dNodeC, dMats, spOf(0), cfg.periodic != 0, dStep, dFlags, bar, ns,
+                                                nMixed, anyLaw0, from, (int)k)
+                               : launch_steps64(stream, N, P, C, I, dMats, spOf(0), cfg.periodic != 0, dStep, dFlags, bar, ns, from, (int)k);
+            if (r) {
+                cudaGetLastError();
+                oneLaunch = false;
+                k = std::min<int64_t>(k, maxChunk);
+            } else
+                launches++;
+        }
+        if (oneLaunch) {
+        } else if (graphChunk) {
             if (!graphExec || graphSteps != k || graphEpoch != nFullRuns) {
                 if (graphExec) cudaGraphExecDestroy(graphExec);
                 graphExec = nullptr;
@@ -1229,14 +1255,18 @@ int Sim::run(int64_t n) {
             }
         }
         WG_CUDA_TRY(cudaGetLastError());
-        WG_CUDA_TRY(cudaMemcpyAsync(hFlags, dFlags, sizeof(int) * 4, cudaMemcpyDeviceToHost, stream));
-        WG_CUDA_TRY(cudaMemcpyAsync(hStepPin, dStep, sizeof(long long), cudaMemcpyDeviceToHost, stream));
+        WG_CUDA_TRY(cudaMemcpyAsync(hFlags, dFlags, CTL_BYTES, cudaMemcpyDeviceToHost, stream));
         WG_CUDA_TRY(cudaStreamSynchronize(stream));
         if (hFlags[FL_ERR]) break;
         int64_t ds = (int64_t)*hStepPin - s0;
         if (ds < 0 || ds > k) return fail(WG_ERR_STATE, "device step counter out of sequence");
         float a;
-        if (graphChunk) {
+        if (oneLaunch) {
+            ph[0] += 1e-6 * (double)(hStepPin[1] - nsA);
+            ph[1] += 1e-6 * (double)(hStepPin[2] - nsB);
+            nsA = hStepPin[1];
+            nsB = hStepPin[2];
+        } else if (graphChunk) {
             cudaEventElapsedTime(&a, E[0], E[1]);
             ph[2] += a;  // whole steps replayed as a graph
         } else
@@ -1247,7 +1277,7 @@ int Sim::run(int64_t n) {
         if (ds < k || hFlags[FL_FULL]) {
             // Leapfrog of step s0+ds ran, its contact loop waits for the collider
             if (!hFlags[FL_FULL]) return fail(WG_ERR_STATE, "queued steps halted without a collider request");
-            if (!graphChunk) {
+            if (!graphChunk && !oneLaunch) {
                 cudaEventElapsedTime(&a, E[3 * ds], E[3 * ds + 1]);
                 ph[0] += a;
             }

@@ -212,7 +212,18 @@ enum { FL_FULL = 0,   // set by Leapfrog: a node moved farther than verletDist, 
        FL_ERR = 1,    // error code raised by a kernel
        FL_HALT = 2,   // set by the contact kernel of a step that found FL_FULL: later queued steps do nothing
        FL_TICKET = 3, // blocks of the last contact kernel of a step that have finished (the last advances the step)
-       FL_WORDS = 4 };
+       FL_BAR = 4,    // arrivals at the barriers of a launch of several steps
+       FL_WORDS = 8 };
+// The step-loop flags and the counters after them are one record, which the host reads in one copy: the
+// step counter, then the nanoseconds a launch of several steps spent in Leapfrog and in the contacts.
+constexpr int CTL_COUNTERS = 3;
+constexpr size_t CTL_BYTES = sizeof(int) * FL_WORDS + sizeof(long long) * CTL_COUNTERS;
+// Scenes of at most so many nodes and active contacts run their steps in one launch (launch_steps64,
+// launch_steps32). Boxes of n spheres, us a step in one launch and in a launch per kernel: FP32 10 000 56 and
+// 69, 40 000 64 and 75, 65 000 73 and 82, 100 000 97 and 100, 250 000 184 and 172; FP64 10 000 74 and 88,
+// 40 000 129 and 133, 65 000 177 and 168, 250 000 530 and 495: one block of 384 or 512 threads a SM has too few
+// warps in flight for the larger ones.
+constexpr int64_t kSmallNodes = 65536, kSmallContacts = 262144;
 
 __host__ __device__ inline int32_t packCellDist(int a, int b, int c) {
     return (int32_t)(((uint32_t)(a + 512) & 1023u) | (((uint32_t)(b + 512) & 1023u) << 10) | (((uint32_t)(c + 512) & 1023u) << 20));
@@ -236,6 +247,18 @@ void launch_contact_fp64(cudaStream_t st, const DevNodes& N, const DevParticles&
                          bool periodic, int block = 0, const EnergyCols* energy = nullptr);
 // perStep: only the heavy particles with a free DOF (guarded by the flags), before Leapfrog;
 // otherwise every particle's DemData.force/torque (reporting at the end of a run).
+// Up to `steps` steps in one cooperative launch (small scenes; no energy tracking, no heavy particle with a
+// free DOF, facets static). It leaves the flags and the step counter as that many launches of the
+// kernels above would: a full run due ends it before that step's contacts. bar: a word that is zero
+// before the launch; ns: nanoseconds spent in Leapfrog and in the contacts, added to. sp: one record, or
+// one per step in a periodic cell. Returns nonzero if it cannot be launched (nothing is then queued).
+int launch_steps64(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
+                   const double4_32a* mats, const ScenePar* sp, bool periodic, long long* dStep, int* dFlags, unsigned* bar,
+                   unsigned long long* ns, int fromEnds, int steps);
+int launch_steps32(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
+                   const DevPackedSS& K, const NodeConst32* nc, const double4_32a* mats, const ScenePar* sp, bool periodic,
+                   long long* dStep, int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool anyLaw0, int fromEnds,
+                   int steps);
 void launch_forces(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevIncidence& I, const ScenePar* sp,
                    const int* dFlags, bool perStep);
 void launch_advance(cudaStream_t st, long long* dStep, const int* dFlags);
@@ -377,8 +400,8 @@ struct Sim {
     std::vector<uint8_t> hParked;      // serving slots: particle holds no job (left out of the collider)
     bool listsDirty = true;            // particle lists of the collider to be rebuilt at the next full run
     bool forceFull = false;            // next step starts with a full collider run
-    long long* dStep = nullptr;
-    int* dFlags = nullptr;   // [0] full run requested, [1] error code
+    int* dFlags = nullptr;   // the step-loop flags (FL_*) and the counters behind them (CTL_BYTES)
+    long long* dStep = nullptr;  // the first of those counters
     int* hFlags = nullptr;   // pinned mirror
     double* hDown = nullptr; // pinned buffers of the threads that download a large state
     std::vector<void*> allocs;

@@ -10,6 +10,7 @@
 #include "wg_ends.cuh"
 #include "wg_energy.cuh"
 #include "wg_geom.cuh"
+#include "wg_grid.cuh"
 
 namespace wg {
 __device__ __forceinline__ double4_32a st4(D3 a, double w) { return make_double4_32a(a.x, a.y, a.z, w); }
@@ -70,11 +71,9 @@ __device__ __noinline__ void resetForce(DevNodes N, int i, double mass, bool gra
     N.torque[i] = make_double4_32a(0., 0., 0., 0.);
 }
 template <bool PERI, bool ENERGY>
-__global__ void __launch_bounds__(128) k_leapfrog(DevNodes N, DevParticles P, DevIncidence I, const ScenePar* __restrict__ spp,
-                                                  int* __restrict__ dFlags, int fromEnds, const long long* __restrict__ dStepC,
-                                                  EnergyCols E) {
-    if (halted(dFlags)) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void leapfrogNode(int i, const DevNodes& N, const DevParticles& P, const DevIncidence& I,
+                                             const ScenePar* __restrict__ spp, int* __restrict__ dFlags, int fromEnds, long long stepAbs,
+                                             const EnergyCols& E) {
     const bool valid = i < N.n;
     const ScenePar& sp = spp[valid ? sceneOfN(N, i) : 0];
     const int nPar = P.n;
@@ -86,7 +85,7 @@ __global__ void __launch_bounds__(128) k_leapfrog(DevNodes N, DevParticles P, De
     // ContactLoop.cpp:250-257), or the stored value
     const bool uni = valid && i < nPar && P.shape[i] != WG_SHAPE_FACET;
     // a scene past its last step (serving slot) is frozen; a node just (re)loaded takes its stored force
-    const bool frozen = valid && (*dStepC - sp.stepBase) >= sp.stepEnd;
+    const bool frozen = valid && (stepAbs - sp.stepBase) >= sp.stepEnd;
     const bool fresh = valid && N.fresh && N.fresh[i];
     int e0 = 0, e1 = 0;
     bool take = false;
@@ -208,6 +207,14 @@ __global__ void __launch_bounds__(128) k_leapfrog(DevNodes N, DevParticles P, De
     const D3 lp = ld3(N.lastPos[i]);
     const double d2 = sqn(lp - pos);
     if (d2 + 0. > sp.maxD2) atomicOr(dFlags + FL_FULL, 1);
+}
+
+template <bool PERI, bool ENERGY>
+__global__ void __launch_bounds__(128) k_leapfrog(DevNodes N, DevParticles P, DevIncidence I, const ScenePar* __restrict__ spp,
+                                                  int* __restrict__ dFlags, int fromEnds, const long long* __restrict__ dStepC,
+                                                  EnergyCols E) {
+    if (halted(dFlags)) return;
+    leapfrogNode<PERI, ENERGY>((int)(blockIdx.x * blockDim.x + threadIdx.x), N, P, I, spp, dFlags, fromEnds, *dStepC, E);
 }
 
 // Threads per block of the FP64 kernels over n items: one warp per block while the blocks of one
@@ -333,24 +340,17 @@ __device__ __noinline__ double2 capShear(double ft1, double ft2, double maxFt, b
 // contact (a zero) takes neither. Drum of 250 000: 0.70 -> 0.49 ms a step; 10 000 settling spheres
 // in one-warp blocks: 45 -> 37 us.
 template <bool PERI, bool ENERGY>
-__global__ void __launch_bounds__(128) k_contact_fp64(DevNodes N, DevParticles P, DevContacts C, DevIncidence I,
-                                                     const double4_32a* __restrict__ mats, const ScenePar* __restrict__ spp,
-                                                     const long long* __restrict__ dStep, int* __restrict__ dFlags,
-                                                     EnergyCols E) {
-    if (dFlags[FL_FULL] || halted(dFlags)) {
-        // the collider runs before this step's contacts; the steps queued after it wait
-        if (blockIdx.x == 0 && threadIdx.x == 0) dFlags[FL_HALT] = 1;
-        return;
-    }
+__device__ __forceinline__ void contactItem(int64_t rk, const DevNodes& N, const DevParticles& P, const DevContacts& C,
+                                            const DevIncidence& I, const double4_32a* __restrict__ mats,
+                                            const ScenePar* __restrict__ spp, long long stepAbs, int* __restrict__ dFlags,
+                                            const EnergyCols& E) {
     int* dErr = dFlags + FL_ERR;
-    const int64_t rk = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (rk >= I.nAct) return;
     // work item: contact index, pA, pB and the static flag bits (type, swap) fixed at the full run
     const int4 wk = I.work[rk];
     const int64_t c = wk.x;
     const int A = wk.y, B = wk.z;
     const ScenePar& sp = spp[sceneOfP(P, B)];
-    if (*dStep - sp.stepBase >= sp.stepEnd) return;  // frozen scene (serving slot past its last step)
+    if (stepAbs - sp.stepBase >= sp.stepEnd) return;  // frozen scene (serving slot past its last step)
     uint32_t fl = C.flags[c];
     if (fl & C_REMOVED) return;
     if ((fl & C_PENDING) && !pendingStays(P, A, B, PERI && sp.periodic, sp.cellSize, dErr)) {
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(128) k_contact_fp64(DevNodes N, DevParticles P
     fl &= ~C_PENDING;
     const uint32_t ty = ctype((uint32_t)wk.w);
     const bool real = fl & C_REAL;
-    const long long step = *dStep - sp.stepBase;
+    const long long step = stepAbs - sp.stepBase;
     const double dt = sp.dt;
     D3 shift2{0, 0, 0}, shiftVel2{0, 0, 0};
     if (PERI) {
@@ -588,6 +588,20 @@ __global__ void __launch_bounds__(128) k_contact_fp64(DevNodes N, DevParticles P
     C.flags[c] = fl | C_REAL;
 }
 
+template <bool PERI, bool ENERGY>
+__global__ void __launch_bounds__(128) k_contact_fp64(DevNodes N, DevParticles P, DevContacts C, DevIncidence I,
+                                                     const double4_32a* __restrict__ mats, const ScenePar* __restrict__ spp,
+                                                     const long long* __restrict__ dStep, int* __restrict__ dFlags,
+                                                     EnergyCols E) {
+    if (dFlags[FL_FULL] || halted(dFlags)) {
+        // the collider runs before this step's contacts; the steps queued after it wait
+        if (blockIdx.x == 0 && threadIdx.x == 0) dFlags[FL_HALT] = 1;
+        return;
+    }
+    const int64_t rk = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (rk < I.nAct) contactItem<PERI, ENERGY>(rk, N, P, C, I, mats, spp, *dStep, dFlags, E);
+}
+
 void launch_contact_fp64(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
                          const double4_32a* mats, const ScenePar* sp, const long long* dStep, int* dFlags, bool periodic, int block,
                          const EnergyCols* energy) {
@@ -602,6 +616,62 @@ void launch_contact_fp64(cudaStream_t st, const DevNodes& N, const DevParticles&
         if (periodic) k_contact_fp64<true, false><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, E);
         else k_contact_fp64<false, false><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, E);
     }
+}
+
+// ---------------------------------------------------------------------------------- many steps in one launch
+// Up to `steps` steps of a small scene in one cooperative launch, as k_steps32 of the FP32-force mode
+// (wg_step32.cu). 10 000 spheres: 50 -> 38 us a step.
+constexpr int kSteps64Threads = 384;  // 170 registers each
+template <bool PERI>
+__global__ void __launch_bounds__(kSteps64Threads, 1) k_steps64(DevNodes N, DevParticles P, DevContacts C, DevIncidence I,
+                                                    const double4_32a* __restrict__ mats, const ScenePar* __restrict__ spp, int seq,
+                                                    long long* dStep, int* dFlags, unsigned* bar, unsigned long long* ns, int fromEnds,
+                                                    int steps) {
+    __shared__ int ok;
+    const long long step0 = *(volatile long long*)dStep;
+    const int lane = threadIdx.x & 31;
+    const int64_t first = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, stride = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const bool clock = blockIdx.x == 0 && threadIdx.x == 0;
+    const EnergyCols none{};
+    unsigned long long tA = 0, tB = 0;
+    int done = 0;
+    for (int s = 0; s < steps; s++) {
+        const ScenePar* __restrict__ sp = spp + (seq ? s : 0);
+        const unsigned long long t0 = clock ? nowNs() : 0ull;
+        for (int64_t c = first; 32 * c < N.n; c += stride)
+            leapfrogNode<PERI, false>((int)(32 * c) + lane, N, P, I, sp, dFlags, s == 0 ? fromEnds : 1, step0 + s, none);
+        if (!gridBarrier(bar, dFlags, &ok)) return;
+        const unsigned long long t1 = clock ? nowNs() : 0ull;
+        tA += t1 - t0;
+        if (flagNow(dFlags + FL_FULL)) break;  // the same for every thread: raised before the barrier, or at the launch
+        for (int64_t c = first; 32 * c < I.nAct; c += stride)
+            if (32 * c + lane < I.nAct) contactItem<PERI, false>(32 * c + lane, N, P, C, I, mats, sp, step0 + s, dFlags, none);
+        if (!gridBarrier(bar, dFlags, &ok)) return;
+        if (clock) tB += nowNs() - t1;
+        if (flagNow(dFlags + FL_ERR)) break;
+        done = s + 1;
+    }
+    if (clock) {
+        *dStep = step0 + done;
+        ns[0] += tA;
+        ns[1] += tB;
+    }
+}
+
+int launch_steps64(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
+                   const double4_32a* mats, const ScenePar* sp, bool periodic, long long* dStep, int* dFlags, unsigned* bar,
+                   unsigned long long* ns, int fromEnds, int steps) {
+    DevNodes n = N;
+    DevParticles p = P;
+    DevContacts c = C;
+    DevIncidence i = I;
+    int seq = periodic ? 1 : 0;
+    void* args[] = {&n, &p, &c, &i, &mats, &sp, &seq, &dStep, &dFlags, &bar, &ns, &fromEnds, &steps};
+    const int64_t items = std::max<int64_t>(N.n, I.nAct);
+    const void* f = periodic ? (const void*)k_steps64<true> : (const void*)k_steps64<false>;
+    const int g = stepsGrid(f, kSteps64Threads, 0, items);
+    if (g < 1) return -1;
+    return cudaLaunchCooperativeKernel(f, dim3((unsigned)g), dim3(kSteps64Threads), args, 0, st) == cudaSuccess ? 0 : -1;
 }
 
 // ---------------------------------------------------------------------------------- energy sums

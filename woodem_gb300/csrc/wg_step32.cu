@@ -10,11 +10,11 @@
 //
 // Compiled with --fmad=true (results are compared to the FP64 oracle within a tolerance).
 #include <algorithm>
-#include <mutex>
 
 #include "wg_ends.cuh"
 #include "wg_energy.cuh"
 #include "wg_geom.cuh"
+#include "wg_grid.cuh"
 
 namespace wg {
 
@@ -125,12 +125,13 @@ __device__ __noinline__ void resetNodeForce(DevNodes N, int i, float mh, float m
 // velocity gradient); the aperiodic instantiation carries none of that FP64 code.
 // ENERGY: Scene.trackEnergy; each node writes its step's energy terms (Leapfrog.cpp:52-97, in FP64
 // from this step's force and torque) into E, as the FP64 Leapfrog does.
-template <bool PERI, bool ENERGY>
-__global__ void __launch_bounds__(256) k_leapfrog32(DevNodes N, DevParticles P, DevIncidence I, const NodeConst32* __restrict__ ncs,
-                                                    const ScenePar* __restrict__ spp, int* __restrict__ dFlags, int fromEnds,
-                                                    const long long* __restrict__ dStepC, EnergyCols E) {
-    __shared__ EndStage<float4, float2, kLeapfrogChunk32> stage[8];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// One node, by all lanes of its warp together (i past the last node: nothing is written). GUARD: the step
+// may have been halted (a launch per kernel); without it the caller knows that it was not.
+template <bool PERI, bool ENERGY, bool GUARD>
+__device__ __forceinline__ void leapfrogNode32(int i, const DevNodes& N, const DevParticles& P, const DevIncidence& I,
+                                               const NodeConst32* __restrict__ ncs, const ScenePar* __restrict__ spp,
+                                               int* __restrict__ dFlags, int fromEnds, long long stepAbs, const EnergyCols& E,
+                                               EndStage<float4, float2, kLeapfrogChunk32>& stage) {
     const bool valid = i < N.n;
     // every load of the node is issued before the step guard (nothing is written before it), so
     // that they are in flight together
@@ -147,9 +148,8 @@ __global__ void __launch_bounds__(256) k_leapfrog32(DevNodes N, DevParticles P, 
         ls0 = I.loStart[pi];
         ls1 = I.loStart[pi + 1];
     }
-    const long long stepAbs = *dStepC;
     const int scene = valid ? sceneOfN(N, i) : 0;
-    if (halted(dFlags)) return;
+    if (GUARD && halted(dFlags)) return;
     const ScenePar& sp = spp[scene];
     const uint32_t flags = nc.flags;
     // DemData.force/torque of this step
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256) k_leapfrog32(DevNodes N, DevParticles P, 
             summed = take;
         }
     }
-    warpSumEnds(I.endAf, I.endBf, take, e0, e1, stage[threadIdx.x >> 5], acc);
+    warpSumEnds(I.endAf, I.endBf, take, e0, e1, stage, acc);
     if (!valid || (flags & F_CLUMPED) || frozen) return;
     if (fresh) N.fresh[i] = 0;
     F3 f, t;
@@ -310,6 +310,15 @@ __global__ void __launch_bounds__(256) k_leapfrog32(DevNodes N, DevParticles P, 
     }
     // force reset of nodes whose force is not rebuilt by the contact sum (facet vertices)
     if (sp.reset && !uni) resetNodeForce(N, i, nc.mh, nc.ml, sp.hasGravity && !(flags & F_GRAVITY_SKIP), spp, scene);
+}
+
+template <bool PERI, bool ENERGY>
+__global__ void __launch_bounds__(256) k_leapfrog32(DevNodes N, DevParticles P, DevIncidence I, const NodeConst32* __restrict__ ncs,
+                                                    const ScenePar* __restrict__ spp, int* __restrict__ dFlags, int fromEnds,
+                                                    const long long* __restrict__ dStepC, EnergyCols E) {
+    __shared__ EndStage<float4, float2, kLeapfrogChunk32> stage[8];
+    leapfrogNode32<PERI, ENERGY, true>((int)(blockIdx.x * blockDim.x + threadIdx.x), N, P, I, ncs, spp, dFlags, fromEnds, *dStepC, E,
+                                       stage[threadIdx.x >> 5]);
 }
 
 void launch_leapfrog32(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevIncidence& I, const NodeConst32* nc,
@@ -719,6 +728,23 @@ __device__ __forceinline__ void ssContact(const SSIn& x, int64_t j, const DevNod
     if ((fl | C_REAL) != fl0) K.flags[j] = (fl | C_REAL) | hiBits;
 }
 
+// the loads of packed contact j but its item
+__device__ __forceinline__ void loadSS(SSIn& x, int64_t j, const DevNodes& N, const DevPackedSS& K, int loadFt) {
+    x.pf = K.flags[j];
+#pragma unroll
+    for (int q = 0; q < CF_NCOL; q++) x.st[q] = K.col[q][j];
+    x.ft1o = 0.;
+    x.ft2o = 0.;
+    if (loadFt) {  // some scene uses IdealElPl
+        x.ft1o = K.ft[0][j];
+        x.ft2o = K.ft[1][j];
+    }
+    x.ma = N.mir[x.it.x];
+    x.mb = N.mir[x.it.y];
+    x.wza = N.wz[x.it.x];
+    x.wzb = N.wz[x.it.y];
+}
+
 // Sphere-sphere contacts of aperiodic scenes (work items [nMixed, nAct)), one per thread: item,
 // flags and state are read at the contact's position in the work list (coalesced), the two
 // particles' mirror records are gathered; every load is issued before the step guard and the
@@ -733,19 +759,7 @@ __global__ void __launch_bounds__(256, MINB) k_contact_ss32(DevNodes N, DevParti
     const int64_t j = in ? j0 : 0;
     SSIn x;
     x.it = K.item[j];
-    x.pf = K.flags[j];
-#pragma unroll
-    for (int q = 0; q < CF_NCOL; q++) x.st[q] = K.col[q][j];
-    x.ft1o = 0.;
-    x.ft2o = 0.;
-    if (loadFt) {  // some scene uses IdealElPl
-        x.ft1o = K.ft[0][j];
-        x.ft2o = K.ft[1][j];
-    }
-    x.ma = N.mir[x.it.x];
-    x.mb = N.mir[x.it.y];
-    x.wza = N.wz[x.it.x];
-    x.wzb = N.wz[x.it.y];
+    loadSS(x, j, N, K, loadFt);
     const long long stepAbs = *dStep;
     if (dFlags[FL_FULL] || halted(dFlags)) {
         if (haltBlock && blockIdx.x == 0 && threadIdx.x == 0) dFlags[FL_HALT] = 1;
@@ -775,19 +789,7 @@ __global__ void __launch_bounds__(256, MINB) k_contact_ss32p(DevNodes N, DevPart
         SSIn x;
         x.it = next;
         if (j + stride < K.n) next = K.item[j + stride];
-        x.pf = K.flags[j];
-#pragma unroll
-        for (int q = 0; q < CF_NCOL; q++) x.st[q] = K.col[q][j];
-        x.ft1o = 0.;
-        x.ft2o = 0.;
-        if (loadFt) {
-            x.ft1o = K.ft[0][j];
-            x.ft2o = K.ft[1][j];
-        }
-        x.ma = N.mir[x.it.x];
-        x.mb = N.mir[x.it.y];
-        x.wza = N.wz[x.it.x];
-        x.wzb = N.wz[x.it.y];
+        loadSS(x, j, N, K, loadFt);
         ssContact<ENERGY>(x, j, N, P, C, I, K, mats, spp, stepAbs, dFlags, nm, E);
     }
     stepTicket(dFlags, dStep, ticketTotal);
@@ -951,7 +953,7 @@ __device__ __forceinline__ bool geomFS32(const DevNodes& N, const DevParticles& 
 template <bool PERI, bool ENERGY>
 __device__ __forceinline__ void mixedContact(int64_t rk, const DevNodes& N, const DevParticles& P, const DevContacts& C,
                                              const DevIncidence& I, const double4_32a* __restrict__ mats,
-                                             const ScenePar* __restrict__ spp, const long long* __restrict__ dStep, int* dFlags,
+                                             const ScenePar* __restrict__ spp, long long stepAbs, int* dFlags,
                                              const EnergyCols& E) {
     int* dErr = dFlags + FL_ERR;
     // work item: contact index, pA, pB and the static flag bits (type, swap) fixed at the full run
@@ -959,7 +961,7 @@ __device__ __forceinline__ void mixedContact(int64_t rk, const DevNodes& N, cons
     const int64_t c = wk.x;
     const int A = wk.y, B = wk.z;
     const ScenePar& sp = spp[sceneOfP(P, B)];
-    if (*dStep - sp.stepBase >= sp.stepEnd) return;  // frozen scene (serving slot past its last step)
+    if (stepAbs - sp.stepBase >= sp.stepEnd) return;  // frozen scene (serving slot past its last step)
     uint32_t fl = C.flags[c];
     if (fl & C_REMOVED) return;
     if ((fl & C_PENDING) && !pendingStays(P, A, B, PERI && sp.periodic, sp.cellSize, dErr)) {
@@ -969,7 +971,7 @@ __device__ __forceinline__ void mixedContact(int64_t rk, const DevNodes& N, cons
     fl &= ~C_PENDING;
     const uint32_t ty = ctype((uint32_t)wk.w);
     const bool real = fl & C_REAL;
-    const long long step = *dStep - sp.stepBase;
+    const long long step = stepAbs - sp.stepBase;
     const float dtf = sp.dtF;
     bool shifted = false;
     D3 shift2{0, 0, 0}, shiftVel2{0, 0, 0};
@@ -1202,24 +1204,14 @@ __global__ void __launch_bounds__(128, 4) k_contact_fp32(DevNodes N, DevParticle
         return;
     }
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const long long stepAbs = *dStep;
     for (int64_t rk = c0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; rk < c1; rk += stride)
-        mixedContact<PERI, ENERGY>(rk, N, P, C, I, mats, spp, dStep, dFlags, E);
+        mixedContact<PERI, ENERGY>(rk, N, P, C, I, mats, spp, stepAbs, dFlags, E);
     stepTicket(dFlags, dStep, ticketTotal);
 }
 
 // minimum resident blocks per SM the one-contact-per-thread kernel is compiled for (register budget)
 constexpr int kSSMinBlocks = 3;
-
-// streaming multiprocessors of the current device
-static int smCount() {
-    static std::mutex mu;
-    static int n[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!n[dev] && (cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n[dev] < 1)) n[dev] = 1;
-    return n[dev];
-}
 
 // sphere-sphere range: block > 0 one contact per thread with that many threads per block;
 // block < 0 the resident-grid kernel with prefetch (256 threads per block)
@@ -1286,6 +1278,89 @@ bool launch_contact_fp32(cudaStream_t st, const SideStream& side, const DevNodes
                                   *energy);
     return contactsFP32<false>(st, side, N, P, C, I, K, mats, sp, dStep, dFlags, nMixed, periodic, anyLaw0, prepFacets, block,
                                EnergyCols{});
+}
+
+// ---------------------------------------------------------------------------------- many steps in one launch
+// Up to `steps` steps of a small scene in one cooperative launch: Leapfrog over the nodes, a barrier of
+// the grid, the contacts, a barrier. The step that finds a node past verletDist ends the launch
+// before its contacts (its collider run comes first), as a halted queue of launches does. A step of a
+// few thousand spheres is bound by latency: three launches, a fork and join of streams and
+// the events between them took 30 us for 10 000 spheres, 19 us here. One block per SM;
+// chunks of 32 items go to the first warp of every block, then to the second and so on, so that few
+// chunks still use every SM and, with four warps a chunk apart, each of its four schedulers.
+// seq: spp holds one record per step (periodic cell). ns: nanoseconds spent in the two phases, added up
+// by the first block.
+constexpr int kSteps32Threads = 512;
+constexpr size_t kSteps32Shared = sizeof(EndStage<float4, float2, kLeapfrogChunk32>) * (kSteps32Threads / 32);
+template <bool PERI>
+__global__ void __launch_bounds__(kSteps32Threads, 1) k_steps32(DevNodes N, DevParticles P, DevContacts C, DevIncidence I, DevPackedSS K,
+                                                    const NodeConst32* __restrict__ ncs, const double4_32a* __restrict__ mats,
+                                                    const ScenePar* __restrict__ spp, int seq, long long* dStep, int* dFlags,
+                                                    unsigned* bar, unsigned long long* ns, int64_t nm, int loadFt, int fromEnds,
+                                                    int steps) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    EndStage<float4, float2, kLeapfrogChunk32>* const stage = (EndStage<float4, float2, kLeapfrogChunk32>*)smem;
+    __shared__ int ok;
+    const long long step0 = *(volatile long long*)dStep;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t first = (int64_t)w * gridDim.x + blockIdx.x, stride = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int64_t cN = (N.n + 31) >> 5, cM = (nm + 31) >> 5, cK = (K.n + 31) >> 5;
+    const bool clock = blockIdx.x == 0 && threadIdx.x == 0;
+    const EnergyCols none{};
+    unsigned long long tA = 0, tB = 0;
+    int done = 0;
+    for (int s = 0; s < steps; s++) {
+        const ScenePar* __restrict__ sp = spp + (seq ? s : 0);
+        const unsigned long long t0 = clock ? nowNs() : 0ull;
+        for (int64_t c = first; c < cN; c += stride)
+            leapfrogNode32<PERI, false, false>((int)(32 * c) + lane, N, P, I, ncs, sp, dFlags, s == 0 ? fromEnds : 1, step0 + s, none,
+                                               stage[w]);
+        if (!gridBarrier(bar, dFlags, &ok)) return;
+        const unsigned long long t1 = clock ? nowNs() : 0ull;
+        tA += t1 - t0;
+        if (flagNow(dFlags + FL_FULL)) break;  // the same for every thread: raised before the barrier, or at the launch
+        for (int64_t c = first; c < cM + cK; c += stride) {
+            if (c < cM) {
+                const int64_t rk = 32 * c + lane;
+                if (rk < nm) mixedContact<PERI, false>(rk, N, P, C, I, mats, sp, step0 + s, dFlags, none);
+            } else {
+                const int64_t j = 32 * (c - cM) + lane;
+                if (j < K.n) {
+                    SSIn x;
+                    x.it = K.item[j];
+                    loadSS(x, j, N, K, loadFt);
+                    ssContact<false>(x, j, N, P, C, I, K, mats, sp, step0 + s, dFlags, nm, none);
+                }
+            }
+        }
+        if (!gridBarrier(bar, dFlags, &ok)) return;
+        if (clock) tB += nowNs() - t1;
+        if (flagNow(dFlags + FL_ERR)) break;
+        done = s + 1;
+    }
+    if (clock) {
+        *dStep = step0 + done;
+        ns[0] += tA;
+        ns[1] += tB;
+    }
+}
+
+int launch_steps32(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
+                   const DevPackedSS& K, const NodeConst32* nc, const double4_32a* mats, const ScenePar* sp, bool periodic, long long* dStep,
+                   int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool anyLaw0, int fromEnds, int steps) {
+    DevNodes n = N;
+    DevParticles p = P;
+    DevContacts c = C;
+    DevIncidence i = I;
+    DevPackedSS k = K;
+    int seq = periodic ? 1 : 0, loadFt = anyLaw0 ? 1 : 0;
+    int64_t nm = periodic ? I.nAct : std::min<int64_t>(nMixed, I.nAct);
+    void* args[] = {&n, &p, &c, &i, &k, &nc, &mats, &sp, &seq, &dStep, &dFlags, &bar, &ns, &nm, &loadFt, &fromEnds, &steps};
+    const int64_t items = std::max<int64_t>(N.n, I.nAct);
+    const void* f = periodic ? (const void*)k_steps32<true> : (const void*)k_steps32<false>;
+    const int g = stepsGrid(f, kSteps32Threads, kSteps32Shared, items);
+    if (g < 1) return -1;
+    return cudaLaunchCooperativeKernel(f, dim3((unsigned)g), dim3(kSteps32Threads), args, kSteps32Shared, st) == cudaSuccess ? 0 : -1;
 }
 
 // ---------------------------------------------------------------------------------- force sum
