@@ -2314,6 +2314,7 @@ int wg_set_contact_state(wg_scene* s, int64_t n, const uint64_t* key, const uint
             }
     }
     S.C.n = n;
+    S.contactsReplaced = true;
     S.K.n = 0;
     S.packDirty = false;
     S.fromEnds = false;    // the first step takes the node forces as written by the host

@@ -32,6 +32,14 @@
 namespace wg {
 
 struct PeriBox;
+// The counts of a full run; the host reads them twice, after the sweep and at the end.
+struct CollideTotals {
+    unsigned long long pairs;  // pairs found (past the buffer's capacity too)
+    unsigned long long real, kept;  // real contacts before the merge, and those of them found among the new pairs
+    unsigned long long act, actReal;  // totals of the work-list scans
+    int32_t heavy, heavyFree;
+    int32_t bad;  // a sphere's box is not finite
+};
 struct CollideWork {
     // sphere and "large" (non-sphere) id lists, built at upload
     int32_t* sphereIds = nullptr;
@@ -43,29 +51,25 @@ struct CollideWork {
     bool largeLargePossible = false;
     std::vector<int32_t> hLarge, hGlobal;
     // grid scratch
-    uint32_t* cellKey = nullptr;
-    uint32_t* cellKeySorted = nullptr;
-    int32_t* cellVal = nullptr;
-    int32_t* sid = nullptr;       // sorted sphere ids
-    double4_32a* smn = nullptr;
-    double4_32a* smx = nullptr;
-    PeriBox* speri = nullptr;     // periodic: the sorted boxes in fractions of the cell
-    float4* smnf = nullptr;       // box min rounded down, mask in w
+    uint32_t* cellKey = nullptr;  // cell of each sphere of sphereIds, and its place within the cell
+    int32_t* cellRank = nullptr;
+    uint32_t* skey = nullptr;     // cells of the spheres in cell order
+    PeriBox* speri = nullptr;     // periodic: the boxes in cell order, in fractions of the cell
+    float4* smnf = nullptr;       // box min rounded down, mask in w (cell order)
     float4* smxf = nullptr;       // box max rounded up, particle id in w
-    int32_t* newLo = nullptr;     // first index of each lo id in the sorted new pairs (merge)
+    int32_t* newLo = nullptr;     // first index of each lo id in the sorted new pairs
     int32_t* oldLo = nullptr;     // the same in the previous contact keys
     int64_t newLoCap = 0, oldLoCap = 0;
-    float4* smnfi = nullptr;      // box min rounded up (inward)
-    float4* smxfi = nullptr;      // box max rounded down (inward)
-    int32_t* cellOff = nullptr;
+    bool oldLoValid = false;
+    int32_t* cellOff = nullptr;   // first sphere of each cell
     int64_t cellOffCap = 0;
-    double* red = nullptr;        // reduction partials
-    double* hRed = nullptr;       // pinned
+    float* red = nullptr;         // reduction partials
     std::vector<int32_t> hChunk;      // grid-reduction chunks of sphereIds (never across scenes)
     std::vector<int32_t> hSceneChunk; // chunks of scene k: [hSceneChunk[k], hSceneChunk[k+1])
     std::vector<int64_t> hSceneSph;   // spheres of scene k: sphereIds[hSceneSph[k] .. hSceneSph[k+1])
     int32_t* dChunk = nullptr;
     Grid* dGrids = nullptr;
+    int32_t* dSceneChunk = nullptr;   // chunks of scene k on the device
     bool chunksDirty = true;
     int32_t* gStart = nullptr;        // walls of scene k in globalIds (batches)
     // pairs
@@ -77,27 +81,34 @@ struct CollideWork {
     int64_t pairCdCap = 0;
     int32_t* newCd = nullptr;         // periodic: cell distance per merged contact
     int64_t newCdCap = 0;
-    unsigned long long* counter = nullptr;
-    unsigned long long* hCounter = nullptr;
+    CollideTotals* tot = nullptr;     // counts a run makes on the device
+    CollideTotals* hTot = nullptr;    // pinned
     // merge scratch
     int32_t* orph = nullptr;      // flags then exclusive scan
     uint64_t* orphKey = nullptr;
     int32_t* orphSrc = nullptr;
     int32_t* src = nullptr;
     int64_t mergeCap = 0, orphCap = 0, srcCap = 0;
+    // FP32-force mode, aperiodic: the packed state of the next set, and where each contact of this and the
+    // next one is packed (plain active contacts alone)
+    DevPackedSS Kb{};
+    int32_t *packIdx = nullptr, *packIdxB = nullptr;
+    int64_t packIdxCap = 0, packIdxCapB = 0;
+    bool packIdxValid = false;
     uint64_t* act = nullptr;      // exclusive scan of the active contacts (low half) and the plain ones of them (high)
     uint64_t* actReal = nullptr;  // FP64 mode: the same of the real contacts
     uint32_t* hiKeys = nullptr;
     uint32_t* hiKeysSorted = nullptr;
     int32_t* hiVals = nullptr;
     int64_t hiCap = 0;
-    int32_t* heavyCount = nullptr;
-    int32_t* hHeavy = nullptr;
     void* cubTmp = nullptr;
     size_t cubBytes = 0;
 };
 
 static const int BS = 256;
+// spheres per block of the grid-bounds reduction: four loads a thread in flight, and a block for every
+// SM from 150 000 spheres on
+constexpr int64_t kGridChunk = 1024;
 
 // ---------------------------------------------------------------- Bo1 functors + verlet
 // Bo1_Sphere_Aabb::go pkg/dem/Sphere.cpp:50-79, Bo1_Wall_Aabb::go pkg/dem/Wall.cpp:24-33,
@@ -194,50 +205,136 @@ __global__ void k_aabb(DevNodes N, DevParticles P, const ScenePar* __restrict__ 
     P.mx[p] = make_double4_32a(mx.x, mx.y, mx.z, 0.);
 }
 
+// the next FP32 number above f
+__device__ __forceinline__ float nextUp(float f) {
+    const int u = __float_as_int(f);
+    return f == 0.f ? __int_as_float(1) : __int_as_float(f > 0.f ? u + 1 : u - 1);
+}
+
 // ---------------------------------------------------------------- grid bounds over spheres
 // partial[b] = {min mn.x, min mn.y, min mn.z, max mn.x, max mn.y, max mn.z, max extent} over the
-// spheres ids[chunk[b] .. chunk[b+1]) (chunks never span two scenes of a batch)
+// spheres ids[chunk[b] .. chunk[b+1]) (chunks never span two scenes of a batch), rounded outward to FP32: the
+// grid only has to hold the boxes, and minima in FP64 bound this pass by its pipe.
 __global__ void k_grid_reduce(DevParticles P, const int32_t* __restrict__ ids, const int32_t* __restrict__ chunk,
-                              double* __restrict__ partial) {
-    __shared__ double s[7][BS];
-    const double inf = __longlong_as_double(0x7ff0000000000000LL);
-    double v[7] = {inf, inf, inf, -inf, -inf, -inf, 0.};
+                              float* __restrict__ partial) {
+    __shared__ float s[7][BS / 32];
+    const unsigned FULL = 0xffffffffu;
+    const float inf = __int_as_float(0x7f800000);
+    float v[7] = {inf, inf, inf, -inf, -inf, -inf, 0.f};
+    bool bad = false;  // a minimum would drop a NaN
     for (int i = chunk[blockIdx.x] + threadIdx.x; i < chunk[blockIdx.x + 1]; i += blockDim.x) {
         const int p = ids[i];
         const double4_32a a = P.mn[p], b = P.mx[p];
-        v[0] = fmin(v[0], a.x); v[1] = fmin(v[1], a.y); v[2] = fmin(v[2], a.z);
-        v[3] = fmax(v[3], a.x); v[4] = fmax(v[4], a.y); v[5] = fmax(v[5], a.z);
-        v[6] = fmax(v[6], fmax(fmax(b.x - a.x, b.y - a.y), b.z - a.z));
-    }
-    for (int q = 0; q < 7; q++) s[q][threadIdx.x] = v[q];
-    __syncthreads();
-    for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-        if (threadIdx.x < st) {
-            for (int q = 0; q < 3; q++) s[q][threadIdx.x] = fmin(s[q][threadIdx.x], s[q][threadIdx.x + st]);
-            for (int q = 3; q < 7; q++) s[q][threadIdx.x] = fmax(s[q][threadIdx.x], s[q][threadIdx.x + st]);
+        const float lo[3] = {__double2float_rd(a.x), __double2float_rd(a.y), __double2float_rd(a.z)};
+        const float hi[3] = {__double2float_ru(b.x), __double2float_ru(b.y), __double2float_ru(b.z)};
+        for (int q = 0; q < 3; q++) {
+            const float up = nextUp(lo[q]), e = __fsub_ru(hi[q], lo[q]);
+            bad = bad || !(e < inf);
+            v[q] = fminf(v[q], lo[q]);
+            v[3 + q] = fmaxf(v[3 + q], up);
+            v[6] = fmaxf(v[6], e);
         }
-        __syncthreads();
     }
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 7; q++) partial[blockIdx.x * 7 + q] = s[q][0];
+    if (bad) v[6] = inf;
+    for (int o = 16; o > 0; o >>= 1) {
+        for (int q = 0; q < 3; q++) v[q] = fminf(v[q], __shfl_down_sync(FULL, v[q], o));
+        for (int q = 3; q < 7; q++) v[q] = fmaxf(v[q], __shfl_down_sync(FULL, v[q], o));
+    }
+    if ((threadIdx.x & 31) == 0)
+        for (int q = 0; q < 7; q++) s[q][threadIdx.x >> 5] = v[q];
+    __syncthreads();
+    if (threadIdx.x < 7) {
+        const int q = threadIdx.x;
+        float m = s[q][0];
+        for (int w = 1; w < BS / 32; w++) m = q < 3 ? fminf(m, s[q][w]) : fmaxf(m, s[q][w]);
+        partial[blockIdx.x * 7 + q] = m;
+    }
 }
 
-__device__ __forceinline__ int cellCoord(double v, double o, double h, int n) {
-    double c = floor((v - o) / h);
-    int ci = (int)c;
+// The grid of each scene from the partial bounds of its chunks: cells slightly larger than the largest
+// sphere box, so that boxes that overlap sit in adjacent cells, and no more than cellBound() of them.
+// A warp per scene, then the first cell keys in scene order. A bound that is not finite sets `bad`.
+__host__ __device__ __forceinline__ int64_t cellBound(int64_t spheres, int scenes) {
+    const int64_t least = scenes > 1 ? 64 : 1 << 16;
+    return 8 * spheres > least ? 8 * spheres : least;
+}
+__global__ void __launch_bounds__(256) k_make_grids(int K, const int32_t* __restrict__ chunk, const int32_t* __restrict__ sceneChunk,
+                                                    const float* __restrict__ partial, const ScenePar* __restrict__ spp, int peri,
+                                                    Grid* __restrict__ out, int* __restrict__ bad) {
+    const unsigned FULL = 0xffffffffu;
+    const float inf = __int_as_float(0x7f800000);
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < K; k += blockDim.x >> 5) {
+        const int c0 = sceneChunk[k], c1 = sceneChunk[k + 1];
+        float v[7] = {inf, inf, inf, -inf, -inf, -inf, 0.f};
+        for (int b = c0 + lane; b < c1; b += 32) {
+            for (int q = 0; q < 3; q++) v[q] = fminf(v[q], partial[7 * b + q]);
+            for (int q = 3; q < 7; q++) v[q] = fmaxf(v[q], partial[7 * b + q]);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            for (int q = 0; q < 3; q++) v[q] = fminf(v[q], __shfl_down_sync(FULL, v[q], o));
+            for (int q = 3; q < 7; q++) v[q] = fmaxf(v[q], __shfl_down_sync(FULL, v[q], o));
+        }
+        if (lane) continue;
+        Grid g{0, 0, 0, 1, 1, 1, 1, 1, 1, 0, 0};
+        if (c0 != c1) {
+            bool fine = true;
+            for (int q = 0; q < 7; q++) fine = fine && isfinite(v[q]);
+            if (!fine) *bad = 1;
+            else {
+                const int64_t most = cellBound((int64_t)chunk[c1] - chunk[c0], K);
+                double h = (double)v[6] * (1 + 1e-9) + 1e-300;
+                const double ext[3] = {(double)v[3] - v[0], (double)v[4] - v[1], (double)v[5] - v[2]};
+                int64_t dims[3];
+                for (;;) {
+                    for (int q = 0; q < 3; q++) {
+                        // the periodic cell [0, size) per axis (unsheared coordinates), or the bounds
+                        const double d = peri ? floor(spp->cellSize[q] / h) : floor(ext[q] / h) + 1;
+                        dims[q] = d < 1. ? 1 : (d > 1e9 ? (int64_t)1000000000 : (int64_t)d);
+                    }
+                    if ((double)dims[0] * (double)dims[1] * (double)dims[2] <= (double)most) break;
+                    h *= 1.25;
+                }
+                g.ox = v[0]; g.oy = v[1]; g.oz = v[2]; g.h = h;
+                g.rh = 1. / h;
+                g.nx = (int32_t)dims[0]; g.ny = (int32_t)dims[1]; g.nz = (int32_t)dims[2];
+                g.ncell = dims[0] * dims[1] * dims[2];
+                if (peri)
+                    for (int q = 0; q < 3; q++)
+                        if (!(h <= 0.49 * spp->cellSize[q])) g.exact = 1;
+            }
+        }
+        out[k] = g;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int64_t base = 0;
+        for (int k = 0; k < K; k++) {
+            out[k].base = base;
+            base += out[k].ncell;
+        }
+    }
+}
+
+// rh = 1/h: the product is off by less than the margin of 1e-9 that h has over the largest box
+__device__ __forceinline__ int cellCoord(double v, double o, double rh, int n) {
+    const int ci = __double2int_rd((v - o) * rh);
     return ci < 0 ? 0 : (ci >= n ? n - 1 : ci);
 }
 
+// The cell of each sphere and its place within it (count: spheres per cell, zero before). The places
+// depend on the atomics' order; the pairs found, sorted afterwards, do not.
 __global__ void k_cellkey(DevParticles P, const int32_t* __restrict__ ids, int n, const Grid* __restrict__ Gs,
-                          uint32_t* __restrict__ key, int32_t* __restrict__ val) {
+                          uint32_t* __restrict__ key, int32_t* __restrict__ rank, int32_t* __restrict__ count) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int p = ids[i];
     const Grid G = Gs[sceneOfP(P, p)];
     const double4_32a a = P.mn[p];
-    const int cx = cellCoord(a.x, G.ox, G.h, G.nx), cy = cellCoord(a.y, G.oy, G.h, G.ny), cz = cellCoord(a.z, G.oz, G.h, G.nz);
-    key[i] = (uint32_t)(G.base + ((int64_t)cz * G.ny + cy) * G.nx + cx);
-    val[i] = p;
+    const int cx = cellCoord(a.x, G.ox, G.rh, G.nx), cy = cellCoord(a.y, G.oy, G.rh, G.ny), cz = cellCoord(a.z, G.oz, G.rh, G.nz);
+    const uint32_t k = (uint32_t)(G.base + ((int64_t)cz * G.ny + cy) * G.nx + cx);
+    key[i] = k;
+    rank[i] = atomicAdd(count + k, 1);
 }
 
 __device__ __forceinline__ int64_t lowerBound32(const uint32_t* a, int64_t n, uint32_t k) {
@@ -257,50 +354,48 @@ __device__ __forceinline__ int64_t lowerBound64(const uint64_t* a, int64_t n, ui
     return lo;
 }
 
-// cellOff[k] = number of sorted spheres with cell key < k, k in [0, ncell]
-__global__ void k_cell_off(const uint32_t* __restrict__ skey, int n, int64_t ncell, int32_t* __restrict__ off) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > ncell) return;
-    off[k] = (int32_t)lowerBound32(skey, n, (uint32_t)k);
-}
-
-__global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ sid, int n, double4_32a* __restrict__ smn,
-                                double4_32a* __restrict__ smx, float4* __restrict__ smnf,
-                                float4* __restrict__ smxf, float4* __restrict__ smnfi, float4* __restrict__ smxfi) {
+// the spheres' boxes in cell order, rounded outward to FP32
+__global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ ids, int n, const uint32_t* __restrict__ key,
+                                const int32_t* __restrict__ rank, const int32_t* __restrict__ off, uint32_t* __restrict__ skey,
+                                float4* __restrict__ smnf, float4* __restrict__ smxf) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int p = sid[i];
+    const int p = ids[i];
     const double4_32a a = P.mn[p], b = P.mx[p];
-    const uint32_t m = P.mask[p];
-    smn[i] = a;
-    smx[i] = b;
-    smnf[i] = make_float4(__double2float_rd(a.x), __double2float_rd(a.y), __double2float_rd(a.z), __uint_as_float(m));
-    smxf[i] = make_float4(__double2float_ru(b.x), __double2float_ru(b.y), __double2float_ru(b.z), __int_as_float(p));
-    smnfi[i] = make_float4(__double2float_ru(a.x), __double2float_ru(a.y), __double2float_ru(a.z), 0.f);
-    smxfi[i] = make_float4(__double2float_rd(b.x), __double2float_rd(b.y), __double2float_rd(b.z), 0.f);
+    const int at = off[key[i]] + rank[i];
+    skey[at] = key[i];
+    smnf[at] = make_float4(__double2float_rd(a.x), __double2float_rd(a.y), __double2float_rd(a.z), __uint_as_float(P.mask[p]));
+    smxf[at] = make_float4(__double2float_ru(b.x), __double2float_ru(b.y), __double2float_ru(b.z), __int_as_float(p));
 }
 
 // Collider::mayCollide pkg/dem/Collision.cpp:19-41 for particles that share no nodes
 __device__ __forceinline__ bool maskOk(uint32_t a, uint32_t b, uint32_t lone) { return (a & b) != 0 && (a & b & lone) == 0; }
 
-__device__ __forceinline__ void emitPair(int a, int b, uint64_t* pairs, int64_t cap, unsigned long long* counter) {
+// a pair as it is sorted: the lo id above the hi id, `bits` bits each (the fewest that hold an id)
+__device__ __forceinline__ uint64_t pairKey(int a, int b, int bits) {
     const int lo = a < b ? a : b, hi = a < b ? b : a;
+    return ((uint64_t)(uint32_t)lo << bits) | (uint32_t)hi;
+}
+__device__ __forceinline__ void emitPair(int a, int b, int bits, uint64_t* pairs, int64_t cap, unsigned long long* counter) {
     const unsigned long long idx = atomicAdd(counter, 1ull);
-    if ((int64_t)idx < cap) pairs[idx] = ((uint64_t)(uint32_t)lo << 32) | (uint32_t)hi;
+    if ((int64_t)idx < cap) pairs[idx] = pairKey(a, b, bits);
 }
 
 // Outward-rounded FP32 boxes overlap whenever the FP64 boxes do, so the FP32 test rejects most
-// candidates exactly; inward-rounded boxes (min up, max down) overlap only if the FP64 boxes do,
-// so they accept most of the rest exactly, and the FP64 test (InsertionSortCollider::spatialOverlap)
-// decides the cases where a bound lies within one FP32 rounding of the other.
+// candidates exactly. One FP32 number inward of each outward bound lies within the FP64 box, so boxes
+// shrunk to those overlap only if the FP64 boxes do, and accept most of the rest exactly; the FP64 test
+// (InsertionSortCollider::spatialOverlap) decides the cases in between.
 __device__ __forceinline__ bool overlapF(const float4& mn1, const float4& mx1, const float4& mn2, const float4& mx2) {
     return (mn1.x <= mx2.x) && (mx1.x >= mn2.x) && (mn1.y <= mx2.y) && (mx1.y >= mn2.y) && (mn1.z <= mx2.z) && (mx1.z >= mn2.z);
 }
-// the FP64 closed overlap of sorted boxes i and j whose outward-rounded boxes overlap
-__device__ __forceinline__ bool overlapSorted(int i, int j, const double4_32a* __restrict__ smn, const double4_32a* __restrict__ smx,
-                                              const float4* __restrict__ smnfi, const float4* __restrict__ smxfi) {
-    if (overlapF(smnfi[i], smxfi[i], smnfi[j], smxfi[j])) return true;
-    return overlap3(smn[i], smx[i], smn[j], smx[j]);
+__device__ __forceinline__ float nextDown(float f) { return -nextUp(-f); }
+__device__ __forceinline__ float4 upOf(const float4& f) { return make_float4(nextUp(f.x), nextUp(f.y), nextUp(f.z), 0.f); }
+__device__ __forceinline__ float4 downOf(const float4& f) { return make_float4(nextDown(f.x), nextDown(f.y), nextDown(f.z), 0.f); }
+// the FP64 closed overlap of particles p and q whose outward-rounded boxes (mn, mx) overlap
+__device__ __forceinline__ bool overlapOuter(const DevParticles& P, int p, int q, const float4& mn1, const float4& mx1, const float4& mn2,
+                                             const float4& mx2) {
+    if (overlapF(upOf(mn1), downOf(mx1), upOf(mn2), downOf(mx2))) return true;
+    return overlap3(P.mn[p], P.mx[p], P.mn[q], P.mx[q]);
 }
 
 // Pairs found by the lanes of a warp are written with one atomic per warp: each lane keeps up to
@@ -328,10 +423,6 @@ __device__ __forceinline__ void flushPairs(uint64_t (&buf)[kPairBuf], int& nb, u
         if (q < nb && (int64_t)(at + q) < cap) pairs[at + q] = buf[q];
     nb = 0;
 }
-__device__ __forceinline__ uint64_t pairKey(int a, int b) {
-    const int lo = a < b ? a : b, hi = a < b ? b : a;
-    return ((uint64_t)(uint32_t)lo << 32) | (uint32_t)hi;
-}
 
 // Appends key to the lane's pair buffer (register-resident: the slot is chosen by unrolled
 // comparisons, never by a runtime index).
@@ -347,11 +438,11 @@ __device__ __forceinline__ void pushPair(uint64_t (&buf)[kPairBuf], int& nb, uin
 // The candidate ranges of a lane are walked as one sequence, kSweepBatch candidates at a time
 // (their boxes are loaded together), so that the warp can flush together.
 constexpr int kSweepBatch = 2;
-__global__ void __launch_bounds__(256, 4) k_pairs_ss(const uint32_t* __restrict__ skey, const double4_32a* __restrict__ smn,
-                           const double4_32a* __restrict__ smx, const float4* __restrict__ smnf, const float4* __restrict__ smxf,
-                           const float4* __restrict__ smnfi, const float4* __restrict__ smxfi,
-                           int n, const Grid* __restrict__ Gs, const int32_t* __restrict__ pscene, const int32_t* __restrict__ off,
-                           uint32_t lone, uint64_t* __restrict__ pairs, int64_t cap, unsigned long long* __restrict__ counter) {
+__global__ void __launch_bounds__(256, 4) k_pairs_ss(DevParticles P, const uint32_t* __restrict__ skey, const float4* __restrict__ smnf,
+                                                     const float4* __restrict__ smxf, int n, const Grid* __restrict__ Gs,
+                                                     const int32_t* __restrict__ off, uint32_t lone, int bits, const int* __restrict__ bad,
+                                                     uint64_t* __restrict__ pairs, int64_t cap, unsigned long long* __restrict__ counter) {
+    if (*bad) return;
     const unsigned FULL = 0xffffffffu;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < n;
@@ -365,7 +456,7 @@ __global__ void __launch_bounds__(256, 4) k_pairs_ss(const uint32_t* __restrict_
         fx1 = smxf[i];
         m1 = __float_as_uint(fn1.w);
         pi = __float_as_int(fx1.w);
-        const Grid G = Gs[pscene ? pscene[pi] : 0];
+        const Grid G = Gs[sceneOfP(P, pi)];
         const uint32_t k = (uint32_t)((int64_t)skey[i] - G.base);
         const int cx = (int)(k % (uint32_t)G.nx);
         const int cy = (int)((k / (uint32_t)G.nx) % (uint32_t)G.ny);
@@ -412,8 +503,8 @@ __global__ void __launch_bounds__(256, 4) k_pairs_ss(const uint32_t* __restrict_
 #pragma unroll
         for (int u = 0; u < kSweepBatch; u++)
             if (jj[u] >= 0 && overlapF(fn1, fx1, a[u], c[u]) && maskOk(m1, __float_as_uint(a[u].w), lone) &&
-                overlapSorted(i, jj[u], smn, smx, smnfi, smxfi))
-                pushPair(buf, nb, pairKey(pi, __float_as_int(c[u].w)));
+                overlapOuter(P, pi, __float_as_int(c[u].w), fn1, fx1, a[u], c[u]))
+                pushPair(buf, nb, pairKey(pi, __float_as_int(c[u].w), bits));
         if (__any_sync(FULL, nb > kPairBuf - kSweepBatch)) flushPairs(buf, nb, pairs, cap, counter);
     }
     flushPairs(buf, nb, pairs, cap, counter);
@@ -422,10 +513,11 @@ __global__ void __launch_bounds__(256, 4) k_pairs_ss(const uint32_t* __restrict_
 // A facet (finite box) against the spheres of the cells its box can reach: a sphere j that
 // overlaps it has mn_j in [mn_f - h, mx_f] on every axis. One warp per facet; its lanes split
 // each x-run of cells.
-__global__ void k_pairs_local(DevParticles P, const int32_t* __restrict__ lids, int nl, const double4_32a* __restrict__ smn,
-                              const double4_32a* __restrict__ smx, const float4* __restrict__ smnf, const float4* __restrict__ smxf,
-                              const float4* __restrict__ smnfi, const float4* __restrict__ smxfi, const Grid* __restrict__ Gs, const int32_t* __restrict__ off, uint32_t lone, uint64_t* __restrict__ pairs,
-                              int64_t cap, unsigned long long* __restrict__ counter) {
+__global__ void k_pairs_local(DevParticles P, const int32_t* __restrict__ lids, int nl, const float4* __restrict__ smnf,
+                              const float4* __restrict__ smxf, const Grid* __restrict__ Gs, const int32_t* __restrict__ off, uint32_t lone,
+                              int bits, const int* __restrict__ bad, uint64_t* __restrict__ pairs, int64_t cap,
+                              unsigned long long* __restrict__ counter) {
+    if (*bad) return;
     const unsigned FULL = 0xffffffffu;
     const int t = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -435,12 +527,10 @@ __global__ void k_pairs_local(DevParticles P, const int32_t* __restrict__ lids, 
     const double4_32a mn1 = P.mn[p], mx1 = P.mx[p];
     const float4 fn1 = make_float4(__double2float_rd(mn1.x), __double2float_rd(mn1.y), __double2float_rd(mn1.z), 0.f);
     const float4 fx1 = make_float4(__double2float_ru(mx1.x), __double2float_ru(mx1.y), __double2float_ru(mx1.z), 0.f);
-    const float4 fni1 = make_float4(__double2float_ru(mn1.x), __double2float_ru(mn1.y), __double2float_ru(mn1.z), 0.f);
-    const float4 fxi1 = make_float4(__double2float_rd(mx1.x), __double2float_rd(mx1.y), __double2float_rd(mx1.z), 0.f);
     const uint32_t m1 = P.mask[p];
-    const int x0 = cellCoord(mn1.x - G.h, G.ox, G.h, G.nx), x1 = cellCoord(mx1.x, G.ox, G.h, G.nx);
-    const int y0 = cellCoord(mn1.y - G.h, G.oy, G.h, G.ny), y1 = cellCoord(mx1.y, G.oy, G.h, G.ny);
-    const int z0 = cellCoord(mn1.z - G.h, G.oz, G.h, G.nz), z1 = cellCoord(mx1.z, G.oz, G.h, G.nz);
+    const int x0 = cellCoord(mn1.x - G.h, G.ox, G.rh, G.nx), x1 = cellCoord(mx1.x, G.ox, G.rh, G.nx);
+    const int y0 = cellCoord(mn1.y - G.h, G.oy, G.rh, G.ny), y1 = cellCoord(mx1.y, G.oy, G.rh, G.ny);
+    const int z0 = cellCoord(mn1.z - G.h, G.oz, G.rh, G.nz), z1 = cellCoord(mx1.z, G.oz, G.rh, G.nz);
     uint64_t buf[kPairBuf];
     int nb = 0;
     for (int z = z0; z <= z1; z++)
@@ -453,8 +543,8 @@ __global__ void k_pairs_local(DevParticles P, const int32_t* __restrict__ lids, 
                     const float4 fn2 = smnf[j], fx2 = smxf[j];
                     const int q = __float_as_int(fx2.w);
                     if (q != p && overlapF(fn1, fx1, fn2, fx2) && maskOk(m1, __float_as_uint(fn2.w), lone) &&
-                        (overlapF(fni1, fxi1, smnfi[j], smxfi[j]) || overlap3(mn1, mx1, smn[j], smx[j])))
-                        pushPair(buf, nb, pairKey(p, q));
+                        overlapOuter(P, p, q, fn1, fx1, fn2, fx2))
+                        pushPair(buf, nb, pairKey(p, q, bits));
                 }
                 if (__any_sync(FULL, nb == kPairBuf)) flushPairs(buf, nb, pairs, cap, counter);
             }
@@ -463,11 +553,13 @@ __global__ void k_pairs_local(DevParticles P, const int32_t* __restrict__ lids, 
 }
 
 // ---------------------------------------------------------------- periodic cell
-__global__ void k_cellkey_peri(DevParticles P, const int32_t* __restrict__ ids, int n, Grid G, const ScenePar* __restrict__ spp,
-                               uint32_t* __restrict__ key, int32_t* __restrict__ val) {
+__global__ void k_cellkey_peri(DevParticles P, const int32_t* __restrict__ ids, int n, const Grid* __restrict__ Gs,
+                               const ScenePar* __restrict__ spp, uint32_t* __restrict__ key, int32_t* __restrict__ rank,
+                               int32_t* __restrict__ count) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const ScenePar& sp = *spp;
+    const Grid G = *Gs;
     const int p = ids[i];
     const double4_32a a = P.mn[p];
     const double w[3] = {cellWrapRelD(a.x, 0., sp.cellSize[0]), cellWrapRelD(a.y, 0., sp.cellSize[1]),
@@ -478,8 +570,9 @@ __global__ void k_cellkey_peri(DevParticles P, const int32_t* __restrict__ ids, 
         const int ci = (int)floor(w[k] / (sp.cellSize[k] / nn[k]));
         c[k] = ci < 0 ? 0 : (ci >= nn[k] ? nn[k] - 1 : ci);
     }
-    key[i] = (uint32_t)(((int64_t)c[2] * G.ny + c[1]) * G.nx + c[0]);
-    val[i] = p;
+    const uint32_t k = (uint32_t)(((int64_t)c[2] * G.ny + c[1]) * G.nx + c[0]);
+    key[i] = k;
+    rank[i] = atomicAdd(count + k, 1);
 }
 // Pairs emitted with their cell distance (periods of the lo particle minus those of the hi one).
 __device__ __forceinline__ void flushPairsCd(uint64_t (&buf)[kPairBuf], int32_t (&cbuf)[kPairBuf], int& nb, uint64_t* pairs,
@@ -515,11 +608,13 @@ struct PeriBox {
 // How far the FP32 fractions above may be from the exact ones: below 3 roundings of 2^-24 each with
 // those of the FP64 quotients behind them; ten times that is decided in FP64.
 constexpr float kPeriEps = 2e-6f;
-__global__ void k_gather_peri(DevParticles P, const int32_t* __restrict__ sid, int n, const ScenePar* __restrict__ spp,
-                              PeriBox* __restrict__ out) {
+__global__ void k_gather_peri(DevParticles P, const int32_t* __restrict__ ids, int n, const uint32_t* __restrict__ key,
+                              const int32_t* __restrict__ rank, const int32_t* __restrict__ off, const ScenePar* __restrict__ spp,
+                              uint32_t* __restrict__ skey, PeriBox* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int q = sid[i];
+    const int q = ids[i], at = off[key[i]] + rank[i];
+    skey[at] = key[i];
     const double4_32a a = P.mn[q], b = P.mx[q];
     const double m[3] = {a.x, a.y, a.z}, x[3] = {b.x, b.y, b.z};
     float u[3], l[3];
@@ -530,9 +625,9 @@ __global__ void k_gather_peri(DevParticles P, const int32_t* __restrict__ sid, i
         u[k] = (float)(f - fl);
         l[k] = (float)((x[k] - m[k]) * d);
     }
-    out[i].u = make_float4(u[0], u[1], u[2], __uint_as_float(P.mask[q]));
-    out[i].l = make_float4(l[0], l[1], l[2], 0.f);
-    out[i].p = make_int4(p[0], p[1], p[2], q);
+    out[at].u = make_float4(u[0], u[1], u[2], __uint_as_float(P.mask[q]));
+    out[at].l = make_float4(l[0], l[1], l[2], 0.f);
+    out[at].p = make_int4(p[0], p[1], p[2], q);
 }
 // out of line: a few pairs in ten thousand come here
 static __device__ __noinline__ int overlapPeriExact(const DevParticles& P, int lo, int hi, const ScenePar* __restrict__ spp, int* per) {
@@ -556,15 +651,18 @@ __device__ __forceinline__ float periGap(float ui, float li, float uj, float lj,
 // the FP32 fractions:
 //   the origin of overlapPeri's wrap is the box that starts first (d > 0: i's, d < 0: j's), so that
 //   the periods are p_i - p_j - r either way, and the overlap is a gap of zero or less.
-// exactOnly: some box is about half the cell or longer on an axis, where overlapPeri raises an error;
+// G.exact: some box is about half the cell or longer on an axis, where overlapPeri raises an error;
 // every candidate then goes through it.
 // Bound by instruction issue over about 85 candidates a sphere. With the exact test on every candidate
 // the sweep took nearly all of a full run of 200 000 spheres: 9.0 -> 0.48 ms.
 __global__ void __launch_bounds__(128) k_pairs_ss_peri(DevParticles P, const uint32_t* __restrict__ skey, const PeriBox* __restrict__ box,
-                                                       int n, Grid G, const int32_t* __restrict__ off, uint32_t lone, int exactOnly,
-                                                       const ScenePar* __restrict__ spp, uint64_t* __restrict__ pairs,
-                                                       int32_t* __restrict__ cds, int64_t cap, unsigned long long* __restrict__ counter,
-                                                       int* __restrict__ dErr) {
+                                                       int n, const Grid* __restrict__ Gs, const int32_t* __restrict__ off, uint32_t lone,
+                                                       int bits, const int* __restrict__ bad, const ScenePar* __restrict__ spp,
+                                                       uint64_t* __restrict__ pairs, int32_t* __restrict__ cds, int64_t cap,
+                                                       unsigned long long* __restrict__ counter, int* __restrict__ dErr) {
+    if (*bad) return;
+    const Grid G = *Gs;
+    const int exactOnly = G.exact;
     const unsigned FULL = 0xffffffffu;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < n;
@@ -623,7 +721,7 @@ __global__ void __launch_bounds__(128) k_pairs_ss_peri(DevParticles P, const uin
                             r = overlapPeriExact(P, pi, pj, spp, per);
                         if (r < 0) atomicCAS(dErr, 0, 103);
                         else if (r > 0) {
-                            const uint64_t key = pairKey(pi, pj);
+                            const uint64_t key = pairKey(pi, pj, bits);
                             const int32_t cd = packCellDist(per[0], per[1], per[2]);
 #pragma unroll
                             for (int v = 0; v < kPairBuf; v++)
@@ -643,7 +741,7 @@ __global__ void __launch_bounds__(128) k_pairs_ss_peri(DevParticles P, const uin
 }
 // Walls against every sphere with the periodic overlap test (pair oriented lo, hi).
 __global__ void k_pairs_global_peri(DevParticles P, const int32_t* __restrict__ gids, int ng, const int32_t* __restrict__ sph, int ns,
-                                    uint32_t lone, const ScenePar* __restrict__ spp, uint64_t* __restrict__ pairs,
+                                    uint32_t lone, int bits, const ScenePar* __restrict__ spp, uint64_t* __restrict__ pairs,
                                     int32_t* __restrict__ cds, int64_t cap, unsigned long long* __restrict__ counter,
                                     int* __restrict__ dErr) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -659,7 +757,7 @@ __global__ void k_pairs_global_peri(DevParticles P, const int32_t* __restrict__ 
         else if (r > 0) {
             const unsigned long long idx = atomicAdd(counter, 1ull);
             if ((int64_t)idx < cap) {
-                pairs[idx] = pairKey(lo, hi);
+                pairs[idx] = pairKey(lo, hi, bits);
                 cds[idx] = packCellDist(per[0], per[1], per[2]);
             }
         }
@@ -670,7 +768,7 @@ __global__ void k_pairs_global_peri(DevParticles P, const int32_t* __restrict__ 
 // gids are grouped by scene: the walls of scene k are gids[gStart[k] .. gStart[k+1]) (gStart null:
 // one scene, all of gids)
 __global__ void k_pairs_global(DevParticles P, const int32_t* __restrict__ gids, int ng, const int32_t* __restrict__ gStart,
-                               const int32_t* __restrict__ sph, int ns, uint32_t lone, uint64_t* __restrict__ pairs, int64_t cap,
+                               const int32_t* __restrict__ sph, int ns, uint32_t lone, int bits, uint64_t* __restrict__ pairs, int64_t cap,
                                unsigned long long* __restrict__ counter) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ns) return;
@@ -682,12 +780,12 @@ __global__ void k_pairs_global(DevParticles P, const int32_t* __restrict__ gids,
     for (int g = g0; g < g1; g++) {
         const int w = gids[g];
         if (w == s) continue;
-        if (overlap3(mn1, mx1, P.mn[w], P.mx[w]) && maskOk(m1, P.mask[w], lone)) emitPair(s, w, pairs, cap, counter);
+        if (overlap3(mn1, mx1, P.mn[w], P.mx[w]) && maskOk(m1, P.mask[w], lone)) emitPair(s, w, bits, pairs, cap, counter);
     }
 }
 
 // Pairs among non-spheres (only launched when their masks allow contact at all).
-__global__ void k_pairs_large_large(DevParticles P, const int32_t* __restrict__ ids, int n, uint32_t lone,
+__global__ void k_pairs_large_large(DevParticles P, const int32_t* __restrict__ ids, int n, uint32_t lone, int bits,
                                     uint64_t* __restrict__ pairs, int64_t cap, unsigned long long* __restrict__ counter) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (int64_t)n * n) return;
@@ -703,7 +801,7 @@ __global__ void k_pairs_large_large(DevParticles P, const int32_t* __restrict__ 
             for (int v = 0; v < 3; v++)
                 if (xa[u] == ya[v]) return;
     }
-    if (overlap3(P.mn[pa], P.mx[pa], P.mn[pb], P.mx[pb]) && maskOk(P.mask[pa], P.mask[pb], lone)) emitPair(pa, pb, pairs, cap, counter);
+    if (overlap3(P.mn[pa], P.mx[pa], P.mn[pb], P.mx[pb]) && maskOk(P.mask[pa], P.mask[pb], lone)) emitPair(pa, pb, bits, pairs, cap, counter);
 }
 
 // ---------------------------------------------------------------- merge with previous contacts
@@ -732,14 +830,19 @@ __device__ __forceinline__ int64_t findInRange(const uint64_t* __restrict__ key,
     }
     return (a < start[lo + 1] && key[a] == k) ? a : -1;
 }
-// pair keys (lo << 32 | hi) to (lo << bits | hi) for the sort, and back
-__global__ void k_pack_keys(uint64_t* __restrict__ k, int64_t n, int bits) {
+// the sorted pairs (lo << bits | hi) as contact keys (lo << 32 | hi), with k_lo_bounds of them
+__global__ void k_unpack_keys(const uint64_t* __restrict__ in, int64_t n, int bits, int nPar, uint64_t* __restrict__ out,
+                              int32_t* __restrict__ start) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) k[i] = ((k[i] >> 32) << bits) | (k[i] & 0xffffffffu);
-}
-__global__ void k_unpack_keys(uint64_t* __restrict__ k, int64_t n, int bits) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) k[i] = ((k[i] >> bits) << 32) | (k[i] & ((1ull << bits) - 1));
+    if (i > n) return;
+    const int prev = i > 0 ? (int)(in[i - 1] >> bits) : -1;
+    int cur = nPar;
+    if (i < n) {
+        const uint64_t k = in[i];
+        cur = (int)(k >> bits);
+        out[i] = ((uint64_t)(uint32_t)cur << 32) | (k & ((1ull << bits) - 1));
+    }
+    for (int q = prev + 1; q <= cur && q <= nPar; q++) start[q] = (int32_t)i;
 }
 __global__ void k_mark_orphans(DevContacts C, const uint64_t* __restrict__ nk, const int32_t* __restrict__ newLo,
                                int32_t* __restrict__ orph, const uint8_t* __restrict__ fresh) {
@@ -759,18 +862,32 @@ __global__ void k_compact_orphans(DevContacts C, const int32_t* __restrict__ orp
         osrc[o] = (int32_t)j;
     }
 }
-__global__ void k_place_new(const uint64_t* __restrict__ nk, int64_t nn, const uint64_t* __restrict__ okey, int64_t no,
-                            const uint64_t* __restrict__ oldKey, const int32_t* __restrict__ oldLo, uint64_t* __restrict__ outKey,
-                            int32_t* __restrict__ src, const int32_t* __restrict__ nkCd, int32_t* __restrict__ outCd,
-                            const uint8_t* __restrict__ fresh) {
+// The place of every new pair in the merged set and the old contact it continues. tot (null: not
+// wanted): the real contacts of the old set, and those of them among the new pairs; where the two differ
+// some real contact lost its overlap.
+__global__ void k_place_new(const uint64_t* __restrict__ nk, int64_t nn, const uint64_t* __restrict__ okey, int64_t no, DevContacts Cold,
+                            const int32_t* __restrict__ oldLo, uint64_t* __restrict__ outKey, int32_t* __restrict__ src,
+                            const int32_t* __restrict__ nkCd, int32_t* __restrict__ outCd, const uint8_t* __restrict__ fresh,
+                            CollideTotals* __restrict__ tot) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nn) return;
-    const uint64_t k = nk[i];
-    const int64_t out = i + lowerBound64(okey, no, k);
-    const int64_t pos = oldLo ? findInRange(oldKey, oldLo, k) : -1;
-    outKey[out] = k;
-    src[out] = (pos >= 0 && !freshPair(fresh, k)) ? (int32_t)pos : -1;
-    if (nkCd) outCd[out] = nkCd[i];
+    bool real = false, kept = false;
+    if (i < nn) {
+        const uint64_t k = nk[i];
+        const int64_t out = i + (no > 0 ? lowerBound64(okey, no, k) : 0);
+        int64_t pos = Cold.n > 0 ? findInRange(Cold.key, oldLo, k) : -1;
+        if (pos >= 0 && freshPair(fresh, k)) pos = -1;
+        kept = tot && pos >= 0 && (Cold.flags[pos] & C_REAL);
+        outKey[out] = k;
+        src[out] = (int32_t)pos;
+        if (nkCd) outCd[out] = nkCd[i];
+    }
+    if (!tot) return;
+    if (i < Cold.n) real = (Cold.flags[i] & C_REAL) && !freshPair(fresh, Cold.key[i]);
+    const int a = __syncthreads_count(real), b = __syncthreads_count(kept);
+    if (threadIdx.x == 0) {
+        if (a) atomicAdd(&tot->real, (unsigned long long)a);
+        if (b) atomicAdd(&tot->kept, (unsigned long long)b);
+    }
 }
 __global__ void k_place_orph(const uint64_t* __restrict__ nk, int64_t nn, const uint64_t* __restrict__ okey,
                              const int32_t* __restrict__ osrc, int64_t no, uint64_t* __restrict__ outKey, int32_t* __restrict__ src) {
@@ -781,56 +898,6 @@ __global__ void k_place_orph(const uint64_t* __restrict__ nk, int64_t nn, const 
     outKey[out] = k;
     src[out] = osrc[o];
 }
-// carry persistent state of surviving contacts; new contacts get their functor type and orientation
-// (CGeomDispatcher functor order: Facet/Wall first, ContactLoop.cpp:145-152)
-__global__ void k_gather(DevContacts Cold, DevContacts Cnew, const int32_t* __restrict__ src, DevParticles P,
-                         const long long* __restrict__ dStep, const int32_t* __restrict__ newCd) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Cnew.n) return;
-    const int32_t s0 = src[i];
-    // a contact removed since the last full run comes back as a new one
-    const int32_t s = (s0 >= 0 && (Cold.flags[s0] & C_REMOVED)) ? -1 : s0;
-    // FP32-force mode carries the state of real contacts only (a contact that is not real has no
-    // state any kernel reads; the listing reports zeros for it)
-    const bool fp32 = Cnew.fcol[0] != nullptr;
-    if (s >= 0) {
-        const uint32_t fo = Cold.flags[s];
-        Cnew.flags[i] = fo & ~(C_PENDING | C_DORMANT);
-        Cnew.step0[i] = Cold.step0[s];
-        Cnew.cdist[i] = Cold.cdist[s];
-        if (!fp32 || (fo & C_REAL)) {
-#pragma unroll
-            for (int q = 0; q < CC_NCOL; q++)
-                if (Cnew.col[q]) Cnew.col[q][i] = Cold.col[q][s];
-#pragma unroll
-            for (int q = 0; q < CF_NCOL; q++)
-                if (Cnew.fcol[q]) Cnew.fcol[q][i] = Cold.fcol[q][s];
-        }
-    } else {
-        const uint64_t k = Cnew.key[i];
-        const int lo = (int)(k >> 32), hi = (int)(k & 0xffffffffu);
-        const int tl = P.shape[lo], th = P.shape[hi];
-        uint32_t fl = 0, ty = CT_NONE;
-        const int a = (tl == WG_SHAPE_SPHERE) ? th : tl;
-        const bool sphLo = (tl == WG_SHAPE_SPHERE), sphHi = (th == WG_SHAPE_SPHERE);
-        if (sphLo && sphHi) ty = CT_SS;
-        else if (sphLo || sphHi) {
-            if (a == WG_SHAPE_FACET) ty = CT_FS;
-            else if (a == WG_SHAPE_WALL) ty = CT_WS;
-            if (sphLo) fl |= C_SWAP;  // the non-sphere (hi) becomes pA
-        }
-        fl |= ty << 2;
-        Cnew.flags[i] = fl;
-        Cnew.step0[i] = (int32_t)(*dStep);
-        Cnew.cdist[i] = newCd ? newCd[i] : packCellDist(0, 0, 0);
-        if (!fp32) {
-#pragma unroll
-            for (int q = 0; q < CC_NCOL; q++)
-                if (Cnew.col[q]) Cnew.col[q][i] = 0.;
-        }
-    }
-}
-
 // Dormant contacts. Between two full runs no node moves farther than verletDist from the position
 // it had at the first of them (the verlet test of Leapfrog triggers the next full run before that),
 // so a pair that is not real and whose surfaces are more than 2*verletDist apart now cannot touch
@@ -838,7 +905,7 @@ __global__ void k_gather(DevContacts Cold, DevContacts Cnew, const int32_t* __re
 // contacts stay in the container (they are potential contacts of the reference) but the contact
 // kernels skip them. The bounds are taken with a relative margin of 1e-9, and only for aperiodic
 // scenes (a periodic cell moves the images of the particles by itself).
-// The FP64 tests of k_dormant (sphere-sphere without mirrors, wall-sphere, facet-sphere), out of
+// The FP64 tests of dormantPair (sphere-sphere without mirrors, wall-sphere, facet-sphere), out of
 // line: inlined, they become predicated FP64 instructions in the warps of mirror-tested pairs.
 __device__ __noinline__ bool dormantFarFP64(const DevNodes& N, const DevParticles& P, const ScenePar* __restrict__ spp, int scene,
                                             uint32_t ty, int A, int B) {
@@ -886,32 +953,80 @@ __device__ __noinline__ bool dormantFarFP64(const DevNodes& N, const DevParticle
     }
     return far;
 }
-__global__ void k_dormant(DevContacts C, DevNodes N, DevParticles P, const ScenePar* __restrict__ spp) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C.n) return;
-    const uint32_t fl = C.flags[c];
-    if (fl & C_REAL) return;
+// whether contact k (flags fl, not real) is dormant
+__device__ __forceinline__ bool dormantPair(const DevNodes& N, const DevParticles& P, const ScenePar* __restrict__ spp, uint64_t k, uint32_t fl) {
     const uint32_t ty = ctype(fl);
-    if (ty == CT_NONE) return;
-    const uint64_t key = C.key[c];
-    const int lo = (int)(key >> 32), hi = (int)(key & 0xffffffffu);
+    if (ty == CT_NONE) return false;
+    const int lo = (int)(k >> 32), hi = (int)(k & 0xffffffffu);
     const int A = (fl & C_SWAP) ? hi : lo, B = (fl & C_SWAP) ? lo : hi;
     const int scene = sceneOfP(P, B);
-    bool far;
-    if (ty == CT_SS && N.mir) {
-        // FP32-force mode: the double-float mirrors of the positions, FP32 arithmetic; the
-        // relative position carries ~47 bits and the squares and sums ~2^-22 relative error
-        const ScenePar& sp = spp[scene];
-        const float4 ha = N.mir[A].ph, la = N.mir[A].pl, hb = N.mir[B].ph, lb = N.mir[B].pl;
-        float sx, tx, sy, ty_, sz, tz;
-        dfDiff(ha.x, la.x, hb.x, lb.x, sx, tx);
-        dfDiff(ha.y, la.y, hb.y, lb.y, sy, ty_);
-        dfDiff(ha.z, la.z, hb.z, lb.z, sz, tz);
-        const float dx = sx + tx, dy = sy + ty_, dz = sz + tz;
-        const float reach = (sp.ssDfAbsF * (ha.w + hb.w) + sp.reach2F) * (1.f + 1e-5f);
-        far = dx * dx + dy * dy + dz * dz > reach * reach;
-    } else far = dormantFarFP64(N, P, spp, scene, ty, A, B);
-    if (far) C.flags[c] = fl | C_DORMANT;
+    if (!(ty == CT_SS && N.mir)) return dormantFarFP64(N, P, spp, scene, ty, A, B);
+    // FP32-force mode: the double-float mirrors of the positions, FP32 arithmetic; the
+    // relative position carries ~47 bits and the squares and sums ~2^-22 relative error
+    const ScenePar& sp = spp[scene];
+    const float4 ha = N.mir[A].ph, la = N.mir[A].pl, hb = N.mir[B].ph, lb = N.mir[B].pl;
+    float sx, tx, sy, ty_, sz, tz;
+    dfDiff(ha.x, la.x, hb.x, lb.x, sx, tx);
+    dfDiff(ha.y, la.y, hb.y, lb.y, sy, ty_);
+    dfDiff(ha.z, la.z, hb.z, lb.z, sz, tz);
+    const float dx = sx + tx, dy = sy + ty_, dz = sz + tz;
+    const float reach = (sp.ssDfAbsF * (ha.w + hb.w) + sp.reach2F) * (1.f + 1e-5f);
+    return dx * dx + dy * dy + dz * dz > reach * reach;
+}
+
+// carry persistent state of surviving contacts; new contacts get their functor type and orientation
+// (CGeomDispatcher functor order: Facet/Wall first, ContactLoop.cpp:145-152); in an aperiodic scene those
+// that are not real are marked dormant where they are. packedState: the state of sphere-sphere contacts
+// goes from the old packed state to the new one (k_pack_ss)
+__global__ void k_gather(DevContacts Cold, DevContacts Cnew, const int32_t* __restrict__ src, DevNodes N, DevParticles P,
+                         const ScenePar* __restrict__ spp, const long long* __restrict__ dStep, const int32_t* __restrict__ newCd,
+                         int peri, int packedState) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= Cnew.n) return;
+    const int32_t s0 = src[i];
+    const uint64_t k = Cnew.key[i];
+    const uint32_t fo = s0 >= 0 ? Cold.flags[s0] : (uint32_t)C_REMOVED;
+    // a contact removed since the last full run comes back as a new one
+    const int32_t s = (fo & C_REMOVED) ? -1 : s0;
+    // FP32-force mode carries the state of real contacts only (a contact that is not real has no
+    // state any kernel reads; the listing reports zeros for it)
+    const bool fp32 = Cnew.fcol[0] != nullptr;
+    uint32_t fl = 0;
+    if (s >= 0) {
+        fl = fo & ~(C_PENDING | C_DORMANT);
+        Cnew.step0[i] = Cold.step0[s];
+        Cnew.cdist[i] = Cold.cdist[s];
+        if (!fp32 || ((fo & C_REAL) && !(packedState && ctype(fo) == CT_SS))) {
+#pragma unroll
+            for (int q = 0; q < CC_NCOL; q++)
+                if (Cnew.col[q]) Cnew.col[q][i] = Cold.col[q][s];
+#pragma unroll
+            for (int q = 0; q < CF_NCOL; q++)
+                if (Cnew.fcol[q]) Cnew.fcol[q][i] = Cold.fcol[q][s];
+        }
+    } else {
+        const int lo = (int)(k >> 32), hi = (int)(k & 0xffffffffu);
+        const int tl = P.shape[lo], th = P.shape[hi];
+        uint32_t ty = CT_NONE;
+        const int a = (tl == WG_SHAPE_SPHERE) ? th : tl;
+        const bool sphLo = (tl == WG_SHAPE_SPHERE), sphHi = (th == WG_SHAPE_SPHERE);
+        if (sphLo && sphHi) ty = CT_SS;
+        else if (sphLo || sphHi) {
+            if (a == WG_SHAPE_FACET) ty = CT_FS;
+            else if (a == WG_SHAPE_WALL) ty = CT_WS;
+            if (sphLo) fl |= C_SWAP;  // the non-sphere (hi) becomes pA
+        }
+        fl |= ty << 2;
+        Cnew.step0[i] = (int32_t)(*dStep);
+        Cnew.cdist[i] = newCd ? newCd[i] : packCellDist(0, 0, 0);
+        if (!fp32) {
+#pragma unroll
+            for (int q = 0; q < CC_NCOL; q++)
+                if (Cnew.col[q]) Cnew.col[q][i] = 0.;
+        }
+    }
+    if (!peri && !(fl & C_REAL) && dormantPair(N, P, spp, k, fl)) fl |= C_DORMANT;
+    Cnew.flags[i] = fl;
 }
 
 // ---------------------------------------------------------------- CSR incidence
@@ -933,12 +1048,10 @@ struct WorkClass {
         return 1ull | (plainContact(fl, cdist[c]) ? 1ull << 32 : 0ull);
     }
 };
-// loStart[p] = active contacts with lo < p
-__global__ void k_lo_start(const uint64_t* __restrict__ key, int64_t n, int nPar, const uint64_t* __restrict__ act,
-                           int32_t* __restrict__ loStart) {
+// loStart[p] = active contacts with lo < p; first[p]: the first contact with a lo id of p or more
+__global__ void k_lo_start(const int32_t* __restrict__ first, int nPar, const uint64_t* __restrict__ act, int32_t* __restrict__ loStart) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p > nPar) return;
-    loStart[p] = (int32_t)(uint32_t)act[lowerBound64(key, n, (uint64_t)(uint32_t)p << 32)];
+    if (p <= nPar) loStart[p] = (int32_t)(uint32_t)act[first[p]];
 }
 // hi id of the active contacts, nPar for the others (sorted past every particle)
 __global__ void k_hi_keys(const uint64_t* __restrict__ key, const uint32_t* __restrict__ flags, int64_t n, uint32_t nPar,
@@ -961,14 +1074,15 @@ __global__ void k_hi_start(const uint32_t* __restrict__ hks, int64_t n, int nPar
 // holds contacts that all go through the functor chain or that all leave after the distance test.
 // Mixed, the FP64 pipe, which takes a warp instruction's time whatever its lanes do, ran the chain
 // for the two fifths of the lanes that were not real (drum of 250 000: contact loop 0.70 -> 0.49 ms a
-// step). The FP32 kernel is bound by the gathered mirror records, which the mixed order reads
-// once for both kinds (1M drum: 0.161 ms a step mixed, 0.168 split).
-// tot, totReal: the counts over all contacts.
+// step). So does a periodic scene in the FP32-force mode, whose contacts are gathered from the contact
+// arrays either way (200 000: 0.12 -> 0.11 ms). The packed FP32 kernel is bound by the gathered mirror
+// records, which neighbours in contact order share: there the real ones come first within tiles of
+// contacts only (k_pack_ss; 1M drum: split over the whole list, the step took 0.168 ms instead of 0.161).
 __global__ void k_slots(const uint64_t* __restrict__ key, const uint32_t* __restrict__ flags, const int32_t* __restrict__ cdist, int64_t n,
-                        const uint64_t* __restrict__ act, const uint64_t* __restrict__ actReal, uint64_t tot, uint64_t totReal,
-                        DevIncidence I) {
+                        const uint64_t* __restrict__ act, const uint64_t* __restrict__ actReal, DevIncidence I) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
+    const uint64_t tot = act[n], totReal = actReal ? actReal[n] : 0;  // over all contacts
     const int nAct = (int)(uint32_t)tot, nPlain = (int)(tot >> 32);
     if (k < nAct) {
         const int32_t ch = I.hiList[k];
@@ -1001,15 +1115,31 @@ __global__ void k_slots(const uint64_t* __restrict__ key, const uint32_t* __rest
 // Particles summed by the block tree; the ones whose node has a free DOF are also summed before
 // every Leapfrog (the others only when the forces are reported).
 __global__ void k_heavy(DevIncidence I, DevParticles P, const uint32_t* __restrict__ nodeFlags, int threshold,
-                        int32_t* __restrict__ count) {
+                        CollideTotals* __restrict__ tot, const uint64_t* __restrict__ act, const uint64_t* __restrict__ actReal, int64_t n) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0) {  // the totals of the work-list scans, for the host
+        tot->act = act[n];
+        tot->actReal = actReal ? actReal[n] : 0;
+    }
     if (p >= P.n) return;
     if (P.shape[p] == WG_SHAPE_FACET) return;
     const int d = (I.hiStart[p + 1] - I.hiStart[p]) + (I.loStart[p + 1] - I.loStart[p]);
     if (d > threshold) {
-        const int q = atomicAdd(count, 1);
+        const int q = atomicAdd(&tot->heavy, 1);
         I.heavy[q] = p;
-        if ((nodeFlags[p] & F_DOF_ALL) != F_DOF_ALL) I.heavyFree[atomicAdd(count + 1, 1)] = p;
+        if ((nodeFlags[p] & F_DOF_ALL) != F_DOF_ALL) I.heavyFree[atomicAdd(&tot->heavyFree, 1)] = p;
+    }
+}
+// every end starts without a contribution: 2 ends of each of the active contacts (*act, low half)
+__global__ void k_zero_ends(DevIncidence I, const uint64_t* __restrict__ act) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 2 * (int64_t)(uint32_t)*act) return;
+    if (I.endA) {
+        I.endA[e] = make_double4_32a(0., 0., 0., 0.);
+        I.endB[e] = make_double2(0., 0.);
+    } else {
+        I.endAf[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        I.endBf[e] = make_float2(0.f, 0.f);
     }
 }
 
@@ -1100,7 +1230,7 @@ static int buildLists(Sim& S) {
     W.chunksDirty = true;
     W.hChunk.assign(1, 0);
     W.hSceneChunk.assign(1, 0);
-    const int64_t CH = 4096;
+    const int64_t CH = kGridChunk;
     for (int k = 0; k < K; k++) {
         for (int64_t b = W.hSceneSph[k]; b < W.hSceneSph[k + 1]; b += CH) W.hChunk.push_back((int32_t)std::min(b + CH, W.hSceneSph[k + 1]));
         W.hSceneChunk.push_back((int32_t)W.hChunk.size() - 1);
@@ -1139,12 +1269,6 @@ static int buildLists(Sim& S) {
 
 int collide_full_run(Sim& S) {
     cudaStream_t st = S.stream;
-    // the contact arrays take back the packed sphere-sphere state before they are merged
-    {
-        int r = S.syncContacts(false);  // the merge below is queued on the same stream
-        if (r) return r;
-        S.K.n = 0;
-    }
     if (!S.cw) {
         S.cw = new CollideWork();
         S.listsDirty = true;
@@ -1155,6 +1279,20 @@ int collide_full_run(Sim& S) {
         S.listsDirty = false;
     }
     CollideWork& W = *S.cw;
+    // The packed sphere-sphere state goes from the old set to the new one; the contact arrays take back its
+    // flags alone. Where they hold another set than the packed one, all of it comes from them.
+    const bool packed = S.prec == WG_PREC_FP32 && !S.cfg.periodic;
+    const bool packedState = packed && S.K.n > 0 && W.packIdxValid && !S.contactsReplaced;
+    if (packedState) {
+        if (S.packDirty) launch_unpack_ss(st, S.C, S.I, S.K, S.nMixed, true);
+        S.packDirty = false;
+    } else {
+        int r = S.syncContacts(false);  // the merge below is queued on the same stream
+        if (r) return r;
+    }
+    const DevPackedSS Kold = S.K;
+    S.K.n = 0;
+    W.packIdxValid = false;
     const uint32_t lone = S.cfg.lone_mask;
     if (S.cfg.periodic && S.hPar.hasShear && !W.hGlobal.empty())
         return S.fail(WG_ERR_UNSUPPORTED, "Walls not supported in skewed (Scene.cell.trsf is not diagonal) periodic boundary conditions.");
@@ -1162,113 +1300,81 @@ int collide_full_run(Sim& S) {
     if (S.nPar > 0) k_aabb<<<(unsigned)((S.nPar + BS - 1) / BS), BS, 0, st>>>(S.N, S.P, S.dPar, S.dFlags + 1);
     // lastPos for node slots not owned by a particle box computation (dummy slots) stays stale:
     // they never move (blocked, zero velocity) and are never tested against a stale reference.
-    // 2. grid over spheres, one per scene of a batch (keys of scene k start at its grid's base)
+    // 2. grid over spheres, one per scene of a batch (keys of scene k start at its grid's base). The grids
+    // are made on the device, so that the host need not wait for the bounds; it knows how many cells there
+    // can be.
     const int K = S.nScenes;
-    std::vector<Grid> hG(K, Grid{0, 0, 0, 1, 1, 1, 1, 1, 0});
-    Grid G = hG[0];
-    bool periExact = false;
     const int ns = W.nSph;
+    const bool peri = S.cfg.periodic != 0;
+    if (!W.tot) {
+        W.tot = (CollideTotals*)S.dalloc(sizeof(CollideTotals));
+        WG_CUDA_TRY(cudaMallocHost(&W.hTot, sizeof(CollideTotals)));
+        if (!W.tot) return S.fail(WG_ERR_CUDA, "out of device memory (counts)");
+    }
+    WG_CUDA_TRY(cudaMemsetAsync(W.tot, 0, sizeof(CollideTotals), st));
+    int* const bad = &W.tot->bad;
     if (ns > 0) {
         const int nb = (int)W.hChunk.size() - 1;
         if (!W.dGrids) {
-            // capacity for the most chunks the particles can form (one per scene plus one per 4096 spheres)
-            const int cap = (int)(S.nPar / 4096 + S.nScenes + 2);
-            W.red = (double*)S.dalloc(sizeof(double) * 7 * cap);
+            // capacity for the most chunks the particles can form (one per scene plus the full ones)
+            const int cap = (int)(S.nPar / kGridChunk + S.nScenes + 2);
+            W.red = (float*)S.dalloc(sizeof(float) * 7 * cap);
             W.dChunk = (int32_t*)S.dalloc(sizeof(int32_t) * (cap + 1));
-            WG_CUDA_TRY(cudaMallocHost(&W.hRed, sizeof(double) * 7 * cap));
+            W.dSceneChunk = (int32_t*)S.dalloc(sizeof(int32_t) * (K + 1));
             W.dGrids = (Grid*)S.dalloc(sizeof(Grid) * K);
-            if (!W.dGrids || !W.dChunk) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
+            const int64_t sph = S.nPar;  // every particle could be an active sphere
+            W.cellKey = (uint32_t*)S.dalloc(sizeof(uint32_t) * sph);
+            W.cellRank = (int32_t*)S.dalloc(sizeof(int32_t) * sph);
+            W.skey = (uint32_t*)S.dalloc(sizeof(uint32_t) * sph);
+            if (peri) W.speri = (PeriBox*)S.dalloc(sizeof(PeriBox) * sph);
+            else {
+                W.smnf = (float4*)S.dalloc(sizeof(float4) * sph);
+                W.smxf = (float4*)S.dalloc(sizeof(float4) * sph);
+            }
+            if (!W.red || !W.dChunk || !W.dSceneChunk || !W.dGrids || !W.cellKey || !W.cellRank || !W.skey ||
+                (peri ? !W.speri : (!W.smnf || !W.smxf)))
+                return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
         }
         if (W.chunksDirty) {
-            WG_CUDA_TRY(cudaMemcpyAsync(W.dChunk, W.hChunk.data(), sizeof(int32_t) * (nb + 1), cudaMemcpyHostToDevice, S.stream));
+            WG_CUDA_TRY(cudaMemcpyAsync(W.dChunk, W.hChunk.data(), sizeof(int32_t) * (nb + 1), cudaMemcpyHostToDevice, st));
+            WG_CUDA_TRY(cudaMemcpyAsync(W.dSceneChunk, W.hSceneChunk.data(), sizeof(int32_t) * (K + 1), cudaMemcpyHostToDevice, st));
             W.chunksDirty = false;
         }
+        int64_t ncell = 0;
+        for (int k = 0; k < K; k++) ncell += cellBound(W.hSceneSph[k + 1] - W.hSceneSph[k], K);
+        if (ncell >= (int64_t(1) << 31) - 2) return S.fail(WG_ERR_CAPACITY, "too many broad-phase cells in the batch");
+        W.cellOff = grow(S, W.cellOff, W.cellOffCap, ncell + 1);
+        if (!W.cellOff) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
+        const unsigned gs = (unsigned)((ns + BS - 1) / BS);
         k_grid_reduce<<<nb, BS, 0, st>>>(S.P, W.sphereIds, W.dChunk, W.red);
-        WG_CUDA_TRY(cudaMemcpyAsync(W.hRed, W.red, sizeof(double) * 7 * nb, cudaMemcpyDeviceToHost, st));
-        WG_CUDA_TRY(cudaStreamSynchronize(st));
-        int64_t base = 0;
-        for (int k = 0; k < K; k++) {
-            double v[7] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, 0.};
-            for (int b = W.hSceneChunk[k]; b < W.hSceneChunk[k + 1]; b++) {
-                for (int q = 0; q < 3; q++) v[q] = std::min(v[q], W.hRed[7 * b + q]);
-                for (int q = 3; q < 7; q++) v[q] = std::max(v[q], W.hRed[7 * b + q]);
-            }
-            Grid& g = hG[k];
-            g.base = base;
-            if (W.hSceneChunk[k] == W.hSceneChunk[k + 1]) continue;  // a scene without spheres
-            if (!(std::isfinite(v[0]) && std::isfinite(v[3]) && std::isfinite(v[6])))
-                return S.fail(WG_ERR_NAN, "InsertionSortCollider: non-finite sphere bounding box (NaN or infinite position)");
-            const int64_t nsk = W.hSceneSph[k + 1] - W.hSceneSph[k];
-            // cell edge slightly above the largest sphere box, so boxes that overlap sit in adjacent cells
-            double h = v[6] * (1 + 1e-9) + 1e-300;
-            double ext[3] = {v[3] - v[0], v[4] - v[1], v[5] - v[2]};
-            int64_t dims[3];
-            for (;;) {
-                if (S.cfg.periodic)  // the periodic cell [0, size) per axis (unsheared coordinates)
-                    for (int q = 0; q < 3; q++) dims[q] = std::max<int64_t>(1, (int64_t)std::floor(S.hPar.cellSize[q] / h));
-                else
-                    for (int q = 0; q < 3; q++) dims[q] = (int64_t)std::floor(ext[q] / h) + 1;
-                int64_t nc = dims[0] * dims[1] * dims[2];
-                if (nc <= std::max<int64_t>(8 * nsk, K > 1 ? 64 : (1 << 16)) && nc < (int64_t(1) << 31)) break;
-                h *= 1.25;
-            }
-            g.ox = v[0]; g.oy = v[1]; g.oz = v[2]; g.h = h;
-            g.nx = (int32_t)dims[0]; g.ny = (int32_t)dims[1]; g.nz = (int32_t)dims[2];
-            g.ncell = dims[0] * dims[1] * dims[2];
-            base += g.ncell;
-        }
-        if (base >= (int64_t(1) << 32) - 1) return S.fail(WG_ERR_CAPACITY, "too many broad-phase cells in the batch");
-        const int64_t ncellAll = base;
-        G = hG[0];
-        WG_CUDA_TRY(cudaMemcpyAsync(W.dGrids, hG.data(), sizeof(Grid) * K, cudaMemcpyHostToDevice, st));
-        // sort spheres by cell
-        if (!W.cellKey) {
-            const int64_t cap = S.nPar;  // every particle could be an active sphere
-            W.cellKey = (uint32_t*)S.dalloc(sizeof(uint32_t) * cap);
-            W.cellKeySorted = (uint32_t*)S.dalloc(sizeof(uint32_t) * cap);
-            W.cellVal = (int32_t*)S.dalloc(sizeof(int32_t) * cap);
-            W.sid = (int32_t*)S.dalloc(sizeof(int32_t) * cap);
-            if (!W.sid) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
-            if (S.cfg.periodic) {
-                W.speri = (PeriBox*)S.dalloc(sizeof(PeriBox) * cap);
-                if (!W.speri) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
-            } else {
-                W.smn = (double4_32a*)S.dalloc(sizeof(double4_32a) * cap);
-                W.smx = (double4_32a*)S.dalloc(sizeof(double4_32a) * cap);
-                W.smnf = (float4*)S.dalloc(sizeof(float4) * cap);
-                W.smxf = (float4*)S.dalloc(sizeof(float4) * cap);
-                W.smnfi = (float4*)S.dalloc(sizeof(float4) * cap);
-                W.smxfi = (float4*)S.dalloc(sizeof(float4) * cap);
-                if (!W.smn || !W.smx || !W.smnf || !W.smxf || !W.smnfi || !W.smxfi) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
-            }
-        }
-        W.cellOff = grow(S, W.cellOff, W.cellOffCap, ncellAll + 1);
-        if (S.cfg.periodic) k_cellkey_peri<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.sphereIds, ns, G, S.dPar, W.cellKey, W.cellVal);
-        else k_cellkey<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, W.cellKey, W.cellVal);
-        int endBit = 1;
-        while ((int64_t(1) << endBit) < ncellAll) endBit++;
+        k_make_grids<<<1, 256, 0, st>>>(K, W.dChunk, W.dSceneChunk, W.red, S.dPar, peri ? 1 : 0, W.dGrids, bad);
+        // spheres in cell order: their number per cell, its running sum, then each to its place
+        WG_CUDA_TRY(cudaMemsetAsync(W.cellOff, 0, sizeof(int32_t) * (ncell + 1), st));
+        if (peri) k_cellkey_peri<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, S.dPar, W.cellKey, W.cellRank, W.cellOff);
+        else k_cellkey<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, W.cellKey, W.cellRank, W.cellOff);
         size_t tb = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, W.cellKey, W.cellKeySorted, W.cellVal, W.sid, ns, 0, endBit, st);
+        cub::DeviceScan::ExclusiveSum(nullptr, tb, W.cellOff, W.cellOff, (int)(ncell + 1), st);
         if (ensureCub(S, tb)) return WG_ERR_CUDA;
         tb = W.cubBytes;
-        WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.cellKey, W.cellKeySorted, W.cellVal, W.sid, ns, 0, endBit, st));
-        k_cell_off<<<(unsigned)((ncellAll + 1 + BS - 1) / BS), BS, 0, st>>>(W.cellKeySorted, ns, ncellAll, W.cellOff);
-        if (S.cfg.periodic) {
-            k_gather_peri<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.sid, ns, S.dPar, W.speri);
-            // the grid's cells are no shorter than the longest box edge
-            for (int q = 0; q < 3; q++) periExact = periExact || !(hG[0].h <= 0.49 * S.hPar.cellSize[q]);
-        } else
-            k_gather_sorted<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.sid, ns, W.smn, W.smx, W.smnf, W.smxf, W.smnfi, W.smxfi);
+        WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, W.cellOff, W.cellOff, (int)(ncell + 1), st));
+        if (peri) k_gather_peri<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.cellKey, W.cellRank, W.cellOff, S.dPar, W.skey, W.speri);
+        else k_gather_sorted<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.cellKey, W.cellRank, W.cellOff, W.skey, W.smnf, W.smxf);
     }
     // lists of large particles: facets with boxes spanning a few cells use the grid, the rest are global
     {
         // decide on the host from the facet sizes measured at the previous full run would need a copy;
         // facet boxes are static in the supported scenes, so classify them once by size here
         if (W.nLarge == 0 && W.nGlobal == 0 && (!W.hLarge.empty() || !W.hGlobal.empty())) {
-            std::vector<double4_32a> mn(S.nPar), mx(S.nPar);
-            WG_CUDA_TRY(cudaMemcpyAsync(mn.data(), S.P.mn, sizeof(double4_32a) * S.nPar, cudaMemcpyDeviceToHost, st));
-            WG_CUDA_TRY(cudaMemcpyAsync(mx.data(), S.P.mx, sizeof(double4_32a) * S.nPar, cudaMemcpyDeviceToHost, st));
-            WG_CUDA_TRY(cudaStreamSynchronize(st));
+            std::vector<double4_32a> mn, mx;
+            std::vector<Grid> hG(K, Grid{0, 0, 0, 1, 1, 1, 1, 1, 1, 0, 0});
+            if (!W.hLarge.empty()) {
+                mn.resize(S.nPar);
+                mx.resize(S.nPar);
+                WG_CUDA_TRY(cudaMemcpyAsync(mn.data(), S.P.mn, sizeof(double4_32a) * S.nPar, cudaMemcpyDeviceToHost, st));
+                WG_CUDA_TRY(cudaMemcpyAsync(mx.data(), S.P.mx, sizeof(double4_32a) * S.nPar, cudaMemcpyDeviceToHost, st));
+                if (ns > 0) WG_CUDA_TRY(cudaMemcpyAsync(hG.data(), W.dGrids, sizeof(Grid) * K, cudaMemcpyDeviceToHost, st));
+                WG_CUDA_TRY(cudaStreamSynchronize(st));
+            }
             std::vector<int32_t> loc, glo = W.hGlobal;
             for (int32_t p : W.hLarge) {
                 double e = std::max({mx[p].x - mn[p].x, mx[p].y - mn[p].y, mx[p].z - mn[p].z});
@@ -1290,20 +1396,18 @@ int collide_full_run(Sim& S) {
         }
     }
     // 3-4. pair generation with a capacity retry
-    if (!W.counter) {
-        W.counter = (unsigned long long*)S.dalloc(sizeof(unsigned long long) * 2);
-        WG_CUDA_TRY(cudaMallocHost(&W.hCounter, sizeof(unsigned long long) * 2));
-    }
     if (W.pairCap == 0) {
         int64_t c0 = std::max<int64_t>(1 << 16, 8 * S.nPar);
         W.pairs = grow(S, W.pairs, W.pairCap, c0);
         int64_t cap2 = 0;
         W.pairsSorted = grow(S, W.pairsSorted, cap2, W.pairCap);
     }
-    const bool peri = S.cfg.periodic != 0;
+    int idBits = 1;  // bits of an id
+    while ((int64_t(1) << idBits) < S.nPar) idBits++;
+    unsigned long long* const counter = &W.tot->pairs;
     int64_t nNew = 0;
     for (int attempt = 0; attempt < 3; attempt++) {
-        WG_CUDA_TRY(cudaMemsetAsync(W.counter, 0, sizeof(unsigned long long), st));
+        if (attempt > 0) WG_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
         if (peri) {
             if (W.pairCdCap < W.pairCap) {
                 int64_t c2 = W.pairCdCap;
@@ -1312,22 +1416,20 @@ int collide_full_run(Sim& S) {
                 if (!W.pairCd || !W.pairCdSorted) return S.fail(WG_ERR_CUDA, "out of device memory (pairs)");
             }
             if (ns > 0)
-                k_pairs_ss_peri<<<(ns + 127) / 128, 128, 0, st>>>(S.P, W.cellKeySorted, W.speri, ns, G, W.cellOff, lone, periExact ? 1 : 0,
-                                                                  S.dPar, W.pairs, W.pairCd, W.pairCap, W.counter, S.dFlags + FL_ERR);
+                k_pairs_ss_peri<<<(ns + 127) / 128, 128, 0, st>>>(S.P, W.skey, W.speri, ns, W.dGrids, W.cellOff, lone, idBits, bad, S.dPar,
+                                                                  W.pairs, W.pairCd, W.pairCap, counter, S.dFlags + FL_ERR);
             if (ns > 0 && W.nGlobal > 0)
-                k_pairs_global_peri<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.globalIds, W.nGlobal, W.sphereIds, ns, lone, S.dPar,
-                                                                     W.pairs, W.pairCd, W.pairCap, W.counter, S.dFlags + FL_ERR);
+                k_pairs_global_peri<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.globalIds, W.nGlobal, W.sphereIds, ns, lone, idBits, S.dPar,
+                                                                     W.pairs, W.pairCd, W.pairCap, counter, S.dFlags + FL_ERR);
         } else if (ns > 0) {
-            k_pairs_ss<<<(ns + BS - 1) / BS, BS, 0, st>>>(W.cellKeySorted, W.smn, W.smx, W.smnf, W.smxf, W.smnfi, W.smxfi, ns, W.dGrids,
-                                                        S.P.scene,
-                                                        W.cellOff, lone, W.pairs, W.pairCap, W.counter);
+            k_pairs_ss<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.skey, W.smnf, W.smxf, ns, W.dGrids, W.cellOff, lone, idBits, bad, W.pairs,
+                                                        W.pairCap, counter);
             if (W.nLarge > 0)
                 k_pairs_local<<<(unsigned)(((int64_t)W.nLarge * 32 + BS - 1) / BS), BS, 0, st>>>(
-                    S.P, W.largeIds, W.nLarge, W.smn, W.smx, W.smnf, W.smxf, W.smnfi, W.smxfi, W.dGrids, W.cellOff, lone, W.pairs,
-                    W.pairCap, W.counter);
+                    S.P, W.largeIds, W.nLarge, W.smnf, W.smxf, W.dGrids, W.cellOff, lone, idBits, bad, W.pairs, W.pairCap, counter);
             if (W.nGlobal > 0)
-                k_pairs_global<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.globalIds, W.nGlobal, K > 1 ? W.gStart : nullptr, W.sphereIds, ns, lone,
-                                                                W.pairs, W.pairCap, W.counter);
+                k_pairs_global<<<(ns + BS - 1) / BS, BS, 0, st>>>(S.P, W.globalIds, W.nGlobal, K > 1 ? W.gStart : nullptr, W.sphereIds, ns,
+                                                                lone, idBits, W.pairs, W.pairCap, counter);
         }
         if (W.largeLargePossible && !peri) {
             // all non-spheres against each other
@@ -1340,224 +1442,227 @@ int collide_full_run(Sim& S) {
                 WG_CUDA_TRY(cudaMemcpyAsync(W.globalIds + W.nGlobal, W.largeIds, sizeof(int32_t) * W.nLarge, cudaMemcpyDeviceToDevice, st));
             }
             int64_t tot = (int64_t)nn * nn;
-            k_pairs_large_large<<<(unsigned)((tot + BS - 1) / BS), BS, 0, st>>>(S.P, ids, nn, lone, W.pairs, W.pairCap, W.counter);
+            k_pairs_large_large<<<(unsigned)((tot + BS - 1) / BS), BS, 0, st>>>(S.P, ids, nn, lone, idBits, W.pairs, W.pairCap, counter);
         }
-        WG_CUDA_TRY(cudaMemcpyAsync(W.hCounter, W.counter, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        WG_CUDA_TRY(cudaMemcpyAsync(W.hTot, W.tot, sizeof(CollideTotals), cudaMemcpyDeviceToHost, st));
         WG_CUDA_TRY(cudaStreamSynchronize(st));
-        nNew = (int64_t)W.hCounter[0];
+        if (W.hTot->bad) return S.fail(WG_ERR_NAN, "InsertionSortCollider: non-finite sphere bounding box (NaN or infinite position)");
+        nNew = (int64_t)W.hTot->pairs;
         if (nNew <= W.pairCap) break;
         int64_t cap2 = W.pairCap;
         W.pairs = grow(S, W.pairs, W.pairCap, nNew + nNew / 4);
         W.pairsSorted = grow(S, W.pairsSorted, cap2, W.pairCap);
         if (!W.pairs || !W.pairsSorted) return S.fail(WG_ERR_CUDA, "out of device memory (pairs)");
     }
-    // sort new pair keys
-    int idBits = 1;
-    while ((int64_t(1) << idBits) < S.nPar) idBits++;
-    if (nNew > 0 && peri) {
+    // sort the pairs, (lo << idBits | hi)
+    if (nNew > 0) {
         size_t tb = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, W.pairs, W.pairsSorted, W.pairCd, W.pairCdSorted, nNew, 0, 32 + idBits, st);
+        if (peri) cub::DeviceRadixSort::SortPairs(nullptr, tb, W.pairs, W.pairsSorted, W.pairCd, W.pairCdSorted, nNew, 0, 2 * idBits, st);
+        else cub::DeviceRadixSort::SortKeys(nullptr, tb, W.pairs, W.pairsSorted, nNew, 0, 2 * idBits, st);
         if (ensureCub(S, tb)) return WG_ERR_CUDA;
         tb = W.cubBytes;
-        WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.pairs, W.pairsSorted, W.pairCd, W.pairCdSorted, nNew, 0,
-                                                    32 + idBits, st));
-    } else if (nNew > 0) {
-        // ids take idBits each: sort (lo << idBits | hi), the same order in fewer radix passes
-        const unsigned pb = (unsigned)((nNew + BS - 1) / BS);
-        k_pack_keys<<<pb, BS, 0, st>>>(W.pairs, nNew, idBits);
-        size_t tb = 0;
-        cub::DeviceRadixSort::SortKeys(nullptr, tb, W.pairs, W.pairsSorted, nNew, 0, 2 * idBits, st);
-        if (ensureCub(S, tb)) return WG_ERR_CUDA;
-        tb = W.cubBytes;
-        WG_CUDA_TRY(cub::DeviceRadixSort::SortKeys(W.cubTmp, tb, W.pairs, W.pairsSorted, nNew, 0, 2 * idBits, st));
-        k_unpack_keys<<<pb, BS, 0, st>>>(W.pairsSorted, nNew, idBits);
+        if (peri)
+            WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.pairs, W.pairsSorted, W.pairCd, W.pairCdSorted, nNew, 0, 2 * idBits,
+                                                        st));
+        else WG_CUDA_TRY(cub::DeviceRadixSort::SortKeys(W.cubTmp, tb, W.pairs, W.pairsSorted, nNew, 0, 2 * idBits, st));
     }
-    // 5. merge with the previous contact set
+    // 5. merge with the previous contact set. Real contacts without an overlap (a law that keeps separated
+    // contacts, or no verletDist) stay: they are looked for first where they can occur, which costs a
+    // scan and a wait; elsewhere the merge counts whether every real contact was among the new pairs, and is
+    // done again with them if the host finds that one was not.
     const int64_t nOld = S.C.n;
-    W.orph = grow(S, W.orph, W.mergeCap, std::max<int64_t>(nOld, 1) * 2 + 2);
-    int64_t capTmp = 0;
-    if (!W.orphKey || W.mergeCap > 0) {
-        // orphKey/orphSrc sized like orph
-        static int64_t dummy;
-        (void)dummy;
-    }
-    int64_t nOrph = 0;
-    // the first index of every lo id in the new pairs and in the old contacts
     W.newLo = grow(S, W.newLo, W.newLoCap, S.nPar + 2);
     W.oldLo = grow(S, W.oldLo, W.oldLoCap, S.nPar + 2);
     if (!W.newLo || !W.oldLo) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
-    k_lo_bounds<<<(unsigned)((nNew + 1 + BS - 1) / BS), BS, 0, st>>>(W.pairsSorted, nNew, (int)S.nPar, W.newLo);
-    k_lo_bounds<<<(unsigned)((nOld + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, nOld, (int)S.nPar, W.oldLo);
-    if (nOld > 0) {
-        int32_t* flagsArr = W.orph;
-        int32_t* scanArr = W.orph + (std::max<int64_t>(nOld, 1) + 1);
-        k_mark_orphans<<<(unsigned)((nOld + BS - 1) / BS), BS, 0, st>>>(S.C, W.pairsSorted, W.newLo, flagsArr, S.P.fresh);
-        size_t tb = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tb, flagsArr, scanArr, (int)nOld, st);
-        if (ensureCub(S, tb)) return WG_ERR_CUDA;
-        tb = W.cubBytes;
-        WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, flagsArr, scanArr, (int)nOld, st));
-        int32_t last[2];
-        WG_CUDA_TRY(cudaMemcpyAsync(&last[0], flagsArr + nOld - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        WG_CUDA_TRY(cudaMemcpyAsync(&last[1], scanArr + nOld - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        WG_CUDA_TRY(cudaStreamSynchronize(st));
-        nOrph = (int64_t)last[0] + last[1];
-        if (nOrph > 0) {
-            if (nOrph > W.orphCap) {
-                int64_t c1 = W.orphCap, c2 = W.orphCap;
-                W.orphKey = grow(S, W.orphKey, c1, nOrph);
-                W.orphSrc = grow(S, W.orphSrc, c2, nOrph);
-                W.orphCap = c1;
-                if (!W.orphKey || !W.orphSrc) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+    // W.pairs takes the sorted pairs back as contact keys
+    const uint64_t* const nk = W.pairs;
+    k_unpack_keys<<<(unsigned)((nNew + 1 + BS - 1) / BS), BS, 0, st>>>(W.pairsSorted, nNew, idBits, (int)S.nPar, W.pairs, W.newLo);
+    if (nOld > 0 && (!W.oldLoValid || S.contactsReplaced))
+        k_lo_bounds<<<(unsigned)((nOld + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, nOld, (int)S.nPar, W.oldLo);
+    S.contactsReplaced = false;
+    bool lookForOrphans = false;
+    for (int k = 0; k < K; k++) {
+        const wg_config& c = K > 1 ? S.cfgs[k] : S.cfg;
+        lookForOrphans = lookForOrphans || !((K > 1 ? S.hPars[k] : S.hPar).verletDist > 0) || (c.law == 0 && c.no_break);
+    }
+    bool law0 = S.cfg.law == 0;
+    for (const wg_config& c : S.cfgs) law0 = law0 || c.law == 0;
+    for (;;) {
+        int64_t nOrph = 0;
+        if (nOld > 0 && lookForOrphans) {
+            W.orph = grow(S, W.orph, W.mergeCap, std::max<int64_t>(nOld, 1) * 2 + 2);
+            if (!W.orph) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+            int32_t* flagsArr = W.orph;
+            int32_t* scanArr = W.orph + (std::max<int64_t>(nOld, 1) + 1);
+            k_mark_orphans<<<(unsigned)((nOld + BS - 1) / BS), BS, 0, st>>>(S.C, nk, W.newLo, flagsArr, S.P.fresh);
+            size_t tb = 0;
+            cub::DeviceScan::ExclusiveSum(nullptr, tb, flagsArr, scanArr, (int)nOld, st);
+            if (ensureCub(S, tb)) return WG_ERR_CUDA;
+            tb = W.cubBytes;
+            WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, flagsArr, scanArr, (int)nOld, st));
+            int32_t last[2];
+            WG_CUDA_TRY(cudaMemcpyAsync(&last[0], flagsArr + nOld - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+            WG_CUDA_TRY(cudaMemcpyAsync(&last[1], scanArr + nOld - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+            WG_CUDA_TRY(cudaStreamSynchronize(st));
+            nOrph = (int64_t)last[0] + last[1];
+            if (nOrph > 0) {
+                if (nOrph > W.orphCap) {
+                    int64_t c1 = W.orphCap, c2 = W.orphCap;
+                    W.orphKey = grow(S, W.orphKey, c1, nOrph);
+                    W.orphSrc = grow(S, W.orphSrc, c2, nOrph);
+                    W.orphCap = c1;
+                    if (!W.orphKey || !W.orphSrc) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+                }
+                k_compact_orphans<<<(unsigned)((nOld + BS - 1) / BS), BS, 0, st>>>(S.C, flagsArr, scanArr, W.orphKey, W.orphSrc);
             }
-            k_compact_orphans<<<(unsigned)((nOld + BS - 1) / BS), BS, 0, st>>>(S.C, flagsArr, scanArr, W.orphKey, W.orphSrc);
         }
-    }
-    (void)capTmp;
-    const int64_t nOut = nNew + nOrph;
-    int r = S.ensureContactCapacity(nOut);
-    if (r) return r;
-    W.src = grow(S, W.src, W.srcCap, std::max<int64_t>(nOut, 1));
-    if (!W.src) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
-    S.Cb.n = nOut;
-    if (peri) {
-        W.newCd = grow(S, W.newCd, W.newCdCap, std::max<int64_t>(nOut, 1));
-        if (!W.newCd) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
-    }
-    if (nNew > 0)
-        k_place_new<<<(unsigned)((nNew + BS - 1) / BS), BS, 0, st>>>(W.pairsSorted, nNew, W.orphKey, nOrph, S.C.key,
-                                                                    nOld > 0 ? W.oldLo : nullptr, S.Cb.key, W.src,
-                                                                    peri ? W.pairCdSorted : nullptr, W.newCd, S.P.fresh);
-    if (nOrph > 0)
-        k_place_orph<<<(unsigned)((nOrph + BS - 1) / BS), BS, 0, st>>>(W.pairsSorted, nNew, W.orphKey, W.orphSrc, nOrph, S.Cb.key,
-                                                                      W.src);
-    if (nOut > 0) k_gather<<<(unsigned)((nOut + BS - 1) / BS), BS, 0, st>>>(S.C, S.Cb, W.src, S.P, S.dStep, peri ? W.newCd : nullptr);
-    std::swap(S.C, S.Cb);
-    if (nOut > 0 && !S.cfg.periodic)
-        k_dormant<<<(unsigned)((nOut + BS - 1) / BS), BS, 0, st>>>(S.C, S.N, S.P, S.dPar);
-    // 6. CSR incidence over the active contacts
-    const int64_t n = S.C.n;
-    if (W.hiCap < std::max<int64_t>(n, 1)) {
-        if (W.hiKeys) {
-            S.dfree(W.hiKeys); S.dfree(W.hiKeysSorted); S.dfree(W.hiVals); S.dfree(S.I.hiList);
-            S.dfree(S.I.slotLo); S.dfree(S.I.slotHi); S.dfree(W.act); S.dfree(W.actReal); S.dfree(S.I.work);
+        const int64_t n = nNew + nOrph;
+        int r = S.ensureContactCapacity(n);
+        if (r) return r;
+        W.src = grow(S, W.src, W.srcCap, std::max<int64_t>(n, 1));
+        if (!W.src) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+        S.Cb.n = n;
+        if (peri) {
+            W.newCd = grow(S, W.newCd, W.newCdCap, std::max<int64_t>(n, 1));
+            if (!W.newCd) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
         }
-        W.hiCap = std::max<int64_t>(n, 1) * 3 / 2 + 1024;
-        W.hiKeys = (uint32_t*)S.dalloc(sizeof(uint32_t) * W.hiCap);
-        W.hiKeysSorted = (uint32_t*)S.dalloc(sizeof(uint32_t) * W.hiCap);
-        W.hiVals = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-        S.I.hiList = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-        S.I.slotLo = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-        S.I.slotHi = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-        W.act = (uint64_t*)S.dalloc(sizeof(uint64_t) * (W.hiCap + 1));
-        W.actReal = S.prec == WG_PREC_FP64 ? (uint64_t*)S.dalloc(sizeof(uint64_t) * (W.hiCap + 1)) : nullptr;
-        S.I.work = (int4*)S.dalloc(sizeof(int4) * W.hiCap);
-        if (!S.I.slotHi || !W.act || !S.I.work || (S.prec == WG_PREC_FP64 && !W.actReal)) return S.fail(WG_ERR_CUDA, "out of device memory (incidence)");
-    }
-    uint64_t tot = 0, totReal = 0;
-    {
-        auto scan = [&](uint32_t real, uint64_t* out, uint64_t* total) -> int {
+        const unsigned gn = (unsigned)((n + BS - 1) / BS);
+        const int64_t places = std::max<int64_t>(nNew, lookForOrphans ? 0 : nOld);
+        if (places > 0)
+            k_place_new<<<(unsigned)((places + BS - 1) / BS), BS, 0, st>>>(nk, nNew, W.orphKey, nOrph, S.C, W.oldLo, S.Cb.key, W.src,
+                                                                          peri ? W.pairCdSorted : nullptr, W.newCd, S.P.fresh,
+                                                                          lookForOrphans ? nullptr : W.tot);
+        if (nOrph > 0)
+            k_place_orph<<<(unsigned)((nOrph + BS - 1) / BS), BS, 0, st>>>(nk, nNew, W.orphKey, W.orphSrc, nOrph, S.Cb.key, W.src);
+        if (n > 0) k_gather<<<gn, BS, 0, st>>>(S.C, S.Cb, W.src, S.N, S.P, S.dPar, S.dStep, peri ? W.newCd : nullptr, peri ? 1 : 0,
+                                             packedState ? 1 : 0);
+        std::swap(S.C, S.Cb);
+        if (nOrph > 0)  // the first index of every lo id in the merged set; without orphans that of the new pairs
+            k_lo_bounds<<<(unsigned)((n + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, n, (int)S.nPar, W.newLo);
+        // 6. CSR incidence over the active contacts. The host does not know their number yet: what is sized by
+        // it is sized for all contacts.
+        if (W.hiCap < std::max<int64_t>(n, 1)) {
+            if (W.hiKeys) {
+                S.dfree(W.hiKeys); S.dfree(W.hiKeysSorted); S.dfree(W.hiVals); S.dfree(S.I.hiList);
+                S.dfree(S.I.slotLo); S.dfree(S.I.slotHi); S.dfree(W.act); S.dfree(W.actReal); S.dfree(S.I.work);
+            }
+            W.hiCap = std::max<int64_t>(n, 1) * 3 / 2 + 1024;
+            W.hiKeys = (uint32_t*)S.dalloc(sizeof(uint32_t) * W.hiCap);
+            W.hiKeysSorted = (uint32_t*)S.dalloc(sizeof(uint32_t) * W.hiCap);
+            W.hiVals = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
+            S.I.hiList = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
+            S.I.slotLo = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
+            S.I.slotHi = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
+            W.act = (uint64_t*)S.dalloc(sizeof(uint64_t) * (W.hiCap + 1));
+            // real contacts first: FP64 mode, and periodic scenes (see k_slots)
+            W.actReal = S.prec == WG_PREC_FP64 || peri ? (uint64_t*)S.dalloc(sizeof(uint64_t) * (W.hiCap + 1)) : nullptr;
+            S.I.work = (int4*)S.dalloc(sizeof(int4) * W.hiCap);
+            if (!S.I.slotHi || !W.act || !S.I.work || ((S.prec == WG_PREC_FP64 || peri) && !W.actReal))
+                return S.fail(WG_ERR_CUDA, "out of device memory (incidence)");
+        }
+        auto scan = [&](uint32_t real, uint64_t* out) -> int {
             const auto in = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), WorkClass{S.C.flags, S.C.cdist, n, real});
             size_t tb = 0;
             cub::DeviceScan::ExclusiveSum(nullptr, tb, in, out, (int)(n + 1), st);
             if (ensureCub(S, tb)) return WG_ERR_CUDA;
             tb = W.cubBytes;
             WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, in, out, (int)(n + 1), st));
-            WG_CUDA_TRY(cudaMemcpyAsync(total, out + n, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
             return 0;
         };
-        int q = scan(0, W.act, &tot);
-        if (q) return q;
-        if (W.actReal) {
-            q = scan(C_REAL, W.actReal, &totReal);
-            if (q) return q;
+        r = scan(0, W.act);
+        if (!r && W.actReal) r = scan(C_REAL, W.actReal);
+        if (r) return r;
+        const uint64_t* const act = W.act + n;  // the totals
+        k_lo_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.newLo, (int)S.nPar, W.act, S.I.loStart);
+        if (S.I.endCap < 2 * std::max<int64_t>(n, 1)) {
+            if (S.I.endA) { S.dfree(S.I.endA); S.dfree(S.I.endB); }
+            if (S.I.endAf) { S.dfree(S.I.endAf); S.dfree(S.I.endBf); }
+            S.I.endA = nullptr; S.I.endB = nullptr; S.I.endAf = nullptr; S.I.endBf = nullptr;
+            S.I.endCap = 2 * std::max<int64_t>(n, 1) * 5 / 4 + 2048;
+            if (S.prec == WG_PREC_FP32) {
+                S.I.endAf = (float4*)S.dalloc(sizeof(float4) * S.I.endCap);
+                S.I.endBf = (float2*)S.dalloc(sizeof(float2) * S.I.endCap);
+                if (!S.I.endAf || !S.I.endBf) return S.fail(WG_ERR_CUDA, "out of device memory (contact ends)");
+            } else {
+                S.I.endA = (double4_32a*)S.dalloc(sizeof(double4_32a) * S.I.endCap);
+                S.I.endB = (double2*)S.dalloc(sizeof(double2) * S.I.endCap);
+                if (!S.I.endA || !S.I.endB) return S.fail(WG_ERR_CUDA, "out of device memory (contact ends)");
+            }
         }
+        int hiBits = 1;  // bits of the largest hi key, nPar
+        while ((int64_t(1) << hiBits) <= S.nPar) hiBits++;
+        if (n > 0) {
+            k_hi_keys<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, n, (uint32_t)S.nPar, W.hiKeys, W.hiVals);
+            size_t tb = 0;
+            cub::DeviceRadixSort::SortPairs(nullptr, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiBits, st);
+            if (ensureCub(S, tb)) return WG_ERR_CUDA;
+            tb = W.cubBytes;
+            WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiBits, st));
+        }
+        k_hi_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.hiKeysSorted, n, (int)S.nPar, S.I.hiStart);
+        if (n > 0) {
+            k_slots<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, S.I);
+            k_zero_ends<<<(unsigned)((2 * n + BS - 1) / BS), BS, 0, st>>>(S.I, act);
+        }
+        // FP32-force mode, aperiodic scenes: the sphere-sphere contacts' state in work-list order
+        if (packed && n > 0) {
+            DevPackedSS& Q = W.Kb;
+            W.packIdxB = grow(S, W.packIdxB, W.packIdxCapB, n);
+            if (!W.packIdxB) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
+            if (Q.cap < n) {
+                S.dfree(Q.item); S.dfree(Q.flags);
+                for (int q = 0; q < CF_NCOL; q++) S.dfree(Q.col[q]);
+                S.dfree(Q.ft[0]); S.dfree(Q.ft[1]);
+                Q = DevPackedSS{};
+                Q.cap = n * 5 / 4 + 4096;
+                Q.item = (int4*)S.dalloc(sizeof(int4) * Q.cap);
+                Q.flags = (uint32_t*)S.dalloc(sizeof(uint32_t) * Q.cap);
+                bool ok = Q.item && Q.flags;
+                for (int q = 0; q < CF_NCOL; q++) {
+                    Q.col[q] = (float*)S.dalloc(sizeof(float) * Q.cap);
+                    ok = ok && Q.col[q];
+                }
+                // the IdealElPl shear force (a serving slot may take a job with that law at any time)
+                Q.ft[0] = (double*)S.dalloc(sizeof(double) * Q.cap);
+                Q.ft[1] = (double*)S.dalloc(sizeof(double) * Q.cap);
+                ok = ok && Q.ft[0] && Q.ft[1];
+                if (!ok) {
+                    Q.cap = 0;
+                    return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
+                }
+            }
+            Q.ftLive = law0;
+            launch_pack_ss(st, S.C, S.I, S.P, Kold, Q, packedState ? W.packIdx : nullptr, W.src, W.packIdxB, act, n);
+        }
+        k_heavy<<<(unsigned)((S.nPar + BS - 1) / BS), BS, 0, st>>>(S.I, S.P, S.N.flags, kHeavyThreshold, W.tot, W.act, W.actReal, n);
+        WG_CUDA_TRY(cudaMemcpyAsync(W.hTot, W.tot, sizeof(CollideTotals), cudaMemcpyDeviceToHost, st));
         WG_CUDA_TRY(cudaStreamSynchronize(st));
-    }
-    const int64_t nAct = (int64_t)(uint32_t)tot, nSS = (int64_t)(tot >> 32);
-    k_lo_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, n, (int)S.nPar, W.act, S.I.loStart);
-    if (S.I.endCap < 2 * std::max<int64_t>(nAct, 1)) {
-        if (S.I.endA) { S.dfree(S.I.endA); S.dfree(S.I.endB); }
-        if (S.I.endAf) { S.dfree(S.I.endAf); S.dfree(S.I.endBf); }
-        S.I.endA = nullptr; S.I.endB = nullptr; S.I.endAf = nullptr; S.I.endBf = nullptr;
-        S.I.endCap = 2 * std::max<int64_t>(nAct, 1) * 3 / 2 + 2048;
-        if (S.prec == WG_PREC_FP32) {
-            S.I.endAf = (float4*)S.dalloc(sizeof(float4) * S.I.endCap);
-            S.I.endBf = (float2*)S.dalloc(sizeof(float2) * S.I.endCap);
-            if (!S.I.endAf || !S.I.endBf) return S.fail(WG_ERR_CUDA, "out of device memory (contact ends)");
-        } else {
-            S.I.endA = (double4_32a*)S.dalloc(sizeof(double4_32a) * S.I.endCap);
-            S.I.endB = (double2*)S.dalloc(sizeof(double2) * S.I.endCap);
-            if (!S.I.endA || !S.I.endB) return S.fail(WG_ERR_CUDA, "out of device memory (contact ends)");
+        const CollideTotals& T = *W.hTot;
+        if (!lookForOrphans && T.real != T.kept) {
+            // again, with the real contacts that have no overlap any more: the old set is in the spare arrays
+            lookForOrphans = true;
+            std::swap(S.C, S.Cb);
+            WG_CUDA_TRY(cudaMemsetAsync(&W.tot->heavy, 0, 2 * sizeof(int32_t), st));
+            continue;
         }
-    }
-    int hiBits = 1;  // bits of the largest hi key, nPar
-    while ((int64_t(1) << hiBits) <= S.nPar) hiBits++;
-    if (n > 0) {
-        k_hi_keys<<<(unsigned)((n + BS - 1) / BS), BS, 0, st>>>(S.C.key, S.C.flags, n, (uint32_t)S.nPar, W.hiKeys, W.hiVals);
-        size_t tb = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiBits, st);
-        if (ensureCub(S, tb)) return WG_ERR_CUDA;
-        tb = W.cubBytes;
-        WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiBits, st));
-    }
-    k_hi_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.hiKeysSorted, n, (int)S.nPar, S.I.hiStart);
-    if (n > 0) k_slots<<<(unsigned)((n + BS - 1) / BS), BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, tot, totReal,
-                                                                           S.I);
-    S.I.nAct = nAct;
-    S.nMixed = nAct - nSS;
-    // every end starts without a contribution; the contact kernel fills the real ones this step
-    const int64_t ne = 2 * std::max<int64_t>(nAct, 1);
-    if (S.prec == WG_PREC_FP32) {
-        WG_CUDA_TRY(cudaMemsetAsync(S.I.endAf, 0, sizeof(float4) * ne, st));
-        WG_CUDA_TRY(cudaMemsetAsync(S.I.endBf, 0, sizeof(float2) * ne, st));
-    } else {
-        WG_CUDA_TRY(cudaMemsetAsync(S.I.endA, 0, sizeof(double4_32a) * ne, st));
-        WG_CUDA_TRY(cudaMemsetAsync(S.I.endB, 0, sizeof(double2) * ne, st));
-    }
-    // FP32-force mode, aperiodic scenes: the sphere-sphere contacts' state in work-list order
-    if (S.prec == WG_PREC_FP32 && !S.cfg.periodic && nSS > 0) {
-        DevPackedSS& K = S.K;
-        if (K.cap < nSS) {
-            S.dfree(K.item); S.dfree(K.flags);
-            for (int q = 0; q < CF_NCOL; q++) S.dfree(K.col[q]);
-            S.dfree(K.ft[0]); S.dfree(K.ft[1]);
-            K = DevPackedSS{};
-            K.cap = nSS * 5 / 4 + 4096;
-            K.item = (int4*)S.dalloc(sizeof(int4) * K.cap);
-            K.flags = (uint32_t*)S.dalloc(sizeof(uint32_t) * K.cap);
-            bool ok = K.item && K.flags;
-            for (int q = 0; q < CF_NCOL; q++) {
-                K.col[q] = (float*)S.dalloc(sizeof(float) * K.cap);
-                ok = ok && K.col[q];
-            }
-            // the IdealElPl shear force (a serving slot may take a job with that law at any time)
-            K.ft[0] = (double*)S.dalloc(sizeof(double) * K.cap);
-            K.ft[1] = (double*)S.dalloc(sizeof(double) * K.cap);
-            ok = ok && K.ft[0] && K.ft[1];
-            if (!ok) {
-                K.cap = 0;
-                return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
-            }
+        const int64_t nAct = (int64_t)(uint32_t)T.act, nSS = (int64_t)(T.act >> 32);
+        S.I.nAct = nAct;
+        S.nMixed = nAct - nSS;
+        if (packed && n > 0) {
+            std::swap(S.K, W.Kb);
+            std::swap(W.packIdx, W.packIdxB);
+            std::swap(W.packIdxCap, W.packIdxCapB);
+            W.packIdxValid = true;
         }
-        K.n = nSS;
-        bool law0 = S.cfg.law == 0;
-        for (const wg_config& c : S.cfgs) law0 = law0 || c.law == 0;
-        K.ftLive = law0;
-        launch_pack_ss(st, S.C, S.I, S.P, K, S.nMixed);
+        S.K.n = packed ? nSS : 0;
+        S.packDirty = packedState && nSS > 0;  // the contact arrays hold no state of those contacts then
+        S.I.nHeavy = S.cfg.apply_forces ? T.heavy : 0;
+        S.I.nHeavyFree = S.cfg.apply_forces ? T.heavyFree : 0;
+        break;
     }
-    S.packDirty = false;
-    // heavy particles
-    if (!W.heavyCount) {
-        W.heavyCount = (int32_t*)S.dalloc(sizeof(int32_t) * 3);
-        WG_CUDA_TRY(cudaMallocHost(&W.hHeavy, sizeof(int32_t) * 3));
-    }
-    WG_CUDA_TRY(cudaMemsetAsync(W.heavyCount, 0, sizeof(int32_t) * 3, st));
-    k_heavy<<<(unsigned)((S.nPar + BS - 1) / BS), BS, 0, st>>>(S.I, S.P, S.N.flags, kHeavyThreshold, W.heavyCount);
-    WG_CUDA_TRY(cudaMemcpyAsync(W.hHeavy, W.heavyCount, sizeof(int32_t) * 3, cudaMemcpyDeviceToHost, st));
-    WG_CUDA_TRY(cudaStreamSynchronize(st));
-    S.I.nHeavy = S.cfg.apply_forces ? W.hHeavy[0] : 0;
-    S.I.nHeavyFree = S.cfg.apply_forces ? W.hHeavy[1] : 0;
+    std::swap(W.newLo, W.oldLo);
+    std::swap(W.newLoCap, W.oldLoCap);
+    W.oldLoValid = true;
     if (S.P.fresh) WG_CUDA_TRY(cudaMemsetAsync(S.P.fresh, 0, S.nPar, st));
     WG_CUDA_TRY(cudaGetLastError());
     S.nFullRuns++;
@@ -1566,9 +1671,7 @@ int collide_full_run(Sim& S) {
 
 void collide_free(Sim& S) {
     if (!S.cw) return;
-    if (S.cw->hRed) cudaFreeHost(S.cw->hRed);
-    if (S.cw->hCounter) cudaFreeHost(S.cw->hCounter);
-    if (S.cw->hHeavy) cudaFreeHost(S.cw->hHeavy);
+    if (S.cw->hTot) cudaFreeHost(S.cw->hTot);
     delete S.cw;
     S.cw = nullptr;
 }

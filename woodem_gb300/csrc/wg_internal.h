@@ -299,10 +299,15 @@ bool launch_contact_fp32(cudaStream_t st, const SideStream& side, const DevNodes
                          const DevIncidence& I, const DevPackedSS& K, const double4_32a* mats, const ScenePar* sp,
                          long long* dStep, int* dFlags, int64_t nMixed, bool periodic, bool anyLaw0, bool prepFacets,
                          int block = 256, const EnergyCols* energy = nullptr);
-// copy the packed sphere-sphere state from (pack) / back to (unpack) the contact arrays
-void launch_pack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevParticles& P, const DevPackedSS& K,
-                    int64_t nMixed);
-void launch_unpack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevPackedSS& K, int64_t nMixed);
+// pack: the packed state K of a new contact set (whose active contacts are counted in the low half of *act
+// on the device, the plain ones in its high half, at most `most`), in tiles with the real ones first
+// (the work list is put in that order too). oldIdx null: from the contact arrays; else from the old packed
+// state Kold, where the contact that contact c continues, src[c], is at oldIdx[src[c]]. idx[c] takes c's place.
+void launch_pack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevParticles& P, const DevPackedSS& Kold,
+                    const DevPackedSS& K, const int32_t* oldIdx, const int32_t* src, int32_t* idx, const uint64_t* act, int64_t most);
+// unpack: the packed state (flagsOnly: its flags alone) back into the contact arrays
+void launch_unpack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevPackedSS& K, int64_t nMixed,
+                      bool flagsOnly = false);
 void launch_forces32(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevIncidence& I, const NodeConst32* nc,
                      const ScenePar* sp, const int* dFlags, bool perStep);
 // FP32-force mode: P.prep from the current vertex positions (before the contact kernels of a step;
@@ -311,10 +316,11 @@ void launch_facet_prep(cudaStream_t st, const DevNodes& N, const DevParticles& P
 
 // ------------------------------------------------------------------ broad phase (wg_collide.cu)
 struct Grid {
-    double ox, oy, oz, h;
+    double ox, oy, oz, h, rh;  // rh = 1/h
     int32_t nx, ny, nz;
     int64_t ncell;
     int64_t base;  // first cell key of this grid (a batch of scenes has one grid per scene)
+    int32_t exact; // periodic: a box reaches about half the cell (see k_pairs_ss_peri)
 };
 struct CollideWork;  // scratch owned by the simulation
 struct Sim;
@@ -398,6 +404,7 @@ struct Sim {
     std::vector<ScenePar> hPars;
     std::vector<double> sceneTime0;    // Scene.time of each scene at upload
     std::vector<uint8_t> hParked;      // serving slots: particle holds no job (left out of the collider)
+    bool contactsReplaced = false;     // the contact arrays were set from outside since the last full run
     bool listsDirty = true;            // particle lists of the collider to be rebuilt at the next full run
     bool forceFull = false;            // next step starts with a full collider run
     int* dFlags = nullptr;   // the step-loop flags (FL_*) and the counters behind them (CTL_BYTES)

@@ -795,29 +795,67 @@ __global__ void __launch_bounds__(256, MINB) k_contact_ss32p(DevNodes N, DevPart
     stepTicket(dFlags, dStep, ticketTotal);
 }
 
-__global__ void k_pack_ss(DevContacts C, DevIncidence I, DevParticles P, DevPackedSS K, int64_t nm, int copyFt) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= K.n) return;
-    const int4 wk = I.work[nm + j];
-    const int64_t c = wk.x;
-    const uint32_t fl = C.flags[c];
-    const int32_t sl = I.slotLo[c], sh = I.slotHi[c];
+constexpr int kPackTile = 1024;
+// One tile of the plain active contacts of a new set per block: its real contacts first, then the others,
+// both in contact order, so that a warp of the contact kernel holds one kind and skips state, velocities and
+// law for the other, while the particles it gathers are still those of its neighbours.
+__global__ void __launch_bounds__(kPackTile) k_pack_ss(DevContacts C, DevIncidence I, DevParticles P, DevPackedSS Kold, DevPackedSS K,
+                                                       const int32_t* __restrict__ oldIdx, const int32_t* __restrict__ src,
+                                                       int32_t* __restrict__ idx, const uint64_t* __restrict__ act, int copyFt) {
+    __shared__ int sh[kPackTile / 32];
+    const uint32_t all = (uint32_t)*act, plain = (uint32_t)(*act >> 32);
+    const int64_t j0 = (int64_t)blockIdx.x * kPackTile, nm = all - plain;
+    if (j0 >= plain) return;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const bool in = j0 + t < plain;
+    int4 wk = make_int4(0, 0, 0, 0);
+    uint32_t fl = 0;
+    if (in) {
+        wk = I.work[nm + j0 + t];
+        fl = C.flags[wk.x];
+    }
+    const bool real = fl & C_REAL;
+    const unsigned m = __ballot_sync(0xffffffffu, real);
+    if (lane == 0) sh[warp] = __popc(m);
+    __syncthreads();
+    int before = __popc(m & ((1u << lane) - 1u)), total = 0;  // real ones before this contact, and in the tile
+    for (int w = 0; w < kPackTile / 32; w++) {
+        if (w < warp) before += sh[w];
+        total += sh[w];
+    }
+    if (!in) return;
+    const int64_t j = j0 + (real ? before : total + (t - before)), c = wk.x;
+    const int32_t sl = I.slotLo[c], shi = I.slotHi[c];
     const bool swap = fl & C_SWAP;
-    K.item[j] = make_int4(wk.y, wk.z, swap ? sh : sl, swap ? sl : sh);
+    I.work[nm + j] = wk;
+    idx[c] = (int32_t)j;
+    K.item[j] = make_int4(wk.y, wk.z, swap ? shi : sl, swap ? sl : shi);
     K.flags[j] = fl | ((uint32_t)sceneOfP(P, wk.z) << 8);
+    if (!real) return;  // no kernel reads the state of a contact that is not
+    if (oldIdx) {
+        const int64_t o = oldIdx[src[c]];
 #pragma unroll
-    for (int q = 0; q < CF_NCOL; q++) K.col[q][j] = C.fcol[q][c];
-    if (copyFt) {
-        K.ft[0][j] = C.col[CC_FT1][c];
-        K.ft[1][j] = C.col[CC_FT2][c];
+        for (int q = 0; q < CF_NCOL; q++) K.col[q][j] = Kold.col[q][o];
+        if (copyFt) {
+            K.ft[0][j] = Kold.ft[0][o];
+            K.ft[1][j] = Kold.ft[1][o];
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < CF_NCOL; q++) K.col[q][j] = C.fcol[q][c];
+        if (copyFt) {
+            K.ft[0][j] = C.col[CC_FT1][c];
+            K.ft[1][j] = C.col[CC_FT2][c];
+        }
     }
 }
 
-__global__ void k_unpack_ss(DevContacts C, DevIncidence I, DevPackedSS K, int64_t nm, int copyFt) {
+__global__ void k_unpack_ss(DevContacts C, DevIncidence I, DevPackedSS K, int64_t nm, int copyFt, int flagsOnly) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= K.n) return;
     const int64_t c = I.work[nm + j].x;
     C.flags[c] = K.flags[j] & 0xffu;
+    if (flagsOnly) return;
 #pragma unroll
     for (int q = 0; q < CF_NCOL; q++) C.fcol[q][c] = K.col[q][j];
     if (copyFt) {
@@ -826,12 +864,14 @@ __global__ void k_unpack_ss(DevContacts C, DevIncidence I, DevPackedSS K, int64_
     }
 }
 
-void launch_pack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevParticles& P, const DevPackedSS& K,
-                    int64_t nMixed) {
-    if (K.n > 0) k_pack_ss<<<(unsigned)((K.n + 255) / 256), 256, 0, st>>>(C, I, P, K, nMixed, K.ftLive ? 1 : 0);
+void launch_pack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevParticles& P, const DevPackedSS& Kold,
+                    const DevPackedSS& K, const int32_t* oldIdx, const int32_t* src, int32_t* idx, const uint64_t* act, int64_t most) {
+    if (most > 0)
+        k_pack_ss<<<(unsigned)((most + kPackTile - 1) / kPackTile), kPackTile, 0, st>>>(C, I, P, Kold, K, oldIdx, src, idx, act,
+                                                                                       K.ftLive ? 1 : 0);
 }
-void launch_unpack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevPackedSS& K, int64_t nMixed) {
-    if (K.n > 0) k_unpack_ss<<<(unsigned)((K.n + 255) / 256), 256, 0, st>>>(C, I, K, nMixed, K.ftLive ? 1 : 0);
+void launch_unpack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevPackedSS& K, int64_t nMixed, bool flagsOnly) {
+    if (K.n > 0) k_unpack_ss<<<(unsigned)((K.n + 255) / 256), 256, 0, st>>>(C, I, K, nMixed, K.ftLive ? 1 : 0, flagsOnly ? 1 : 0);
 }
 
 // FacetPrep of every facet (Facet.cpp:240-246: normal; CompUtils.cpp:92-110: the barycentric
