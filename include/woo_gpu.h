@@ -149,12 +149,11 @@ int wg_set_config(wg_scene* s, const wg_config* c);
    batched. Replaces wg_set_config; call before the first run. */
 int wg_set_scenes(wg_scene* s, int32_t n_scenes, const wg_config* cfgs, const int64_t* particle_start);
 /* Launch shape (no counterpart in the reference): threads per block of the contact kernels
-   (0 = default, 64, 128, 256; -256: the FP32 sphere-sphere contacts through a resident grid whose
-   threads prefetch their next contact), steps
-   queued per host check of the collider request (1..1024), and flags: WG_LAUNCH_GRAPH replays each
-   such chunk of steps as one CUDA graph, WG_LAUNCH_SERIAL runs the facet/wall contacts before the
-   sphere-sphere ones instead of beside them on a second stream. Results do not depend on these;
-   only the speed does. */
+   (0 = default, 64, 128, 256; -256: the FP32 contacts through a resident grid whose threads prefetch
+   their next contact, as by default), steps queued per host check of the collider request (1..1024), and
+   flags: WG_LAUNCH_GRAPH replays each such chunk of steps as one CUDA graph, WG_LAUNCH_SERIAL, with a
+   positive block size, runs the facet/wall contacts before the sphere-sphere ones instead of beside them
+   on a second stream. Results do not depend on these; only the speed does. */
 #define WG_LAUNCH_GRAPH 1
 #define WG_LAUNCH_SERIAL 2
 int wg_set_launch(wg_scene* s, int32_t contact_block, int32_t chunk_steps, int32_t launch_flags);

@@ -9,8 +9,8 @@
 // (ContactContainer::removePending, ContactContainer.hpp:78-93). This file computes exactly
 // that set on the GPU:
 //   1. Bo1 functors + verlet enlargement per particle            (k_aabb)
-//   2. spheres bucketed into a uniform grid whose cell is at least the largest sphere box,
-//      keyed by the cell of the box minimum and radix-sorted      (k_cellkey + cub radix sort)
+//   2. spheres bucketed into a uniform grid whose cell is at least the largest sphere box, by a counting
+//      sort on the cell of the box minimum                        (k_make_grids, k_cellkey .. )
 //   3. half-shell sweep over the sorted cells: every candidate pair is tested once with the
 //      reference's closed-interval comparisons                   (k_pairs_ss)
 //   4. facets query the cells their box covers; walls (infinite boxes) test every sphere

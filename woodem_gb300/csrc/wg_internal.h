@@ -245,8 +245,6 @@ void launch_leapfrog(cudaStream_t st, const DevNodes& N, const DevParticles& P, 
 void launch_contact_fp64(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C,
                          const DevIncidence& I, const double4_32a* mats, const ScenePar* sp, const long long* dStep, int* dFlags,
                          bool periodic, int block = 0, const EnergyCols* energy = nullptr);
-// perStep: only the heavy particles with a free DOF (guarded by the flags), before Leapfrog;
-// otherwise every particle's DemData.force/torque (reporting at the end of a run).
 // Up to `steps` steps in one cooperative launch (small scenes; no energy tracking, no heavy particle with a
 // free DOF, facets static). It leaves the flags and the step counter as that many launches of the
 // kernels above would: a full run due ends it before that step's contacts. bar: a word that is zero
@@ -259,6 +257,8 @@ int launch_steps32(cudaStream_t st, const DevNodes& N, const DevParticles& P, co
                    const DevPackedSS& K, const NodeConst32* nc, const double4_32a* mats, const ScenePar* sp, bool periodic,
                    long long* dStep, int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool anyLaw0, int fromEnds,
                    int steps);
+// perStep: only the heavy particles with a free DOF (guarded by the flags), before Leapfrog;
+// otherwise every particle's DemData.force/torque (reporting at the end of a run).
 void launch_forces(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevIncidence& I, const ScenePar* sp,
                    const int* dFlags, bool perStep);
 void launch_advance(cudaStream_t st, long long* dStep, const int* dFlags);
@@ -420,10 +420,11 @@ struct Sim {
     bool fromEnds = false;   // the end slots hold the forces of the last contact loop
     // launch shape (wg_set_launch): threads per block of the contact kernels, steps queued per host
     // check, and whether a chunk of steps is replayed as a CUDA graph
-    int contactBlock = 0;    // 0: default (FP32: the resident-grid sphere-sphere kernel; FP64: by the contacts' number)
+    int contactBlock = 0;    // 0: default (FP32: the resident grid over both ranges; FP64: by the contacts' number)
     int chunkSteps = 32;
+    int64_t lastFullStep = -1, runInterval = 0;  // the last full run's step, and its distance from the one before
     bool useGraph = false;
-    bool concurrentContacts = true;   // facet/wall contacts beside, not before, the sphere-sphere ones
+    bool concurrentContacts = true;   // contactBlock > 0: facet/wall contacts beside, not before, the sphere-sphere ones
     bool facetsStatic = false;        // every facet vertex is fully blocked and at rest: FacetPrep is made once
     cudaGraphExec_t graphExec = nullptr;
     int64_t graphSteps = 0;  // steps in the captured chunk, 0: none valid

@@ -745,6 +745,26 @@ __device__ __forceinline__ void loadSS(SSIn& x, int64_t j, const DevNodes& N, co
     x.wzb = N.wz[x.it.y];
 }
 
+// The same for a contact whose flags are there already: one that is not real needs the two positions
+// alone (its state, the velocities and the angular velocities enter with the frame's update).
+__device__ __forceinline__ void loadSSKnown(SSIn& x, int64_t j, const DevNodes& N, const DevPackedSS& K, int loadFt) {
+    if (x.pf & C_REAL) {
+        const uint32_t pf = x.pf;
+        loadSS(x, j, N, K, loadFt);
+        x.pf = pf;
+        return;
+    }
+    x.ma.ph = N.mir[x.it.x].ph;
+    x.ma.pl = N.mir[x.it.x].pl;
+    x.mb.ph = N.mir[x.it.y].ph;
+    x.mb.pl = N.mir[x.it.y].pl;
+    x.ft1o = x.ft2o = 0.;
+    x.ma.vh = x.ma.vl = x.mb.vh = x.mb.vl = make_float4(0.f, 0.f, 0.f, 0.f);
+    x.wza = x.wzb = 0.f;
+#pragma unroll
+    for (int q = 0; q < CF_NCOL; q++) x.st[q] = 0.f;
+}
+
 // Sphere-sphere contacts of aperiodic scenes (work items [nMixed, nAct)), one per thread: item,
 // flags and state are read at the contact's position in the work list (coalesced), the two
 // particles' mirror records are gathered; every load is issued before the step guard and the
@@ -769,33 +789,15 @@ __global__ void __launch_bounds__(256, MINB) k_contact_ss32(DevNodes N, DevParti
     ssContact<ENERGY>(x, j, N, P, C, I, K, mats, spp, stepAbs, dFlags, nm, E);
 }
 
-// The same contacts through a resident grid, each thread walking the range with the grid's
-// stride: the next contact's packed item is loaded while the current contact's state and mirror
-// records are in flight, so each contact waits for one memory round trip instead of two.
-template <int MINB, bool ENERGY>
-__global__ void __launch_bounds__(256, MINB) k_contact_ss32p(DevNodes N, DevParticles P, DevContacts C, DevIncidence I, DevPackedSS K,
-                                                             const double4_32a* __restrict__ mats, const ScenePar* __restrict__ spp,
-                                                             long long* __restrict__ dStep, int* __restrict__ dFlags, int64_t nm,
-                                                             int haltBlock, int loadFt, int ticketTotal, EnergyCols E) {
-    const long long stepAbs = *dStep;
-    if (dFlags[FL_FULL] || halted(dFlags)) {  // the same for every thread of the grid
-        if (haltBlock && blockIdx.x == 0 && threadIdx.x == 0) dFlags[FL_HALT] = 1;
-        return;
-    }
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int4 next = j < K.n ? K.item[j] : make_int4(0, 0, 0, 0);
-    for (; j < K.n; j += stride) {
-        SSIn x;
-        x.it = next;
-        if (j + stride < K.n) next = K.item[j + stride];
-        loadSS(x, j, N, K, loadFt);
-        ssContact<ENERGY>(x, j, N, P, C, I, K, mats, spp, stepAbs, dFlags, nm, E);
-    }
-    stepTicket(dFlags, dStep, ticketTotal);
-}
-
+// The first contact of chunk c of 32: the chunks of a tile in an order of the tile's own, so that the warps of
+// a resident grid, whose stride may be a number of whole tiles, meet real and other contacts alike.
 constexpr int kPackTile = 1024;
+__device__ __forceinline__ int64_t packedChunk(int64_t c) {
+    const uint32_t tile = (uint32_t)(c >> 5);
+    return ((int64_t)tile << 10) + (int64_t)((((uint32_t)c + ((tile * 0x9E3779B1u) >> 27)) & 31u) << 5);
+}
+static_assert(kPackTile == 32 * 32, "packedChunk");
+
 // One tile of the plain active contacts of a new set per block: its real contacts first, then the others,
 // both in contact order, so that a warp of the contact kernel holds one kind and skips state, velocities and
 // law for the other, while the particles it gathers are still those of its neighbours.
@@ -1250,29 +1252,80 @@ __global__ void __launch_bounds__(128, 4) k_contact_fp32(DevNodes N, DevParticle
     stepTicket(dFlags, dStep, ticketTotal);
 }
 
-// minimum resident blocks per SM the one-contact-per-thread kernel is compiled for (register budget)
+// minimum resident blocks per SM the sphere-sphere kernels are compiled for (register budget)
 constexpr int kSSMinBlocks = 3;
 
-// sphere-sphere range: block > 0 one contact per thread with that many threads per block;
-// block < 0 the resident-grid kernel with prefetch (256 threads per block)
-// Returns true when the launch also advances the step counter (advance requested and possible).
-// grid of the resident sphere-sphere kernel (block < 0), or 0 for the one-contact-per-thread kernel
-static int ssGrid(const DevPackedSS& K, int block, int blocksPerSM) {
-    return block < 0 ? (int)std::min<int64_t>((K.n + 255) / 256, (int64_t)blocksPerSM * smCount()) : 0;
-}
-template <bool ENERGY>
-static void launchSS(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
-                     const DevPackedSS& K, const double4_32a* mats, const ScenePar* sp, long long* dStep, int* dFlags, int64_t nm,
-                     int halt, int loadFt, int block, int grid, int ticketTotal, const EnergyCols& E) {
-    if (block < 0) {
-        k_contact_ss32p<kSSMinBlocks, ENERGY><<<(unsigned)grid, 256, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, halt, loadFt,
-                                                                              ticketTotal, E);
+// Both ranges of an aperiodic scene in one resident grid, each warp walking chunks of 32 contacts with the
+// grid's stride. The next contact's packed item and flags are loaded while the current one's state and
+// mirror records are in flight, so a contact waits for one memory round trip instead of two. The warps are of
+// one kind, real or not, but for one in a tile (k_pack_ss); those that are not load two positions and leave.
+// A chunk of 32 facet and wall contacts, a long chain of FP64 geometry, takes the place of kMixedRows chunks
+// of packed contacts in the rows that the warps walk: row r < kMixedRows holds the mixed chunks (the same ones,
+// done once) and then packed chunks, every later row packed ones alone.
+// Bound by the latency of the gathered mirror records at the occupancy its registers allow (3 blocks of 256 a
+// SM). 1M drum, both ranges: 0.160 -> 0.125 ms a step; as two kernels on two streams the mixed one, a block of
+// 128 registers a thread on each SM, left room for two blocks of this one beside it instead of three.
+constexpr int kMixedRows = 4;
+template <int MINB>
+__global__ void __launch_bounds__(256, MINB) k_contact_all32(DevNodes N, DevParticles P, DevContacts C, DevIncidence I, DevPackedSS K,
+                                                             const double4_32a* __restrict__ mats, const ScenePar* __restrict__ spp,
+                                                             long long* __restrict__ dStep, int* __restrict__ dFlags, int64_t nm,
+                                                             int loadFt) {
+    const EnergyCols none{};
+    const long long stepAbs = *dStep;
+    if (dFlags[FL_FULL] || halted(dFlags)) {  // the same for every thread of the grid
+        if (blockIdx.x == 0 && threadIdx.x == 0) dFlags[FL_HALT] = 1;
         return;
     }
-    k_contact_ss32<kSSMinBlocks, ENERGY><<<(unsigned)((K.n + block - 1) / block), (unsigned)block, 0, st>>>(
-        N, P, C, I, K, mats, sp, dStep, dFlags, nm, halt, loadFt, E);
+    const int64_t chunks = ((K.n + kPackTile - 1) / kPackTile) * (kPackTile / 32), mixed = (nm + 31) >> 5;
+    const int64_t W = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const int64_t w = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // mixed chunks: an SM's first warps
+    const int64_t m = mixed < W ? mixed : W;                                 // warps that start with one
+    for (int64_t q = w; q < mixed; q += W) {
+        const int64_t rk = 32 * q + lane;
+        if (rk < nm) mixedContact<false, false>(rk, N, P, C, I, mats, spp, stepAbs, dFlags, none);
+    }
+    int64_t c;
+    int row;
+    if (w < m) {
+        row = kMixedRows;
+        c = kMixedRows * (W - m) + w;
+    } else {
+        row = 0;
+        c = w - m;
+    }
+    auto advance = [&]() {  // the chunk of the next row
+        row++;
+        c = row < kMixedRows ? row * (W - m) + (w - m) : kMixedRows * (W - m) + (row - kMixedRows) * W + w;
+    };
+    int64_t j = packedChunk(c) + lane;
+    int4 next = make_int4(0, 0, 0, 0);
+    uint32_t nextPf = 0;
+    if (c < chunks && j < K.n) {
+        next = K.item[j];
+        nextPf = K.flags[j];
+    }
+    while (c < chunks) {
+        const int64_t now = j;
+        SSIn x;
+        x.it = next;
+        x.pf = nextPf;
+        advance();
+        j = packedChunk(c) + lane;
+        if (c < chunks && j < K.n) {
+            next = K.item[j];
+            nextPf = K.flags[j];
+        }
+        if (now >= K.n) continue;
+        loadSSKnown(x, now, N, K, loadFt);
+        ssContact<false>(x, now, N, P, C, I, K, mats, spp, stepAbs, dFlags, nm, none);
+    }
+    stepTicket(dFlags, dStep, gridDim.x);
 }
 
+// block < 0 (never with energy tracking): both ranges by k_contact_all32; block > 0: one packed contact per thread, that many threads a
+// block. Returns true when the launch also advances the step counter.
 template <bool ENERGY>
 static bool contactsFP32(cudaStream_t st, const SideStream& side, const DevNodes& N, const DevParticles& P, const DevContacts& C,
                          const DevIncidence& I, const DevPackedSS& K, const double4_32a* mats, const ScenePar* sp,
@@ -1280,33 +1333,37 @@ static bool contactsFP32(cudaStream_t st, const SideStream& side, const DevNodes
                          int block, const EnergyCols& E) {
     const int64_t nm = periodic ? I.nAct : std::min<int64_t>(nMixed, I.nAct);
     const int64_t ns = periodic ? 0 : K.n;
+    if constexpr (!ENERGY) if (ns > 0 && block < 0) {
+        if (nm > 0 && prepFacets) launch_facet_prep(st, N, P, dFlags);
+        const int64_t want = ((ns + 31) / 32 + (nm + 31) / 32 + 7) / 8;
+        const int g = (int)std::min<int64_t>(want, (int64_t)kSSMinBlocks * smCount());
+        k_contact_all32<kSSMinBlocks><<<(unsigned)g, 256, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, anyLaw0);
+        return true;
+    }
+    const unsigned gS = ns > 0 ? (unsigned)((ns + block - 1) / block) : 0u;
     if (ns > 0 && nm > 0 && side.st) {
-        // the mixed range (facets and walls, FP64 geometry) beside the sphere-sphere range: one block
-        // of 128 threads per SM, and two resident sphere-sphere blocks per SM beside it; the
-        // sphere-sphere launch raises FL_HALT when a full run is due; the last block of either
-        // advances the step counter
+        // the mixed range (facets and walls, FP64 geometry) beside the sphere-sphere range: one block of 128
+        // threads per SM; the sphere-sphere launch raises FL_HALT when a full run is due
         const int gM = (int)std::min<int64_t>((nm + 127) / 128, smCount());
-        const int gS = ssGrid(K, block, kSSMinBlocks - 1);
-        const int total = gS > 0 ? gM + gS : 0;
         cudaEventRecord(side.fork, st);
         cudaStreamWaitEvent(side.st, side.fork, 0);
         if (prepFacets) launch_facet_prep(side.st, N, P, dFlags);
-        k_contact_fp32<false, ENERGY><<<(unsigned)gM, 128, 0, side.st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 0, total, E);
-        launchSS<ENERGY>(st, N, P, C, I, K, mats, sp, dStep, dFlags, nm, 1, anyLaw0, block, gS, total, E);
+        k_contact_fp32<false, ENERGY><<<(unsigned)gM, 128, 0, side.st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 0, 0, E);
+        k_contact_ss32<kSSMinBlocks, ENERGY><<<gS, (unsigned)block, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, 1, anyLaw0, E);
         cudaEventRecord(side.join, side.st);
         cudaStreamWaitEvent(st, side.join, 0);
-        return total > 0;
+        return false;
     }
-    // the first launch also raises FL_HALT when a full run is due (it always runs); the last
-    // kernel of the step advances the step counter
+    // the first launch also raises FL_HALT when a full run is due (it always runs); where it is the step's
+    // last one it advances the step counter
     if (nm > 0 && prepFacets) launch_facet_prep(st, N, P, dFlags);
-    const int gS = ns > 0 ? ssGrid(K, block, kSSMinBlocks) : 0;
     const int gM = (int)std::max<int64_t>(1, std::min<int64_t>((nm + 127) / 128, 4 * smCount()));
-    const int totalM = ns > 0 ? 0 : gM;
-    if (periodic) k_contact_fp32<true, ENERGY><<<(unsigned)gM, 128, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 1, totalM, E);
-    else k_contact_fp32<false, ENERGY><<<(unsigned)gM, 128, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 1, totalM, E);
-    if (ns > 0) launchSS<ENERGY>(st, N, P, C, I, K, mats, sp, dStep, dFlags, nm, 0, anyLaw0, block, gS, gS, E);
-    return totalM > 0 || gS > 0;
+    const int total = ns > 0 ? 0 : gM;
+    if (periodic) k_contact_fp32<true, ENERGY><<<(unsigned)gM, 128, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 1, total, E);
+    else k_contact_fp32<false, ENERGY><<<(unsigned)gM, 128, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 1, total, E);
+    if (ns > 0)
+        k_contact_ss32<kSSMinBlocks, ENERGY><<<gS, (unsigned)block, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, 0, anyLaw0, E);
+    return total > 0;
 }
 
 bool launch_contact_fp32(cudaStream_t st, const SideStream& side, const DevNodes& N, const DevParticles& P, const DevContacts& C,

@@ -13,8 +13,8 @@ import numpy as np
 
 DEFAULT_CANDIDATES = (
     # (contact threads per block, steps per chunk, CUDA graph, facet/wall contacts on a second
-    # stream beside the sphere-sphere ones); block -256 selects the resident-grid FP32
-    # sphere-sphere kernel whose threads prefetch their next contact
+    # stream beside the sphere-sphere ones, for a positive block); block -256 selects the resident
+    # FP32 grid over both, whose threads prefetch their next contact
     (-256, 32, False, True),
     (-256, 32, False, False),
     (256, 32, False, True),
