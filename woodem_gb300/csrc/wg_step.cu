@@ -333,12 +333,11 @@ __device__ __noinline__ double2 capShear(double ft1, double ft2, double maxFt, b
     return make_double2(ft1 * ratio, ft2 * ratio);
 }
 
-// Bound by the FP64 pipe (82 % busy at 20 of 32 lanes, mixed with contacts that are not real). What it
-// costs is warps times FP64 instructions: the work list puts the real contacts together (k_slots),
-// quotients by a common divisor share its reciprocal (wg_div.cuh), the four branches of
-// the frame's quaternion one square root and one division, and the shear cap of a compressed Hertz
-// contact (a zero) takes neither. Drum of 250 000: 0.70 -> 0.49 ms a step; 10 000 settling spheres
-// in one-warp blocks: 45 -> 37 us.
+// Bound by the FP64 pipe (81 % busy at 28 of 32 lanes in a drum of 250 000). What it costs is warps times FP64
+// instructions: the block puts contacts with work left together (contactsOfBlock), quotients by a common
+// divisor share its reciprocal (wg_div.cuh), the four branches of the frame's quaternion one square root and
+// one division, and the shear cap of a compressed Hertz contact (a zero) takes neither. Drum of 250 000: 0.70
+// -> 0.46 ms a step.
 template <bool PERI, bool ENERGY>
 __device__ __forceinline__ void contactItem(int64_t rk, const DevNodes& N, const DevParticles& P, const DevContacts& C,
                                             const DevIncidence& I, const double4_32a* __restrict__ mats,
@@ -588,39 +587,130 @@ __device__ __forceinline__ void contactItem(int64_t rk, const DevNodes& N, const
     C.flags[c] = fl | C_REAL;
 }
 
+// What is left to do for a contact in this step: nothing, an update, or perhaps a creation. These are the tests
+// with which contactItem begins.
+enum { CK_NONE, CK_REAL, CK_NEW };
+static __device__ __noinline__ bool otherTouches(const DevNodes& N, const DevParticles& P, uint32_t ty, int A, int B, D3 shift2, int* dErr) {
+    Geo g;
+    return ty == CT_WS ? geomWS(N, P, 0., A, B, shift2, false, g) : geomFS(N, P, A, B, shift2, false, g, dErr);
+}
+template <bool PERI>
+__device__ __forceinline__ int contactKind(int64_t rk, const DevNodes& N, const DevParticles& P, const DevContacts& C,
+                                           const DevIncidence& I, const ScenePar* __restrict__ spp, long long stepAbs, int* dErr) {
+    const int4 wk = I.work[rk];
+    const int64_t c = wk.x;
+    const int A = wk.y, B = wk.z;
+    const ScenePar& sp = spp[sceneOfP(P, B)];
+    if (stepAbs - sp.stepBase >= sp.stepEnd) return CK_NONE;
+    const uint32_t was = C.flags[c];
+    if (was & C_REMOVED) return CK_NONE;
+    if (was & C_REAL) return CK_REAL;
+    if (was & C_PENDING) return CK_NEW;  // the law has just let it go: few lanes of many warps, divisions in a periodic cell
+    const uint32_t ty = ctype((uint32_t)wk.w);
+    D3 shift2{0, 0, 0};
+    if (PERI) {
+        const int32_t pcd = C.cdist[c];
+        if (pcd != packCellDist(0, 0, 0)) {
+            int a, b, cc;
+            unpackCellDist(pcd, a, b, cc);
+            if (was & C_SWAP) { a = -a; b = -b; cc = -cc; }
+            shift2 = mul(ldm(sp.hSize), D3{(double)a, (double)b, (double)cc});
+        }
+    }
+    Geo g;
+    if (ty == CT_SS ? geomSS(N, A, B, shift2, false, sp.ssDistFactor, g) : otherTouches(N, P, ty, A, B, shift2, dErr))
+        return CK_NEW;
+    return CK_NONE;
+}
+
+// A block's share of the work list: chunks blockIdx.x, + gridDim.x, ... of 32 items. The block tests `rounds`
+// chunks a warp, puts the contacts with work left into its list, real ones from the front and new ones from the
+// back, and its warps take the list. The work list has the contacts that were real at the last full run in
+// front, but they come and go between two runs: a Hertz contact of the drum lasts some 40 steps, and one new
+// contact costs its warp the divisions of the creation and the whole law. In one launch per kernel 200 000
+// sheared spheres 0.56 -> 0.45 ms a step 60 steps after a run, 0.43 -> 0.42 just after one; in k_steps64 10 000
+// settled spheres 29 -> 20 us, 30 000 63 -> 33. (Four lists, with the walls, facets and pairs across a periodic
+// boundary apart, gain less than their last, partly filled warps cost: 0.455 and 0.460 ms.) Every thread of the
+// block calls it.
+constexpr int kRounds = 4;
+template <int THREADS>
+struct ContactList {
+    int32_t at[THREADS * kRounds];
+    int n[2];
+};
+template <bool PERI, bool ENERGY, int THREADS>
+__device__ __forceinline__ void contactsOfBlock(ContactList<THREADS>& L, int rounds, const DevNodes& N, const DevParticles& P,
+                                                const DevContacts& C, const DevIncidence& I, const double4_32a* __restrict__ mats,
+                                                const ScenePar* __restrict__ spp, long long stepAbs, int* __restrict__ dFlags,
+                                                const EnergyCols& E) {
+    constexpr int LAST = THREADS * kRounds - 1;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int64_t chunks = (I.nAct + 31) >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    for (int64_t q0 = 0; q0 * nw * gridDim.x + blockIdx.x < chunks; q0 += rounds) {
+        if (threadIdx.x < 2) L.n[threadIdx.x] = 0;
+        __syncthreads();
+        for (int q = 0; q < rounds; q++) {
+            const int64_t c = ((q0 + q) * nw + w) * gridDim.x + blockIdx.x;
+            if (c >= chunks) break;
+            const int64_t rk = 32 * c + lane;
+            const int k = rk < I.nAct ? contactKind<PERI>(rk, N, P, C, I, spp, stepAbs, dFlags + FL_ERR) : CK_NONE;
+            const unsigned is1 = __ballot_sync(0xffffffffu, k == CK_REAL), is2 = __ballot_sync(0xffffffffu, k == CK_NEW);
+            int at = 0;
+            if (lane == 0 && is1) at = atomicAdd(&L.n[0], __popc(is1));
+            if (lane == 1 && is2) at = atomicAdd(&L.n[1], __popc(is2));
+            const int at1 = __shfl_sync(0xffffffffu, at, 0), at2 = __shfl_sync(0xffffffffu, at, 1);
+            if (k == CK_REAL) L.at[at1 + __popc(is1 & below)] = (int32_t)rk;
+            if (k == CK_NEW) L.at[LAST - (at2 + __popc(is2 & below))] = (int32_t)rk;
+        }
+        __syncthreads();
+        const int n1 = L.n[0], n2 = L.n[1], w1 = (n1 + 31) >> 5, w2 = (n2 + 31) >> 5;
+        for (int t = w; t < w1 + w2; t += nw) {
+            const bool first = t < w1;
+            const int k = 32 * (first ? t : t - w1) + lane;
+            if (k < (first ? n1 : n2))
+                contactItem<PERI, ENERGY>(L.at[first ? k : LAST - k], N, P, C, I, mats, spp, stepAbs, dFlags, E);
+        }
+        __syncthreads();
+    }
+}
+
 template <bool PERI, bool ENERGY>
 __global__ void __launch_bounds__(128) k_contact_fp64(DevNodes N, DevParticles P, DevContacts C, DevIncidence I,
                                                      const double4_32a* __restrict__ mats, const ScenePar* __restrict__ spp,
-                                                     const long long* __restrict__ dStep, int* __restrict__ dFlags,
+                                                     const long long* __restrict__ dStep, int* __restrict__ dFlags, int rounds,
                                                      EnergyCols E) {
-    if (dFlags[FL_FULL] || halted(dFlags)) {
+    if (__syncthreads_or(dFlags[FL_FULL] || halted(dFlags))) {  // the same for all: an error may be raised meanwhile
         // the collider runs before this step's contacts; the steps queued after it wait
         if (blockIdx.x == 0 && threadIdx.x == 0) dFlags[FL_HALT] = 1;
         return;
     }
-    const int64_t rk = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (rk < I.nAct) contactItem<PERI, ENERGY>(rk, N, P, C, I, mats, spp, *dStep, dFlags, E);
+    __shared__ ContactList<128> list;
+    contactsOfBlock<PERI, ENERGY, 128>(list, rounds, N, P, C, I, mats, spp, *dStep, dFlags, E);
 }
 
 void launch_contact_fp64(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
                          const double4_32a* mats, const ScenePar* sp, const long long* dStep, int* dFlags, bool periodic, int block,
                          const EnergyCols* energy) {
     const int bs = block > 0 ? block : fp64Block(I.nAct);
+    // a block's list is longer, and its last warp fuller, the more it tests: up to kRounds items a thread while
+    // every SM has its three blocks
+    const int rounds = (int)std::min<int64_t>(kRounds, std::max<int64_t>(1, I.nAct / ((int64_t)bs * 3 * smCount())));
     // launched even without contacts: it raises FL_HALT when a full run is due
-    const unsigned g = (unsigned)std::max<int64_t>(1, (I.nAct + bs - 1) / bs);
+    const unsigned g = (unsigned)std::max<int64_t>(1, (I.nAct + bs * rounds - 1) / (bs * rounds));
     const EnergyCols E = energy ? *energy : EnergyCols{};
     if (energy) {
-        if (periodic) k_contact_fp64<true, true><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, E);
-        else k_contact_fp64<false, true><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, E);
+        if (periodic) k_contact_fp64<true, true><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, rounds, E);
+        else k_contact_fp64<false, true><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, rounds, E);
     } else {
-        if (periodic) k_contact_fp64<true, false><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, E);
-        else k_contact_fp64<false, false><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, E);
+        if (periodic) k_contact_fp64<true, false><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, rounds, E);
+        else k_contact_fp64<false, false><<<g, bs, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, rounds, E);
     }
 }
 
 // ---------------------------------------------------------------------------------- many steps in one launch
 // Up to `steps` steps of a small scene in one cooperative launch, as k_steps32 of the FP32-force mode
-// (wg_step32.cu). 10 000 spheres: 50 -> 38 us a step.
+// (wg_step32.cu). 10 000 spheres: 50 -> 38 us a step while they fall, 35 settled (44 without the list of the block).
 constexpr int kSteps64Threads = 384;  // 170 registers each
 template <bool PERI>
 __global__ void __launch_bounds__(kSteps64Threads, 1) k_steps64(DevNodes N, DevParticles P, DevContacts C, DevIncidence I,
@@ -628,6 +718,7 @@ __global__ void __launch_bounds__(kSteps64Threads, 1) k_steps64(DevNodes N, DevP
                                                     long long* dStep, int* dFlags, unsigned* bar, unsigned long long* ns, int fromEnds,
                                                     int steps) {
     __shared__ int ok;
+    __shared__ ContactList<kSteps64Threads> list;
     const long long step0 = *(volatile long long*)dStep;
     const int lane = threadIdx.x & 31;
     const int64_t first = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x, stride = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -644,8 +735,7 @@ __global__ void __launch_bounds__(kSteps64Threads, 1) k_steps64(DevNodes N, DevP
         const unsigned long long t1 = clock ? nowNs() : 0ull;
         tA += t1 - t0;
         if (flagNow(dFlags + FL_FULL)) break;  // the same for every thread: raised before the barrier, or at the launch
-        for (int64_t c = first; 32 * c < I.nAct; c += stride)
-            if (32 * c + lane < I.nAct) contactItem<PERI, false>(32 * c + lane, N, P, C, I, mats, sp, step0 + s, dFlags, none);
+        contactsOfBlock<PERI, false, kSteps64Threads>(list, kRounds, N, P, C, I, mats, sp, step0 + s, dFlags, none);
         if (!gridBarrier(bar, dFlags, &ok)) return;
         if (clock) tB += nowNs() - t1;
         if (flagNow(dFlags + FL_ERR)) break;
