@@ -92,7 +92,9 @@ __device__ __forceinline__ void leapfrogNode(int i, const DevNodes& N, const Dev
     D3 f{0, 0, 0}, t{0, 0, 0};
     if (fromEnds && uni && !fresh && !frozen) {
         if (sp.hasGravity && !(flags & F_GRAVITY_SKIP)) f = mass * D3{sp.g[0], sp.g[1], sp.g[2]};
-        if (sp.applyForces) {
+        // a blocked node's force moves nothing: the lane of a wall with 60 contacts would hold up its warp
+        // (2803 spheres in a box: 27 -> 15 us)
+        if (sp.applyForces && (ENERGY || (flags & F_DOF_ALL) != F_DOF_ALL)) {
             endRange(I, i, e0, e1);
             take = (e1 - e0) <= kHeavyThreshold;
             if (!take) {  // summed by the block tree before this kernel

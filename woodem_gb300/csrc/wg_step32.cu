@@ -163,7 +163,7 @@ __device__ __forceinline__ void leapfrogNode32(int i, const DevNodes& N, const D
     if (fromEnds && uni && !fresh && !frozen) {
         if (sp.hasGravity && !(flags & F_GRAVITY_SKIP)) acc.initGravity(nc.mh, nc.ml, sp.gH, sp.gL);
         summed = true;
-        if (sp.applyForces) {
+        if (sp.applyForces && (ENERGY || (flags & F_DOF_ALL) != F_DOF_ALL)) {  // a blocked node's force moves nothing
             e0 = hs0 + ls0;
             e1 = hs1 + ls1;
             take = (e1 - e0) <= kHeavyThreshold;
