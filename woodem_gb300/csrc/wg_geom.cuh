@@ -54,6 +54,38 @@ __device__ __forceinline__ int overlapPeri(const double4_32a& mn1, const double4
     }
     return res;
 }
+// The same decision from FP32 fractions of the cell, where it is clear: 1 overlap, 0 none, 2 not decided here. Boxes
+// of less than 0.4 periods span no boundary of the origin that overlapPeri chooses (the box minimum within half a
+// period below the other), and overlap there if that offset is no more than the lower box. Which box is the lower
+// one is open only at offsets of 0 (boxes above 1e-4: both overlap) and 1/2 (neither does). The fractions are off by
+// at most 3e-7 (1 + periods between the boxes), the FP64 routine by 1e-9 for minima within 1e6 periods.
+// overlapPeri divides 18 times in FP64, some 450 instructions for the one lane of a warp whose contact the law has
+// just let go: 200 000 sheared spheres in FP32-force mode 0.104 -> 0.098 ms a step of contacts.
+__host__ __device__ __forceinline__ int overlapPeriQuick(const double4_32a& mn1, const double4_32a& mx1, const double4_32a& mn2,
+                                                         const double4_32a& mx2, const double* size) {
+    const double m1a[3] = {mn1.x, mn1.y, mn1.z}, x1a[3] = {mx1.x, mx1.y, mx1.z};
+    const double m2a[3] = {mn2.x, mn2.y, mn2.z}, x2a[3] = {mx2.x, mx2.y, mx2.z};
+    int res = 1;
+    for (int axis = 0; axis < 3; axis++) {
+        const float dim = (float)size[axis], m1 = (float)m1a[axis], m2 = (float)m2a[axis];
+        const float e1 = (float)(x1a[axis] - m1a[axis]) / dim, e2 = (float)(x2a[axis] - m2a[axis]) / dim;
+        const float d = (float)(m2a[axis] - m1a[axis]) / dim;
+        const float lim = 1e6f * dim;
+        if (!(dim > 1e-30f && dim < 1e30f && fabsf(m1) < lim && fabsf(m2) < lim && e1 > 1e-4f && e1 < 0.4f && e2 > 1e-4f && e2 < 0.4f))
+            return 2;
+        const float f = d - rintf(d);
+        const float over = f >= 0.f ? e1 - f : e2 + f;
+        if (!(fabsf(over) > 2e-6f * (1.f + fabsf(d)))) return 2;
+        if (over < 0.f) res = 0;
+    }
+    return res;
+}
+static __device__ __noinline__ bool overlapPeriOut(const DevParticles& P, int lo, int hi, const double* cellSize, int* dErr) {
+    int per[3];
+    const int r = overlapPeri(P.mn[lo], P.mx[lo], P.mn[hi], P.mx[hi], cellSize, per);
+    if (r < 0) atomicCAS(dErr, 0, 103);
+    return r > 0;
+}
 // ContactContainer::removePending (pkg/dem/ContactContainer.hpp:78-93 with
 // InsertionSortCollider::shouldBeRemoved, InsertionSortCollider.hpp:209-214): a contact that the
 // law removed in the last step leaves the container at the next collider run unless the boxes of
@@ -61,10 +93,8 @@ __device__ __forceinline__ int overlapPeri(const double4_32a& mn1, const double4
 __device__ __forceinline__ bool pendingStays(const DevParticles& P, int A, int B, bool periodic, const double* cellSize, int* dErr) {
     const int lo = A < B ? A : B, hi = A < B ? B : A;
     if (!periodic) return overlap3(P.mn[lo], P.mx[lo], P.mn[hi], P.mx[hi]);
-    int per[3];
-    const int r = overlapPeri(P.mn[lo], P.mx[lo], P.mn[hi], P.mx[hi], cellSize, per);
-    if (r < 0) atomicCAS(dErr, 0, 103);
-    return r > 0;
+    const int q = overlapPeriQuick(P.mn[lo], P.mx[lo], P.mn[hi], P.mx[hi], cellSize);
+    return q < 2 ? q == 1 : overlapPeriOut(P, lo, hi, cellSize, dErr);
 }
 // Cg2_Sphere_Sphere_L6Geom::go, pkg/dem/Sphere.cpp:88-109
 __device__ __forceinline__ bool geomSS(const DevNodes& N, int A, int B, D3 shift2, bool real, double ssDf, Geo& g) {
