@@ -29,6 +29,7 @@ BUILD = {
     "warp": (_box(26), 3000),  # 26 spheres and 6 walls: 32 nodes
     "warp+1": (_box(27), 3000),
     "part": (_box(700), 3000),
+    "many": (_box(100003), 40),
     "no verlet": (_box(100, 0.0), 3000),
     "periodic": (_peri, 300),
     "drum": (lambda p: scenes.hertz_drum(n=1500, seed=2, diameter=0.3, length=0.12, div=31, axDiv=6, fill_fraction=0.3, precision=p), 300),
@@ -68,5 +69,26 @@ def test_one_launch_is_many_in_a_batch(precision, gpu_lib):
         out.append([[S.dem._nodes.soa.col(k).copy() for k in KEYS] for S in mix])
         B.close()
     for a, b in zip(*out):
+        for x, y in zip(a, b):
+            assert np.array_equal(x, y)
+
+
+def test_simulations_side_by_side(gpu_lib):
+    """Scenes of both precisions in threads of their own, each launch with a grid barrier beside the others'."""
+    from concurrent.futures import ThreadPoolExecutor
+    jobs = [(n, p) for n in (700, 4000, 26) for p in ("fp64", "fp32")]
+
+    def go(job):
+        S = scenes.box_settle_scaled(job[0], 5e-3, seed=job[0], precision=job[1])
+        for _ in range(20):
+            S.run(100)
+        S.sync()
+        out = [S.dem._nodes.soa.col(k).copy() for k in KEYS]
+        S.close()
+        return out
+    alone = [go(j) for j in jobs]
+    with ThreadPoolExecutor(len(jobs)) as ex:
+        beside = list(ex.map(go, jobs))
+    for a, b in zip(alone, beside):
         for x, y in zip(a, b):
             assert np.array_equal(x, y)

@@ -1143,9 +1143,9 @@ int Sim::run(int64_t n) {
         }
         // a small scene runs its steps in one launch, which ends by itself where a full run is due: the
         // chunk only bounds its length (in a periodic cell every step has its own record)
-        const bool small = N.n <= kSmallNodes && I.nAct <= kSmallContacts && !trackE && !useGraph && contactBlock <= 0 &&
-                           I.nHeavyFree == 0 && (!fp32 || P.nFacets == 0 || facetsStatic);
-        int64_t k = std::min<int64_t>(n - done, small && !cfg.periodic && !anyZeroVd ? 8 * maxChunk : maxChunk);
+        const bool small = N.n <= kSmallNodes && I.nAct <= (fp32 && !cfg.periodic ? kSmallContacts32 : kSmallContacts) && !trackE &&
+                           !useGraph && contactBlock <= 0 && I.nHeavyFree == 0 && (!fp32 || P.nFacets == 0 || facetsStatic);
+        int64_t k = std::min<int64_t>(n - done, small && N.n <= 65536 && !cfg.periodic && !anyZeroVd ? 8 * maxChunk : maxChunk);
         // Steps queued past a full run's request do nothing, at two or three empty launches each (2 us apiece), and
         // a chunk that ends before it waits for the host (15 us): one chunk up to where the last interval
         // between two runs ended, then shorter ones. 64 scenes with a run every 2 steps: 32 steps

@@ -219,11 +219,13 @@ enum { FL_FULL = 0,   // set by Leapfrog: a node moved farther than verletDist, 
 constexpr int CTL_COUNTERS = 3;
 constexpr size_t CTL_BYTES = sizeof(int) * FL_WORDS + sizeof(long long) * CTL_COUNTERS;
 // Scenes of at most so many nodes and active contacts run their steps in one launch (launch_steps64,
-// launch_steps32). Boxes of n spheres, us a step in one launch and in a launch per kernel: FP32 10 000 56 and
-// 69, 40 000 64 and 75, 65 000 73 and 82, 100 000 97 and 100, 250 000 184 and 172; FP64 10 000 74 and 88,
-// 40 000 129 and 133, 65 000 177 and 168, 250 000 530 and 495: one block of 384 or 512 threads a SM has too few
-// warps in flight for the larger ones.
-constexpr int64_t kSmallNodes = 65536, kSmallContacts = 262144;
+// launch_steps32). Us a step in one launch and in a launch per
+// kernel: FP32 falling boxes of 10 000 spheres 54 and 65, 100 000 96 and 99, 150 000 122 and 127, 250 000 (2.5 M
+// potential contacts) 183 and 172, drums of 30 000 36 and 49, 100 000 57 and 66, 200 000 85 and 93, periodic
+// shear of 200 000 175 and 183; FP64 falling boxes of 65 000 126 and 151, 250 000 383 and 390, settled ones
+// 168 and 197, a drum of 250 000 625 and 645. 64 scenes of 980 000 spheres in FP32 lose (0.46 and 0.43 ms): one block
+// a SM has fewer warps in flight, and prefetches less, than k_contact_all32.
+constexpr int64_t kSmallNodes = 262144, kSmallContacts = 2097152, kSmallContacts32 = 1048576;
 
 __host__ __device__ inline int32_t packCellDist(int a, int b, int c) {
     return (int32_t)(((uint32_t)(a + 512) & 1023u) | (((uint32_t)(b + 512) & 1023u) << 10) | (((uint32_t)(c + 512) & 1023u) << 20));

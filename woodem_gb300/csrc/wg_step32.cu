@@ -1252,7 +1252,7 @@ __global__ void __launch_bounds__(128, 4) k_contact_fp32(DevNodes N, DevParticle
     stepTicket(dFlags, dStep, ticketTotal);
 }
 
-// minimum resident blocks per SM the sphere-sphere kernels are compiled for (register budget)
+// minimum resident blocks per SM the sphere-sphere kernels are compiled for, which bounds their registers
 constexpr int kSSMinBlocks = 3;
 
 // Both ranges of an aperiodic scene in one resident grid, each warp walking chunks of 32 contacts with the
