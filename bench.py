@@ -713,10 +713,10 @@ def main():
     ap.add_argument("--serve-low-seconds", type=float, default=60.0)
     ap.add_argument("--contact-block", type=int, default=0,
                     help="launch shape of the contact kernels (wg_set_launch): 128/256 one contact per thread, "
-                         "-256 the resident-grid FP32 sphere-sphere kernel with prefetch")
+                         "-256 the resident FP32 grid over all contacts, with prefetch (the default)")
     ap.add_argument("--chunk-steps", type=int, default=32, help="steps queued per host check of the collider request")
     ap.add_argument("--serial-contacts", action="store_true",
-                    help="facet/wall contacts before the sphere-sphere ones (default: beside them on a second stream)")
+                    help="with --contact-block 128/256: facet/wall contacts before the sphere-sphere ones, not beside them")
     ap.add_argument("--write-state", default=None, help=argparse.SUPPRESS)
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
@@ -838,9 +838,9 @@ def main():
         dist.destroy_process_group()
 
 
-# the kernels behind each roofline entry (the contact loop of the FP32-force mode is the facet/wall
-# kernel beside the sphere-sphere kernel, timed together by the phase events)
-KERNELS = {"contact_loop": "k_contact_fp32 (facets, walls) + k_contact_ss32p (sphere-sphere)", "k_contact_fp64": "k_contact_fp64",
+# the kernels behind each roofline entry (the contact loop of the FP32-force mode is one launch over the facet,
+# wall and sphere-sphere contacts)
+KERNELS = {"contact_loop": "k_contact_all32 (facets, walls, sphere-sphere)", "k_contact_fp64": "k_contact_fp64",
            "k_leapfrog32": "k_leapfrog32", "k_leapfrog": "k_leapfrog"}
 
 

@@ -1070,12 +1070,11 @@ __global__ void k_hi_start(const uint32_t* __restrict__ hks, int64_t n, int nPar
 // at hiStart[p+1] + (active contacts before c) (see DevIncidence); inactive contacts have no slot (-1).
 // The work list holds the nOther active contacts that are not plain (walls, facets, spheres of
 // different periods) and then the plain ones, each group in ascending contact order. In the FP64 mode
-// (actReal) the real contacts of a group come before its others: a warp of the contact kernel then
-// holds contacts that all go through the functor chain or that all leave after the distance test.
-// Mixed, the FP64 pipe, which takes a warp instruction's time whatever its lanes do, ran the chain
-// for the two fifths of the lanes that were not real (drum of 250 000: contact loop 0.70 -> 0.49 ms a
-// step). So does a periodic scene in the FP32-force mode, whose contacts are gathered from the contact
-// arrays either way (200 000: 0.12 -> 0.11 ms). The packed FP32 kernel is bound by the gathered mirror
+// (actReal) the real contacts of a group come before its others: a warp of the contact kernel then tests contacts
+// of one kind, and most that are real pass it by. Before the kernel sorted what is left to do (contactsOfBlock),
+// this order alone took the contact loop of a drum of 250 000 from 0.70 to 0.49 ms a step; with both it takes
+// 0.46. A periodic scene in the FP32-force mode, whose contacts are gathered from the contact arrays either
+// way, has it too (200 000: 0.12 -> 0.11 ms). The packed FP32 kernel is bound by the gathered mirror
 // records, which neighbours in contact order share: there the real ones come first within tiles of
 // contacts only (k_pack_ss; 1M drum: split over the whole list, the step took 0.168 ms instead of 0.161).
 __global__ void k_slots(const uint64_t* __restrict__ key, const uint32_t* __restrict__ flags, const int32_t* __restrict__ cdist, int64_t n,
