@@ -8,6 +8,7 @@
 #include <cstring>
 #include <limits>
 #include <string>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -280,7 +281,11 @@ static cudaError_t copyState(double* stage, int64_t na, double* const host[6], i
 constexpr int64_t kDownloadChunk = int64_t(1) << 18;  // doubles: 2 MB
 constexpr int kDownloadThreads = 8;
 static int downloadState(Sim& S, double* stage, int64_t na, double* const host[6]) {
-    if (!S.hDown) WG_CUDA_TRY(cudaMallocHost(&S.hDown, sizeof(double) * kDownloadChunk * kDownloadThreads));
+    if (!S.hDown && cudaMallocHost(&S.hDown, sizeof(double) * kDownloadChunk * kDownloadThreads) != cudaSuccess) {
+        cudaGetLastError();
+        S.hDown = nullptr;
+        return 1;  // no page-locked memory left: the driver's way
+    }
     const int64_t off[7] = {0, 3, 7, 10, 13, 16, 19};
     struct Piece {
         double *to, *from;
@@ -1961,7 +1966,14 @@ int wg_get_nodes(wg_scene* s, double* pos, double* ori, double* vel, double* ang
             bytes += (int64_t)sizeof(double) * w[q] * na;
             locked = locked && pageLocked(dst[q]);
         }
-    if (!locked && bytes >= (int64_t(4) << 20)) return downloadState(S, X.dStage, na, dst);
+    if (!locked && bytes >= (int64_t(4) << 20)) {
+        try {
+            const int r = downloadState(S, X.dStage, na, dst);
+            if (r <= 0) return r;
+        } catch (const std::exception& e) {  // its lists, before any thread has started
+            return S.fail(WG_ERR_STATE, e.what());
+        }
+    }
     WG_CUDA_TRY(copyState(X.dStage, na, dst, 0, 6, false, S.stream));
     WG_CUDA_TRY(cudaGetLastError());
     WG_CUDA_TRY(cudaStreamSynchronize(S.stream));
