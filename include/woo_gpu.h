@@ -245,6 +245,10 @@ int wg_get_aabbs(wg_scene* s, double* mn, double* mx);
 /* Run only the broad phase on the current positions (full run), no stepping. */
 int wg_collide_only(wg_scene* s);
 
+/* For tests of what a failed call leaves behind: the n-th device allocation of the scene from now on (0: the
+   next one) fails as if no memory were left. -1: none does. */
+int wg_fail_alloc(wg_scene* s, int64_t n);
+
 /* Mark the region a profiler started with "profile from start off" captures (1 = start, 0 = stop). */
 int wg_profiler(int on);
 

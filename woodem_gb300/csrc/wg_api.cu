@@ -34,6 +34,7 @@ static thread_local std::string g_createError;
 
 void* Sim::dalloc(size_t bytes) {
     void* p = nullptr;
+    if (failAlloc >= 0 && failAlloc-- == 0) return nullptr;
     if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
@@ -353,20 +354,31 @@ int Sim::ensureContactCapacity(int64_t need) {
     // FP64 plain: every FP64 column. FP32-force: the FP32 columns plus the FP64 shear force
     // (IdealElPl) and contact point (facet and wall contacts).
     auto needD = [&](int q) { return prec == WG_PREC_FP64 || q == CC_FT1 || q == CC_FT2 || q == CC_CPX || q == CC_CPY || q == CC_CPZ; };
+    auto give = [&](DevContacts& d) {
+        dfree(d.key); dfree(d.flags); dfree(d.step0); dfree(d.cdist);
+        for (int q = 0; q < CC_NCOL; q++) dfree(d.col[q]);
+        for (int q = 0; q < CF_NCOL; q++) dfree(d.fcol[q]);
+    };
+    bool ok = true;
     for (DevContacts* d : {&nc, &nb}) {
         d->key = (uint64_t*)dalloc(sizeof(uint64_t) * cap);
         d->flags = (uint32_t*)dalloc(sizeof(uint32_t) * cap);
         d->step0 = (int32_t*)dalloc(sizeof(int32_t) * cap);
         d->cdist = (int32_t*)dalloc(sizeof(int32_t) * cap);
-        if (!d->cdist) return fail(WG_ERR_CUDA, "out of device memory (contacts)");
+        ok = ok && d->key && d->flags && d->step0 && d->cdist;
         for (int q = 0; q < CC_NCOL; q++) {
             d->col[q] = needD(q) ? (double*)dalloc(sizeof(double) * cap) : nullptr;
-            if (needD(q) && !d->col[q]) return fail(WG_ERR_CUDA, "out of device memory (contacts)");
+            ok = ok && (!needD(q) || d->col[q]);
         }
         for (int q = 0; q < CF_NCOL; q++) {
             d->fcol[q] = (prec == WG_PREC_FP32) ? (float*)dalloc(sizeof(float) * cap) : nullptr;
-            if (prec == WG_PREC_FP32 && !d->fcol[q]) return fail(WG_ERR_CUDA, "out of device memory (contacts)");
+            ok = ok && (prec != WG_PREC_FP32 || d->fcol[q]);
         }
+    }
+    if (!ok) {
+        give(nc);
+        give(nb);
+        return fail(WG_ERR_CUDA, "out of device memory (contacts)");
     }
     if (C.key && C.n > 0) {
         WG_CUDA_TRY(cudaMemcpyAsync(nc.key, C.key, sizeof(uint64_t) * C.n, cudaMemcpyDeviceToDevice, stream));
@@ -380,12 +392,8 @@ int Sim::ensureContactCapacity(int64_t need) {
     }
     WG_CUDA_TRY(cudaStreamSynchronize(stream));
     nc.n = C.n;
-    for (DevContacts* d : {&C, &Cb}) {
-        if (!d->key) continue;
-        dfree(d->key); dfree(d->flags); dfree(d->step0); dfree(d->cdist);
-        for (int q = 0; q < CC_NCOL; q++) dfree(d->col[q]);
-        for (int q = 0; q < CF_NCOL; q++) dfree(d->fcol[q]);
-    }
+    give(C);
+    give(Cb);
     C = nc;
     Cb = nb;
     cCap = cap;
@@ -1192,6 +1200,7 @@ int Sim::run(int64_t n) {
         }
         const bool needFull = !initialized || anyZeroVd || forceFull;
         k_set_flags<<<1, 1, 0, stream>>>(dFlags, needFull ? 1 : 0);
+        const HostCell cell0 = X.cell;
         if (cfg.periodic) {
             // Cell::integrateAndUpdate then setNextGradV for every queued step (Scene::doOneStep)
             for (int64_t j = 0; j < k; j++) {
@@ -1300,7 +1309,23 @@ int Sim::run(int64_t n) {
             }
             WG_CUDA_TRY(cudaEventRecord(E[3 * maxChunk], stream));
             int r = collide_full_run(*this);
-            if (r) return r;
+            if (r) {
+                // the steps before this one are done; it starts anew in the next call
+                if (cfg.periodic) X.cell = ds > 0 ? cellEnd[ds - 1] : cell0;
+                for (int64_t j = 0; j < ds; j++) {
+                    if (dd.on) dd.activated(step + j, timeAbs);
+                    time += cfg.dt;
+                    timeAbs += cfg.dt;
+                    for (int q = 0; q < nScenes && nScenes > 1; q++)
+                        if (!sceneFrozen(q, step + j)) {
+                            if (bdd[q].on) bdd[q].activated(sceneStep(q, step + j), bTime[q]);
+                            bTime[q] += hPars[q].dt;
+                        }
+                }
+                fromEnds = fromEnds || ds > 0;
+                step += ds;
+                return r;
+            }
             if (lastFullStep >= 0 && step + ds > lastFullStep) runInterval = step + ds - lastFullStep;
             lastFullStep = step + ds;
             if (trackE) {
@@ -2406,6 +2431,12 @@ int wg_get_aabbs(wg_scene* s, double* mn, double* mx) {
         mn[3 * i] = a[i].x; mn[3 * i + 1] = a[i].y; mn[3 * i + 2] = a[i].z;
         mx[3 * i] = b[i].x; mx[3 * i + 1] = b[i].y; mx[3 * i + 2] = b[i].z;
     }
+    return WG_OK;
+}
+
+int wg_fail_alloc(wg_scene* s, int64_t n) {
+    if (!s) return WG_ERR_ARG;
+    SIM(s)->failAlloc = n;
     return WG_OK;
 }
 

@@ -23,6 +23,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "wg_internal.h"
 #include "wg_math.cuh"
@@ -78,9 +79,7 @@ struct CollideWork {
     int64_t pairCap = 0;
     int32_t* pairCd = nullptr;        // periodic: cell distance of each new pair
     int32_t* pairCdSorted = nullptr;
-    int64_t pairCdCap = 0;
     int32_t* newCd = nullptr;         // periodic: cell distance per merged contact
-    int64_t newCdCap = 0;
     CollideTotals* tot = nullptr;     // counts a run makes on the device
     CollideTotals* hTot = nullptr;    // pinned
     // merge scratch
@@ -94,7 +93,6 @@ struct CollideWork {
     DevPackedSS Kb{};
     int32_t *packIdx = nullptr, *packIdxB = nullptr;
     int64_t packIdxCap = 0, packIdxCapB = 0;
-    bool packIdxValid = false;
     uint64_t* act = nullptr;      // exclusive scan of the active contacts (low half) and the plain ones of them (high)
     uint64_t* actReal = nullptr;  // FP64 mode: the same of the real contacts
     uint32_t* hiKeys = nullptr;
@@ -1129,16 +1127,32 @@ __global__ void k_heavy(DevIncidence I, DevParticles P, const uint32_t* __restri
         if ((nodeFlags[p] & F_DOF_ALL) != F_DOF_ALL) I.heavyFree[atomicAdd(&tot->heavyFree, 1)] = p;
     }
 }
-// every end starts without a contribution: 2 ends of each of the active contacts (*act, low half)
-__global__ void k_zero_ends(DevIncidence I, const uint64_t* __restrict__ act) {
+// every end starts without a contribution
+__global__ void k_zero_ends(DevIncidence I, int64_t ends) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= 2 * (int64_t)(uint32_t)*act) return;
+    if (e >= ends) return;
     if (I.endA) {
         I.endA[e] = make_double4_32a(0., 0., 0., 0.);
         I.endB[e] = make_double2(0., 0.);
     } else {
         I.endAf[e] = make_float4(0.f, 0.f, 0.f, 0.f);
         I.endBf[e] = make_float2(0.f, 0.f);
+    }
+}
+
+// the packed state K back into the contact arrays of its set, contact c from idx[c] (whatever the work list holds)
+__global__ void k_unpack_set(DevContacts C, DevPackedSS K, const int32_t* __restrict__ idx, int copyFt) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= C.n) return;
+    const uint32_t fl = C.flags[c];
+    if (!activeContact(fl) || !plainContact(fl, C.cdist[c])) return;
+    const int64_t j = idx[c];
+    C.flags[c] = K.flags[j] & 0xffu;
+#pragma unroll
+    for (int q = 0; q < CF_NCOL; q++) C.fcol[q][c] = K.col[q][j];
+    if (copyFt) {
+        C.col[CC_FT1][c] = K.ft[0][j];
+        C.col[CC_FT2][c] = K.ft[1][j];
     }
 }
 
@@ -1194,21 +1208,62 @@ int count_contacts(Sim& S, int64_t p0, int64_t p1, int64_t out[2]) {
 }
 
 // ---------------------------------------------------------------- host orchestration
+// Larger arrays in place of others, all of them or none: where one cannot be had, the old ones stay.
+class Larger {
+    Sim& S;
+    std::vector<std::pair<void*, void*>> fresh;  // where the pointer is kept, and the new array
+    bool ok = true;
+
+public:
+    explicit Larger(Sim& s) : S(s) {}
+    ~Larger() {
+        for (auto& f : fresh) S.dfree(f.second);
+    }
+    template <class T>
+    void add(T*& p, int64_t n) {
+        void* const q = S.dalloc(sizeof(T) * n);
+        ok = ok && q;
+        if (q) fresh.push_back({&p, q});
+    }
+    bool put() {
+        if (!ok) return false;
+        for (auto& f : fresh) {
+            void* old;
+            std::memcpy(&old, f.first, sizeof old);
+            std::memcpy(f.first, &f.second, sizeof old);
+            S.dfree(old);
+        }
+        fresh.clear();
+        return true;
+    }
+};
+
 static int ensureCub(Sim& S, size_t bytes) {
     CollideWork& W = *S.cw;
     if (bytes <= W.cubBytes) return 0;
-    if (W.cubTmp) S.dfree(W.cubTmp);
-    W.cubBytes = bytes * 3 / 2 + 1024;
-    W.cubTmp = S.dalloc(W.cubBytes);
-    return W.cubTmp ? 0 : S.fail(WG_ERR_CUDA, "out of device memory (collider scratch)");
+    Larger L(S);
+    char* tmp = (char*)W.cubTmp;
+    const size_t want = bytes * 3 / 2 + 1024;
+    L.add(tmp, (int64_t)want);
+    if (!L.put()) return S.fail(WG_ERR_CUDA, "out of device memory (collider scratch)");
+    W.cubTmp = tmp;
+    W.cubBytes = want;
+    return 0;
 }
 
-template <class T>
-static T* grow(Sim& S, T* p, int64_t& cap, int64_t need) {
-    if (need <= cap && p) return p;
-    if (p) S.dfree(p);
-    cap = std::max<int64_t>(need, cap * 3 / 2 + 1024);
-    return (T*)S.dalloc(sizeof(T) * cap);
+// Scratch of one capacity whose contents need not last: given up before the larger one is asked for, all of it
+// or none (cap is 0 then). False: out of device memory.
+template <class... T>
+static bool scratch(Sim& S, int64_t& cap, int64_t need, T*&... p) {
+    if (need <= cap) return true;
+    const int64_t want = std::max<int64_t>(need, cap * 3 / 2 + 1024);
+    ((S.dfree(p), p = nullptr), ...);
+    ((p = (T*)S.dalloc(sizeof(T) * want)), ...);
+    cap = want;
+    if ((... && (p != nullptr))) return true;
+    ((S.dfree(p), p = nullptr), ...);
+    cap = 0;
+    return false;
 }
 
 static int buildLists(Sim& S) {
@@ -1238,11 +1293,12 @@ static int buildLists(Sim& S) {
     W.hGlobal = glob;
     // capacity for every particle: the lists are rebuilt when serving slots change
     if (!W.sphereIds) {
-        W.sphereIds = (int32_t*)S.dalloc(sizeof(int32_t) * std::max<int64_t>(1, S.nPar));
-        W.largeIds = (int32_t*)S.dalloc(sizeof(int32_t) * std::max<int64_t>(1, S.nPar));
-        W.globalIds = (int32_t*)S.dalloc(sizeof(int32_t) * std::max<int64_t>(1, S.nPar));
-        W.gStart = (int32_t*)S.dalloc(sizeof(int32_t) * (S.nScenes + 1));
-        if (!W.sphereIds || !W.largeIds || !W.globalIds || !W.gStart) return S.fail(WG_ERR_CUDA, "out of device memory");
+        Larger L(S);
+        L.add(W.sphereIds, S.nPar);
+        L.add(W.largeIds, S.nPar);
+        L.add(W.globalIds, S.nPar);
+        L.add(W.gStart, S.nScenes + 1);
+        if (!L.put()) return S.fail(WG_ERR_CUDA, "out of device memory");
     }
     W.nLarge = W.nGlobal = 0;
     if (!sph.empty()) WG_CUDA_TRY(cudaMemcpyAsync(W.sphereIds, sph.data(), sizeof(int32_t) * sph.size(), cudaMemcpyHostToDevice, S.stream));
@@ -1266,7 +1322,140 @@ static int buildLists(Sim& S) {
     return 0;
 }
 
-int collide_full_run(Sim& S) {
+// ---------------------------------------------------------------- the second half of a run, over a set of n contacts
+static int hiKeyBits(const Sim& S) {  // bits of the largest hi key, nPar
+    int bits = 1;
+    while ((int64_t(1) << bits) <= S.nPar) bits++;
+    return bits;
+}
+// Room for the incidence of n contacts; the arrays in use stay until all of the larger ones are there.
+static int incidenceRoom(Sim& S, int64_t n) {
+    CollideWork& W = *S.cw;
+    const bool realFirst = S.prec == WG_PREC_FP64 || S.cfg.periodic;  // see k_slots
+    if (W.hiCap < std::max<int64_t>(n, 1)) {
+        const int64_t cap = std::max<int64_t>(n, 1) * 3 / 2 + 1024;
+        Larger L(S);
+        L.add(W.hiKeys, cap);
+        L.add(W.hiKeysSorted, cap);
+        L.add(W.hiVals, cap);
+        L.add(S.I.hiList, cap);
+        L.add(S.I.slotLo, cap);
+        L.add(S.I.slotHi, cap);
+        L.add(W.act, cap + 1);
+        if (realFirst) L.add(W.actReal, cap + 1);
+        L.add(S.I.work, cap);
+        if (!L.put()) return S.fail(WG_ERR_CUDA, "out of device memory (incidence)");
+        W.hiCap = cap;
+    }
+    size_t a = 0, b = 0;
+    const auto in = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), WorkClass{S.C.flags, S.C.cdist, n, 0});
+    cub::DeviceScan::ExclusiveSum(nullptr, a, in, W.act, (int)(n + 1), S.stream);
+    if (n > 0) cub::DeviceRadixSort::SortPairs(nullptr, b, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiKeyBits(S), S.stream);
+    return ensureCub(S, std::max(a, b));
+}
+// CSR incidence and work list of the n contacts of S.C; first: the first contact of every lo id. The room is there.
+// The host does not know the number of active contacts before the end.
+static int incidence(Sim& S, int64_t n, const int32_t* first) {
+    CollideWork& W = *S.cw;
+    cudaStream_t st = S.stream;
+    const unsigned gn = (unsigned)((n + BS - 1) / BS);
+    auto scan = [&](uint32_t real, uint64_t* out) -> int {
+        const auto in = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), WorkClass{S.C.flags, S.C.cdist, n, real});
+        size_t tb = W.cubBytes;
+        WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, in, out, (int)(n + 1), st));
+        return 0;
+    };
+    int r = scan(0, W.act);
+    if (!r && W.actReal) r = scan(C_REAL, W.actReal);
+    if (r) return r;
+    k_lo_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(first, (int)S.nPar, W.act, S.I.loStart);
+    if (n > 0) {
+        k_hi_keys<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, n, (uint32_t)S.nPar, W.hiKeys, W.hiVals);
+        size_t tb = W.cubBytes;
+        WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiKeyBits(S), st));
+    }
+    k_hi_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.hiKeysSorted, n, (int)S.nPar, S.I.hiStart);
+    if (n > 0) k_slots<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, S.I);
+    k_heavy<<<(unsigned)((S.nPar + BS - 1) / BS), BS, 0, st>>>(S.I, S.P, S.N.flags, kHeavyThreshold, W.tot, W.act, W.actReal, n);
+    return 0;
+}
+// Room for the ends of nAct contacts; the old ends stay until the new ones are there.
+static int endRoom(Sim& S, int64_t nAct) {
+    if (S.I.endCap >= 2 * std::max<int64_t>(nAct, 1)) return 0;
+    const int64_t cap = 2 * std::max<int64_t>(nAct, 1) * 5 / 4 + 2048;
+    Larger L(S);
+    if (S.prec == WG_PREC_FP32) {
+        L.add(S.I.endAf, cap);
+        L.add(S.I.endBf, cap);
+    } else {
+        L.add(S.I.endA, cap);
+        L.add(S.I.endB, cap);
+    }
+    if (!L.put()) return S.fail(WG_ERR_CUDA, "out of device memory (contact ends)");
+    S.I.endCap = cap;
+    return 0;
+}
+// Room in Q, whose contents need not last, for n packed contacts.
+static int packRoom(Sim& S, DevPackedSS& Q, int64_t n) {
+    if (Q.cap >= n) return 0;
+    S.dfree(Q.item); S.dfree(Q.flags);
+    for (int q = 0; q < CF_NCOL; q++) S.dfree(Q.col[q]);
+    S.dfree(Q.ft[0]); S.dfree(Q.ft[1]);
+    Q = DevPackedSS{};
+    const int64_t cap = n * 5 / 4 + 4096;
+    Larger L(S);
+    L.add(Q.item, cap);
+    L.add(Q.flags, cap);
+    for (int q = 0; q < CF_NCOL; q++) L.add(Q.col[q], cap);
+    // the IdealElPl shear force (a serving slot may take a job with that law at any time)
+    L.add(Q.ft[0], cap);
+    L.add(Q.ft[1], cap);
+    if (!L.put()) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
+    Q.cap = cap;
+    return 0;
+}
+
+// A run that ends early after the incidence of the new set was begun: the old set, from its keys and flags, takes
+// its incidence and work list again (the ends and the packed state are still those of the old set).
+struct Undo {
+    Sim& S;
+    const bool packedState;
+    bool swapped = false, incidence = false, off = false;
+    Undo(Sim& s, bool p) : S(s), packedState(p) {}
+    void swap() {
+        std::swap(S.C, S.Cb);
+        swapped = !swapped;
+    }
+    ~Undo() {
+        if (off) return;
+        if (swapped) swap();
+        if (!incidence) return;
+        const std::string why = S.err;  // what the run failed for
+        if (restore()) S.K.n = 0;       // the device is gone
+        S.err = why;
+    }
+    int restore() {
+        CollideWork& W = *S.cw;
+        const int64_t n = S.C.n;
+        if (S.contactsReplaced) {  // set from outside and never run: it has no forces to list
+            WG_CUDA_TRY(cudaMemsetAsync(S.I.slotLo, 0xff, sizeof(int32_t) * W.hiCap, S.stream));
+            WG_CUDA_TRY(cudaMemsetAsync(S.I.slotHi, 0xff, sizeof(int32_t) * W.hiCap, S.stream));
+            return 0;
+        }
+        if (packedState && n > 0) k_unpack_set<<<(unsigned)((n + BS - 1) / BS), BS, 0, S.stream>>>(S.C, S.K, W.packIdx, S.K.ftLive ? 1 : 0);
+        k_lo_bounds<<<(unsigned)((n + 1 + BS - 1) / BS), BS, 0, S.stream>>>(S.C.key, n, (int)S.nPar, W.oldLo);
+        WG_CUDA_TRY(cudaMemsetAsync(&W.tot->heavy, 0, 2 * sizeof(int32_t), S.stream));
+        int r = incidenceRoom(S, n);
+        if (!r) r = wg::incidence(S, n, W.oldLo);
+        if (r) return r;
+        launch_pack_ss(S.stream, S.C, S.I, S.P, S.K, S.K, nullptr, nullptr, W.packIdx, W.act + n, S.K.n);
+        S.packDirty = false;
+        WG_CUDA_TRY(cudaGetLastError());
+        return 0;
+    }
+};
+
+static int fullRun(Sim& S) {
     cudaStream_t st = S.stream;
     if (!S.cw) {
         S.cw = new CollideWork();
@@ -1279,19 +1468,10 @@ int collide_full_run(Sim& S) {
     }
     CollideWork& W = *S.cw;
     // The packed sphere-sphere state goes from the old set to the new one; the contact arrays take back its
-    // flags alone. Where they hold another set than the packed one, all of it comes from them.
+    // flags alone. Until the new set is in place the packed state stays that of the old one.
     const bool packed = S.prec == WG_PREC_FP32 && !S.cfg.periodic;
-    const bool packedState = packed && S.K.n > 0 && W.packIdxValid && !S.contactsReplaced;
-    if (packedState) {
-        if (S.packDirty) launch_unpack_ss(st, S.C, S.I, S.K, S.nMixed, true);
-        S.packDirty = false;
-    } else {
-        int r = S.syncContacts(false);  // the merge below is queued on the same stream
-        if (r) return r;
-    }
-    const DevPackedSS Kold = S.K;
-    S.K.n = 0;
-    W.packIdxValid = false;
+    const bool packedState = S.K.n > 0;  // none where the contact arrays were set from outside
+    if (packedState && S.packDirty) launch_unpack_ss(st, S.C, S.I, S.K, S.nMixed, true);
     const uint32_t lone = S.cfg.lone_mask;
     if (S.cfg.periodic && S.hPar.hasShear && !W.hGlobal.empty())
         return S.fail(WG_ERR_UNSUPPORTED, "Walls not supported in skewed (Scene.cell.trsf is not diagonal) periodic boundary conditions.");
@@ -1305,11 +1485,8 @@ int collide_full_run(Sim& S) {
     const int K = S.nScenes;
     const int ns = W.nSph;
     const bool peri = S.cfg.periodic != 0;
-    if (!W.tot) {
-        W.tot = (CollideTotals*)S.dalloc(sizeof(CollideTotals));
-        WG_CUDA_TRY(cudaMallocHost(&W.hTot, sizeof(CollideTotals)));
-        if (!W.tot) return S.fail(WG_ERR_CUDA, "out of device memory (counts)");
-    }
+    if (!W.hTot) WG_CUDA_TRY(cudaMallocHost(&W.hTot, sizeof(CollideTotals)));
+    if (!W.tot && !(W.tot = (CollideTotals*)S.dalloc(sizeof(CollideTotals)))) return S.fail(WG_ERR_CUDA, "out of device memory (counts)");
     WG_CUDA_TRY(cudaMemsetAsync(W.tot, 0, sizeof(CollideTotals), st));
     int* const bad = &W.tot->bad;
     if (ns > 0) {
@@ -1317,22 +1494,21 @@ int collide_full_run(Sim& S) {
         if (!W.dGrids) {
             // capacity for the most chunks the particles can form (one per scene plus the full ones)
             const int cap = (int)(S.nPar / kGridChunk + S.nScenes + 2);
-            W.red = (float*)S.dalloc(sizeof(float) * 7 * cap);
-            W.dChunk = (int32_t*)S.dalloc(sizeof(int32_t) * (cap + 1));
-            W.dSceneChunk = (int32_t*)S.dalloc(sizeof(int32_t) * (K + 1));
-            W.dGrids = (Grid*)S.dalloc(sizeof(Grid) * K);
             const int64_t sph = S.nPar;  // every particle could be an active sphere
-            W.cellKey = (uint32_t*)S.dalloc(sizeof(uint32_t) * sph);
-            W.cellRank = (int32_t*)S.dalloc(sizeof(int32_t) * sph);
-            W.skey = (uint32_t*)S.dalloc(sizeof(uint32_t) * sph);
-            if (peri) W.speri = (PeriBox*)S.dalloc(sizeof(PeriBox) * sph);
+            Larger L(S);
+            L.add(W.red, 7 * (int64_t)cap);
+            L.add(W.dChunk, cap + 1);
+            L.add(W.dSceneChunk, K + 1);
+            L.add(W.dGrids, K);
+            L.add(W.cellKey, sph);
+            L.add(W.cellRank, sph);
+            L.add(W.skey, sph);
+            if (peri) L.add(W.speri, sph);
             else {
-                W.smnf = (float4*)S.dalloc(sizeof(float4) * sph);
-                W.smxf = (float4*)S.dalloc(sizeof(float4) * sph);
+                L.add(W.smnf, sph);
+                L.add(W.smxf, sph);
             }
-            if (!W.red || !W.dChunk || !W.dSceneChunk || !W.dGrids || !W.cellKey || !W.cellRank || !W.skey ||
-                (peri ? !W.speri : (!W.smnf || !W.smxf)))
-                return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
+            if (!L.put()) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
         }
         if (W.chunksDirty) {
             WG_CUDA_TRY(cudaMemcpyAsync(W.dChunk, W.hChunk.data(), sizeof(int32_t) * (nb + 1), cudaMemcpyHostToDevice, st));
@@ -1342,8 +1518,7 @@ int collide_full_run(Sim& S) {
         int64_t ncell = 0;
         for (int k = 0; k < K; k++) ncell += cellBound(W.hSceneSph[k + 1] - W.hSceneSph[k], K);
         if (ncell >= (int64_t(1) << 31) - 2) return S.fail(WG_ERR_CAPACITY, "too many broad-phase cells in the batch");
-        W.cellOff = grow(S, W.cellOff, W.cellOffCap, ncell + 1);
-        if (!W.cellOff) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
+        if (!scratch(S, W.cellOffCap, ncell + 1, W.cellOff)) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
         const unsigned gs = (unsigned)((ns + BS - 1) / BS);
         k_grid_reduce<<<nb, BS, 0, st>>>(S.P, W.sphereIds, W.dChunk, W.red);
         k_make_grids<<<1, 256, 0, st>>>(K, W.dChunk, W.dSceneChunk, W.red, S.dPar, peri ? 1 : 0, W.dGrids, bad);
@@ -1395,12 +1570,11 @@ int collide_full_run(Sim& S) {
         }
     }
     // 3-4. pair generation with a capacity retry
-    if (W.pairCap == 0) {
-        int64_t c0 = std::max<int64_t>(1 << 16, 8 * S.nPar);
-        W.pairs = grow(S, W.pairs, W.pairCap, c0);
-        int64_t cap2 = 0;
-        W.pairsSorted = grow(S, W.pairsSorted, cap2, W.pairCap);
-    }
+    auto pairRoom = [&](int64_t need) {
+        return peri ? scratch(S, W.pairCap, need, W.pairs, W.pairsSorted, W.pairCd, W.pairCdSorted)
+                    : scratch(S, W.pairCap, need, W.pairs, W.pairsSorted);
+    };
+    if (!pairRoom(std::max<int64_t>(1 << 16, 8 * S.nPar))) return S.fail(WG_ERR_CUDA, "out of device memory (pairs)");
     int idBits = 1;  // bits of an id
     while ((int64_t(1) << idBits) < S.nPar) idBits++;
     unsigned long long* const counter = &W.tot->pairs;
@@ -1408,12 +1582,6 @@ int collide_full_run(Sim& S) {
     for (int attempt = 0; attempt < 3; attempt++) {
         if (attempt > 0) WG_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
         if (peri) {
-            if (W.pairCdCap < W.pairCap) {
-                int64_t c2 = W.pairCdCap;
-                W.pairCd = grow(S, W.pairCd, W.pairCdCap, W.pairCap);
-                W.pairCdSorted = grow(S, W.pairCdSorted, c2, W.pairCap);
-                if (!W.pairCd || !W.pairCdSorted) return S.fail(WG_ERR_CUDA, "out of device memory (pairs)");
-            }
             if (ns > 0)
                 k_pairs_ss_peri<<<(ns + 127) / 128, 128, 0, st>>>(S.P, W.skey, W.speri, ns, W.dGrids, W.cellOff, lone, idBits, bad, S.dPar,
                                                                   W.pairs, W.pairCd, W.pairCap, counter, S.dFlags + FL_ERR);
@@ -1448,10 +1616,7 @@ int collide_full_run(Sim& S) {
         if (W.hTot->bad) return S.fail(WG_ERR_NAN, "InsertionSortCollider: non-finite sphere bounding box (NaN or infinite position)");
         nNew = (int64_t)W.hTot->pairs;
         if (nNew <= W.pairCap) break;
-        int64_t cap2 = W.pairCap;
-        W.pairs = grow(S, W.pairs, W.pairCap, nNew + nNew / 4);
-        W.pairsSorted = grow(S, W.pairsSorted, cap2, W.pairCap);
-        if (!W.pairs || !W.pairsSorted) return S.fail(WG_ERR_CUDA, "out of device memory (pairs)");
+        if (!pairRoom(nNew + nNew / 4)) return S.fail(WG_ERR_CUDA, "out of device memory (pairs)");
     }
     // sort the pairs, (lo << idBits | hi)
     if (nNew > 0) {
@@ -1470,15 +1635,13 @@ int collide_full_run(Sim& S) {
     // scan and a wait; elsewhere the merge counts whether every real contact was among the new pairs, and is
     // done again with them if the host finds that one was not.
     const int64_t nOld = S.C.n;
-    W.newLo = grow(S, W.newLo, W.newLoCap, S.nPar + 2);
-    W.oldLo = grow(S, W.oldLo, W.oldLoCap, S.nPar + 2);
-    if (!W.newLo || !W.oldLo) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+    if (!scratch(S, W.newLoCap, S.nPar + 2, W.newLo) || !scratch(S, W.oldLoCap, S.nPar + 2, W.oldLo))
+        return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
     // W.pairs takes the sorted pairs back as contact keys
     const uint64_t* const nk = W.pairs;
     k_unpack_keys<<<(unsigned)((nNew + 1 + BS - 1) / BS), BS, 0, st>>>(W.pairsSorted, nNew, idBits, (int)S.nPar, W.pairs, W.newLo);
     if (nOld > 0 && (!W.oldLoValid || S.contactsReplaced))
         k_lo_bounds<<<(unsigned)((nOld + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, nOld, (int)S.nPar, W.oldLo);
-    S.contactsReplaced = false;
     bool lookForOrphans = false;
     for (int k = 0; k < K; k++) {
         const wg_config& c = K > 1 ? S.cfgs[k] : S.cfg;
@@ -1486,13 +1649,13 @@ int collide_full_run(Sim& S) {
     }
     bool law0 = S.cfg.law == 0;
     for (const wg_config& c : S.cfgs) law0 = law0 || c.law == 0;
+    Undo undo(S, packedState);
     for (;;) {
         int64_t nOrph = 0;
         if (nOld > 0 && lookForOrphans) {
-            W.orph = grow(S, W.orph, W.mergeCap, std::max<int64_t>(nOld, 1) * 2 + 2);
-            if (!W.orph) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+            if (!scratch(S, W.mergeCap, nOld * 2 + 2, W.orph)) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
             int32_t* flagsArr = W.orph;
-            int32_t* scanArr = W.orph + (std::max<int64_t>(nOld, 1) + 1);
+            int32_t* scanArr = W.orph + (nOld + 1);
             k_mark_orphans<<<(unsigned)((nOld + BS - 1) / BS), BS, 0, st>>>(S.C, nk, W.newLo, flagsArr, S.P.fresh);
             size_t tb = 0;
             cub::DeviceScan::ExclusiveSum(nullptr, tb, flagsArr, scanArr, (int)nOld, st);
@@ -1505,26 +1668,18 @@ int collide_full_run(Sim& S) {
             WG_CUDA_TRY(cudaStreamSynchronize(st));
             nOrph = (int64_t)last[0] + last[1];
             if (nOrph > 0) {
-                if (nOrph > W.orphCap) {
-                    int64_t c1 = W.orphCap, c2 = W.orphCap;
-                    W.orphKey = grow(S, W.orphKey, c1, nOrph);
-                    W.orphSrc = grow(S, W.orphSrc, c2, nOrph);
-                    W.orphCap = c1;
-                    if (!W.orphKey || !W.orphSrc) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
-                }
+                if (!scratch(S, W.orphCap, nOrph, W.orphKey, W.orphSrc)) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
                 k_compact_orphans<<<(unsigned)((nOld + BS - 1) / BS), BS, 0, st>>>(S.C, flagsArr, scanArr, W.orphKey, W.orphSrc);
             }
         }
         const int64_t n = nNew + nOrph;
         int r = S.ensureContactCapacity(n);
         if (r) return r;
-        W.src = grow(S, W.src, W.srcCap, std::max<int64_t>(n, 1));
-        if (!W.src) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+        if (!(peri ? scratch(S, W.srcCap, std::max<int64_t>(n, 1), W.src, W.newCd) : scratch(S, W.srcCap, std::max<int64_t>(n, 1), W.src)))
+            return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+        r = incidenceRoom(S, n);
+        if (r) return r;
         S.Cb.n = n;
-        if (peri) {
-            W.newCd = grow(S, W.newCd, W.newCdCap, std::max<int64_t>(n, 1));
-            if (!W.newCd) return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
-        }
         const unsigned gn = (unsigned)((n + BS - 1) / BS);
         const int64_t places = std::max<int64_t>(nNew, lookForOrphans ? 0 : nOld);
         if (places > 0)
@@ -1535,128 +1690,47 @@ int collide_full_run(Sim& S) {
             k_place_orph<<<(unsigned)((nOrph + BS - 1) / BS), BS, 0, st>>>(nk, nNew, W.orphKey, W.orphSrc, nOrph, S.Cb.key, W.src);
         if (n > 0) k_gather<<<gn, BS, 0, st>>>(S.C, S.Cb, W.src, S.N, S.P, S.dPar, S.dStep, peri ? W.newCd : nullptr, peri ? 1 : 0,
                                              packedState ? 1 : 0);
-        std::swap(S.C, S.Cb);
+        undo.swap();
         if (nOrph > 0)  // the first index of every lo id in the merged set; without orphans that of the new pairs
             k_lo_bounds<<<(unsigned)((n + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, n, (int)S.nPar, W.newLo);
-        // 6. CSR incidence over the active contacts. The host does not know their number yet: what is sized by
-        // it is sized for all contacts.
-        if (W.hiCap < std::max<int64_t>(n, 1)) {
-            if (W.hiKeys) {
-                S.dfree(W.hiKeys); S.dfree(W.hiKeysSorted); S.dfree(W.hiVals); S.dfree(S.I.hiList);
-                S.dfree(S.I.slotLo); S.dfree(S.I.slotHi); S.dfree(W.act); S.dfree(W.actReal); S.dfree(S.I.work);
-            }
-            W.hiCap = std::max<int64_t>(n, 1) * 3 / 2 + 1024;
-            W.hiKeys = (uint32_t*)S.dalloc(sizeof(uint32_t) * W.hiCap);
-            W.hiKeysSorted = (uint32_t*)S.dalloc(sizeof(uint32_t) * W.hiCap);
-            W.hiVals = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-            S.I.hiList = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-            S.I.slotLo = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-            S.I.slotHi = (int32_t*)S.dalloc(sizeof(int32_t) * W.hiCap);
-            W.act = (uint64_t*)S.dalloc(sizeof(uint64_t) * (W.hiCap + 1));
-            // real contacts first: FP64 mode, and periodic scenes (see k_slots)
-            W.actReal = S.prec == WG_PREC_FP64 || peri ? (uint64_t*)S.dalloc(sizeof(uint64_t) * (W.hiCap + 1)) : nullptr;
-            S.I.work = (int4*)S.dalloc(sizeof(int4) * W.hiCap);
-            if (!S.I.slotHi || !W.act || !S.I.work || ((S.prec == WG_PREC_FP64 || peri) && !W.actReal))
-                return S.fail(WG_ERR_CUDA, "out of device memory (incidence)");
-        }
-        auto scan = [&](uint32_t real, uint64_t* out) -> int {
-            const auto in = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), WorkClass{S.C.flags, S.C.cdist, n, real});
-            size_t tb = 0;
-            cub::DeviceScan::ExclusiveSum(nullptr, tb, in, out, (int)(n + 1), st);
-            if (ensureCub(S, tb)) return WG_ERR_CUDA;
-            tb = W.cubBytes;
-            WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, in, out, (int)(n + 1), st));
-            return 0;
-        };
-        r = scan(0, W.act);
-        if (!r && W.actReal) r = scan(C_REAL, W.actReal);
+        // 6. CSR incidence over the active contacts
+        undo.incidence = true;
+        r = incidence(S, n, W.newLo);
         if (r) return r;
-        const uint64_t* const act = W.act + n;  // the totals
-        k_lo_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.newLo, (int)S.nPar, W.act, S.I.loStart);
-        if (S.I.endCap < 2 * std::max<int64_t>(n, 1)) {
-            if (S.I.endA) { S.dfree(S.I.endA); S.dfree(S.I.endB); }
-            if (S.I.endAf) { S.dfree(S.I.endAf); S.dfree(S.I.endBf); }
-            S.I.endA = nullptr; S.I.endB = nullptr; S.I.endAf = nullptr; S.I.endBf = nullptr;
-            S.I.endCap = 2 * std::max<int64_t>(n, 1) * 5 / 4 + 2048;
-            if (S.prec == WG_PREC_FP32) {
-                S.I.endAf = (float4*)S.dalloc(sizeof(float4) * S.I.endCap);
-                S.I.endBf = (float2*)S.dalloc(sizeof(float2) * S.I.endCap);
-                if (!S.I.endAf || !S.I.endBf) return S.fail(WG_ERR_CUDA, "out of device memory (contact ends)");
-            } else {
-                S.I.endA = (double4_32a*)S.dalloc(sizeof(double4_32a) * S.I.endCap);
-                S.I.endB = (double2*)S.dalloc(sizeof(double2) * S.I.endCap);
-                if (!S.I.endA || !S.I.endB) return S.fail(WG_ERR_CUDA, "out of device memory (contact ends)");
-            }
-        }
-        int hiBits = 1;  // bits of the largest hi key, nPar
-        while ((int64_t(1) << hiBits) <= S.nPar) hiBits++;
-        if (n > 0) {
-            k_hi_keys<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, n, (uint32_t)S.nPar, W.hiKeys, W.hiVals);
-            size_t tb = 0;
-            cub::DeviceRadixSort::SortPairs(nullptr, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiBits, st);
-            if (ensureCub(S, tb)) return WG_ERR_CUDA;
-            tb = W.cubBytes;
-            WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiBits, st));
-        }
-        k_hi_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.hiKeysSorted, n, (int)S.nPar, S.I.hiStart);
-        if (n > 0) {
-            k_slots<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, S.I);
-            k_zero_ends<<<(unsigned)((2 * n + BS - 1) / BS), BS, 0, st>>>(S.I, act);
-        }
-        // FP32-force mode, aperiodic scenes: the sphere-sphere contacts' state in work-list order
-        if (packed && n > 0) {
-            DevPackedSS& Q = W.Kb;
-            W.packIdxB = grow(S, W.packIdxB, W.packIdxCapB, n);
-            if (!W.packIdxB) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
-            if (Q.cap < n) {
-                S.dfree(Q.item); S.dfree(Q.flags);
-                for (int q = 0; q < CF_NCOL; q++) S.dfree(Q.col[q]);
-                S.dfree(Q.ft[0]); S.dfree(Q.ft[1]);
-                Q = DevPackedSS{};
-                Q.cap = n * 5 / 4 + 4096;
-                Q.item = (int4*)S.dalloc(sizeof(int4) * Q.cap);
-                Q.flags = (uint32_t*)S.dalloc(sizeof(uint32_t) * Q.cap);
-                bool ok = Q.item && Q.flags;
-                for (int q = 0; q < CF_NCOL; q++) {
-                    Q.col[q] = (float*)S.dalloc(sizeof(float) * Q.cap);
-                    ok = ok && Q.col[q];
-                }
-                // the IdealElPl shear force (a serving slot may take a job with that law at any time)
-                Q.ft[0] = (double*)S.dalloc(sizeof(double) * Q.cap);
-                Q.ft[1] = (double*)S.dalloc(sizeof(double) * Q.cap);
-                ok = ok && Q.ft[0] && Q.ft[1];
-                if (!ok) {
-                    Q.cap = 0;
-                    return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
-                }
-            }
-            Q.ftLive = law0;
-            launch_pack_ss(st, S.C, S.I, S.P, Kold, Q, packedState ? W.packIdx : nullptr, W.src, W.packIdxB, act, n);
-        }
-        k_heavy<<<(unsigned)((S.nPar + BS - 1) / BS), BS, 0, st>>>(S.I, S.P, S.N.flags, kHeavyThreshold, W.tot, W.act, W.actReal, n);
         WG_CUDA_TRY(cudaMemcpyAsync(W.hTot, W.tot, sizeof(CollideTotals), cudaMemcpyDeviceToHost, st));
         WG_CUDA_TRY(cudaStreamSynchronize(st));
         const CollideTotals& T = *W.hTot;
         if (!lookForOrphans && T.real != T.kept) {
             // again, with the real contacts that have no overlap any more: the old set is in the spare arrays
             lookForOrphans = true;
-            std::swap(S.C, S.Cb);
+            undo.swap();
             WG_CUDA_TRY(cudaMemsetAsync(&W.tot->heavy, 0, 2 * sizeof(int32_t), st));
             continue;
         }
         const int64_t nAct = (int64_t)(uint32_t)T.act, nSS = (int64_t)(T.act >> 32);
-        S.I.nAct = nAct;
-        S.nMixed = nAct - nSS;
-        if (packed && n > 0) {
+        // what takes memory for the active contacts, then the new set takes the old one's place
+        r = endRoom(S, nAct);
+        if (r) return r;
+        if (packed) {
+            DevPackedSS& Q = W.Kb;
+            if (!scratch(S, W.packIdxCapB, n, W.packIdxB)) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
+            r = packRoom(S, Q, nSS);
+            if (r) return r;
+            Q.n = nSS;
+            Q.ftLive = law0;
+            launch_pack_ss(st, S.C, S.I, S.P, S.K, Q, packedState ? W.packIdx : nullptr, W.src, W.packIdxB, W.act + n, nSS);
             std::swap(S.K, W.Kb);
             std::swap(W.packIdx, W.packIdxB);
             std::swap(W.packIdxCap, W.packIdxCapB);
-            W.packIdxValid = true;
         }
-        S.K.n = packed ? nSS : 0;
+        undo.off = true;
+        if (nAct > 0) k_zero_ends<<<(unsigned)((2 * nAct + BS - 1) / BS), BS, 0, st>>>(S.I, 2 * nAct);
+        S.I.nAct = nAct;
+        S.nMixed = nAct - nSS;
         S.packDirty = packedState && nSS > 0;  // the contact arrays hold no state of those contacts then
         S.I.nHeavy = S.cfg.apply_forces ? T.heavy : 0;
         S.I.nHeavyFree = S.cfg.apply_forces ? T.heavyFree : 0;
+        S.contactsReplaced = false;
         break;
     }
     std::swap(W.newLo, W.oldLo);
@@ -1666,6 +1740,14 @@ int collide_full_run(Sim& S) {
     WG_CUDA_TRY(cudaGetLastError());
     S.nFullRuns++;
     return 0;
+}
+
+// A run that fails leaves the contacts, their state and their forces as they were; the boxes and the verlet
+// reference positions are those of the failed run, so that the next step starts with a full run.
+int collide_full_run(Sim& S) {
+    const int r = fullRun(S);
+    if (r) S.forceFull = true;
+    return r;
 }
 
 void collide_free(Sim& S) {

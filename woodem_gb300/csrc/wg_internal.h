@@ -414,6 +414,7 @@ struct Sim {
     int* hFlags = nullptr;   // pinned mirror
     double* hDown = nullptr; // pinned buffers of the threads that download a large state
     std::vector<void*> allocs;
+    int64_t failAlloc = -1;  // wg_fail_alloc: the allocations left before one fails, -1: none does
     CollideWork* cw = nullptr;
     bool uploaded = false, initialized = false;
     int64_t step = 0;
