@@ -1084,6 +1084,8 @@ int Sim::run(int64_t n) {
     const bool fp32 = prec == WG_PREC_FP32;
     bool anyLaw0 = cfg.law == 0;
     for (const wg_config& c : cfgs) anyLaw0 = anyLaw0 || c.law == 0;
+    // a job with that law may just have come into a slot: the full run before its first contacts makes room
+    auto loadFt = [&]() { return anyLaw0 && K.ft[0]; };
     auto stepLeapfrog = [&](int fromEndsArg, ScenePar* sp) {
         if (fromEndsArg) {
             if (fp32) launch_forces32(stream, N, P, I, dNodeC, sp, dFlags, true);
@@ -1112,7 +1114,7 @@ int Sim::run(int64_t n) {
             // the energy sums after the contact kernels read the step counter those advance: they
             // run with the step advance at the end instead
             cudaMemsetAsync(eCon.col, 0, sizeof(double) * EN_CON_NCOL * eCon.cap, stream);
-            launch_contact_fp32(stream, SideStream{}, N, P, C, I, K, dMats, sp, dStep, dFlags, nMixed, cfg.periodic != 0, anyLaw0,
+            launch_contact_fp32(stream, SideStream{}, N, P, C, I, K, dMats, sp, dStep, dFlags, nMixed, cfg.periodic != 0, loadFt(),
                                 !facetsStatic, 128, &eCon);
             launch_energy_sum(stream, eCon, 1, I.nAct, dEPartial, dEnergy, dECreated, dFlags, false);
             launches += 2;
@@ -1123,7 +1125,7 @@ int Sim::run(int64_t n) {
             }
         } else if (fp32)
             advanced = launch_contact_fp32(stream, concurrentContacts ? side : SideStream{}, N, P, C, I, K, dMats, sp, dStep, dFlags,
-                                           nMixed, cfg.periodic != 0, anyLaw0, !facetsStatic, contactBlock != 0 ? contactBlock : -256);
+                                           nMixed, cfg.periodic != 0, loadFt(), !facetsStatic, contactBlock != 0 ? contactBlock : -256);
         else if (trackE) {
             cudaMemsetAsync(eCon.col, 0, sizeof(double) * EN_CON_NCOL * eCon.cap, stream);
             launch_contact_fp64(stream, N, P, C, I, dMats, sp, dStep, dFlags, cfg.periodic != 0,
@@ -1228,7 +1230,7 @@ int Sim::run(int64_t n) {
             unsigned long long* ns = (unsigned long long*)dNs;
             const int from = fromEnds ? 1 : 0;
             const int r = fp32 ? launch_steps32(stream, N, P, C, I, K, dNodeC, dMats, spOf(0), cfg.periodic != 0, dStep, dFlags, bar, ns,
-                                                nMixed, anyLaw0, from, (int)k)
+                                                nMixed, loadFt(), from, (int)k)
                                : launch_steps64(stream, N, P, C, I, dMats, spOf(0), cfg.periodic != 0, dStep, dFlags, bar, ns, from, (int)k);
             if (r) {
                 cudaGetLastError();

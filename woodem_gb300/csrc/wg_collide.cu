@@ -1395,22 +1395,24 @@ static int endRoom(Sim& S, int64_t nAct) {
     S.I.endCap = cap;
     return 0;
 }
-// Room in Q, whose contents need not last, for n packed contacts.
-static int packRoom(Sim& S, DevPackedSS& Q, int64_t n) {
-    if (Q.cap >= n) return 0;
-    S.dfree(Q.item); S.dfree(Q.flags);
-    for (int q = 0; q < CF_NCOL; q++) S.dfree(Q.col[q]);
-    S.dfree(Q.ft[0]); S.dfree(Q.ft[1]);
+// Room in Q, whose contents need not last, for n packed contacts, in one block of memory. ft: with the IdealElPl
+// shear force.
+static int packRoom(Sim& S, DevPackedSS& Q, int64_t n, bool ft) {
+    if (Q.cap >= n && (Q.ft[0] || !ft)) return 0;
+    S.dfree(Q.item);
     Q = DevPackedSS{};
-    const int64_t cap = n * 5 / 4 + 4096;
-    Larger L(S);
-    L.add(Q.item, cap);
-    L.add(Q.flags, cap);
-    for (int q = 0; q < CF_NCOL; q++) L.add(Q.col[q], cap);
-    // the IdealElPl shear force (a serving slot may take a job with that law at any time)
-    L.add(Q.ft[0], cap);
-    L.add(Q.ft[1], cap);
-    if (!L.put()) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
+    const int64_t cap = (n * 5 / 4 + 4096) / 64 * 64;  // every column is aligned
+    char* p = (char*)S.dalloc((size_t)cap * (sizeof(int4) + (ft ? 2 * sizeof(double) : 0) + sizeof(uint32_t) + CF_NCOL * sizeof(float)));
+    if (!p) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
+    auto take = [&](size_t bytes) {
+        void* const at = p;
+        p += bytes * cap;
+        return at;
+    };
+    Q.item = (int4*)take(sizeof(int4));
+    for (int q = 0; ft && q < 2; q++) Q.ft[q] = (double*)take(sizeof(double));
+    Q.flags = (uint32_t*)take(sizeof(uint32_t));
+    for (int q = 0; q < CF_NCOL; q++) Q.col[q] = (float*)take(sizeof(float));
     Q.cap = cap;
     return 0;
 }
@@ -1714,7 +1716,7 @@ static int fullRun(Sim& S) {
         if (packed) {
             DevPackedSS& Q = W.Kb;
             if (!scratch(S, W.packIdxCapB, n, W.packIdxB)) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
-            r = packRoom(S, Q, nSS);
+            r = packRoom(S, Q, nSS, law0 || S.P.fresh);  // a serving slot may take a job with that law at any time
             if (r) return r;
             Q.n = nSS;
             Q.ftLive = law0;

@@ -197,13 +197,14 @@ constexpr int kLeapfrogChunk32 = 256;
 // [nMixed, nAct)) held in work-list order, so that the per-step kernel loads and stores it
 // coalesced, with the particle ids and end slots beside it. Filled from the contact arrays at
 // each full collider run and written back before the next one and before the host reads the
-// contacts; the contact arrays hold the state of those contacts only after such a write-back.
+// contacts; the contact arrays hold the state of those contacts only after such a write-back. One block of
+// memory, which begins with the items.
 struct DevPackedSS {
     int64_t n = 0, cap = 0;
     int4* item = nullptr;      // (pA, pB, end slot of pA, end slot of pB)
     uint32_t* flags = nullptr; // contact flags | scene << 8
     float* col[CF_NCOL] = {};
-    double* ft[2] = {};        // IdealElPl shear force
+    double* ft[2] = {};        // IdealElPl shear force; none where no scene can use that law
     bool ftLive = false;       // ft is copied (some scene used IdealElPl at the last full run); it is
                                // read only for contacts of scenes with that law
 };
@@ -257,7 +258,7 @@ int launch_steps64(cudaStream_t st, const DevNodes& N, const DevParticles& P, co
                    unsigned long long* ns, int fromEnds, int steps);
 int launch_steps32(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
                    const DevPackedSS& K, const NodeConst32* nc, const double4_32a* mats, const ScenePar* sp, bool periodic,
-                   long long* dStep, int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool anyLaw0, int fromEnds,
+                   long long* dStep, int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool loadFt, int fromEnds,
                    int steps);
 // perStep: only the heavy particles with a free DOF (guarded by the flags), before Leapfrog;
 // otherwise every particle's DemData.force/torque (reporting at the end of a run).
@@ -299,7 +300,7 @@ struct SideStream {
 // Returns true when the sphere-sphere kernel, last of the step, also advanced the step counter.
 bool launch_contact_fp32(cudaStream_t st, const SideStream& side, const DevNodes& N, const DevParticles& P, const DevContacts& C,
                          const DevIncidence& I, const DevPackedSS& K, const double4_32a* mats, const ScenePar* sp,
-                         long long* dStep, int* dFlags, int64_t nMixed, bool periodic, bool anyLaw0, bool prepFacets,
+                         long long* dStep, int* dFlags, int64_t nMixed, bool periodic, bool loadFt, bool prepFacets,
                          int block = 256, const EnergyCols* energy = nullptr);
 // pack: the packed state K of a new contact set (whose active contacts are counted in the low half of *act
 // on the device, the plain ones in its high half, at most `most`), in tiles with the real ones first

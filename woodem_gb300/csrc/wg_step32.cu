@@ -870,7 +870,7 @@ void launch_pack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I
                     const DevPackedSS& K, const int32_t* oldIdx, const int32_t* src, int32_t* idx, const uint64_t* act, int64_t most) {
     if (most > 0)
         k_pack_ss<<<(unsigned)((most + kPackTile - 1) / kPackTile), kPackTile, 0, st>>>(C, I, P, Kold, K, oldIdx, src, idx, act,
-                                                                                       K.ftLive ? 1 : 0);
+                                                                                       K.ftLive && (!oldIdx || Kold.ft[0]) ? 1 : 0);
 }
 void launch_unpack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevPackedSS& K, int64_t nMixed, bool flagsOnly) {
     if (K.n > 0) k_unpack_ss<<<(unsigned)((K.n + 255) / 256), 256, 0, st>>>(C, I, K, nMixed, K.ftLive ? 1 : 0, flagsOnly ? 1 : 0);
@@ -1329,7 +1329,7 @@ __global__ void __launch_bounds__(256, MINB) k_contact_all32(DevNodes N, DevPart
 template <bool ENERGY>
 static bool contactsFP32(cudaStream_t st, const SideStream& side, const DevNodes& N, const DevParticles& P, const DevContacts& C,
                          const DevIncidence& I, const DevPackedSS& K, const double4_32a* mats, const ScenePar* sp,
-                         long long* dStep, int* dFlags, int64_t nMixed, bool periodic, bool anyLaw0, bool prepFacets,
+                         long long* dStep, int* dFlags, int64_t nMixed, bool periodic, bool loadFt, bool prepFacets,
                          int block, const EnergyCols& E) {
     const int64_t nm = periodic ? I.nAct : std::min<int64_t>(nMixed, I.nAct);
     const int64_t ns = periodic ? 0 : K.n;
@@ -1337,7 +1337,7 @@ static bool contactsFP32(cudaStream_t st, const SideStream& side, const DevNodes
         if (nm > 0 && prepFacets) launch_facet_prep(st, N, P, dFlags);
         const int64_t want = ((ns + 31) / 32 + (nm + 31) / 32 + 7) / 8;
         const int g = (int)std::min<int64_t>(want, (int64_t)kSSMinBlocks * smCount());
-        k_contact_all32<kSSMinBlocks><<<(unsigned)g, 256, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, anyLaw0);
+        k_contact_all32<kSSMinBlocks><<<(unsigned)g, 256, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, loadFt);
         return true;
     }
     const unsigned gS = ns > 0 ? (unsigned)((ns + block - 1) / block) : 0u;
@@ -1349,7 +1349,7 @@ static bool contactsFP32(cudaStream_t st, const SideStream& side, const DevNodes
         cudaStreamWaitEvent(side.st, side.fork, 0);
         if (prepFacets) launch_facet_prep(side.st, N, P, dFlags);
         k_contact_fp32<false, ENERGY><<<(unsigned)gM, 128, 0, side.st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 0, 0, E);
-        k_contact_ss32<kSSMinBlocks, ENERGY><<<gS, (unsigned)block, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, 1, anyLaw0, E);
+        k_contact_ss32<kSSMinBlocks, ENERGY><<<gS, (unsigned)block, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, 1, loadFt, E);
         cudaEventRecord(side.join, side.st);
         cudaStreamWaitEvent(st, side.join, 0);
         return false;
@@ -1362,18 +1362,18 @@ static bool contactsFP32(cudaStream_t st, const SideStream& side, const DevNodes
     if (periodic) k_contact_fp32<true, ENERGY><<<(unsigned)gM, 128, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 1, total, E);
     else k_contact_fp32<false, ENERGY><<<(unsigned)gM, 128, 0, st>>>(N, P, C, I, mats, sp, dStep, dFlags, 0, nm, 1, total, E);
     if (ns > 0)
-        k_contact_ss32<kSSMinBlocks, ENERGY><<<gS, (unsigned)block, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, 0, anyLaw0, E);
+        k_contact_ss32<kSSMinBlocks, ENERGY><<<gS, (unsigned)block, 0, st>>>(N, P, C, I, K, mats, sp, dStep, dFlags, nm, 0, loadFt, E);
     return total > 0;
 }
 
 bool launch_contact_fp32(cudaStream_t st, const SideStream& side, const DevNodes& N, const DevParticles& P, const DevContacts& C,
                          const DevIncidence& I, const DevPackedSS& K, const double4_32a* mats, const ScenePar* sp,
-                         long long* dStep, int* dFlags, int64_t nMixed, bool periodic, bool anyLaw0, bool prepFacets,
+                         long long* dStep, int* dFlags, int64_t nMixed, bool periodic, bool loadFt, bool prepFacets,
                          int block, const EnergyCols* energy) {
     if (energy)
-        return contactsFP32<true>(st, side, N, P, C, I, K, mats, sp, dStep, dFlags, nMixed, periodic, anyLaw0, prepFacets, block,
+        return contactsFP32<true>(st, side, N, P, C, I, K, mats, sp, dStep, dFlags, nMixed, periodic, loadFt, prepFacets, block,
                                   *energy);
-    return contactsFP32<false>(st, side, N, P, C, I, K, mats, sp, dStep, dFlags, nMixed, periodic, anyLaw0, prepFacets, block,
+    return contactsFP32<false>(st, side, N, P, C, I, K, mats, sp, dStep, dFlags, nMixed, periodic, loadFt, prepFacets, block,
                                EnergyCols{});
 }
 
@@ -1444,15 +1444,15 @@ __global__ void __launch_bounds__(kSteps32Threads, 1) k_steps32(DevNodes N, DevP
 
 int launch_steps32(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
                    const DevPackedSS& K, const NodeConst32* nc, const double4_32a* mats, const ScenePar* sp, bool periodic, long long* dStep,
-                   int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool anyLaw0, int fromEnds, int steps) {
+                   int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool loadFt, int fromEnds, int steps) {
     DevNodes n = N;
     DevParticles p = P;
     DevContacts c = C;
     DevIncidence i = I;
     DevPackedSS k = K;
-    int seq = periodic ? 1 : 0, loadFt = anyLaw0 ? 1 : 0;
+    int seq = periodic ? 1 : 0, ft = loadFt ? 1 : 0;
     int64_t nm = periodic ? I.nAct : std::min<int64_t>(nMixed, I.nAct);
-    void* args[] = {&n, &p, &c, &i, &k, &nc, &mats, &sp, &seq, &dStep, &dFlags, &bar, &ns, &nm, &loadFt, &fromEnds, &steps};
+    void* args[] = {&n, &p, &c, &i, &k, &nc, &mats, &sp, &seq, &dStep, &dFlags, &bar, &ns, &nm, &ft, &fromEnds, &steps};
     const int64_t items = std::max<int64_t>(N.n, I.nAct);
     const void* f = periodic ? (const void*)k_steps32<true> : (const void*)k_steps32<false>;
     const int g = stepsGrid(f, kSteps32Threads, kSteps32Shared, items);

@@ -20,8 +20,9 @@ import numpy as np
 
 from . import _native, _plan
 
-# device bytes per particle held by the GPU path (state, mirrors, contacts with ~6 potential
-# contacts per sphere, incidence, collider scratch); used for admission
+# device bytes per particle held by the GPU path (state, mirrors, contacts, incidence, collider scratch), used for
+# admission: an estimate for scenes with few potential contacts. Measured with 5 of them per sphere: 3500 (drum of a
+# million, FP32-force mode), 3600 (batch), 3800 to 3900 (periodic FP32, FP64 drum), 4700 (periodic FP64)
 BYTES_PER_PARTICLE = 3000
 
 

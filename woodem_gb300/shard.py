@@ -23,8 +23,8 @@ import threading
 
 import numpy as np
 
-# device bytes per particle of the GPU path (state, mirrors, ~6 potential contacts per sphere,
-# incidence, collider scratch), the unit of the footprint
+# device bytes per particle of the GPU path (state, mirrors, contacts, incidence, collider scratch), the unit of the
+# footprint: scenes with 5 potential contacts per sphere take 3500 to 4700
 BYTES_PER_PARTICLE = 3000
 
 
