@@ -242,6 +242,9 @@ int wg_get_contacts(wg_scene* s, int32_t* id_lo, int32_t* id_hi, int32_t* id_a, 
                     int32_t* cell_dist, double* fglob, double* local, double* cpt, double* trsf);
 /* Aabb.min/max per particle from the last full run (verletDist included), 3 doubles each. */
 int wg_get_aabbs(wg_scene* s, double* mn, double* mx);
+/* The uniform grid of the last full run over the spheres of scene k: its origin, the edge of its cells (slightly more
+   than the largest sphere box, unless that made too many of them) and their number per axis. */
+int wg_get_grid(wg_scene* s, int32_t k, double* origin3, double* cell, int32_t* dims3);
 /* Run only the broad phase on the current positions (full run), no stepping. */
 int wg_collide_only(wg_scene* s);
 

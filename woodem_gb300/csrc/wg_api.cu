@@ -2436,6 +2436,19 @@ int wg_get_aabbs(wg_scene* s, double* mn, double* mx) {
     return WG_OK;
 }
 
+int wg_get_grid(wg_scene* s, int32_t k, double* origin3, double* cell, int32_t* dims3) {
+    if (!s || !origin3 || !cell || !dims3) return WG_ERR_ARG;
+    Sim& S = *SIM(s);
+    if (k < 0 || k >= S.nScenes) return S.fail(WG_ERR_ARG, "scene index out of range");
+    Grid g;
+    const int r = read_grid(S, k, g);
+    if (r) return r;
+    origin3[0] = g.ox; origin3[1] = g.oy; origin3[2] = g.oz;
+    *cell = g.h;
+    dims3[0] = g.nx; dims3[1] = g.ny; dims3[2] = g.nz;
+    return WG_OK;
+}
+
 int wg_fail_alloc(wg_scene* s, int64_t n) {
     if (!s) return WG_ERR_ARG;
     SIM(s)->failAlloc = n;

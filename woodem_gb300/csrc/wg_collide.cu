@@ -64,7 +64,7 @@ struct CollideWork {
     bool oldLoValid = false;
     int32_t* cellOff = nullptr;   // first sphere of each cell
     int64_t cellOffCap = 0;
-    float* red = nullptr;         // reduction partials
+    double* red = nullptr;        // reduction partials
     std::vector<int32_t> hChunk;      // grid-reduction chunks of sphereIds (never across scenes)
     std::vector<int32_t> hSceneChunk; // chunks of scene k: [hSceneChunk[k], hSceneChunk[k+1])
     std::vector<int64_t> hSceneSph;   // spheres of scene k: sphereIds[hSceneSph[k] .. hSceneSph[k+1])
@@ -209,43 +209,46 @@ __device__ __forceinline__ float nextUp(float f) {
     return f == 0.f ? __int_as_float(1) : __int_as_float(f > 0.f ? u + 1 : u - 1);
 }
 
+// An integer that orders FP64 numbers as they are (the same function takes it back). Minima and maxima of
+// doubles would occupy the FP64 pipe, which those of integers do not.
+__device__ __forceinline__ long long orderOf(long long bits) { return bits ^ ((bits >> 63) & 0x7fffffffffffffffLL); }
+
 // ---------------------------------------------------------------- grid bounds over spheres
 // partial[b] = {min mn.x, min mn.y, min mn.z, max mn.x, max mn.y, max mn.z, max extent} over the
-// spheres ids[chunk[b] .. chunk[b+1]) (chunks never span two scenes of a batch), rounded outward to FP32: the
-// grid only has to hold the boxes, and minima in FP64 bound this pass by its pipe.
+// spheres ids[chunk[b] .. chunk[b+1]) (chunks never span two scenes of a batch), in FP64: rounded to FP32 where
+// they stand, boxes of 1 cm at coordinates of 1e6 m would make the cells ten times too long.
 __global__ void k_grid_reduce(DevParticles P, const int32_t* __restrict__ ids, const int32_t* __restrict__ chunk,
-                              float* __restrict__ partial) {
-    __shared__ float s[7][BS / 32];
+                              double* __restrict__ partial) {
+    __shared__ long long s[7][BS / 32];
     const unsigned FULL = 0xffffffffu;
-    const float inf = __int_as_float(0x7f800000);
-    float v[7] = {inf, inf, inf, -inf, -inf, -inf, 0.f};
-    bool bad = false;  // a minimum would drop a NaN
+    const long long INF = 0x7ff0000000000000LL, most = orderOf(INF), least = orderOf(INF | (1LL << 63));
+    long long v[7] = {most, most, most, least, least, least, 0};
+    bool bad = false;  // an edge that is not finite: a NaN or infinite position
     for (int i = chunk[blockIdx.x] + threadIdx.x; i < chunk[blockIdx.x + 1]; i += blockDim.x) {
         const int p = ids[i];
         const double4_32a a = P.mn[p], b = P.mx[p];
-        const float lo[3] = {__double2float_rd(a.x), __double2float_rd(a.y), __double2float_rd(a.z)};
-        const float hi[3] = {__double2float_ru(b.x), __double2float_ru(b.y), __double2float_ru(b.z)};
+        const double lo[3] = {a.x, a.y, a.z}, hi[3] = {b.x, b.y, b.z};
         for (int q = 0; q < 3; q++) {
-            const float up = nextUp(lo[q]), e = __fsub_ru(hi[q], lo[q]);
-            bad = bad || !(e < inf);
-            v[q] = fminf(v[q], lo[q]);
-            v[3 + q] = fmaxf(v[3 + q], up);
-            v[6] = fmaxf(v[6], e);
+            const long long u = orderOf(__double_as_longlong(lo[q])), e = __double_as_longlong(hi[q] - lo[q]);
+            bad = bad || (e & INF) == INF;
+            v[q] = min(v[q], u);
+            v[3 + q] = max(v[3 + q], u);
+            v[6] = max(v[6], e);
         }
     }
-    if (bad) v[6] = inf;
+    if (bad) v[6] = INF;
     for (int o = 16; o > 0; o >>= 1) {
-        for (int q = 0; q < 3; q++) v[q] = fminf(v[q], __shfl_down_sync(FULL, v[q], o));
-        for (int q = 3; q < 7; q++) v[q] = fmaxf(v[q], __shfl_down_sync(FULL, v[q], o));
+        for (int q = 0; q < 3; q++) v[q] = min(v[q], __shfl_down_sync(FULL, v[q], o));
+        for (int q = 3; q < 7; q++) v[q] = max(v[q], __shfl_down_sync(FULL, v[q], o));
     }
     if ((threadIdx.x & 31) == 0)
         for (int q = 0; q < 7; q++) s[q][threadIdx.x >> 5] = v[q];
     __syncthreads();
     if (threadIdx.x < 7) {
         const int q = threadIdx.x;
-        float m = s[q][0];
-        for (int w = 1; w < BS / 32; w++) m = q < 3 ? fminf(m, s[q][w]) : fmaxf(m, s[q][w]);
-        partial[blockIdx.x * 7 + q] = m;
+        long long m = s[q][0];
+        for (int w = 1; w < BS / 32; w++) m = q < 3 ? min(m, s[q][w]) : max(m, s[q][w]);
+        partial[blockIdx.x * 7 + q] = __longlong_as_double(orderOf(m));
     }
 }
 
@@ -256,22 +259,23 @@ __host__ __device__ __forceinline__ int64_t cellBound(int64_t spheres, int scene
     const int64_t least = scenes > 1 ? 64 : 1 << 16;
     return 8 * spheres > least ? 8 * spheres : least;
 }
+constexpr double kCellMargin = 2e-6;
 __global__ void __launch_bounds__(256) k_make_grids(int K, const int32_t* __restrict__ chunk, const int32_t* __restrict__ sceneChunk,
-                                                    const float* __restrict__ partial, const ScenePar* __restrict__ spp, int peri,
+                                                    const double* __restrict__ partial, const ScenePar* __restrict__ spp, int peri,
                                                     Grid* __restrict__ out, int* __restrict__ bad) {
     const unsigned FULL = 0xffffffffu;
-    const float inf = __int_as_float(0x7f800000);
+    const double inf = __longlong_as_double(0x7ff0000000000000LL);
     const int lane = threadIdx.x & 31;
     for (int k = threadIdx.x >> 5; k < K; k += blockDim.x >> 5) {
         const int c0 = sceneChunk[k], c1 = sceneChunk[k + 1];
-        float v[7] = {inf, inf, inf, -inf, -inf, -inf, 0.f};
+        double v[7] = {inf, inf, inf, -inf, -inf, -inf, 0.};  // these drop a NaN, whose edge is infinite here
         for (int b = c0 + lane; b < c1; b += 32) {
-            for (int q = 0; q < 3; q++) v[q] = fminf(v[q], partial[7 * b + q]);
-            for (int q = 3; q < 7; q++) v[q] = fmaxf(v[q], partial[7 * b + q]);
+            for (int q = 0; q < 3; q++) v[q] = fmin(v[q], partial[7 * b + q]);
+            for (int q = 3; q < 7; q++) v[q] = fmax(v[q], partial[7 * b + q]);
         }
         for (int o = 16; o > 0; o >>= 1) {
-            for (int q = 0; q < 3; q++) v[q] = fminf(v[q], __shfl_down_sync(FULL, v[q], o));
-            for (int q = 3; q < 7; q++) v[q] = fmaxf(v[q], __shfl_down_sync(FULL, v[q], o));
+            for (int q = 0; q < 3; q++) v[q] = fmin(v[q], __shfl_down_sync(FULL, v[q], o));
+            for (int q = 3; q < 7; q++) v[q] = fmax(v[q], __shfl_down_sync(FULL, v[q], o));
         }
         if (lane) continue;
         Grid g{0, 0, 0, 1, 1, 1, 1, 1, 1, 0, 0};
@@ -281,8 +285,8 @@ __global__ void __launch_bounds__(256) k_make_grids(int K, const int32_t* __rest
             if (!fine) *bad = 1;
             else {
                 const int64_t most = cellBound((int64_t)chunk[c1] - chunk[c0], K);
-                double h = (double)v[6] * (1 + 1e-9) + 1e-300;
-                const double ext[3] = {(double)v[3] - v[0], (double)v[4] - v[1], (double)v[5] - v[2]};
+                double h = v[6] * (1 + kCellMargin) + 1e-300;
+                const double ext[3] = {v[3] - v[0], v[4] - v[1], v[5] - v[2]};
                 int64_t dims[3];
                 for (;;) {
                     for (int q = 0; q < 3; q++) {
@@ -297,6 +301,10 @@ __global__ void __launch_bounds__(256) k_make_grids(int K, const int32_t* __rest
                 g.rh = 1. / h;
                 g.nx = (int32_t)dims[0]; g.ny = (int32_t)dims[1]; g.nz = (int32_t)dims[2];
                 g.ncell = dims[0] * dims[1] * dims[2];
+                // coordinates that FP32 numbers resolve badly, compared with a cell: the boxes in cell order are
+                // kept relative to the grid's origin
+                for (int q = 0; q < 6; q++)
+                    if (fabs(v[q]) > 4096. * h) g.far = 1;
                 if (peri)
                     for (int q = 0; q < 3; q++)
                         if (!(h <= 0.49 * spp->cellSize[q])) g.exact = 1;
@@ -314,7 +322,7 @@ __global__ void __launch_bounds__(256) k_make_grids(int K, const int32_t* __rest
     }
 }
 
-// rh = 1/h: the product is off by less than the margin of 1e-9 that h has over the largest box
+// rh = 1/h: over 2^31 cells the product is off by less than half the margin that h has over the largest box
 __device__ __forceinline__ int cellCoord(double v, double o, double rh, int n) {
     const int ci = __double2int_rd((v - o) * rh);
     return ci < 0 ? 0 : (ci >= n ? n - 1 : ci);
@@ -352,14 +360,24 @@ __device__ __forceinline__ int64_t lowerBound64(const uint64_t* a, int64_t n, ui
     return lo;
 }
 
-// the spheres' boxes in cell order, rounded outward to FP32
-__global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ ids, int n, const uint32_t* __restrict__ key,
+// the spheres' boxes in cell order, rounded outward to FP32 (of a grid far from zero, relative to its origin: the
+// subtraction keeps their order, and so what overlapF and overlapOuter conclude from it)
+__device__ __forceinline__ double4_32a relative(const Grid& G, const double4_32a& a) {
+    return make_double4_32a(a.x - G.ox, a.y - G.oy, a.z - G.oz, 0.);
+}
+__global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ ids, int n, const Grid* __restrict__ Gs,
+                                const uint32_t* __restrict__ key,
                                 const int32_t* __restrict__ rank, const int32_t* __restrict__ off, uint32_t* __restrict__ skey,
                                 float4* __restrict__ smnf, float4* __restrict__ smxf) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int p = ids[i];
-    const double4_32a a = P.mn[p], b = P.mx[p];
+    double4_32a a = P.mn[p], b = P.mx[p];
+    const Grid& G = Gs[sceneOfP(P, p)];
+    if (G.far) {
+        a = relative(G, a);
+        b = relative(G, b);
+    }
     const int at = off[key[i]] + rank[i];
     skey[at] = key[i];
     smnf[at] = make_float4(__double2float_rd(a.x), __double2float_rd(a.y), __double2float_rd(a.z), __uint_as_float(P.mask[p]));
@@ -523,8 +541,9 @@ __global__ void k_pairs_local(DevParticles P, const int32_t* __restrict__ lids, 
     const int p = lids[t];
     const Grid G = Gs[sceneOfP(P, p)];
     const double4_32a mn1 = P.mn[p], mx1 = P.mx[p];
-    const float4 fn1 = make_float4(__double2float_rd(mn1.x), __double2float_rd(mn1.y), __double2float_rd(mn1.z), 0.f);
-    const float4 fx1 = make_float4(__double2float_ru(mx1.x), __double2float_ru(mx1.y), __double2float_ru(mx1.z), 0.f);
+    const double4_32a rn = G.far ? relative(G, mn1) : mn1, rx = G.far ? relative(G, mx1) : mx1;
+    const float4 fn1 = make_float4(__double2float_rd(rn.x), __double2float_rd(rn.y), __double2float_rd(rn.z), 0.f);
+    const float4 fx1 = make_float4(__double2float_ru(rx.x), __double2float_ru(rx.y), __double2float_ru(rx.z), 0.f);
     const uint32_t m1 = P.mask[p];
     const int x0 = cellCoord(mn1.x - G.h, G.ox, G.rh, G.nx), x1 = cellCoord(mx1.x, G.ox, G.rh, G.nx);
     const int y0 = cellCoord(mn1.y - G.h, G.oy, G.rh, G.ny), y1 = cellCoord(mx1.y, G.oy, G.rh, G.ny);
@@ -1186,6 +1205,13 @@ __global__ void k_count_packed(DevPackedSS K, int64_t p0, int64_t p1, unsigned l
     }
     addCounts(!(fl & C_REMOVED), (fl & C_REAL) && !(fl & C_REMOVED), out);
 }
+int read_grid(Sim& S, int k, Grid& g) {
+    if (!S.cw || !S.cw->dGrids) return S.fail(WG_ERR_STATE, "no grid before the first full run");
+    WG_CUDA_TRY(cudaSetDevice(S.device));
+    WG_CUDA_TRY(cudaMemcpyAsync(&g, S.cw->dGrids + k, sizeof g, cudaMemcpyDeviceToHost, S.stream));
+    WG_CUDA_TRY(cudaStreamSynchronize(S.stream));
+    return 0;
+}
 int count_contacts(Sim& S, int64_t p0, int64_t p1, int64_t out[2]) {
     out[0] = out[1] = 0;
     if (!S.uploaded || S.C.n == 0) return 0;
@@ -1534,7 +1560,7 @@ static int fullRun(Sim& S) {
         tb = W.cubBytes;
         WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, W.cellOff, W.cellOff, (int)(ncell + 1), st));
         if (peri) k_gather_peri<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.cellKey, W.cellRank, W.cellOff, S.dPar, W.skey, W.speri);
-        else k_gather_sorted<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.cellKey, W.cellRank, W.cellOff, W.skey, W.smnf, W.smxf);
+        else k_gather_sorted<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, W.cellKey, W.cellRank, W.cellOff, W.skey, W.smnf, W.smxf);
     }
     // lists of large particles: facets with boxes spanning a few cells use the grid, the rest are global
     {

@@ -323,11 +323,14 @@ struct Grid {
     int32_t nx, ny, nz;
     int64_t ncell;
     int64_t base;  // first cell key of this grid (a batch of scenes has one grid per scene)
+    int32_t far;   // the boxes in cell order are relative to the origin
     int32_t exact; // periodic: a box reaches about half the cell (see k_pairs_ss_peri)
 };
 struct CollideWork;  // scratch owned by the simulation
 struct Sim;
 int collide_full_run(Sim& S);
+// the grid of scene k
+int read_grid(Sim& S, int k, Grid& g);
 // contacts with their lo id in [p0, p1): out[0] not removed, out[1] real
 int count_contacts(Sim& S, int64_t p0, int64_t p1, int64_t out[2]);
 
