@@ -150,7 +150,9 @@ int wg_set_config(wg_scene* s, const wg_config* c);
 int wg_set_scenes(wg_scene* s, int32_t n_scenes, const wg_config* cfgs, const int64_t* particle_start);
 /* Launch shape (no counterpart in the reference): threads per block of the contact kernels
    (0 = default, 64, 128, 256; -256: the FP32 contacts through a resident grid whose threads prefetch
-   their next contact, as by default), steps queued per host check of the collider request (1..1024), and
+   their next contact, as by default), steps queued per host check of the collider request (1..1024: at
+   most, fewer about where the last interval between full runs ended; a launch of many steps at once, as small
+   scenes have by default, holds up to eight times as many), and
    flags: WG_LAUNCH_GRAPH replays each such chunk of steps as one CUDA graph, WG_LAUNCH_SERIAL, with a
    positive block size, runs the facet/wall contacts before the sphere-sphere ones instead of beside them
    on a second stream. Results do not depend on these; only the speed does. */
@@ -248,6 +250,9 @@ int wg_get_grid(wg_scene* s, int32_t k, double* origin3, double* cell, int32_t* 
 /* Run only the broad phase on the current positions (full run), no stepping. */
 int wg_collide_only(wg_scene* s);
 
+/* The rule behind that number where the steps are queued as single launches: at most `most` steps, `since` steps
+   after the last full run, which came `interval` steps after the one before it (0: not known). */
+int64_t wg_steps_to_queue(int64_t most, int64_t since, int64_t interval);
 /* For tests of what a failed call leaves behind: the n-th device allocation of the scene from now on (0: the
    next one) fails as if no memory were left. -1: none does. */
 int wg_fail_alloc(wg_scene* s, int64_t n);

@@ -1043,6 +1043,18 @@ int Sim::runDynDt(int64_t stepNow) {
     return 0;
 }
 
+// Steps to queue before the host looks for a full run's request, of at most `most`: since, the steps from the last full
+// run, interval, those between the two before (0: unknown). Steps queued past a request do nothing, at two or three
+// empty launches each (2 us apiece), and a chunk that ends before it waits for the host (15 us): one chunk up to where
+// the last interval ended, then chunks that grow with the steps gone by, so that a scene that comes to rest soon
+// queues `most` again. 64 scenes with a run every 2 steps: 32 steps queued each time cost 0.13 ms of the 0.45 a
+// step and run took. 30 000 spheres that came to rest after a run every 4 steps, with a launch per kernel: chunks of
+// two steps for good 40 us a step in FP32 and 39 in FP64, growing ones 32 and 31.
+static int64_t stepsToQueue(int64_t most, int64_t since, int64_t interval) {
+    if (interval <= 0) return most;
+    return std::min(most, since < interval ? interval - since + 1 : std::max<int64_t>(2, since / 4));
+}
+
 int Sim::run(int64_t n) {
     Sim& S = *this;
     SimEx& X = static_cast<SimEx&>(*this);
@@ -1161,12 +1173,7 @@ int Sim::run(int64_t n) {
         const bool small = N.n <= kSmallNodes && I.nAct <= (fp32 && !cfg.periodic ? kSmallContacts32 : kSmallContacts) && !trackE &&
                            !useGraph && contactBlock <= 0 && I.nHeavyFree == 0 && (!fp32 || P.nFacets == 0 || facetsStatic);
         int64_t k = std::min<int64_t>(n - done, small && N.n <= 65536 && !cfg.periodic && !anyZeroVd ? 8 * maxChunk : maxChunk);
-        // Steps queued past a full run's request do nothing, at two or three empty launches each (2 us apiece), and
-        // a chunk that ends before it waits for the host (15 us): one chunk up to where the last interval
-        // between two runs ended, then shorter ones. 64 scenes with a run every 2 steps: 32 steps
-        // queued each time cost 0.13 ms of the 0.45 a step and run took.
-        if (!small && !useGraph && runInterval > 0)
-            k = std::min(k, step - lastFullStep < runInterval ? runInterval - (step - lastFullStep) + 1 : std::max<int64_t>(2, runInterval / 4));
+        if (!small && !useGraph) k = stepsToQueue(k, step - lastFullStep, runInterval);
         // dt may change after a step (Scene.nextDt, DynDt): such a step ends its chunk
         if (std::isfinite(nextDt)) k = 1;
         // wg_run_host's early copy-out: the run's last step gets a chunk of its own, whose first
@@ -1328,7 +1335,8 @@ int Sim::run(int64_t n) {
                 step += ds;
                 return r;
             }
-            if (lastFullStep >= 0 && step + ds > lastFullStep) runInterval = step + ds - lastFullStep;
+            // a run that was forced (a slot's new job, contacts set from outside) says nothing about the spheres' motion
+            if (!needFull && lastFullStep >= 0 && step + ds > lastFullStep) runInterval = step + ds - lastFullStep;
             lastFullStep = step + ds;
             if (trackE) {
                 r = ensureEnergyCapacity();
@@ -2448,6 +2456,8 @@ int wg_get_grid(wg_scene* s, int32_t k, double* origin3, double* cell, int32_t* 
     dims3[0] = g.nx; dims3[1] = g.ny; dims3[2] = g.nz;
     return WG_OK;
 }
+
+int64_t wg_steps_to_queue(int64_t most, int64_t since, int64_t interval) { return stepsToQueue(most, since, interval); }
 
 int wg_fail_alloc(wg_scene* s, int64_t n) {
     if (!s) return WG_ERR_ARG;
