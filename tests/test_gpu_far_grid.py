@@ -62,3 +62,28 @@ def test_one_sphere_far_away(at, gpu_lib):
     S = spheres(300)
     S.dem._nodes.soa.col("pos")[7] = (at, -.5 * at, 0.)
     collide(S)
+
+
+def test_one_scene_of_a_batch_far_away(gpu_lib):
+    """Its pairs and those of the others are what each scene has alone."""
+    from woodem_gb300.batch import Batch
+    from woodem_gb300 import _plan
+    at = (0., 1e6, 3.)
+    pairs = []
+    for q in at:
+        S = spheres(400)
+        S.dem._nodes.soa.col("pos")[:] += q
+        sim = S._ensure_sim()
+        sim.H.check(sim.H.L.wg_collide_only(sim.H.h), "collide_only")
+        c = _plan.read_contacts(sim.H.L, sim.H.h, "wg")
+        pairs.append((c["id_lo"], c["id_hi"]))
+        S.close()
+    mix = [spheres(400) for _ in at]
+    for S, q in zip(mix, at):
+        S.dem._nodes.soa.col("pos")[:] += q
+    B = Batch(mix)
+    B.H.check(B.H.L.wg_collide_only(B.H.h), "collide_only")
+    for k, (lo, hi) in enumerate(pairs):
+        c = B.contacts(k)
+        assert len(lo) > 100 and np.array_equal(c["id_lo"], lo) and np.array_equal(c["id_hi"], hi)
+    B.close()

@@ -40,6 +40,7 @@ struct CollideTotals {
     unsigned long long act, actReal;  // totals of the work-list scans
     int32_t heavy, heavyFree;
     int32_t bad;  // a sphere's box is not finite
+    int32_t far;  // some grid is far from zero (Grid::far)
 };
 struct CollideWork {
     // sphere and "large" (non-sphere) id lists, built at upload
@@ -64,7 +65,7 @@ struct CollideWork {
     bool oldLoValid = false;
     int32_t* cellOff = nullptr;   // first sphere of each cell
     int64_t cellOffCap = 0;
-    double* red = nullptr;        // reduction partials
+    long long* red = nullptr;     // reduction partials
     std::vector<int32_t> hChunk;      // grid-reduction chunks of sphereIds (never across scenes)
     std::vector<int32_t> hSceneChunk; // chunks of scene k: [hSceneChunk[k], hSceneChunk[k+1])
     std::vector<int64_t> hSceneSph;   // spheres of scene k: sphereIds[hSceneSph[k] .. hSceneSph[k+1])
@@ -216,9 +217,9 @@ __device__ __forceinline__ long long orderOf(long long bits) { return bits ^ ((b
 // ---------------------------------------------------------------- grid bounds over spheres
 // partial[b] = {min mn.x, min mn.y, min mn.z, max mn.x, max mn.y, max mn.z, max extent} over the
 // spheres ids[chunk[b] .. chunk[b+1]) (chunks never span two scenes of a batch), in FP64: rounded to FP32 where
-// they stand, boxes of 1 cm at coordinates of 1e6 m would make the cells ten times too long.
+// they stand, boxes of 1 cm at coordinates of 1e6 m would make the cells ten times too long. As orderOf().
 __global__ void k_grid_reduce(DevParticles P, const int32_t* __restrict__ ids, const int32_t* __restrict__ chunk,
-                              double* __restrict__ partial) {
+                              long long* __restrict__ partial) {
     __shared__ long long s[7][BS / 32];
     const unsigned FULL = 0xffffffffu;
     const long long INF = 0x7ff0000000000000LL, most = orderOf(INF), least = orderOf(INF | (1LL << 63));
@@ -248,41 +249,43 @@ __global__ void k_grid_reduce(DevParticles P, const int32_t* __restrict__ ids, c
         const int q = threadIdx.x;
         long long m = s[q][0];
         for (int w = 1; w < BS / 32; w++) m = q < 3 ? min(m, s[q][w]) : max(m, s[q][w]);
-        partial[blockIdx.x * 7 + q] = __longlong_as_double(orderOf(m));
+        partial[blockIdx.x * 7 + q] = m;
     }
 }
 
 // The grid of each scene from the partial bounds of its chunks: cells slightly larger than the largest
 // sphere box, so that boxes that overlap sit in adjacent cells, and no more than cellBound() of them.
-// A warp per scene, then the first cell keys in scene order. A bound that is not finite sets `bad`.
+// A warp per scene, then the first cell keys in scene order. A bound that is not finite sets tot->bad.
 __host__ __device__ __forceinline__ int64_t cellBound(int64_t spheres, int scenes) {
     const int64_t least = scenes > 1 ? 64 : 1 << 16;
     return 8 * spheres > least ? 8 * spheres : least;
 }
 constexpr double kCellMargin = 2e-6;
-__global__ void __launch_bounds__(256) k_make_grids(int K, const int32_t* __restrict__ chunk, const int32_t* __restrict__ sceneChunk,
-                                                    const double* __restrict__ partial, const ScenePar* __restrict__ spp, int peri,
-                                                    Grid* __restrict__ out, int* __restrict__ bad) {
+__global__ void __launch_bounds__(1024) k_make_grids(int K, const int32_t* __restrict__ chunk, const int32_t* __restrict__ sceneChunk,
+                                                     const long long* __restrict__ partial, const ScenePar* __restrict__ spp, int peri,
+                                                     Grid* __restrict__ out, CollideTotals* __restrict__ tot) {
     const unsigned FULL = 0xffffffffu;
-    const double inf = __longlong_as_double(0x7ff0000000000000LL);
+    const long long INF = 0x7ff0000000000000LL, most0 = orderOf(INF), least0 = orderOf(INF | (1LL << 63));
     const int lane = threadIdx.x & 31;
     for (int k = threadIdx.x >> 5; k < K; k += blockDim.x >> 5) {
         const int c0 = sceneChunk[k], c1 = sceneChunk[k + 1];
-        double v[7] = {inf, inf, inf, -inf, -inf, -inf, 0.};  // these drop a NaN, whose edge is infinite here
+        long long u[7] = {most0, most0, most0, least0, least0, least0, 0};
         for (int b = c0 + lane; b < c1; b += 32) {
-            for (int q = 0; q < 3; q++) v[q] = fmin(v[q], partial[7 * b + q]);
-            for (int q = 3; q < 7; q++) v[q] = fmax(v[q], partial[7 * b + q]);
+            for (int q = 0; q < 3; q++) u[q] = min(u[q], partial[7 * b + q]);
+            for (int q = 3; q < 7; q++) u[q] = max(u[q], partial[7 * b + q]);
         }
         for (int o = 16; o > 0; o >>= 1) {
-            for (int q = 0; q < 3; q++) v[q] = fmin(v[q], __shfl_down_sync(FULL, v[q], o));
-            for (int q = 3; q < 7; q++) v[q] = fmax(v[q], __shfl_down_sync(FULL, v[q], o));
+            for (int q = 0; q < 3; q++) u[q] = min(u[q], __shfl_down_sync(FULL, u[q], o));
+            for (int q = 3; q < 7; q++) u[q] = max(u[q], __shfl_down_sync(FULL, u[q], o));
         }
         if (lane) continue;
+        double v[7];
+        for (int q = 0; q < 7; q++) v[q] = __longlong_as_double(orderOf(u[q]));
         Grid g{0, 0, 0, 1, 1, 1, 1, 1, 1, 0, 0};
         if (c0 != c1) {
             bool fine = true;
             for (int q = 0; q < 7; q++) fine = fine && isfinite(v[q]);
-            if (!fine) *bad = 1;
+            if (!fine) tot->bad = 1;
             else {
                 const int64_t most = cellBound((int64_t)chunk[c1] - chunk[c0], K);
                 double h = v[6] * (1 + kCellMargin) + 1e-300;
@@ -304,7 +307,7 @@ __global__ void __launch_bounds__(256) k_make_grids(int K, const int32_t* __rest
                 // coordinates that FP32 numbers resolve badly, compared with a cell: the boxes in cell order are
                 // kept relative to the grid's origin
                 for (int q = 0; q < 6; q++)
-                    if (fabs(v[q]) > 4096. * h) g.far = 1;
+                    if (fabs(v[q]) > 4096. * h) g.far = tot->far = 1;
                 if (peri)
                     for (int q = 0; q < 3; q++)
                         if (!(h <= 0.49 * spp->cellSize[q])) g.exact = 1;
@@ -313,12 +316,18 @@ __global__ void __launch_bounds__(256) k_make_grids(int K, const int32_t* __rest
         out[k] = g;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t base = 0;
-        for (int k = 0; k < K; k++) {
-            out[k].base = base;
-            base += out[k].ncell;
+    if (threadIdx.x >= 32) return;
+    int64_t base = 0;
+    for (int k0 = 0; k0 < K; k0 += 32) {
+        const int k = k0 + lane;
+        const int64_t mine = k < K ? out[k].ncell : 0;
+        int64_t upTo = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t w = __shfl_up_sync(FULL, upTo, o);
+            if (lane >= o) upTo += w;
         }
+        if (k < K) out[k].base = base + upTo - mine;
+        base += __shfl_sync(FULL, upTo, 31);
     }
 }
 
@@ -365,7 +374,7 @@ __device__ __forceinline__ int64_t lowerBound64(const uint64_t* a, int64_t n, ui
 __device__ __forceinline__ double4_32a relative(const Grid& G, const double4_32a& a) {
     return make_double4_32a(a.x - G.ox, a.y - G.oy, a.z - G.oz, 0.);
 }
-__global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ ids, int n, const Grid* __restrict__ Gs,
+__global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ ids, int n, const Grid* __restrict__ Gs, const int* __restrict__ far,
                                 const uint32_t* __restrict__ key,
                                 const int32_t* __restrict__ rank, const int32_t* __restrict__ off, uint32_t* __restrict__ skey,
                                 float4* __restrict__ smnf, float4* __restrict__ smxf) {
@@ -373,10 +382,12 @@ __global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ ids,
     if (i >= n) return;
     const int p = ids[i];
     double4_32a a = P.mn[p], b = P.mx[p];
-    const Grid& G = Gs[sceneOfP(P, p)];
-    if (G.far) {
-        a = relative(G, a);
-        b = relative(G, b);
+    if (*far) {
+        const Grid& G = Gs[sceneOfP(P, p)];
+        if (G.far) {
+            a = relative(G, a);
+            b = relative(G, b);
+        }
     }
     const int at = off[key[i]] + rank[i];
     skey[at] = key[i];
@@ -1146,10 +1157,13 @@ __global__ void k_heavy(DevIncidence I, DevParticles P, const uint32_t* __restri
         if ((nodeFlags[p] & F_DOF_ALL) != F_DOF_ALL) I.heavyFree[atomicAdd(&tot->heavyFree, 1)] = p;
     }
 }
-// every end starts without a contribution
-__global__ void k_zero_ends(DevIncidence I, int64_t ends) {
+// Every end starts without a contribution, once nothing can call the old set back: the active contacts (the totals
+// *act, as k_pack_ss has them) and the plain ones of them fit where they go, and with tot no real contact is missing.
+__global__ void k_zero_ends(DevIncidence I, const uint64_t* __restrict__ act, const CollideTotals* __restrict__ tot, int64_t mostAct,
+                            int64_t mostPlain) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= ends) return;
+    const int64_t all = (uint32_t)*act, plain = *act >> 32;
+    if (e >= 2 * all || all > mostAct || plain > mostPlain || (tot && tot->real != tot->kept)) return;
     if (I.endA) {
         I.endA[e] = make_double4_32a(0., 0., 0., 0.);
         I.endB[e] = make_double2(0., 0.);
@@ -1549,7 +1563,7 @@ static int fullRun(Sim& S) {
         if (!scratch(S, W.cellOffCap, ncell + 1, W.cellOff)) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
         const unsigned gs = (unsigned)((ns + BS - 1) / BS);
         k_grid_reduce<<<nb, BS, 0, st>>>(S.P, W.sphereIds, W.dChunk, W.red);
-        k_make_grids<<<1, 256, 0, st>>>(K, W.dChunk, W.dSceneChunk, W.red, S.dPar, peri ? 1 : 0, W.dGrids, bad);
+        k_make_grids<<<1, 32 * std::min(K, 32), 0, st>>>(K, W.dChunk, W.dSceneChunk, W.red, S.dPar, peri ? 1 : 0, W.dGrids, W.tot);
         // spheres in cell order: their number per cell, its running sum, then each to its place
         WG_CUDA_TRY(cudaMemsetAsync(W.cellOff, 0, sizeof(int32_t) * (ncell + 1), st));
         if (peri) k_cellkey_peri<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, S.dPar, W.cellKey, W.cellRank, W.cellOff);
@@ -1560,7 +1574,7 @@ static int fullRun(Sim& S) {
         tb = W.cubBytes;
         WG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(W.cubTmp, tb, W.cellOff, W.cellOff, (int)(ncell + 1), st));
         if (peri) k_gather_peri<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.cellKey, W.cellRank, W.cellOff, S.dPar, W.skey, W.speri);
-        else k_gather_sorted<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, W.cellKey, W.cellRank, W.cellOff, W.skey, W.smnf, W.smxf);
+        else k_gather_sorted<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, &W.tot->far, W.cellKey, W.cellRank, W.cellOff, W.skey, W.smnf, W.smxf);
     }
     // lists of large particles: facets with boxes spanning a few cells use the grid, the rest are global
     {
@@ -1725,6 +1739,23 @@ static int fullRun(Sim& S) {
         undo.incidence = true;
         r = incidence(S, n, W.newLo);
         if (r) return r;
+        DevPackedSS& Q = W.Kb;
+        auto pack = [&](int64_t most) {
+            Q.ftLive = law0;
+            launch_pack_ss(st, S.C, S.I, S.P, S.K, Q, packedState ? W.packIdx : nullptr, W.src, W.packIdxB, W.act + n, most);
+        };
+        auto zero = [&](const CollideTotals* tot, int64_t mostAct, int64_t mostPlain) {
+            const int64_t most = 2 * std::min(mostAct, n);
+            if (most > 0) k_zero_ends<<<(unsigned)((most + BS - 1) / BS), BS, 0, st>>>(S.I, W.act + n, tot, mostAct, mostPlain);
+        };
+        // Both are done before the host knows the numbers, where the room is there that is probably enough
+        const bool ft = law0 || S.P.fresh;  // a serving slot may take a job with that law at any time
+        const int64_t roomAct = S.I.endCap ? S.I.endCap / 2 : -1, roomPlain = !packed ? n : (Q.ft[0] || !ft ? Q.cap : -1);
+        if (packed) {
+            if (!scratch(S, W.packIdxCapB, n, W.packIdxB)) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
+            pack(std::min(n, roomPlain));
+        }
+        zero(lookForOrphans ? nullptr : W.tot, roomAct, roomPlain);
         WG_CUDA_TRY(cudaMemcpyAsync(W.hTot, W.tot, sizeof(CollideTotals), cudaMemcpyDeviceToHost, st));
         WG_CUDA_TRY(cudaStreamSynchronize(st));
         const CollideTotals& T = *W.hTot;
@@ -1736,23 +1767,21 @@ static int fullRun(Sim& S) {
             continue;
         }
         const int64_t nAct = (int64_t)(uint32_t)T.act, nSS = (int64_t)(T.act >> 32);
-        // what takes memory for the active contacts, then the new set takes the old one's place
-        r = endRoom(S, nAct);
-        if (r) return r;
-        if (packed) {
-            DevPackedSS& Q = W.Kb;
-            if (!scratch(S, W.packIdxCapB, n, W.packIdxB)) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
-            r = packRoom(S, Q, nSS, law0 || S.P.fresh);  // a serving slot may take a job with that law at any time
+        // the new set takes the old one's place, after what takes more memory
+        if (nAct > roomAct || nSS > roomPlain) {
+            r = endRoom(S, nAct);
+            if (!r && packed) r = packRoom(S, Q, nSS, ft);
             if (r) return r;
+            if (packed && nSS > roomPlain) pack(nSS);
+            zero(nullptr, nAct, nSS);
+        }
+        undo.off = true;
+        if (packed) {
             Q.n = nSS;
-            Q.ftLive = law0;
-            launch_pack_ss(st, S.C, S.I, S.P, S.K, Q, packedState ? W.packIdx : nullptr, W.src, W.packIdxB, W.act + n, nSS);
             std::swap(S.K, W.Kb);
             std::swap(W.packIdx, W.packIdxB);
             std::swap(W.packIdxCap, W.packIdxCapB);
         }
-        undo.off = true;
-        if (nAct > 0) k_zero_ends<<<(unsigned)((2 * nAct + BS - 1) / BS), BS, 0, st>>>(S.I, 2 * nAct);
         S.I.nAct = nAct;
         S.nMixed = nAct - nSS;
         S.packDirty = packedState && nSS > 0;  // the contact arrays hold no state of those contacts then

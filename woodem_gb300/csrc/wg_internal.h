@@ -304,8 +304,9 @@ bool launch_contact_fp32(cudaStream_t st, const SideStream& side, const DevNodes
                          int block = 256, const EnergyCols* energy = nullptr);
 // pack: the packed state K of a new contact set (whose active contacts are counted in the low half of *act
 // on the device, the plain ones in its high half, at most `most`), in tiles with the real ones first
-// (the work list is put in that order too). oldIdx null: from the contact arrays; else from the old packed
-// state Kold, where the contact that contact c continues, src[c], is at oldIdx[src[c]]. idx[c] takes c's place.
+// (the work list is put in that order too); nothing where K has no room for them. oldIdx null: from the contact
+// arrays; else from the old packed state Kold, where the contact that contact c continues, src[c], is at
+// oldIdx[src[c]]. idx[c] takes c's place.
 void launch_pack_ss(cudaStream_t st, const DevContacts& C, const DevIncidence& I, const DevParticles& P, const DevPackedSS& Kold,
                     const DevPackedSS& K, const int32_t* oldIdx, const int32_t* src, int32_t* idx, const uint64_t* act, int64_t most);
 // unpack: the packed state (flagsOnly: its flags alone) back into the contact arrays

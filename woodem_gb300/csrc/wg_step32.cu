@@ -807,7 +807,7 @@ __global__ void __launch_bounds__(kPackTile) k_pack_ss(DevContacts C, DevInciden
     __shared__ int sh[kPackTile / 32];
     const uint32_t all = (uint32_t)*act, plain = (uint32_t)(*act >> 32);
     const int64_t j0 = (int64_t)blockIdx.x * kPackTile, nm = all - plain;
-    if (j0 >= plain) return;
+    if (j0 >= plain || plain > K.cap) return;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const bool in = j0 + t < plain;
     int4 wk = make_int4(0, 0, 0, 0);
