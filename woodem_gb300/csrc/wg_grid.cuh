@@ -59,15 +59,17 @@ static int smCount() {
     return n[dev];
 }
 
-// blocks of a cooperative launch of kernel f: one on each SM, and no more than the chunks of 32 items
-// need; 0 if it cannot be launched
-static int stepsGrid(const void* f, int threads, size_t shared, int64_t items) {
+// blocks that a launch of several steps over so many items can use: one on each SM, a warp for 32 items
+static int stepsBlocks(int64_t items) { return (int)std::min<int64_t>(std::max<int64_t>((items + 31) / 32, 1), smCount()); }
+
+// Whether kernel f can be launched with a block on every SM at once.
+static bool stepsFit(const void* f, int threads, size_t shared) {
     int most = 0;
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, f, threads, shared) != cudaSuccess || most < 1) {
         cudaGetLastError();
-        return 0;
+        return false;
     }
-    return (int)std::min<int64_t>(std::max<int64_t>((items + 31) / 32, 1), smCount());
+    return true;
 }
 }  // namespace wg

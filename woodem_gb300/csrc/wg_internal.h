@@ -227,6 +227,7 @@ constexpr size_t CTL_BYTES = sizeof(int) * FL_WORDS + sizeof(long long) * CTL_CO
 // 168 and 197, a drum of 250 000 625 and 645. 64 scenes of 980 000 spheres in FP32 lose (0.46 and 0.43 ms): one block
 // a SM has fewer warps in flight, and prefetches less, than k_contact_all32.
 constexpr int64_t kSmallNodes = 262144, kSmallContacts = 2097152, kSmallContacts32 = 1048576;
+constexpr int64_t kSmallBeside = 65536;  // nodes, while several others are in a run on the device (RunShare)
 
 __host__ __device__ inline int32_t packCellDist(int a, int b, int c) {
     return (int32_t)(((uint32_t)(a + 512) & 1023u) | (((uint32_t)(b + 512) & 1023u) << 10) | (((uint32_t)(c + 512) & 1023u) << 20));
@@ -252,14 +253,15 @@ void launch_contact_fp64(cudaStream_t st, const DevNodes& N, const DevParticles&
 // free DOF, facets static). It leaves the flags and the step counter as that many launches of the
 // kernels above would: a full run due ends it before that step's contacts. bar: a word that is zero
 // before the launch; ns: nanoseconds spent in Leapfrog and in the contacts, added to. sp: one record, or
-// one per step in a periodic cell. Returns nonzero if it cannot be launched (nothing is then queued).
+// one per step in a periodic cell. blocks: of the launch, at most one on each SM; the results do not depend on it.
+// Returns nonzero if it cannot be launched (nothing is then queued).
 int launch_steps64(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
                    const double4_32a* mats, const ScenePar* sp, bool periodic, long long* dStep, int* dFlags, unsigned* bar,
-                   unsigned long long* ns, int fromEnds, int steps);
+                   unsigned long long* ns, int fromEnds, int steps, int blocks);
 int launch_steps32(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
                    const DevPackedSS& K, const NodeConst32* nc, const double4_32a* mats, const ScenePar* sp, bool periodic,
                    long long* dStep, int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool loadFt, int fromEnds,
-                   int steps);
+                   int steps, int blocks);
 // perStep: only the heavy particles with a free DOF (guarded by the flags), before Leapfrog;
 // otherwise every particle's DemData.force/torque (reporting at the end of a run).
 void launch_forces(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevIncidence& I, const ScenePar* sp,

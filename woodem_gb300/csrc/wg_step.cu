@@ -752,18 +752,16 @@ __global__ void __launch_bounds__(kSteps64Threads, 1) k_steps64(DevNodes N, DevP
 
 int launch_steps64(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
                    const double4_32a* mats, const ScenePar* sp, bool periodic, long long* dStep, int* dFlags, unsigned* bar,
-                   unsigned long long* ns, int fromEnds, int steps) {
+                   unsigned long long* ns, int fromEnds, int steps, int blocks) {
     DevNodes n = N;
     DevParticles p = P;
     DevContacts c = C;
     DevIncidence i = I;
     int seq = periodic ? 1 : 0;
     void* args[] = {&n, &p, &c, &i, &mats, &sp, &seq, &dStep, &dFlags, &bar, &ns, &fromEnds, &steps};
-    const int64_t items = std::max<int64_t>(N.n, I.nAct);
     const void* f = periodic ? (const void*)k_steps64<true> : (const void*)k_steps64<false>;
-    const int g = stepsGrid(f, kSteps64Threads, 0, items);
-    if (g < 1) return -1;
-    return cudaLaunchCooperativeKernel(f, dim3((unsigned)g), dim3(kSteps64Threads), args, 0, st) == cudaSuccess ? 0 : -1;
+    if (!stepsFit(f, kSteps64Threads, 0)) return -1;
+    return cudaLaunchCooperativeKernel(f, dim3((unsigned)blocks), dim3(kSteps64Threads), args, 0, st) == cudaSuccess ? 0 : -1;
 }
 
 // ---------------------------------------------------------------------------------- energy sums

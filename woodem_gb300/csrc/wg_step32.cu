@@ -1444,7 +1444,7 @@ __global__ void __launch_bounds__(kSteps32Threads, 1) k_steps32(DevNodes N, DevP
 
 int launch_steps32(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevContacts& C, const DevIncidence& I,
                    const DevPackedSS& K, const NodeConst32* nc, const double4_32a* mats, const ScenePar* sp, bool periodic, long long* dStep,
-                   int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool loadFt, int fromEnds, int steps) {
+                   int* dFlags, unsigned* bar, unsigned long long* ns, int64_t nMixed, bool loadFt, int fromEnds, int steps, int blocks) {
     DevNodes n = N;
     DevParticles p = P;
     DevContacts c = C;
@@ -1453,11 +1453,9 @@ int launch_steps32(cudaStream_t st, const DevNodes& N, const DevParticles& P, co
     int seq = periodic ? 1 : 0, ft = loadFt ? 1 : 0;
     int64_t nm = periodic ? I.nAct : std::min<int64_t>(nMixed, I.nAct);
     void* args[] = {&n, &p, &c, &i, &k, &nc, &mats, &sp, &seq, &dStep, &dFlags, &bar, &ns, &nm, &ft, &fromEnds, &steps};
-    const int64_t items = std::max<int64_t>(N.n, I.nAct);
     const void* f = periodic ? (const void*)k_steps32<true> : (const void*)k_steps32<false>;
-    const int g = stepsGrid(f, kSteps32Threads, kSteps32Shared, items);
-    if (g < 1) return -1;
-    return cudaLaunchCooperativeKernel(f, dim3((unsigned)g), dim3(kSteps32Threads), args, kSteps32Shared, st) == cudaSuccess ? 0 : -1;
+    if (!stepsFit(f, kSteps32Threads, kSteps32Shared)) return -1;
+    return cudaLaunchCooperativeKernel(f, dim3((unsigned)blocks), dim3(kSteps32Threads), args, kSteps32Shared, st) == cudaSuccess ? 0 : -1;
 }
 
 // ---------------------------------------------------------------------------------- force sum
