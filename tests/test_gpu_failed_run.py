@@ -10,7 +10,7 @@ from woodem_gb300.dem import DemField, FrictMat
 
 pytestmark = pytest.mark.gpu
 
-R, PAIRS, LOOSE = 5e-3, 24, 300
+R, PAIRS, LOOSE = 5e-3, 24, 480
 KEYS = ("pos", "ori", "vel", "angVel", "force", "torque")
 
 
@@ -73,7 +73,7 @@ def crowd(nodes):
     """The loose spheres brought together (their boxes overlap many others), and every third pair parted."""
     out = [a.copy() for a in nodes]
     rng = np.random.default_rng(3)
-    at = np.stack(np.meshgrid(*[np.arange(7)] * 3, indexing="ij"), -1).reshape(-1, 3)[:LOOSE] * 2.05 * R + [.1, .1, .6]
+    at = np.stack(np.meshgrid(*[np.arange(8)] * 3, indexing="ij"), -1).reshape(-1, 3)[:LOOSE] * 2.05 * R + [.1, .1, .6]
     out[0][2 * PAIRS:] = at + rng.uniform(-.02 * R, .02 * R, at.shape)
     out[0][1:2 * PAIRS:6] += 3 * R
     return out

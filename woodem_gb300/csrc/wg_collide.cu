@@ -1457,7 +1457,7 @@ static int packRoom(Sim& S, DevPackedSS& Q, int64_t n, bool ft) {
     return 0;
 }
 
-// A run that ends early after the incidence of the new set was begun: the old set, from its keys and flags, takes
+// A run that ends early after room for the incidence of the new set was made: the old set, from its keys and flags, takes
 // its incidence and work list again (the ends and the packed state are still those of the old set).
 struct Undo {
     Sim& S;
@@ -1480,6 +1480,7 @@ struct Undo {
         CollideWork& W = *S.cw;
         const int64_t n = S.C.n;
         if (S.contactsReplaced) {  // set from outside and never run: it has no forces to list
+            if (!W.hiCap) return 0;
             WG_CUDA_TRY(cudaMemsetAsync(S.I.slotLo, 0xff, sizeof(int32_t) * W.hiCap, S.stream));
             WG_CUDA_TRY(cudaMemsetAsync(S.I.slotHi, 0xff, sizeof(int32_t) * W.hiCap, S.stream));
             return 0;
@@ -1719,6 +1720,7 @@ static int fullRun(Sim& S) {
         if (r) return r;
         if (!(peri ? scratch(S, W.srcCap, std::max<int64_t>(n, 1), W.src, W.newCd) : scratch(S, W.srcCap, std::max<int64_t>(n, 1), W.src)))
             return S.fail(WG_ERR_CUDA, "out of device memory (merge)");
+        undo.incidence = true;  // the arrays that are in use may be others from here on
         r = incidenceRoom(S, n);
         if (r) return r;
         S.Cb.n = n;
@@ -1736,7 +1738,6 @@ static int fullRun(Sim& S) {
         if (nOrph > 0)  // the first index of every lo id in the merged set; without orphans that of the new pairs
             k_lo_bounds<<<(unsigned)((n + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, n, (int)S.nPar, W.newLo);
         // 6. CSR incidence over the active contacts
-        undo.incidence = true;
         r = incidence(S, n, W.newLo);
         if (r) return r;
         DevPackedSS& Q = W.Kb;
@@ -1769,8 +1770,8 @@ static int fullRun(Sim& S) {
         const int64_t nAct = (int64_t)(uint32_t)T.act, nSS = (int64_t)(T.act >> 32);
         // the new set takes the old one's place, after what takes more memory
         if (nAct > roomAct || nSS > roomPlain) {
-            r = endRoom(S, nAct);
-            if (!r && packed) r = packRoom(S, Q, nSS, ft);
+            r = packed ? packRoom(S, Q, nSS, ft) : 0;
+            if (!r) r = endRoom(S, nAct);  // last: the old ends are gone then
             if (r) return r;
             if (packed && nSS > roomPlain) pack(nSS);
             zero(nullptr, nAct, nSS);
