@@ -1094,6 +1094,21 @@ __global__ void k_hi_start(const uint32_t* __restrict__ hks, int64_t n, int nPar
     if (p > nPar) return;
     hiStart[p] = (int32_t)lowerBound32(hks, n, (uint32_t)p);
 }
+__device__ __forceinline__ void clearEnd(const DevIncidence& I, int64_t e) {
+    if (I.endA) {
+        I.endA[e] = make_double4_32a(0., 0., 0., 0.);
+        I.endB[e] = make_double2(0., 0.);
+    } else {
+        I.endAf[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        I.endBf[e] = make_float2(0.f, 0.f);
+    }
+}
+// Room that a run has before the host knows what the new set needs: for so many active contacts and plain ones
+// (act < 0: nothing is to be cleared). tot: the real contacts are counted, and none must be missing.
+struct Room {
+    int64_t act = -1, plain = -1;
+    const CollideTotals* tot = nullptr;
+};
 // end slots: active contact c with hi==p sits at loStart[p] + (its index k in hiList); with lo==p
 // at hiStart[p+1] + (active contacts before c) (see DevIncidence); inactive contacts have no slot (-1).
 // The work list holds the nOther active contacts that are not plain (walls, facets, spheres of
@@ -1105,23 +1120,29 @@ __global__ void k_hi_start(const uint32_t* __restrict__ hks, int64_t n, int nPar
 // way, has it too (200 000: 0.12 -> 0.11 ms). The packed FP32 kernel is bound by the gathered mirror
 // records, which neighbours in contact order share: there the real ones come first within tiles of
 // contacts only (k_pack_ss; 1M drum: split over the whole list, the step took 0.168 ms instead of 0.161).
+// The ends start without a contribution, once nothing can call the old set back.
 __global__ void k_slots(const uint64_t* __restrict__ key, const uint32_t* __restrict__ flags, const int32_t* __restrict__ cdist, int64_t n,
-                        const uint64_t* __restrict__ act, const uint64_t* __restrict__ actReal, DevIncidence I) {
+                        const uint64_t* __restrict__ act, const uint64_t* __restrict__ actReal, DevIncidence I, Room room) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint64_t tot = act[n], totReal = actReal ? actReal[n] : 0;  // over all contacts
     const int nAct = (int)(uint32_t)tot, nPlain = (int)(tot >> 32);
+    const bool clear = nAct <= room.act && nPlain <= room.plain && !(room.tot && room.tot->real != room.tot->kept);
     if (k < nAct) {
         const int32_t ch = I.hiList[k];
         const int hiP = (int)(key[ch] & 0xffffffffu);
-        I.slotHi[ch] = I.loStart[hiP] + (int32_t)k;
+        const int32_t slot = I.loStart[hiP] + (int32_t)k;
+        I.slotHi[ch] = slot;
+        if (clear) clearEnd(I, slot);
     }
     const uint32_t fl = flags[k];
     if (activeContact(fl)) {
         const uint64_t a = act[k];
         const int all = (int)(uint32_t)a, plain = (int)(a >> 32);
         const int loP = (int)(key[k] >> 32), hiP = (int)(key[k] & 0xffffffffu);
-        I.slotLo[k] = I.hiStart[loP + 1] + all;
+        const int32_t slot = I.hiStart[loP + 1] + all;
+        I.slotLo[k] = slot;
+        if (clear) clearEnd(I, slot);
         const bool isPlain = plainContact(fl, cdist[k]);
         int w = isPlain ? plain : all - plain;  // place within the group
         if (actReal) {
@@ -1157,20 +1178,10 @@ __global__ void k_heavy(DevIncidence I, DevParticles P, const uint32_t* __restri
         if ((nodeFlags[p] & F_DOF_ALL) != F_DOF_ALL) I.heavyFree[atomicAdd(&tot->heavyFree, 1)] = p;
     }
 }
-// Every end starts without a contribution, once nothing can call the old set back: the active contacts (the totals
-// *act, as k_pack_ss has them) and the plain ones of them fit where they go, and with tot no real contact is missing.
-__global__ void k_zero_ends(DevIncidence I, const uint64_t* __restrict__ act, const CollideTotals* __restrict__ tot, int64_t mostAct,
-                            int64_t mostPlain) {
+// every end starts without a contribution
+__global__ void k_zero_ends(DevIncidence I, int64_t ends) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t all = (uint32_t)*act, plain = *act >> 32;
-    if (e >= 2 * all || all > mostAct || plain > mostPlain || (tot && tot->real != tot->kept)) return;
-    if (I.endA) {
-        I.endA[e] = make_double4_32a(0., 0., 0., 0.);
-        I.endB[e] = make_double2(0., 0.);
-    } else {
-        I.endAf[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-        I.endBf[e] = make_float2(0.f, 0.f);
-    }
+    if (e < ends) clearEnd(I, e);
 }
 
 // the packed state K back into the contact arrays of its set, contact c from idx[c] (whatever the work list holds)
@@ -1394,8 +1405,8 @@ static int incidenceRoom(Sim& S, int64_t n) {
     return ensureCub(S, std::max(a, b));
 }
 // CSR incidence and work list of the n contacts of S.C; first: the first contact of every lo id. The room is there.
-// The host does not know the number of active contacts before the end.
-static int incidence(Sim& S, int64_t n, const int32_t* first) {
+// The host does not know the number of active contacts before the end; the ends are cleared as far as room says.
+static int incidence(Sim& S, int64_t n, const int32_t* first, const Room& room) {
     CollideWork& W = *S.cw;
     cudaStream_t st = S.stream;
     const unsigned gn = (unsigned)((n + BS - 1) / BS);
@@ -1415,7 +1426,7 @@ static int incidence(Sim& S, int64_t n, const int32_t* first) {
         WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiKeyBits(S), st));
     }
     k_hi_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.hiKeysSorted, n, (int)S.nPar, S.I.hiStart);
-    if (n > 0) k_slots<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, S.I);
+    if (n > 0) k_slots<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, S.I, room);
     k_heavy<<<(unsigned)((S.nPar + BS - 1) / BS), BS, 0, st>>>(S.I, S.P, S.N.flags, kHeavyThreshold, W.tot, W.act, W.actReal, n);
     return 0;
 }
@@ -1489,7 +1500,7 @@ struct Undo {
         k_lo_bounds<<<(unsigned)((n + 1 + BS - 1) / BS), BS, 0, S.stream>>>(S.C.key, n, (int)S.nPar, W.oldLo);
         WG_CUDA_TRY(cudaMemsetAsync(&W.tot->heavy, 0, 2 * sizeof(int32_t), S.stream));
         int r = incidenceRoom(S, n);
-        if (!r) r = wg::incidence(S, n, W.oldLo);
+        if (!r) r = wg::incidence(S, n, W.oldLo, Room{});
         if (r) return r;
         launch_pack_ss(S.stream, S.C, S.I, S.P, S.K, S.K, nullptr, nullptr, W.packIdx, W.act + n, S.K.n);
         S.packDirty = false;
@@ -1738,25 +1749,22 @@ static int fullRun(Sim& S) {
         if (nOrph > 0)  // the first index of every lo id in the merged set; without orphans that of the new pairs
             k_lo_bounds<<<(unsigned)((n + 1 + BS - 1) / BS), BS, 0, st>>>(S.C.key, n, (int)S.nPar, W.newLo);
         // 6. CSR incidence over the active contacts
-        r = incidence(S, n, W.newLo);
-        if (r) return r;
         DevPackedSS& Q = W.Kb;
         auto pack = [&](int64_t most) {
             Q.ftLive = law0;
             launch_pack_ss(st, S.C, S.I, S.P, S.K, Q, packedState ? W.packIdx : nullptr, W.src, W.packIdxB, W.act + n, most);
         };
-        auto zero = [&](const CollideTotals* tot, int64_t mostAct, int64_t mostPlain) {
-            const int64_t most = 2 * std::min(mostAct, n);
-            if (most > 0) k_zero_ends<<<(unsigned)((most + BS - 1) / BS), BS, 0, st>>>(S.I, W.act + n, tot, mostAct, mostPlain);
-        };
-        // Both are done before the host knows the numbers, where the room is there that is probably enough
+        // The ends are cleared and the packed state is made before the host knows the numbers, where the room that
+        // is there suffices
         const bool ft = law0 || S.P.fresh;  // a serving slot may take a job with that law at any time
-        const int64_t roomAct = S.I.endCap ? S.I.endCap / 2 : -1, roomPlain = !packed ? n : (Q.ft[0] || !ft ? Q.cap : -1);
-        if (packed) {
-            if (!scratch(S, W.packIdxCapB, n, W.packIdxB)) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
-            pack(std::min(n, roomPlain));
-        }
-        zero(lookForOrphans ? nullptr : W.tot, roomAct, roomPlain);
+        Room room;
+        room.act = S.I.endCap ? S.I.endCap / 2 : -1;
+        room.plain = !packed ? n : (Q.ft[0] || !ft ? Q.cap : -1);
+        room.tot = lookForOrphans ? nullptr : W.tot;
+        if (packed && !scratch(S, W.packIdxCapB, n, W.packIdxB)) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
+        r = incidence(S, n, W.newLo, room);
+        if (r) return r;
+        if (packed) pack(std::min(n, room.plain));
         WG_CUDA_TRY(cudaMemcpyAsync(W.hTot, W.tot, sizeof(CollideTotals), cudaMemcpyDeviceToHost, st));
         WG_CUDA_TRY(cudaStreamSynchronize(st));
         const CollideTotals& T = *W.hTot;
@@ -1769,12 +1777,12 @@ static int fullRun(Sim& S) {
         }
         const int64_t nAct = (int64_t)(uint32_t)T.act, nSS = (int64_t)(T.act >> 32);
         // the new set takes the old one's place, after what takes more memory
-        if (nAct > roomAct || nSS > roomPlain) {
+        if (nAct > room.act || nSS > room.plain) {
             r = packed ? packRoom(S, Q, nSS, ft) : 0;
             if (!r) r = endRoom(S, nAct);  // last: the old ends are gone then
             if (r) return r;
-            if (packed && nSS > roomPlain) pack(nSS);
-            zero(nullptr, nAct, nSS);
+            if (packed && nSS > room.plain) pack(nSS);
+            if (nAct > 0) k_zero_ends<<<(unsigned)((2 * nAct + BS - 1) / BS), BS, 0, st>>>(S.I, 2 * nAct);
         }
         undo.off = true;
         if (packed) {
