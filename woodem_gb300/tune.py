@@ -16,12 +16,10 @@ DEFAULT_CANDIDATES = (
     # stream beside the sphere-sphere ones, for a positive block); block -256 selects the resident
     # FP32 grid over both, whose threads prefetch their next contact
     (-256, 32, False, True),
-    (-256, 32, False, False),
     (256, 32, False, True),
     (128, 32, False, True),
     (-256, 8, True, True),
     (-256, 32, True, True),
-    (-256, 32, True, False),
     (-256, 64, True, True),
 )
 
