@@ -465,7 +465,9 @@ int64_t wg_pack_rsa_device(int64_t n, const double* radii, const double* lo, con
         return -1;
     k_move_window<<<1, kSpec, 0, st>>>(dWin, n, W, dState, dList);
     for (;;) {
-        if (cudaMemcpyAsync(&win, dWin, sizeof(Window), cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+        // a launch that was refused would leave the window where it is for good
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMemcpyAsync(&win, dWin, sizeof(Window), cudaMemcpyDeviceToHost, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
             return -1;
         if (win.done) break;
         if (win.nU <= kSpec) {
