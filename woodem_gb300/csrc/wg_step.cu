@@ -220,9 +220,9 @@ __global__ void __launch_bounds__(128) k_leapfrog(DevNodes N, DevParticles P, De
 }
 
 // Threads per block of the FP64 kernels over n items: one warp per block while the blocks of one
-// warp can all be resident (32 a SM on 152 SMs), so that a small scene's warps spread over every
+// warp can all be resident (32 a SM), so that a small scene's warps spread over every
 // SM's FP64 pipe instead of queueing for a few of them; 128 beyond that.
-static int fp64Block(int64_t n) { return n <= 152 * 32 * 32 ? 32 : 128; }
+static int fp64Block(int64_t n) { return n <= (int64_t)smCount() * 32 * 32 ? 32 : 128; }
 
 void launch_leapfrog(cudaStream_t st, const DevNodes& N, const DevParticles& P, const DevIncidence& I, const ScenePar* sp,
                      int* dFlags, int fromEnds, const long long* dStep, bool periodic, const EnergyCols* energy) {
