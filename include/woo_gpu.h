@@ -257,6 +257,13 @@ int64_t wg_steps_to_queue(int64_t most, int64_t since, int64_t interval);
    next one) fails as if no memory were left. -1: none does. */
 int wg_fail_alloc(wg_scene* s, int64_t n);
 
+/* Compiled device functions on arrays, for the tests. Quotients: per item i, with a = a3[3i..], b = b3[3i..] and the rounded
+   reciprocals rb3 of b: a / b[0] (3), a / b by component (3), a normalised (3), and the quaternion (b[0], a) normalised
+   (w, x, y, z). Overlap: two boxes per item in a periodic cell, min6/max6: quick 1 overlap, 0 none, 2 not decided in
+   FP32; exact: the FP64 test, negative where a box reaches half the cell. Without exact nothing runs on a GPU. */
+int wg_selftest_quotients(int64_t n, const double* a3, const double* b3, const double* rb3, double* out13);
+int wg_selftest_overlap(int64_t n, const double* min6, const double* max6, const double* size3, int32_t* quick, int32_t* exact);
+
 /* Mark the region a profiler started with "profile from start off" captures (1 = start, 0 = stop). */
 int wg_profiler(int on);
 

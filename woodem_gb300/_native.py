@@ -117,6 +117,8 @@ def lib():
         "wg_get_timing": (C.c_int, [C.c_void_p, P_D, P_D, P_I64]),
         "wg_get_grid": (C.c_int, [C.c_void_p, C.c_int32, P_D, P_D, P_I32]),
         "wg_steps_to_queue": (C.c_int64, [C.c_int64, C.c_int64, C.c_int64]),
+        "wg_selftest_quotients": (C.c_int, [C.c_int64, P_D, P_D, P_D, P_D]),
+        "wg_selftest_overlap": (C.c_int, [C.c_int64, P_D, P_D, P_D, P_I32, P_I32]),
         "wg_fail_alloc": (C.c_int, [C.c_void_p, C.c_int64]),
         "wg_profiler": (C.c_int, [C.c_int]),
         "wg_contact_state_cols": (C.c_int32, [C.c_void_p]),

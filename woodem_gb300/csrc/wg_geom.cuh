@@ -57,8 +57,10 @@ __device__ __forceinline__ int overlapPeri(const double4_32a& mn1, const double4
 // The same decision from FP32 fractions of the cell, where it is clear: 1 overlap, 0 none, 2 not decided here. Boxes
 // of less than 0.4 periods span no boundary of the origin that overlapPeri chooses (the box minimum within half a
 // period below the other), and overlap there if that offset is no more than the lower box. Which box is the lower
-// one is open only at offsets of 0 (boxes above 1e-4: both overlap) and 1/2 (neither does). The fractions are off by
-// at most 3e-7 (1 + periods between the boxes), the FP64 routine by 1e-9 for minima within 1e6 periods.
+// one is open at offsets of 1/2, where neither overlaps, and of 0: there the rounding of the FP64 routine may put a
+// box's minimum just below a boundary that the box then spans, which is an error, and it decides itself. The
+// fractions are off by at most 3e-7 (1 + periods between the boxes), the FP64 routine by 1e-9 for minima within 1e6
+// periods.
 // overlapPeri divides 18 times in FP64, some 450 instructions for the one lane of a warp whose contact the law has
 // just let go: 200 000 sheared spheres in FP32-force mode 0.104 -> 0.098 ms a step of contacts.
 __host__ __device__ __forceinline__ int overlapPeriQuick(const double4_32a& mn1, const double4_32a& mx1, const double4_32a& mn2,
@@ -75,7 +77,7 @@ __host__ __device__ __forceinline__ int overlapPeriQuick(const double4_32a& mn1,
             return 2;
         const float f = d - rintf(d);
         const float over = f >= 0.f ? e1 - f : e2 + f;
-        if (!(fabsf(over) > 2e-6f * (1.f + fabsf(d)))) return 2;
+        if (!(fminf(fabsf(over), fabsf(f)) > 2e-6f * (1.f + fabsf(d)))) return 2;
         if (over < 0.f) res = 0;
     }
     return res;

@@ -1530,4 +1530,37 @@ void launch_forces32(cudaStream_t st, const DevNodes& N, const DevParticles& P, 
     if (I.nHeavy > 0) k_forces32_heavy<<<I.nHeavy, 256, 0, st>>>(N, I, I.heavy, sp, nullptr);
 }
 
+// ---------------------------------------------------------------------------------- for the tests
+// Two boxes an item: the decision from FP32 fractions of the cell and the FP64 test's, as this file's kernels compile them.
+__global__ void k_selftest_overlap(int64_t n, const double4_32a* __restrict__ mn, const double4_32a* __restrict__ mx, double sx, double sy,
+                                   double sz, int32_t* __restrict__ quick, int32_t* __restrict__ exact) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double size[3] = {sx, sy, sz};
+    int per[3];
+    quick[i] = overlapPeriQuick(mn[2 * i], mx[2 * i], mn[2 * i + 1], mx[2 * i + 1], size);
+    exact[i] = overlapPeri(mn[2 * i], mx[2 * i], mn[2 * i + 1], mx[2 * i + 1], size, per);
+}
+int selftest_overlap32(int64_t n, const double4_32a* mn, const double4_32a* mx, const double* size, int32_t* quick, int32_t* exact) {
+    if (n == 0) return 0;
+    const size_t boxes = sizeof(double4_32a) * 2 * n, ints = sizeof(int32_t) * n;
+    char* d = nullptr;
+    if (cudaMalloc(&d, 2 * boxes + 2 * ints) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
+    double4_32a *dmn = (double4_32a*)d, *dmx = (double4_32a*)(d + boxes);
+    int32_t *dq = (int32_t*)(d + 2 * boxes), *de = dq + n;
+    cudaError_t r = cudaMemcpy(dmn, mn, boxes, cudaMemcpyHostToDevice);
+    if (r == cudaSuccess) r = cudaMemcpy(dmx, mx, boxes, cudaMemcpyHostToDevice);
+    if (r == cudaSuccess) {
+        k_selftest_overlap<<<(unsigned)((n + 255) / 256), 256>>>(n, dmn, dmx, size[0], size[1], size[2], dq, de);
+        r = cudaGetLastError();
+    }
+    if (r == cudaSuccess) r = cudaMemcpy(quick, dq, ints, cudaMemcpyDeviceToHost);
+    if (r == cudaSuccess) r = cudaMemcpy(exact, de, ints, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return r == cudaSuccess ? 0 : -1;
+}
+
 }  // namespace wg
