@@ -255,7 +255,8 @@ __global__ void k_grid_reduce(DevParticles P, const int32_t* __restrict__ ids, c
 
 // The grid of each scene from the partial bounds of its chunks: cells slightly larger than the largest
 // sphere box, so that boxes that overlap sit in adjacent cells, and no more than cellBound() of them.
-// A warp per scene, then the first cell keys in scene order. A bound that is not finite sets tot->bad.
+// A warp per scene, several where there are fewer than 32, then the first cell keys in scene order. A bound that is not
+// finite sets tot->bad.
 __host__ __device__ __forceinline__ int64_t cellBound(int64_t spheres, int scenes) {
     const int64_t least = scenes > 1 ? 64 : 1 << 16;
     return 8 * spheres > least ? 8 * spheres : least;
@@ -264,20 +265,37 @@ constexpr double kCellMargin = 2e-6;
 __global__ void __launch_bounds__(1024) k_make_grids(int K, const int32_t* __restrict__ chunk, const int32_t* __restrict__ sceneChunk,
                                                      const long long* __restrict__ partial, const ScenePar* __restrict__ spp, int peri,
                                                      Grid* __restrict__ out, CollideTotals* __restrict__ tot) {
+    __shared__ long long s[32][7];
     const unsigned FULL = 0xffffffffu;
     const long long INF = 0x7ff0000000000000LL, most0 = orderOf(INF), least0 = orderOf(INF | (1LL << 63));
-    const int lane = threadIdx.x & 31;
-    for (int k = threadIdx.x >> 5; k < K; k += blockDim.x >> 5) {
-        const int c0 = sceneChunk[k], c1 = sceneChunk[k + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int each = K < 32 ? 32 / K : 1, groups = 32 / each;  // warps a scene, and scenes at once
+    for (int k0 = 0; k0 < K; k0 += groups) {
+        const int k = k0 + warp / each, part = warp % each;
+        const bool in = k < K && warp < groups * each;
+        const int c0 = in ? sceneChunk[k] : 0, c1 = in ? sceneChunk[k + 1] : 0;
         long long u[7] = {most0, most0, most0, least0, least0, least0, 0};
-        for (int b = c0 + lane; b < c1; b += 32) {
+        auto across = [&]() {  // to the first lane
+            for (int o = 16; o > 0; o >>= 1) {
+                for (int q = 0; q < 3; q++) u[q] = min(u[q], __shfl_down_sync(FULL, u[q], o));
+                for (int q = 3; q < 7; q++) u[q] = max(u[q], __shfl_down_sync(FULL, u[q], o));
+            }
+        };
+        for (int b = c0 + 32 * part + lane; b < c1; b += 32 * each) {
             for (int q = 0; q < 3; q++) u[q] = min(u[q], partial[7 * b + q]);
             for (int q = 3; q < 7; q++) u[q] = max(u[q], partial[7 * b + q]);
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            for (int q = 0; q < 3; q++) u[q] = min(u[q], __shfl_down_sync(FULL, u[q], o));
-            for (int q = 3; q < 7; q++) u[q] = max(u[q], __shfl_down_sync(FULL, u[q], o));
+        across();
+        if (each > 1) {  // then groups >= K: every thread comes here once
+            if (lane == 0)
+                for (int q = 0; q < 7; q++) s[warp][q] = u[q];
+            __syncthreads();
+            if (part || !in) continue;  // a warp left over has no others after it
+            if (lane < each)
+                for (int q = 0; q < 7; q++) u[q] = s[warp + lane][q];
+            across();
         }
+        if (!in) continue;
         if (lane) continue;
         double v[7];
         for (int q = 0; q < 7; q++) v[q] = __longlong_as_double(orderOf(u[q]));
@@ -371,22 +389,20 @@ __device__ __forceinline__ int64_t lowerBound64(const uint64_t* a, int64_t n, ui
 
 // the spheres' boxes in cell order, rounded outward to FP32 (of a grid far from zero, relative to its origin: the
 // subtraction keeps their order, and so what overlapF and overlapOuter conclude from it)
-__device__ __forceinline__ double4_32a relative(const Grid& G, const double4_32a& a) {
-    return make_double4_32a(a.x - G.ox, a.y - G.oy, a.z - G.oz, 0.);
-}
 __global__ void k_gather_sorted(DevParticles P, const int32_t* __restrict__ ids, int n, const Grid* __restrict__ Gs, const int* __restrict__ far,
                                 const uint32_t* __restrict__ key,
                                 const int32_t* __restrict__ rank, const int32_t* __restrict__ off, uint32_t* __restrict__ skey,
                                 float4* __restrict__ smnf, float4* __restrict__ smxf) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    const int anyFar = *far;
     const int p = ids[i];
     double4_32a a = P.mn[p], b = P.mx[p];
-    if (*far) {
+    if (anyFar) {
         const Grid& G = Gs[sceneOfP(P, p)];
         if (G.far) {
-            a = relative(G, a);
-            b = relative(G, b);
+            a = make_double4_32a(a.x - G.ox, a.y - G.oy, a.z - G.oz, 0.);
+            b = make_double4_32a(b.x - G.ox, b.y - G.oy, b.z - G.oz, 0.);
         }
     }
     const int at = off[key[i]] + rank[i];
@@ -537,6 +553,12 @@ __global__ void __launch_bounds__(256, 4) k_pairs_ss(DevParticles P, const uint3
     flushPairs(buf, nb, pairs, cap, counter);
 }
 
+// A box relative to its grid's origin (out of line: inlined, the subtractions become predicated FP64 instructions of
+// every warp).
+static __device__ __noinline__ void makeRelative(const Grid& G, double4_32a& a, double4_32a& b) {
+    a = make_double4_32a(a.x - G.ox, a.y - G.oy, a.z - G.oz, 0.);
+    b = make_double4_32a(b.x - G.ox, b.y - G.oy, b.z - G.oz, 0.);
+}
 // A facet (finite box) against the spheres of the cells its box can reach: a sphere j that
 // overlaps it has mn_j in [mn_f - h, mx_f] on every axis. One warp per facet; its lanes split
 // each x-run of cells.
@@ -552,7 +574,8 @@ __global__ void k_pairs_local(DevParticles P, const int32_t* __restrict__ lids, 
     const int p = lids[t];
     const Grid G = Gs[sceneOfP(P, p)];
     const double4_32a mn1 = P.mn[p], mx1 = P.mx[p];
-    const double4_32a rn = G.far ? relative(G, mn1) : mn1, rx = G.far ? relative(G, mx1) : mx1;
+    double4_32a rn = mn1, rx = mx1;
+    if (G.far) makeRelative(G, rn, rx);
     const float4 fn1 = make_float4(__double2float_rd(rn.x), __double2float_rd(rn.y), __double2float_rd(rn.z), 0.f);
     const float4 fx1 = make_float4(__double2float_ru(rx.x), __double2float_ru(rx.y), __double2float_ru(rx.z), 0.f);
     const uint32_t m1 = P.mask[p];
@@ -1108,7 +1131,14 @@ __device__ __forceinline__ void clearEnd(const DevIncidence& I, int64_t e) {
 struct Room {
     int64_t act = -1, plain = -1;
     const CollideTotals* tot = nullptr;
+    // whether the set whose active contacts and plain ones are counted in act (low and high half) is the new one
+    __device__ __forceinline__ bool suffices(uint64_t n) const {
+        return (int64_t)(uint32_t)n <= act && (int64_t)(n >> 32) <= plain && !(tot && tot->real != tot->kept);
+    }
 };
+// Up to so many contacts the kernel that gives out the slots clears the ends (a launch less: 10 000 spheres 245 -> 238 us
+// a run); beyond, a kernel of its own does, which writes them in order (1M drum: 76 us for both, 121 in one).
+constexpr int64_t kClearInSlots = 1 << 19;
 // end slots: active contact c with hi==p sits at loStart[p] + (its index k in hiList); with lo==p
 // at hiStart[p+1] + (active contacts before c) (see DevIncidence); inactive contacts have no slot (-1).
 // The work list holds the nOther active contacts that are not plain (walls, facets, spheres of
@@ -1121,13 +1151,14 @@ struct Room {
 // records, which neighbours in contact order share: there the real ones come first within tiles of
 // contacts only (k_pack_ss; 1M drum: split over the whole list, the step took 0.168 ms instead of 0.161).
 // The ends start without a contribution, once nothing can call the old set back.
+template <bool CLEAR>
 __global__ void k_slots(const uint64_t* __restrict__ key, const uint32_t* __restrict__ flags, const int32_t* __restrict__ cdist, int64_t n,
                         const uint64_t* __restrict__ act, const uint64_t* __restrict__ actReal, DevIncidence I, Room room) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint64_t tot = act[n], totReal = actReal ? actReal[n] : 0;  // over all contacts
     const int nAct = (int)(uint32_t)tot, nPlain = (int)(tot >> 32);
-    const bool clear = nAct <= room.act && nPlain <= room.plain && !(room.tot && room.tot->real != room.tot->kept);
+    const bool clear = CLEAR && room.suffices(tot);
     if (k < nAct) {
         const int32_t ch = I.hiList[k];
         const int hiP = (int)(key[ch] & 0xffffffffu);
@@ -1178,10 +1209,10 @@ __global__ void k_heavy(DevIncidence I, DevParticles P, const uint32_t* __restri
         if ((nodeFlags[p] & F_DOF_ALL) != F_DOF_ALL) I.heavyFree[atomicAdd(&tot->heavyFree, 1)] = p;
     }
 }
-// every end starts without a contribution
-__global__ void k_zero_ends(DevIncidence I, int64_t ends) {
+// every end of the active contacts (counted in the low half of *act) starts without a contribution
+__global__ void k_zero_ends(DevIncidence I, const uint64_t* __restrict__ act, Room room) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < ends) clearEnd(I, e);
+    if (e < 2 * (int64_t)(uint32_t)*act && room.suffices(*act)) clearEnd(I, e);
 }
 
 // the packed state K back into the contact arrays of its set, contact c from idx[c] (whatever the work list holds)
@@ -1426,7 +1457,8 @@ static int incidence(Sim& S, int64_t n, const int32_t* first, const Room& room) 
         WG_CUDA_TRY(cub::DeviceRadixSort::SortPairs(W.cubTmp, tb, W.hiKeys, W.hiKeysSorted, W.hiVals, S.I.hiList, n, 0, hiKeyBits(S), st));
     }
     k_hi_start<<<(unsigned)((S.nPar + 1 + BS - 1) / BS), BS, 0, st>>>(W.hiKeysSorted, n, (int)S.nPar, S.I.hiStart);
-    if (n > 0) k_slots<<<gn, BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, S.I, room);
+    if (n > 0 && room.act >= 0) k_slots<true><<<gn, BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, S.I, room);
+    else if (n > 0) k_slots<false><<<gn, BS, 0, st>>>(S.C.key, S.C.flags, S.C.cdist, n, W.act, W.actReal, S.I, room);
     k_heavy<<<(unsigned)((S.nPar + BS - 1) / BS), BS, 0, st>>>(S.I, S.P, S.N.flags, kHeavyThreshold, W.tot, W.act, W.actReal, n);
     return 0;
 }
@@ -1575,7 +1607,7 @@ static int fullRun(Sim& S) {
         if (!scratch(S, W.cellOffCap, ncell + 1, W.cellOff)) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
         const unsigned gs = (unsigned)((ns + BS - 1) / BS);
         k_grid_reduce<<<nb, BS, 0, st>>>(S.P, W.sphereIds, W.dChunk, W.red);
-        k_make_grids<<<1, 32 * std::min(K, 32), 0, st>>>(K, W.dChunk, W.dSceneChunk, W.red, S.dPar, peri ? 1 : 0, W.dGrids, W.tot);
+        k_make_grids<<<1, 1024, 0, st>>>(K, W.dChunk, W.dSceneChunk, W.red, S.dPar, peri ? 1 : 0, W.dGrids, W.tot);
         // spheres in cell order: their number per cell, its running sum, then each to its place
         WG_CUDA_TRY(cudaMemsetAsync(W.cellOff, 0, sizeof(int32_t) * (ncell + 1), st));
         if (peri) k_cellkey_peri<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, S.dPar, W.cellKey, W.cellRank, W.cellOff);
@@ -1762,8 +1794,13 @@ static int fullRun(Sim& S) {
         room.plain = !packed ? n : (Q.ft[0] || !ft ? Q.cap : -1);
         room.tot = lookForOrphans ? nullptr : W.tot;
         if (packed && !scratch(S, W.packIdxCapB, n, W.packIdxB)) return S.fail(WG_ERR_CUDA, "out of device memory (packed contacts)");
-        r = incidence(S, n, W.newLo, room);
+        auto zero = [&](const Room& rm) {
+            const int64_t most = 2 * std::min(rm.act, n);
+            if (most > 0) k_zero_ends<<<(unsigned)((most + BS - 1) / BS), BS, 0, st>>>(S.I, W.act + n, rm);
+        };
+        r = incidence(S, n, W.newLo, n <= kClearInSlots ? room : Room{});
         if (r) return r;
+        if (n > kClearInSlots) zero(room);
         if (packed) pack(std::min(n, room.plain));
         WG_CUDA_TRY(cudaMemcpyAsync(W.hTot, W.tot, sizeof(CollideTotals), cudaMemcpyDeviceToHost, st));
         WG_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1782,7 +1819,7 @@ static int fullRun(Sim& S) {
             if (!r) r = endRoom(S, nAct);  // last: the old ends are gone then
             if (r) return r;
             if (packed && nSS > room.plain) pack(nSS);
-            if (nAct > 0) k_zero_ends<<<(unsigned)((2 * nAct + BS - 1) / BS), BS, 0, st>>>(S.I, 2 * nAct);
+            zero(Room{nAct, nSS, nullptr});
         }
         undo.off = true;
         if (packed) {
