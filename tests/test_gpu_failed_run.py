@@ -55,6 +55,13 @@ class Raw:
     def put(self, nodes):
         self.sim.H.check(self.L.wg_put_state(self.h, *[_native.ptr(a) for a in nodes]), "put_state")
 
+    def apart(self):
+        """Whether the boxes of each pair of the last full run are apart."""
+        mn, mx = np.empty((self.n, 3)), np.empty((self.n, 3))
+        self.sim.H.check(self.L.wg_get_aabbs(self.h, _native.ptr(mn), _native.ptr(mx)), "get_aabbs")
+        a, b = np.arange(0, 2 * PAIRS, 2), np.arange(1, 2 * PAIRS, 2)
+        return np.any((mn[a] > mx[b]) | (mx[a] < mn[b]), axis=1)
+
     def contacts(self):
         from woodem_gb300 import _plan
         c = _plan.read_contacts(self.L, self.h, "wg")
@@ -121,6 +128,8 @@ def fails_and_goes_on(precision, periodic, cause, read):
     checkpoint.restore_contacts(T, snap)
     for steps in (1, 2, 40):
         assert raw.run(steps) == 0 and t.run(steps) == 0
+        if steps == 1:  # the run met real contacts without an overlap, which the merge finds by being repeated
+            assert np.all(raw.apart()[::3]) and not np.any(raw.apart()[1::3])
         for a, b, k in zip(raw.nodes(), t.nodes(), KEYS):
             assert np.array_equal(a, b), k
         same(raw.contacts()[1], t.contacts()[1])
