@@ -255,7 +255,7 @@ __global__ void k_grid_reduce(DevParticles P, const int32_t* __restrict__ ids, c
 
 // The grid of each scene from the partial bounds of its chunks: cells slightly larger than the largest
 // sphere box, so that boxes that overlap sit in adjacent cells, and no more than cellBound() of them.
-// A warp per scene, several where there are fewer than 32, then the first cell keys in scene order. A bound that is not
+// A warp per scene, all warps of the block for a single one, then the first cell keys in scene order. A bound that is not
 // finite sets tot->bad.
 __host__ __device__ __forceinline__ int64_t cellBound(int64_t spheres, int scenes) {
     const int64_t least = scenes > 1 ? 64 : 1 << 16;
@@ -269,11 +269,9 @@ __global__ void __launch_bounds__(1024) k_make_grids(int K, const int32_t* __res
     const unsigned FULL = 0xffffffffu;
     const long long INF = 0x7ff0000000000000LL, most0 = orderOf(INF), least0 = orderOf(INF | (1LL << 63));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int each = K < 32 ? 32 / K : 1, groups = 32 / each;  // warps a scene, and scenes at once
-    for (int k0 = 0; k0 < K; k0 += groups) {
-        const int k = k0 + warp / each, part = warp % each;
-        const bool in = k < K && warp < groups * each;
-        const int c0 = in ? sceneChunk[k] : 0, c1 = in ? sceneChunk[k + 1] : 0;
+    const int warps = blockDim.x >> 5, each = K == 1 ? warps : 1, part = K == 1 ? warp : 0;  // warps of a scene
+    for (int k = K == 1 ? 0 : warp; k < K; k += K == 1 ? 1 : warps) {
+        const int c0 = sceneChunk[k], c1 = sceneChunk[k + 1];
         long long u[7] = {most0, most0, most0, least0, least0, least0, 0};
         auto across = [&]() {  // to the first lane
             for (int o = 16; o > 0; o >>= 1) {
@@ -286,16 +284,15 @@ __global__ void __launch_bounds__(1024) k_make_grids(int K, const int32_t* __res
             for (int q = 3; q < 7; q++) u[q] = max(u[q], partial[7 * b + q]);
         }
         across();
-        if (each > 1) {  // then groups >= K: every thread comes here once
+        if (K == 1) {
             if (lane == 0)
                 for (int q = 0; q < 7; q++) s[warp][q] = u[q];
             __syncthreads();
-            if (part || !in) continue;  // a warp left over has no others after it
-            if (lane < each)
-                for (int q = 0; q < 7; q++) u[q] = s[warp + lane][q];
+            if (warp) continue;
+            if (lane < warps)
+                for (int q = 0; q < 7; q++) u[q] = s[lane][q];
             across();
         }
-        if (!in) continue;
         if (lane) continue;
         double v[7];
         for (int q = 0; q < 7; q++) v[q] = __longlong_as_double(orderOf(u[q]));
@@ -1607,7 +1604,7 @@ static int fullRun(Sim& S) {
         if (!scratch(S, W.cellOffCap, ncell + 1, W.cellOff)) return S.fail(WG_ERR_CUDA, "out of device memory (grid)");
         const unsigned gs = (unsigned)((ns + BS - 1) / BS);
         k_grid_reduce<<<nb, BS, 0, st>>>(S.P, W.sphereIds, W.dChunk, W.red);
-        k_make_grids<<<1, 1024, 0, st>>>(K, W.dChunk, W.dSceneChunk, W.red, S.dPar, peri ? 1 : 0, W.dGrids, W.tot);
+        k_make_grids<<<1, K == 1 ? 1024 : 32 * std::min(K, 32), 0, st>>>(K, W.dChunk, W.dSceneChunk, W.red, S.dPar, peri ? 1 : 0, W.dGrids, W.tot);
         // spheres in cell order: their number per cell, its running sum, then each to its place
         WG_CUDA_TRY(cudaMemsetAsync(W.cellOff, 0, sizeof(int32_t) * (ncell + 1), st));
         if (peri) k_cellkey_peri<<<gs, BS, 0, st>>>(S.P, W.sphereIds, ns, W.dGrids, S.dPar, W.cellKey, W.cellRank, W.cellOff);
