@@ -188,7 +188,9 @@ int wg_set_particles(wg_scene* s, int64_t n, const int32_t* shape, const int32_t
                      const double* half_thick, const double* fake_vel, const int32_t* mat,
                      const uint32_t* mask);
 
-/* Advance n steps with device-resident state. */
+/* Advance n steps with device-resident state. Where a collider run fails (a box that is not finite, no memory left),
+   the steps before it are done and the contacts stay as after them; the step itself begins anew, with a full run, in the
+   next call. */
 int wg_run(wg_scene* s, int64_t n_steps);
 /* Same step loop driven from host buffers (the reference keeps state in host objects):
    copies the node state in from host memory, runs n steps, copies it back out. */
