@@ -189,8 +189,8 @@ int wg_set_particles(wg_scene* s, int64_t n, const int32_t* shape, const int32_t
                      const uint32_t* mask);
 
 /* Advance n steps with device-resident state. Where a collider run fails (a box that is not finite, no memory left),
-   the steps before it are done and the contacts stay as after them; the step itself begins anew, with a full run, in the
-   next call. */
+   the steps before it are done and the contacts stay as after them; the next call goes on with that run, unless nodes,
+   contacts or a slot are set in between: it then begins with a step, and a full run in it. */
 int wg_run(wg_scene* s, int64_t n_steps);
 /* Same step loop driven from host buffers (the reference keeps state in host objects):
    copies the node state in from host memory, runs n steps, copies it back out. */

@@ -43,6 +43,7 @@ class Raw:
         self.S, self.sim = S, S._ensure_sim()
         self.L, self.h = self.sim.H.L, self.sim.H.h
         self.n = len(S.dem._nodes.soa)
+        self.due = 0
 
     def run(self, n):
         return self.L.wg_run(self.h, n)
@@ -51,6 +52,11 @@ class Raw:
         out = [np.empty((self.n, w)) for w in (3, 4, 3, 3, 3, 3)]
         self.sim.H.check(self.L.wg_get_nodes(self.h, *[_native.ptr(a) for a in out]), "get_nodes")
         return out
+
+    def energy(self):
+        v, c = np.zeros(32), np.zeros(32, np.int32)
+        self.sim.H.check(self.L.wg_get_energy(self.h, _native.ptr(v), _native.ptr(c, _native.P_I32)), "get_energy")
+        return np.concatenate([v, c])
 
     def put(self, nodes):
         self.sim.H.check(self.L.wg_put_state(self.h, *[_native.ptr(a) for a in nodes]), "put_state")
@@ -196,3 +202,36 @@ def test_no_memory_at_the_first_run(precision, periodic, gpu_lib):
         if done:
             break
     assert k > 25
+
+
+@pytest.mark.parametrize("precision,periodic", MODES)
+def test_goes_on_as_if_it_had_not_failed(precision, periodic, gpu_lib):
+    """Failed runs, the first ones of a scene and later ones, and the steps after them beside a scene that never failed."""
+    def go(fails):
+        S = build(precision, periodic)
+        S.trackEnergy = not periodic
+        raw = Raw(S)
+        assert raw.run(0) == 0
+        failed = 0
+        for steps, crowded in ((4, False), (3, True), (1, False), (30, False)):
+            if crowded:
+                raw.put(crowd(raw.nodes()))
+            for k in fails:
+                raw.L.wg_fail_alloc(raw.h, k)
+                failed += raw.run(steps) != 0
+                raw.L.wg_fail_alloc(raw.h, -1)
+                if raw.sim.clock()[0] == raw.due + steps:
+                    break
+            rest = raw.due + steps - raw.sim.clock()[0]
+            assert raw.run(rest) == 0
+            raw.due += steps
+        out = (raw.nodes(), raw.contacts()[0], raw.sim.clock()[:2], raw.energy())
+        S.close()
+        return out, failed
+    want, none = go([])
+    got, failed = go([0, 7, 3])
+    assert none == 0 and failed >= 6
+    for a, b in zip(got[0], want[0]):
+        assert np.array_equal(a, b)
+    same(got[1], want[1])
+    assert got[2] == want[2] and np.array_equal(got[3], want[3])

@@ -847,11 +847,12 @@ int Sim::syncContacts(bool hostWait) {
 int Sim::ensureEnergyCapacity() {
     Sim& S = *this;
     if (!dEnergy) {
-        dEnergy = (double*)dalloc(sizeof(double) * WG_ENERGY_N);
-        dECreated = (int32_t*)dalloc(sizeof(int32_t) * WG_ENERGY_N);
-        dEPartial = (double*)dalloc(sizeof(double) * EN_CON_NCOL * 256);
-        dEPrev = (double*)dalloc(sizeof(double) * 10);
-        if (!dEnergy || !dECreated || !dEPartial || !dEPrev) return fail(WG_ERR_CUDA, "out of device memory (energy)");
+        if (!dECreated) dECreated = (int32_t*)dalloc(sizeof(int32_t) * WG_ENERGY_N);
+        if (!dEPartial) dEPartial = (double*)dalloc(sizeof(double) * EN_CON_NCOL * 256);
+        if (!dEPrev) dEPrev = (double*)dalloc(sizeof(double) * 10);
+        if (!dECreated || !dEPartial || !dEPrev) return fail(WG_ERR_CUDA, "out of device memory (energy)");
+        dEnergy = (double*)dalloc(sizeof(double) * WG_ENERGY_N);  // last: it stands for all four
+        if (!dEnergy) return fail(WG_ERR_CUDA, "out of device memory (energy)");
         WG_CUDA_TRY(cudaMemsetAsync(dEnergy, 0, sizeof(double) * WG_ENERGY_N, S.stream));
         WG_CUDA_TRY(cudaMemsetAsync(dECreated, 0, sizeof(int32_t) * WG_ENERGY_N, S.stream));
         // ContactLoop.prevStress = 0, prevVol = NaN (ContactLoop.hpp:119-123)
@@ -861,7 +862,7 @@ int Sim::ensureEnergyCapacity() {
     }
     if (cfg.periodic && cfg.eval_stress) {
         const int64_t need = 9 * (std::max<int64_t>(1, (I.nAct + 255) / 256) + 1);
-        if (stressCap < need) {
+        if (stressCap < need || !dStress) {
             if (dStress) dfree(dStress);
             stressCap = need + need / 2;
             dStress = (double*)dalloc(sizeof(double) * stressCap);
@@ -872,7 +873,7 @@ int Sim::ensureEnergyCapacity() {
             }
         }
     }
-    if (eNode.cap < N.n) {
+    if (eNode.cap < N.n || !eNode.col) {
         if (eNode.col) dfree(eNode.col);
         eNode.cap = std::max<int64_t>(N.n, 1);
         eNode.col = (double*)dalloc(sizeof(double) * EN_NODE_NCOL * eNode.cap);
@@ -1204,8 +1205,10 @@ int Sim::run(int64_t n) {
                            !useGraph && contactBlock <= 0 && I.nHeavyFree == 0 && (!fp32 || P.nFacets == 0 || facetsStatic);
         int64_t k = std::min<int64_t>(n - done, small && N.n <= 65536 && !cfg.periodic && !anyZeroVd ? 8 * maxChunk : maxChunk);
         if (!small && !useGraph) k = stepsToQueue(k, step - lastFullStep, runInterval);
-        // dt may change after a step (Scene.nextDt, DynDt): such a step ends its chunk
-        if (std::isfinite(nextDt)) k = 1;
+        // dt may change after a step (Scene.nextDt, DynDt): such a step ends its chunk; one that goes on from its
+        // collider run, which failed in the last call, is one of its own
+        const bool resume = midStep;
+        if (std::isfinite(nextDt) || resume) k = 1;
         // wg_run_host's early copy-out: the run's last step gets a chunk of its own, whose first
         // Leapfrog always runs (a halt only stops the steps after a full-run request)
         if (earlyWanted && !earlyIssued && done < n - 1) k = std::min<int64_t>(k, n - 1 - done);
@@ -1259,9 +1262,9 @@ int Sim::run(int64_t n) {
         const int64_t s0 = step;
         // a chunk that starts from the end slots and is not due for a full run is replayed as a
         // CUDA graph (re-captured after every full run, whose contact arrays it refers to)
-        const bool lastEarly = earlyWanted && !earlyIssued && done + k == n && k == 1;
+        const bool lastEarly = earlyWanted && !earlyIssued && done + k == n && k == 1 && !resume;
         const bool graphChunk = useGraph && fromEnds && !needFull && k == maxChunk && !cfg.periodic && !lastEarly;
-        bool oneLaunch = small && !lastEarly;
+        bool oneLaunch = small && !lastEarly && !resume;
         const int blocks = share.part(oneLaunch ? stepsBlocks(std::max<int64_t>(N.n, I.nAct)) : smCount(), N.n > kSmallBeside);
         if (oneLaunch) {
             unsigned* bar = (unsigned*)(dFlags + FL_BAR);
@@ -1278,7 +1281,7 @@ int Sim::run(int64_t n) {
             } else
                 launches++;
         }
-        if (oneLaunch) {
+        if (oneLaunch || resume) {
         } else if (graphChunk) {
             if (!graphExec || graphSteps != k || graphEpoch != nFullRuns) {
                 if (graphExec) cudaGraphExecDestroy(graphExec);
@@ -1338,7 +1341,7 @@ int Sim::run(int64_t n) {
         if (ds < k || hFlags[FL_FULL]) {
             // Leapfrog of step s0+ds ran, its contact loop waits for the collider
             if (!hFlags[FL_FULL]) return fail(WG_ERR_STATE, "queued steps halted without a collider request");
-            if (!graphChunk && !oneLaunch) {
+            if (!graphChunk && !oneLaunch && !resume) {
                 cudaEventElapsedTime(&a, E[3 * ds], E[3 * ds + 1]);
                 ph[0] += a;
             }
@@ -1350,8 +1353,10 @@ int Sim::run(int64_t n) {
             }
             WG_CUDA_TRY(cudaEventRecord(E[3 * maxChunk], stream));
             int r = collide_full_run(*this);
+            if (!r && trackE) r = ensureEnergyCapacity();
             if (r) {
-                // the steps before this one are done; it starts anew in the next call
+                // the steps before this one are done, and of it Leapfrog: the next call goes on with the collider
+                midStep = forceFull = true;
                 if (cfg.periodic) X.cell = ds > 0 ? cellEnd[ds - 1] : cell0;
                 for (int64_t j = 0; j < ds; j++) {
                     if (dd.on) dd.activated(step + j, timeAbs);
@@ -1370,12 +1375,8 @@ int Sim::run(int64_t n) {
             // a run that was forced (a slot's new job, contacts set from outside) says nothing about the spheres' motion
             if (!needFull && lastFullStep >= 0 && step + ds > lastFullStep) runInterval = step + ds - lastFullStep;
             lastFullStep = step + ds;
-            if (trackE) {
-                r = ensureEnergyCapacity();
-                if (r) return r;
-            }
             initialized = true;
-            forceFull = false;
+            forceFull = midStep = false;
             launches += 12;
             WG_CUDA_TRY(cudaEventRecord(E[3 * maxChunk + 1], stream));
             k_set_flags<<<1, 1, 0, stream>>>(dFlags, 0);
@@ -1466,7 +1467,7 @@ int Sim::run(int64_t n) {
     // ContactLoop.stress of the last step (periodic cells with evalStress)
     if (cfg.periodic && cfg.eval_stress && fromEnds && done > 0) {
         const int64_t need = 9 * (std::max<int64_t>(1, (I.nAct + 255) / 256) + 1);
-        if (stressCap < need) {
+        if (stressCap < need || !dStress) {
             if (dStress) dfree(dStress);
             stressCap = need + need / 2;
             dStress = (double*)dalloc(sizeof(double) * stressCap);
@@ -1706,6 +1707,7 @@ static int writeSlot(Sim& S, int64_t p0, int64_t cap, int64_t n, const double* p
     if (cudaStreamSynchronize(S.stream) != cudaSuccess) return S.fail(WG_ERR_CUDA, "slot upload failed");
     S.listsDirty = true;
     S.forceFull = true;
+    S.midStep = false;  // the new job's nodes begin with Leapfrog
     return 0;
 }
 
@@ -1993,6 +1995,7 @@ int wg_put_state(wg_scene* s, const double* pos, const double* ori, const double
     }
     k_put_state<<<(unsigned)((na + 255) / 256), 256, 0, S.stream>>>(S.N, X.dApiMap, na, stagedArrays(X.dStage, na));
     S.fromEnds = false;  // the next step starts from the forces written here
+    S.midStep = false;
     if (vel) S.facetsStatic = false;  // facet vertices may have been given a velocity
     launch_facet_prep(S.stream, S.N, S.P, nullptr);
     WG_CUDA_TRY(cudaGetLastError());
@@ -2405,6 +2408,7 @@ int wg_set_contact_state(wg_scene* s, int64_t n, const uint64_t* key, const uint
     S.K.n = 0;
     S.packDirty = false;
     S.fromEnds = false;    // the first step takes the node forces as written by the host
+    S.midStep = false;
     S.forceFull = true;    // and starts with a full run that merges these contacts
     return WG_OK;
 }

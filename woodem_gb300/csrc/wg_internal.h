@@ -416,6 +416,7 @@ struct Sim {
     bool contactsReplaced = false;     // the contact arrays were set from outside since the last full run
     bool listsDirty = true;            // particle lists of the collider to be rebuilt at the next full run
     bool forceFull = false;            // next step starts with a full collider run
+    bool midStep = false;              // Leapfrog of the next step is done: its collider run failed
     int* dFlags = nullptr;   // the step-loop flags (FL_*) and the counters behind them (CTL_BYTES)
     long long* dStep = nullptr;  // the first of those counters
     int* hFlags = nullptr;   // pinned mirror
