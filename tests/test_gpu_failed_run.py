@@ -1,6 +1,8 @@
 """A collider run that fails (a box that is not finite, no memory left) leaves the contacts, their state and their
 forces as they were: they list as before, and with the cause mended the scene goes on as one restored from them.
 The run is one that parts touching pairs (real contacts without an overlap) and brings many new ones (every array grows)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -235,3 +237,50 @@ def test_goes_on_as_if_it_had_not_failed(precision, periodic, gpu_lib):
         assert np.array_equal(a, b)
     same(got[1], want[1])
     assert got[2] == want[2] and np.array_equal(got[3], want[3])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("scenes_", [1, 3])
+def test_failure_among_queued_steps(scenes_, precision, gpu_lib):
+    """Spheres fall into a heap; whenever a run needs larger arrays, it first fails: every step, time and DynDt count as if
+    it had not, in a scene and in a batch."""
+    from woodem_gb300 import scenes
+    from woodem_gb300.batch import Batch
+
+    def go(fail):
+        mix = []
+        for q in range(scenes_):
+            S = scenes.box_settle_scaled(500 + 150 * q, 5e-3, seed=q, precision=precision)
+            S.engines = utils.defaultEngines(damping=.2, verletDist=-.1, dynDtPeriod=70)
+            nd = S.dem._nodes.soa
+            nd.col("vel")[6:] = np.random.default_rng(q).uniform(-.3, .3, (len(nd) - 6, 3)) + [0, 0, -1.]
+            mix.append(S)
+        B = Batch(mix) if scenes_ > 1 else mix[0]._ensure_sim()
+        H, step, time = B.H, C.c_int64(), C.c_double()
+        done = failed = inside = 0
+        while done < 2500:
+            if fail:
+                H.L.wg_fail_alloc(H.h, 0)
+            r = H.L.wg_run(H.h, 2500 - done)
+            H.L.wg_fail_alloc(H.h, -1)
+            H.check(H.L.wg_get_clock(H.h, 0, C.byref(step), C.byref(time), None, None), "get_clock")
+            failed += r != 0
+            inside += r != 0 and step.value > done
+            done = step.value
+            if r:  # once more with memory, up to the next need
+                H.check(H.L.wg_run(H.h, min(10, 2500 - done)), "run")
+                done += min(10, 2500 - done)
+        times = []
+        for k in range(scenes_):
+            H.check(H.L.wg_get_clock(H.h, k, C.byref(step), C.byref(time), None, None), "get_clock")
+            times += [step.value, time.value]
+        n = sum(len(S.dem._nodes.soa) for S in mix)
+        out = [np.empty((n, w)) for w in (3, 4, 3, 3, 3, 3)]
+        H.check(H.L.wg_get_nodes(H.h, *[_native.ptr(a) for a in out]), "get_nodes")
+        (B if scenes_ > 1 else mix[0]).close()
+        return out, times, failed, inside
+    want, got = go(False), go(True)
+    assert want[2] == 0 and got[2] >= 3 and got[3] >= 1
+    assert got[1] == want[1]
+    for a, b in zip(got[0], want[0]):
+        assert np.array_equal(a, b)

@@ -928,22 +928,29 @@ int Sim::applyDtScene(int k, double ndt) {
     return 0;
 }
 
+// Scratch of the critical timesteps of scenes with DynDt, grown to the contact ends (before a step that may need it)
+int Sim::ensureDynDtCapacity() {
+    bool on = dd.on;
+    for (const DynDtState& q : bdd) on = on || q.on;
+    if (!on) return 0;
+    if (I.endCap > kCap || !dKA || !dKB) {
+        dfree(dKA);
+        dfree(dKB);
+        kCap = std::max<int64_t>(I.endCap, 1);
+        dKA = (double4_32a*)dalloc(sizeof(double4_32a) * kCap);
+        dKB = (double2*)dalloc(sizeof(double2) * kCap);
+    }
+    if (!dCrit) dCrit = (unsigned long long*)dalloc(sizeof(unsigned long long));
+    if (nScenes > 1 && !dCritB) dCritB = (unsigned long long*)dalloc(sizeof(unsigned long long) * nScenes);
+    if (!dKA || !dKB || !dCrit || (nScenes > 1 && !dCritB)) return fail(WG_ERR_CUDA, "out of device memory (DynDt)");
+    return 0;
+}
+
 // DynDt::run (pkg/dem/DynDt.cpp:93-113) for the scenes of a batch whose DynDt is due after the
 // contact loop of device step deviceStep: one stiffness pass over all scenes, the critical
 // timestep of each scene (the minimum over its own nodes), then each due scene's rule.
 int Sim::runDynDtScenes(const std::vector<char>& due, long long deviceStep) {
     Sim& S = *this;
-    if (I.endCap > kCap || !dCritB) {
-        if (I.endCap > kCap) {
-            if (dKA) dfree(dKA);
-            if (dKB) dfree(dKB);
-            kCap = std::max<int64_t>(I.endCap, 1);
-            dKA = (double4_32a*)dalloc(sizeof(double4_32a) * kCap);
-            dKB = (double2*)dalloc(sizeof(double2) * kCap);
-        }
-        if (!dCritB) dCritB = (unsigned long long*)dalloc(sizeof(unsigned long long) * nScenes);
-        if (!dKA || !dKB || !dCritB) return fail(WG_ERR_CUDA, "out of device memory (DynDt)");
-    }
     const double inf = std::numeric_limits<double>::infinity();
     unsigned long long bits;
     std::memcpy(&bits, &inf, sizeof bits);
@@ -1002,15 +1009,6 @@ int Sim::applyDt(double ndt) {
 // nextDt = min(crDt*dtSafety, dt*(1+maxRelInc)^(steps since the previous run)).
 int Sim::runDynDt(int64_t stepNow) {
     Sim& S = *this;
-    if (I.endCap > kCap || !dCrit) {
-        if (dKA) dfree(dKA);
-        if (dKB) dfree(dKB);
-        kCap = std::max<int64_t>(I.endCap, 1);
-        dKA = (double4_32a*)dalloc(sizeof(double4_32a) * kCap);
-        dKB = (double2*)dalloc(sizeof(double2) * kCap);
-        if (!dCrit) dCrit = (unsigned long long*)dalloc(sizeof(unsigned long long));
-        if (!dKA || !dKB || !dCrit) return fail(WG_ERR_CUDA, "out of device memory (DynDt)");
-    }
     const double inf = std::numeric_limits<double>::infinity();
     unsigned long long bits;
     std::memcpy(&bits, &inf, sizeof bits);
@@ -1198,6 +1196,7 @@ int Sim::run(int64_t n) {
             int r = ensureEnergyCapacity();
             if (r) return r;
         }
+        if (int r = ensureDynDtCapacity()) return r;
         // a small scene runs its steps in one launch, which ends by itself where a full run is due: the
         // chunk only bounds its length (in a periodic cell every step has its own record)
         const bool small = N.n <= (share.crowded() ? kSmallBeside : kSmallNodes) &&
@@ -1354,6 +1353,7 @@ int Sim::run(int64_t n) {
             WG_CUDA_TRY(cudaEventRecord(E[3 * maxChunk], stream));
             int r = collide_full_run(*this);
             if (!r && trackE) r = ensureEnergyCapacity();
+            if (!r) r = ensureDynDtCapacity();
             if (r) {
                 // the steps before this one are done, and of it Leapfrog: the next call goes on with the collider
                 midStep = forceFull = true;

@@ -472,6 +472,7 @@ struct Sim {
     double* dEPartial = nullptr;    // EN_CON_NCOL * 256 block partials
     double* dEPrev = nullptr;       // periodic gradV work: previous stress (9) and volume
     int ensureEnergyCapacity();
+    int ensureDynDtCapacity();
     // timing
     std::vector<cudaEvent_t> evPool;  // per queued step: before Leapfrog, before contacts, after
     cudaEvent_t ev[8];
