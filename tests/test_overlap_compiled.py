@@ -55,7 +55,7 @@ def decide(mn, mx, size, device):
 
 @pytest.mark.parametrize("scale", [1., 1e-3, 1e5])
 @pytest.mark.parametrize("kind", KINDS)
-def test_on_the_host(kind, scale):
+def test_on_the_host(kind, scale, gpu_lib):
     size = SIZE * scale
     mn, mx = boxes(kind, 2000, size)
     q, _ = decide(mn, mx, size, False)

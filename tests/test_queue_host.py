@@ -7,7 +7,7 @@ from woodem_gb300 import _native
 
 @pytest.mark.parametrize("most", [1, 2, 32, 1024])
 @pytest.mark.parametrize("interval", [0, 1, 2, 3, 8, 40, 5000])
-def test_chunks(most, interval):
+def test_chunks(most, interval, gpu_lib):
     q = _native.lib().wg_steps_to_queue
     since = waits = 0
     while since < 100000:
